@@ -100,17 +100,18 @@ cudaError_t diff_march16(const StepDims& d, const Geometry& g, const float* u, f
     return cudaGetLastError();
 }
 
-// FP64 8^3 blocks: the k-march kernel, in place (any k-chunk depth asked for)
-inline cudaError_t diff_march64_8(const StepDims& d, const Geometry& g, double* u, StepScalars* sc, cudaStream_t st) {
-    using S = M64Shape<8, 8, 8>;
+// FP64: the k-march kernel, in place (any k-chunk depth asked for)
+template <int N, int VPT>
+cudaError_t diff_march64(const StepDims& d, const Geometry& g, double* u, StepScalars* sc, cudaStream_t st) {
+    using S = M64Shape<N, N, N, VPT>;
     static bool attr = false;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_diffusion_march64<8, 8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)S::smem);
+        cudaError_t e = cudaFuncSetAttribute(k_diffusion_march64<N, N, N, VPT>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    k_diffusion_march64<8, 8, 8><<<d.nblocks, S::NT, S::smem, st>>>(u, g, sc);
+    k_diffusion_march64<N, N, N, VPT><<<d.nblocks, S::NT, S::smem, st>>>(u, g, sc);
     return cudaGetLastError();
 }
 
@@ -119,22 +120,24 @@ cudaError_t diff_any(const StepDims& d, const Geometry& g, const T* u, T* out, i
                      StepScalars* sc, int kpar, cudaStream_t st, int cfl_next = 0) {
     if (push.tgt != nullptr && out == u) return cudaErrorInvalidValue;   // pushing needs out != u
     if constexpr (Pol<T>::exact) {
-        if (d.ni == 8 && d.nj == 8 && d.nk == 8 && out == u && push.tgt == nullptr)
-            return diff_march64_8(d, g, out, sc, st);
+        if (out != u || push.tgt != nullptr) return cudaErrorInvalidValue;   // the exact path runs in place
+        if (d.ni == 8 && d.nj == 8 && d.nk == 8) return diff_march64<8, 1>(d, g, out, sc, st);
+        if (d.ni == 16 && d.nj == 16 && d.nk == 16) return diff_march64<16, 4>(d, g, out, sc, st);
+        return cudaErrorInvalidValue;
     }
     if constexpr (!Pol<T>::exact) {
         if (d.ni == 16 && d.nj == 16 && d.nk == 16)
             return kpar == 1 ? diff_march16<1>(d, g, u, out, lo, push, sc, cfl_next, st)
                              : diff_march16<2>(d, g, u, out, lo, push, sc, cfl_next, st);
     }
-#define FALCON_DIFF_CASE(N, K) \
-    if (d.ni == N && kpar == K) return diff_n<T, N, K>(d, g, u, out, lo, push, sc, cfl_next, st);
-    if (d.ni != d.nj || d.ni != d.nk) return cudaErrorInvalidValue;
-    FALCON_DIFF_CASE(8, 2) FALCON_DIFF_CASE(8, 4)
-    FALCON_DIFF_CASE(16, 1)
-    // (16, 4) would need more than 227 KB of shared memory for its face arrays
-    if constexpr (!Pol<T>::exact) { FALCON_DIFF_CASE(8, 8) }
-#undef FALCON_DIFF_CASE
+    if constexpr (!Pol<T>::exact) {
+        if (d.ni != 8 || d.nj != 8 || d.nk != 8) return cudaErrorInvalidValue;
+        switch (kpar) {
+        case 2: return diff_n<T, 8, 2>(d, g, u, out, lo, push, sc, cfl_next, st);
+        case 4: return diff_n<T, 8, 4>(d, g, u, out, lo, push, sc, cfl_next, st);
+        case 8: return diff_n<T, 8, 8>(d, g, u, out, lo, push, sc, cfl_next, st);
+        }
+    }
     return cudaErrorInvalidValue;
 }
 

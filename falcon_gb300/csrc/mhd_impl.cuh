@@ -46,6 +46,104 @@ __device__ __forceinline__ T minmod(T ul, T u, T ur) {
     return (s + T(0.5)) * copysign(m, a);
 }
 
+// ---- exact FP64 results with fewer instructions on the FP64 pipe -------------
+// GB300 issues one FP64 warp instruction per 16 cycles and SM; compares, minima,
+// sign and exponent changes of doubles run on the integer pipes instead (a
+// positive double orders as its bit pattern), and a division by a value that
+// many cells share goes through its reciprocal. Every function below gives the
+// bits of the expression that it stands for.
+__device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ bool is_zero(double x) { return abs_bits(x) == 0ull; }
+__device__ __forceinline__ double with_sign_of(unsigned long long mag, double s) {
+    return __longlong_as_double((long long)(mag | ((unsigned long long)__double_as_longlong(s) & 0x8000000000000000ull)));
+}
+constexpr unsigned long long kExpOne = 1ull << 52;   // one step of the exponent field: a factor of 2
+
+// A positive divisor b and y = RN(1/b). lim: 0 sends every quotient to the
+// plain division (b outside 2^-300 .. 2^300).
+struct Divisor {
+    double b, y;
+    unsigned lim;
+};
+__device__ __forceinline__ Divisor divisor(double b) {
+    return Divisor{b, 1.0 / b, b > 0.0 && (unsigned)(exp_field(b) - 723) <= 600u ? 1000u : 0u};
+}
+// a / b correctly rounded in 5 FP64 instructions instead of the about 10 of a
+// division (P. Markstein, IBM J. R&D 34 (1990) 111): with y = RN(1/b) and q
+// within one ulp of a/b, RN(q + (a - b q) y) = RN(a/b), the residual a - b q
+// being exact in an FMA. The first correction brings q = RN(a y) within an
+// ulp. Quotients whose residual could underflow (exponent of a outside
+// 2^-523 .. 2^477) are divided; a zero keeps its sign.
+// The rare divisions are calls: inlined, the compiler runs their FP64
+// instructions for every warp that holds a zero.
+static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
+__device__ __forceinline__ double div_by(double a, const Divisor& d) {
+    double q = a * d.y;
+    q = fma(fma(-d.b, q, a), d.y, q);
+    q = fma(fma(-d.b, q, a), d.y, q);
+    if ((unsigned)(exp_field(a) - 500) >= d.lim) {
+        if (is_zero(a) && d.lim) q = a;
+        else q = div_plain(a, d.b);
+    }
+    return q;
+}
+
+// Half the minmod slope of a cell (minmod() below times 0.5) from its
+// differences dl = u - ul, dr = ur - u and da = ur - ul. With a = da/2, b =
+// 2 dr, c = 2 dl the selector max(0,ab) max(0,bc) 1e10 >= 1e-30 needs equal
+// signs and |a| |b|^2 |c| >= 1e-40: the exponents' sum E puts that product in
+// [2^E, 2^(E+4)), which decides it unless E is -136 .. -133 (1e-40 = 2^-132.88).
+// The minimum and the factors of 2 are integer operations on the bit patterns.
+// Magnitudes above 2^200, infinities and NaNs and the undecided products take
+// the formula itself.
+static __device__ __noinline__ double half_minmod_formula(double dl, double dr, double da) {
+    const double a = da * 0.5, b = 2.0 * dr, c = 2.0 * dl;
+    const double t = fmax(0.0, a * b) * fmax(0.0, b * c) * 1.e10 - (double)1.e-30f;
+    return ((copysign(0.5, t) + 0.5) * copysign(fmin(fmin(fabs(a), fabs(b)), fabs(c)), a)) * 0.5;
+}
+__device__ __forceinline__ double half_minmod(double dl, double dr, double da) {
+    const int ea = exp_field(da), eb = exp_field(dr), ec = exp_field(dl);
+    const int E = ea + 2 * eb + ec - 4 * 1023 + 2;   // a: -1, b twice: +2, c: +1
+    if (max(max(ea, eb), ec) > 1223 || (unsigned)(E + 136) <= 3u) return half_minmod_formula(dl, dr, da);
+    const int ha = __double2hiint(da);
+    const bool same = ((ha ^ __double2hiint(dr)) | (ha ^ __double2hiint(dl))) >= 0;
+    // min(|da|/2, 2 |dr|, 2 |dl|) / 2, each factor on the exponent of |da|
+    unsigned long long m = min(abs_bits(da), min(abs_bits(dr), abs_bits(dl)) + 2 * kExpOne) - 2 * kExpOne;
+    if (!same || E < -132) m = 0ull;
+    return with_sign_of(m, da);
+}
+// The limited flux through a face (face_flux_s below) from the cell values fl,
+// fr, their difference den = fr - fl, the half slopes and the sum of the two
+// cells' speeds. phi = max(0, 1 + 2 (num/den - 1)) is 0 unless num/den > 1/2 --
+// decided by sign and magnitude, and 0/0 counts as 0 -- and 1 for num = den
+// (both slopes 0), so only the faces near an extremum divide. Halving is exact,
+// so -(phi/2 num) speed / 2 is formed as (-phi/4 num) speed.
+static __device__ __noinline__ double flux_formula(double num, double den, double speed) {
+    return -(0.5 * fmax(0.0, 1.0 + 2.0 * (num / den - 1.0)) * num) * speed * 0.5;
+}
+__device__ __forceinline__ double face_flux_h(double fl, double fr, double den, double hL, double hR, double speed) {
+    const double num = ((fr - hR) - fl) - hL;
+    const unsigned long long an = abs_bits(num), ad = abs_bits(den);
+    const bool opposite = (__double2hiint(num) ^ __double2hiint(den)) < 0;
+    double q;   // -phi/4
+    if ((an | ad) == 0ull) {
+        q = -0.0;   // 0/0
+    } else if (ad - 600 * kExpOne >= 1000 * kExpOne || an >= 1600 * kExpOne) {
+        // den tiny or huge, or a value that is not finite: the formula
+        return flux_formula(num, den, speed);
+    } else if (opposite || an <= ad - kExpOne) {
+        q = -0.0;
+    } else if (an == ad) {
+        q = -0.25;
+    } else {
+        q = -fma(0.5, num / den - 1.0, 0.25);   // num/den > 1/2: not negative
+    }
+    return q * num * speed;
+}
+
 // FP32 minmod with the reference's selector written as a compare: the
 // reference forms t = max(0,ab)max(0,bc)*1e10 - 1e-30 and returns
 // (sign(t)/2 + 1/2) * sign(a) min(|a|,|b|,|c|), which is min(...) with a's
@@ -179,16 +277,27 @@ struct Shape {
     static constexpr uint32_t PLB = PL * (uint32_t)sizeof(T);   // bytes of one variable plane
     static_assert(PLB % 16 == 0, "plane must be a multiple of 16 bytes");
     static_assert(NK % KPAR == 0, "KPAR must divide NK");
-    // FP64 path: Br/sin(theta) and (v x B)_r/sin(theta) per point, [2][WP][PL]
-    // (the k-derivatives of the curls divide them by the cell's sin(theta),
-    // which its k-neighbours share: formed once per point, not per use)
-    static constexpr int NXS = sizeof(T) == 8 ? 2 : 0;
-    // shared memory: mbarriers | A1/A2 (double) | tile[NV][W][PL] | p1[WP][PL] | xs[NXS][WP][PL] | gi | gj | gs
+    // FP64 path: the fields that several cells' derivatives read, formed once
+    // per point instead of at each use. Br/sin(theta) and E_r/sin(theta) (E = v
+    // x B; the k-derivatives of the curls divide them by the cell's sin(theta),
+    // which its k-neighbours share) and E_theta over the p1 window: [WP][PLI]
+    // twice and [WP][NJ][NIP]; E_r and E_phi of the chunk's own planes, on the
+    // points that i- and j-derivatives reach: [KPAR][NJP][NI] and [KPAR][PL].
+    // With the derivatives' FMAs and the quotients by rho0 and sin(theta)
+    // through reciprocals a cell takes 377 FP64 instructions instead of 548
+    // (442,368 cells: 477 -> 359 us per stage in 8^3 blocks, 652 -> 482 in 16^3).
+    static constexpr bool kPoint = sizeof(T) == 8;
+    static constexpr int NXS = kPoint ? 2 * WP * PLI : 0, NE2 = kPoint ? WP * NJ * NIP : 0;
+    static constexpr int NE1 = kPoint ? KPAR * NJP * NI : 0, NE3 = kPoint ? KPAR * PL : 0;
+    // shared memory: mbarriers | A1/A2 (double) | tile[NV][W][PL] | p1[WP][PL] | xs | e2 | e1 | e3 | gi | gj | gs
     static constexpr size_t off_a12 = 16;
     static constexpr size_t off_tile = off_a12 + ((2 * NIP * sizeof(double) + 15) / 16) * 16;
     static constexpr size_t off_p1 = off_tile + (size_t)NV * W * PL * sizeof(T);
     static constexpr size_t off_xs = off_p1 + (size_t)WP * PL * sizeof(T);
-    static constexpr size_t off_gi = off_xs + (size_t)NXS * WP * PL * sizeof(T);
+    static constexpr size_t off_e2 = off_xs + (size_t)NXS * sizeof(T);
+    static constexpr size_t off_e1 = off_e2 + (size_t)NE2 * sizeof(T);
+    static constexpr size_t off_e3 = off_e1 + (size_t)NE1 * sizeof(T);
+    static constexpr size_t off_gi = off_e3 + (size_t)NE3 * sizeof(T);
     static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * NIP * sizeof(T);
     static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * NJP * sizeof(T);
     static constexpr size_t smem_stage = off_gs + GS_COUNT * sizeof(T);
@@ -481,6 +590,9 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
     T* tile = reinterpret_cast<T*>(smem + S::off_tile);
     T* tp1 = reinterpret_cast<T*>(smem + S::off_p1);
     T* txs = reinterpret_cast<T*>(smem + S::off_xs);   // FP64: [0] Br/sin, [1] E_r/sin (E = v x B)
+    T* te2 = reinterpret_cast<T*>(smem + S::off_e2);   // FP64: E_theta, E_r, E_phi
+    T* te1 = reinterpret_cast<T*>(smem + S::off_e1);
+    T* te3 = reinterpret_cast<T*>(smem + S::off_e3);
     T* gi = reinterpret_cast<T*>(smem + S::off_gi);
     T* gj = reinterpret_cast<T*>(smem + S::off_gj);
     T* gs = reinterpret_cast<T*>(smem + S::off_gs);
@@ -535,12 +647,20 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
     const T rho0c = GRHO0[ii], rho0inv = gi[GI_RHO0INV * NIP + ii];
     const T gor0 = gi[GI_GOR0 * NIP + ii], heat = gi[GI_HEAT * NIP + ii], xi2inv = gi[GI_XI2INV * NIP + ii];
     const double dt = sc->dt;
-    const double divs = (double)(5.0f - (float)stage);
-    // x / divs for divs = 4, 2, 1 (stages 1, 3, 4) is x times the exact
-    // reciprocal, the same bits without an FP64 division; stage 2 divides by 3
-    const bool div_pow2 = stage != 2;
-    const double rdivs = 1.0 / divs;
-    auto over_divs = [&](double x) { return div_pow2 ? x * rdivs : x / divs; };
+    // (dt R) / (5 - stage): for 4, 2, 1 (stages 1, 3, 4) the division is exact
+    // and goes into dt, the same bits; stage 2 divides by 3
+    const Divisor three{3.0, 1.0 / 3.0, 1000u};
+    const double dts = stage == 2 ? dt : dt / (double)(5.0f - (float)stage);
+    auto advance = [&](double R) {   // (dt R) / (5 - stage)
+        const double x = dts * R;
+        return stage == 2 ? div_by(x, three) : x;
+    };
+    Divisor by_rho0{1.0, 1.0, 0u};   // FP64: quotients by the cell's rho0
+    if constexpr (Pol<T>::exact) by_rho0 = divisor((double)rho0c);
+    auto over_rho0 = [&](T x) -> T {
+        if constexpr (Pol<T>::exact) return (T)div_by((double)x, by_rho0);
+        else return Pol<T>::dv(x, rho0c, rho0inv);
+    };
     const float dtk = sc->dt_stage_f[stage - 1];
 
     constexpr int nchunk = NK / KPAR;
@@ -588,18 +708,33 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
                 const double s1v = (double)tile[(V_S1 * W + slot) * PL + c];
                 tp1[(kp % WP) * PL + c] = (T)(a12[ic] * r1 + a12[NIP + ic] * s1v);
                 const int jc = c / NIP;
-                if (ic >= 2 && ic < NI + 2 && jc >= 2 && jc < NJ + 2) {   // the k-neighbours of interior cells
+                if (jc >= 2 && jc < NJ + 2) {   // the k-neighbours of interior cells, and E_theta's i-neighbours
                     auto at = [&](int v) { return tile[(v * W + slot) * PL + c]; };
-                    const T sn = gj[GJ_SIN * S::NJP + jc];
-                    txs[(0 * WP + kp % WP) * PL + c] = Pol<T>::dv(at(V_BR), sn, T(0));
-                    txs[(1 * WP + kp % WP) * PL + c] =
-                        Pol<T>::dv(at(V_VT) * at(V_BP) - at(V_VP) * at(V_BT), sn, T(0));
+                    const T vr = at(V_VR), vp = at(V_VP), br = at(V_BR), bp = at(V_BP);
+                    te2[((kp % WP) * NJ + jc - 2) * NIP + ic] = vp * br - vr * bp;
+                    if (ic >= 2 && ic < NI + 2) {
+                        const Divisor by_sin{gj[GJ_SIN * S::NJP + jc], gj[GJ_SININV * S::NJP + jc], 1000u};
+                        T* xs = txs + (kp % WP) * S::PLI + (jc - 2) * NI + ic - 2;
+                        xs[0] = div_by(br, by_sin);
+                        xs[WP * S::PLI] = div_by(at(V_VT) * bp - vp * at(V_BT), by_sin);
+                    }
                 }
             } else {
                 const float* f = reinterpret_cast<const float*>(a12);
                 tp1[(kp % WP) * PL + c] = p1_ff(f[ic], f[NIP + ic], f[2 * NIP + ic], f[3 * NIP + ic],
                                                 (float)tile[(V_RHO1 * W + slot) * PL + c],
                                                 (float)tile[(V_S1 * W + slot) * PL + c]);
+            }
+        }
+        if constexpr (Pol<T>::exact) {   // E_r and E_phi of the chunk's planes
+            for (int x = tid; x < KPAR * PL; x += S::NT) {
+                const int q = x / PL, c = x % PL, ic = c % NIP, jc = c / NIP, slot = (k0 + 1 + q) % W;
+                const bool in_i = ic >= 2 && ic < NI + 2, in_j = jc >= 2 && jc < NJ + 2;
+                if (!in_i && !in_j) continue;
+                auto at = [&](int v) { return tile[(v * W + slot) * PL + c]; };
+                const T vt = at(V_VT), bt = at(V_BT);
+                te3[q * PL + c] = at(V_VR) * bt - vt * at(V_BR);
+                if (in_i) te1[(q * S::NJP + jc) * NI + ic - 2] = vt * at(V_BP) - at(V_VP) * bt;
             }
         }
         __syncthreads();
@@ -612,7 +747,11 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         };
         auto P = [&](int di, int dj, int dk) -> T { return tp1[sp[dk + 2] * PL + (jj + dj) * NIP + ii + di]; };
         // ModDerivative_1st_O4_3D (3_6/ModDerivative.f90:16-32)
-        auto D = [&](T c, auto f) -> T { return c * (((-f(2) + T(8) * f(1)) - T(8) * f(-1)) + f(-2)); };
+        auto D = [&](T c, auto f) -> T {
+            // 8 f is exact, so the FP64 FMAs round where the reference's sums do
+            if constexpr (Pol<T>::exact) return c * (fma(-8.0, f(-1), fma(8.0, f(1), -f(2))) + f(-2));
+            else return c * (((-f(2) + T(8) * f(1)) - T(8) * f(-1)) + f(-2));
+        };
         const T vr = A(V_VR, 0, 0, 0), vt = A(V_VT, 0, 0, 0), vp = A(V_VP, 0, 0, 0);
         const T br = A(V_BR, 0, 0, 0), bt = A(V_BT, 0, 0, 0), bp = A(V_BP, 0, 0, 0);
         const T rho1 = A(V_RHO1, 0, 0, 0);
@@ -667,16 +806,16 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
             T g3 = D(c3, [&](int m) { return P(0, 0, m); });
             g3 = g3 * rinv;
             g3 = g3 * sinv;
-            Rvr = Rvr - Pol<T>::dv(g1, rho0c, rho0inv);
-            Rvt = Rvt - Pol<T>::dv(g2, rho0c, rho0inv);
-            Rvp = Rvp - Pol<T>::dv(g3, rho0c, rho0inv);
+            Rvr = Rvr - over_rho0(g1);
+            Rvt = Rvt - over_rho0(g2);
+            Rvp = Rvp - over_rho0(g3);
         }
         // Lorentz force (curl B) x B / rho0 (3_6/ModEquation.f90:97-116, curl :38-102)
         {
             T k1 = D(c2, [&](int m) { return A(V_BP, 0, m, 0) * GSIN[jj + m]; }) -
                    D(c3, [&](int m) { return A(V_BT, 0, 0, m); });
             auto brs = [&](int m) -> T {   // Br / sin(theta) at the k-neighbour m
-                if constexpr (Pol<T>::exact) return txs[(0 * WP + sp[m + 2]) * PL + jj * NIP + ii];
+                if constexpr (Pol<T>::exact) return txs[sp[m + 2] * S::PLI + j * NI + i];
                 else return Pol<T>::dv(A(V_BR, 0, 0, m), sin_c, sinv);
             };
             T k2 = D(c3, brs) -
@@ -688,9 +827,9 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
             const T x1 = k2 * bp - k3 * bt;
             const T x2 = k3 * br - k1 * bp;
             const T x3 = k1 * bt - k2 * br;
-            Rvr = Rvr + Pol<T>::dv(x1, rho0c, rho0inv);
-            Rvt = Rvt + Pol<T>::dv(x2, rho0c, rho0inv);
-            Rvp = Rvp + Pol<T>::dv(x3, rho0c, rho0inv);
+            Rvr = Rvr + over_rho0(x1);
+            Rvt = Rvt + over_rho0(x2);
+            Rvp = Rvp + over_rho0(x3);
         }
         // Buoyancy -(g/rho0) rho1 (3_6/ModEquation.f90:121-127)
         Rvr = Rvr - gor0 * rho1;
@@ -701,12 +840,22 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         // Induction curl(v x B) (3_6/ModEquation.f90:154-162)
         T RBr, RBt, RBp;
         {
-            auto E1 = [&](int a, int bq, int c) { return A(V_VT, a, bq, c) * A(V_BP, a, bq, c) - A(V_VP, a, bq, c) * A(V_BT, a, bq, c); };
-            auto E2 = [&](int a, int bq, int c) { return A(V_VP, a, bq, c) * A(V_BR, a, bq, c) - A(V_VR, a, bq, c) * A(V_BP, a, bq, c); };
-            auto E3 = [&](int a, int bq, int c) { return A(V_VR, a, bq, c) * A(V_BT, a, bq, c) - A(V_VT, a, bq, c) * A(V_BR, a, bq, c); };
+            // FP64: from the point arrays (E1 along j, E2 along i and k, E3 along i and j)
+            auto E1 = [&](int a, int bq, int c) -> T {
+                if constexpr (Pol<T>::exact) return te1[(kq * S::NJP + jj + bq) * NI + i];
+                else return A(V_VT, a, bq, c) * A(V_BP, a, bq, c) - A(V_VP, a, bq, c) * A(V_BT, a, bq, c);
+            };
+            auto E2 = [&](int a, int bq, int c) -> T {
+                if constexpr (Pol<T>::exact) return te2[(sp[c + 2] * NJ + j) * NIP + ii + a];
+                else return A(V_VP, a, bq, c) * A(V_BR, a, bq, c) - A(V_VR, a, bq, c) * A(V_BP, a, bq, c);
+            };
+            auto E3 = [&](int a, int bq, int c) -> T {
+                if constexpr (Pol<T>::exact) return te3[kq * PL + (jj + bq) * NIP + ii + a];
+                else return A(V_VR, a, bq, c) * A(V_BT, a, bq, c) - A(V_VT, a, bq, c) * A(V_BR, a, bq, c);
+            };
             T q1 = D(c2, [&](int m) { return E3(0, m, 0) * GSIN[jj + m]; }) - D(c3, [&](int m) { return E2(0, 0, m); });
             auto e1s = [&](int m) -> T {   // E1 / sin(theta) at the k-neighbour m
-                if constexpr (Pol<T>::exact) return txs[(1 * WP + sp[m + 2]) * PL + jj * NIP + ii];
+                if constexpr (Pol<T>::exact) return txs[(WP + sp[m + 2]) * S::PLI + j * NI + i];
                 else return Pol<T>::dv(E1(0, 0, m), sin_c, sinv);
             };
             T q2 = D(c3, e1s) -
@@ -761,7 +910,7 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
             const size_t pc = (size_t)b * NCELL + (size_t)kp * PL + jj * NIP + ii;
             const T pn = static_cast<const T*>(psi.un)[pc];
             T po;
-            if constexpr (Pol<T>::exact) po = (T)((double)pn + over_divs(dt * (double)Rpsi));
+            if constexpr (Pol<T>::exact) po = (T)((double)pn + advance((double)Rpsi));
             else po = fmaf((float)dtk, (float)Rpsi, (float)pn);
             static_cast<T*>(psi.out)[pc] = po;
         }
@@ -771,7 +920,7 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         T o[NV];
         if constexpr (Pol<T>::exact) {
 #pragma unroll
-            for (int v = 0; v < NV; ++v) o[v] = (T)((double)u0s[v] + over_divs(dt * (double)R[v]));
+            for (int v = 0; v < NV; ++v) o[v] = (T)((double)u0s[v] + advance((double)R[v]));
         } else if (ulo != nullptr && stage == 4) {
             // u^{n+1} = u^n + dt*R with u^n and u^{n+1} compensated
             int8_t* ql = ulo + (size_t)b * NV * S::NINT + ((size_t)(kp - 2) * NJ + (jj - 2)) * NI + (ii - 2);
@@ -1551,42 +1700,51 @@ __global__ void __launch_bounds__(NI * NJ) k_push_state(float* u, PushTable push
 // ---------------------------------------------------------------------------
 // FP64 artificial diffusion (3_6/ModDiffusion.f90:9-150) of one block as a k
 // march, in place (the exact path: no pushes, no fused CFL minimum, no u^n
-// correction). One thread per (cell column, variable): NI*NJ*NV threads. The
-// k window, slope and face of the thread's column and variable stay in
-// registers; across each plane every i and j slope is formed once, then every
-// i and j face flux, then each cell sums its six faces. The fluxes are the
-// chunked kernel's functions of the same four values and the sum runs in the
-// reference's order (i, j, k, each as a division by its denominator), so the
-// result is the same bit for bit, with 3 minmod slopes per cell and variable
-// where the chunked kernel forms 5 or 6.
-template <int NI, int NJ, int NK>
+// correction). A thread takes VPT variables of one cell column: 8^3 blocks run
+// one variable per thread (512 threads), 16^3 blocks four (512 threads, one
+// CTA per SM by shared memory). The k window, slope and face of the thread's
+// column stay in registers; across each plane every i and j slope is formed
+// once, then every i and j face flux, then each cell sums its six faces in the
+// reference's order. Bound by the FP64 pipe, so what counts is FP64
+// instructions per cell and variable: the slopes are half_minmod (3 of them
+// plus one integer selector, 17 in the formula), a face's difference is the
+// slopes' own, its speed sum is formed once for all variables, only faces near
+// an extremum divide (face_flux_h) and the sums divide by reciprocals (div_by).
+// 442,368 cells, CUDA events: 8^3 blocks 1678 -> 768 us (251 -> 105 FP64
+// instructions per cell and variable), 16^3 blocks 2385 (chunked kernel) -> 971 us.
+template <int NI, int NJ, int NK, int VPT>
 struct M64Shape {
     static constexpr int NG = 2, NIP = NI + 4, NJP = NJ + 4, NKP = NK + 4;
     static constexpr int PL = NIP * NJP, NCELL = PL * NKP;
-    static constexpr int NCOL = NI * NJ, NT = NCOL * NV;
+    static constexpr int NCOL = NI * NJ, NT = NCOL * NV / VPT;
     static constexpr int W = 5;                          // plane ring slots
     static constexpr uint32_t PLB = PL * 8u;
     static constexpr int P = NI + 2;                     // row pitch of the slope and face arrays
-    // per variable: SI[NJ][P] (cells i = -1..NI at i + 1), SJ[NJ + 2][P]
-    // (rows j = -1..NJ at j + 1), FI[NJ][P] (faces i - 1/2, i = 0..NI), FJ[NJ + 1][P]
+    // per variable: half slopes SI[NJ][P] (cells i = -1..NI at i + 1), SJ[NJ + 2][P]
+    // (rows j = -1..NJ at j + 1), fluxes FI[NJ][P] (faces i - 1/2, i = 0..NI), FJ[NJ + 1][P];
+    // speed sums of the plane's faces: VI[NJ][P], VJ[NJ + 1][P], VK[NJ][P] (the face above)
     static constexpr int NSI = NJ * P, NSJ = (NJ + 2) * P, NFI = NJ * P, NFJ = (NJ + 1) * P;
-    // shared memory: mbarriers | tile[NV][W][PL] | SI | SJ | FI | FJ | gi | gj | gs
+    // shared memory: mbarriers | tile[NV][W][PL] | SI | SJ | FI | FJ | VI | VJ | VK | gi | gj | gs
     static constexpr size_t off_tile = 64;
     static constexpr size_t off_si = off_tile + (size_t)NV * W * PL * 8;
     static constexpr size_t off_sj = off_si + (size_t)NV * NSI * 8;
     static constexpr size_t off_fi = off_sj + (size_t)NV * NSJ * 8;
     static constexpr size_t off_fj = off_fi + (size_t)NV * NFI * 8;
-    static constexpr size_t off_gi = off_fj + (size_t)NV * NFJ * 8;
+    static constexpr size_t off_vi = off_fj + (size_t)NV * NFJ * 8;
+    static constexpr size_t off_vj = off_vi + (size_t)NFI * 8;
+    static constexpr size_t off_vk = off_vj + (size_t)NFJ * 8;
+    static constexpr size_t off_gi = off_vk + (size_t)NFI * 8;
     static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * NIP * 8;
     static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * NJP * 8;
     static constexpr size_t smem = off_gs + GS_COUNT * 8;
-    static_assert(NT <= 1024, "one thread per column and variable");
+    static_assert(NT <= 1024 && NV % VPT == 0, "whole columns");
+    static_assert(smem <= 232448, "227 KB of shared memory per CTA");
 };
 
-template <int NI, int NJ, int NK>
-__global__ void __launch_bounds__(NI * NJ * NV)
+template <int NI, int NJ, int NK, int VPT>
+__global__ void __launch_bounds__(NI * NJ * NV / VPT)
 k_diffusion_march64(double* u, Geometry g, StepScalars* sc) {
-    using S = M64Shape<NI, NJ, NK>;
+    using S = M64Shape<NI, NJ, NK, VPT>;
     constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, P = S::P;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
@@ -1595,6 +1753,9 @@ k_diffusion_march64(double* u, Geometry g, StepScalars* sc) {
     double* SJ = reinterpret_cast<double*>(smem + S::off_sj);
     double* FI = reinterpret_cast<double*>(smem + S::off_fi);
     double* FJ = reinterpret_cast<double*>(smem + S::off_fj);
+    double* VI = reinterpret_cast<double*>(smem + S::off_vi);
+    double* VJ = reinterpret_cast<double*>(smem + S::off_vj);
+    double* VK = reinterpret_cast<double*>(smem + S::off_vk);
     double* gi = reinterpret_cast<double*>(smem + S::off_gi);
     double* gj = reinterpret_cast<double*>(smem + S::off_gj);
     double* gs = reinterpret_cast<double*>(smem + S::off_gs);
@@ -1612,12 +1773,13 @@ k_diffusion_march64(double* u, Geometry g, StepScalars* sc) {
     }
     load_geometry<double, S>(g, b, gi, gj, gs, nullptr);
     __syncthreads();
-    const int c = tid % S::NCOL, v = tid / S::NCOL;
+    const int c = tid % S::NCOL, v0 = tid / S::NCOL * VPT;
     const int i = c % NI, j = c / NI, ii = i + 2, jj = j + 2;
     const double* GCS = gi + GI_CS * NIP;
     const double cs = GCS[ii];
     const double rc = gi[GI_R * NIP + ii];
-    const double den[3] = {gs[GS_DXI], gs[GS_DXJ] * rc, gs[GS_DXK] * rc * gj[GJ_SIN * S::NJP + jj]};
+    const Divisor den0 = divisor(gs[GS_DXI]), den1 = divisor(gs[GS_DXJ] * rc),
+                  den2 = divisor(gs[GS_DXK] * rc * gj[GJ_SIN * S::NJP + jj]);
     const double hdt = 0.5 * sc->dt;
     const int polls = sc->wait_polls;
     int late = 0;
@@ -1628,78 +1790,106 @@ k_diffusion_march64(double* u, Geometry g, StepScalars* sc) {
             mbar_wait(&bars[p % W], (uint32_t)((p / W) & 1), kWaitPolls);
         for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
     };
-    double* SIv = SI + v * S::NSI;
-    double* SJv = SJ + v * S::NSJ;
-    double* FIv = FI + v * S::NFI;
-    double* FJv = FJ + v * S::NFJ;
-    const double* col = tile + (size_t)v * W * PL + jj * NIP + ii;         // this column, this variable
+    const double* col = tile + (size_t)v0 * W * PL + jj * NIP + ii;        // this column, the first variable
     const double* colvp = tile + (size_t)V_VP * W * PL + jj * NIP + ii;    // this column's v_phi
     for (int p = 0; p < 4; ++p) late |= mbar_wait(&bars[p], 0u, polls) ? 0 : 1;
-    double u0, u1, dk0, fk0;
+    // per variable: u at kp and kp + 1, their difference, the half slope at kp, the flux below kp
+    double u0[VPT], u1[VPT], dk[VPT], hk0[VPT], fk0[VPT];
     {
-        const double a0 = col[0], a1 = col[PL], a2 = col[2 * PL], a3 = col[3 * PL];
-        const double d1 = face_slope(a0, a1, a2), d2 = face_slope(a1, a2, a3);
-        u0 = a2;
-        u1 = a3;
-        dk0 = d2;
-        fk0 = face_flux_s(a1, a2, d1, d2, fabs(colvp[PL]) + cs, fabs(colvp[2 * PL]) + cs);
+        const double speed = (fabs(colvp[2 * PL]) + cs) + (fabs(colvp[PL]) + cs);
+#pragma unroll
+        for (int q = 0; q < VPT; ++q) {
+            const double* a = col + q * W * PL;
+            const double a0 = a[0], a1 = a[PL], a2 = a[2 * PL], a3 = a[3 * PL];
+            const double d0 = a1 - a0, d1 = a2 - a1, d2 = a3 - a2;
+            u0[q] = a2;
+            u1[q] = a3;
+            dk[q] = d2;
+            hk0[q] = half_minmod(d1, d2, a3 - a1);
+            fk0[q] = face_flux_h(a1, a2, d1, half_minmod(d0, d1, a2 - a0), hk0[q], speed);
+        }
     }
     for (int kp = 2; kp < NK + 2; ++kp) {
         const int p2 = kp + 2;
         late |= mbar_wait(&bars[p2 % W], (uint32_t)((p2 / W) & 1), polls) ? 0 : 1;
         const int s0 = (kp % W) * PL, s1 = ((kp + 1) % W) * PL, s2 = (p2 % W) * PL;
         const double* tc = col + s0;   // this cell in plane kp
-        // ---- phase A: k slope and face from the window; i and j slopes
-        const double u2 = col[s2];
-        const double dk1 = face_slope(u0, u1, u2);
-        const double fk1 = face_flux_s(u0, u1, dk0, dk1, fabs(colvp[s0]) + cs, fabs(colvp[s1]) + cs);
-        SIv[j * P + i + 1] = face_slope(tc[-1], u0, tc[1]);
-        SJv[(j + 1) * P + i] = face_slope(tc[-NIP], u0, tc[NIP]);
-        // ghost-cell slopes: i = -1, NI of every row, j = -1, NJ of every column
+        // ---- phase A: the k slope of plane kp + 1, the i and j slopes, the speed sums
+        double u2[VPT], dk1[VPT], hk1[VPT], dli[VPT], dlj[VPT];
+#pragma unroll
+        for (int q = 0; q < VPT; ++q) {
+            const double* a = tc + q * W * PL;
+            u2[q] = col[q * W * PL + s2];
+            dk1[q] = u2[q] - u1[q];
+            hk1[q] = half_minmod(dk[q], dk1[q], u2[q] - u0[q]);
+            const double l = a[-1], r = a[1], d = a[-NIP], t = a[NIP];
+            dli[q] = u0[q] - l;
+            dlj[q] = u0[q] - d;
+            SI[(v0 + q) * S::NSI + j * P + i + 1] = half_minmod(dli[q], r - u0[q], r - l);
+            SJ[(v0 + q) * S::NSJ + (j + 1) * P + i] = half_minmod(dlj[q], t - u0[q], t - d);
+        }
+        // ghost-cell slopes: i = -1, NI of every row, j = -1, NJ of every
+        // column; then the faces' speed sums, |v_dir| + c_s on either side
         constexpr int NEI = 2 * NJ * NV, NEJ = 2 * NI * NV;
-        for (int x = tid; x < NEI + NEJ; x += S::NT) {
-            if (x < NEI) {
-                const int side = x & 1, r = (x >> 1) % NJ, w = (x >> 1) / NJ;
-                const double* q = tile + (size_t)w * W * PL + s0 + (r + 2) * NIP + (side ? NI + 2 : 1);
-                SI[w * S::NSI + r * P + (side ? NI + 1 : 0)] = face_slope(q[-1], q[0], q[1]);
+        constexpr int NVI = NJ * (NI + 1), NVJ = (NJ + 1) * NI, NVK = NJ * NI;
+        for (int x = tid; x < NEI + NEJ + NVI + NVJ + NVK; x += S::NT) {
+            if (x < NEI + NEJ) {
+                const bool on_i = x < NEI;
+                const int y = on_i ? x : x - NEI, n = on_i ? NJ : NI;
+                const int side = y & 1, r = (y >> 1) % n, w = (y >> 1) / n, st = on_i ? 1 : NIP;
+                const double* q = tile + (size_t)w * W * PL + s0 +
+                                  (on_i ? (r + 2) * NIP + (side ? NI + 2 : 1) : (side ? NJ + 2 : 1) * NIP + r + 2);
+                const double l = q[-st], m = q[0], t = q[st];
+                double* dst = on_i ? SI + w * S::NSI + r * P + (side ? NI + 1 : 0)
+                                   : SJ + w * S::NSJ + (side ? NJ + 1 : 0) * P + r;
+                *dst = half_minmod(m - l, t - m, t - l);
+                continue;
+            }
+            const int y = x - NEI - NEJ;
+            if (y < NVI) {
+                const int r = y / (NI + 1), e = y % (NI + 1);
+                const double* a = tile + (size_t)V_VR * W * PL + s0 + (r + 2) * NIP + e + 1;
+                VI[r * P + e] = (fabs(a[1]) + GCS[e + 2]) + (fabs(a[0]) + GCS[e + 1]);
+            } else if (y < NVI + NVJ) {
+                const int r = (y - NVI) / NI, e = (y - NVI) % NI;
+                const double* a = tile + (size_t)V_VT * W * PL + s0 + (r + 1) * NIP + e + 2;
+                VJ[r * P + e] = (fabs(a[NIP]) + GCS[e + 2]) + (fabs(a[0]) + GCS[e + 2]);
             } else {
-                const int y = x - NEI, side = y & 1, r = (y >> 1) % NI, w = (y >> 1) / NI;
-                const double* q = tile + (size_t)w * W * PL + s0 + (side ? NJ + 2 : 1) * NIP + r + 2;
-                SJ[w * S::NSJ + (side ? NJ + 1 : 0) * P + r] = face_slope(q[-NIP], q[0], q[NIP]);
+                const int r = (y - NVI - NVJ) / NI, e = (y - NVI - NVJ) % NI;
+                const double* a = tile + (size_t)V_VP * W * PL + (r + 2) * NIP + e + 2;
+                VK[r * P + e] = (fabs(a[s1]) + GCS[e + 2]) + (fabs(a[s0]) + GCS[e + 2]);
             }
         }
         if (__syncthreads_or(late)) {
             abort_cta();
             return;
         }
-        // ---- phase B: this cell's faces i - 1/2 and j - 1/2; the last faces
-        // of the rows and columns
-        const double* vr = tile + (size_t)V_VR * W * PL + s0 + jj * NIP + ii;
-        const double* vt = tile + (size_t)V_VT * W * PL + s0 + jj * NIP + ii;
-        const double fi0 = face_flux_s(tc[-1], u0, SIv[j * P + i], SIv[j * P + i + 1], fabs(vr[-1]) + GCS[ii - 1],
-                                       fabs(vr[0]) + cs);
-        const double fj0 =
-            face_flux_s(tc[-NIP], u0, SJv[j * P + i], SJv[(j + 1) * P + i], fabs(vt[-NIP]) + cs, fabs(vt[0]) + cs);
-        FIv[j * P + i] = fi0;
-        FJv[j * P + i] = fj0;
+        // ---- phase B: the face above this cell and its faces i - 1/2 and j -
+        // 1/2; the last faces of the rows and columns
+        double fk1[VPT], fi0[VPT], fj0[VPT];
+        const double vi = VI[j * P + i], vj = VJ[j * P + i], vk = VK[j * P + i];
+#pragma unroll
+        for (int q = 0; q < VPT; ++q) {
+            const double* a = tc + q * W * PL;
+            const double* si = SI + (v0 + q) * S::NSI + j * P + i;
+            const double* sj = SJ + (v0 + q) * S::NSJ + j * P + i;
+            fk1[q] = face_flux_h(u0[q], u1[q], dk[q], hk0[q], hk1[q], vk);
+            fi0[q] = face_flux_h(a[-1], u0[q], dli[q], si[0], si[1], vi);
+            fj0[q] = face_flux_h(a[-NIP], u0[q], dlj[q], sj[0], sj[P], vj);
+            FI[(v0 + q) * S::NFI + j * P + i] = fi0[q];
+            FJ[(v0 + q) * S::NFJ + j * P + i] = fj0[q];
+        }
         constexpr int NFE = NJ * NV + NI * NV;
         for (int x = tid; x < NFE; x += S::NT) {
-            if (x < NJ * NV) {
-                const int r = x % NJ, w = x / NJ;
-                const double* a = tile + (size_t)w * W * PL + s0 + (r + 2) * NIP + NI + 1;   // last interior cell of row r
-                const double* vrr = tile + (size_t)V_VR * W * PL + s0 + (r + 2) * NIP + NI + 1;
-                FI[w * S::NFI + r * P + NI] =
-                    face_flux_s(a[0], a[1], SI[w * S::NSI + r * P + NI], SI[w * S::NSI + r * P + NI + 1],
-                                fabs(vrr[0]) + GCS[NI + 1], fabs(vrr[1]) + GCS[NI + 2]);
-            } else {
-                const int y = x - NJ * NV, r = y % NI, w = y / NI;
-                const double* a = tile + (size_t)w * W * PL + s0 + (NJ + 1) * NIP + r + 2;   // last interior row, column r
-                const double* vtt = tile + (size_t)V_VT * W * PL + s0 + (NJ + 1) * NIP + r + 2;
-                const double c2 = GCS[r + 2];
-                FJ[w * S::NFJ + NJ * P + r] =
-                    face_flux_s(a[0], a[NIP], SJ[w * S::NSJ + NJ * P + r], SJ[w * S::NSJ + (NJ + 1) * P + r],
-                                fabs(vtt[0]) + c2, fabs(vtt[NIP]) + c2);
-            }
+            const bool on_i = x < NJ * NV;
+            const int y = on_i ? x : x - NJ * NV, n = on_i ? NJ : NI, r = y % n, w = y / n;
+            const double* a = tile + (size_t)w * W * PL + s0 +
+                              (on_i ? (r + 2) * NIP + NI + 1 : (NJ + 1) * NIP + r + 2);   // last interior cell
+            const double l = a[0], t = on_i ? a[1] : a[NIP];
+            const double* h = on_i ? SI + w * S::NSI + r * P + NI : SJ + w * S::NSJ + NJ * P + r;
+            const double speed = on_i ? VI[r * P + NI] : VJ[NJ * P + r];
+            double* dst = on_i ? FI + w * S::NFI + r * P + NI : FJ + w * S::NFJ + NJ * P + r;
+            *dst = face_flux_h(l, t, t - l, h[0], on_i ? h[1] : h[P], speed);
         }
         __syncthreads();
         if (tid == 0) {
@@ -1707,15 +1897,18 @@ k_diffusion_march64(double* u, Geometry g, StepScalars* sc) {
                 issue_planes<double, S>(blk, tile, issued, issued + 1, &bars[issued % W]);
         }
         // ---- phase C: the six faces in the reference's order, the update in place
-        double R = 0.0;
-        R = R + Pol<double>::dv(fi0 - FIv[j * P + i + 1], den[0], 0.0);
-        R = R + Pol<double>::dv(fj0 - FJv[(j + 1) * P + i], den[1], 0.0);
-        R = R + Pol<double>::dv(fk0 - fk1, den[2], 0.0);
-        blk[(size_t)v * NCELL + (size_t)kp * PL + jj * NIP + ii] = u0 + hdt * R;
-        u0 = u1;
-        u1 = u2;
-        dk0 = dk1;
-        fk0 = fk1;
+#pragma unroll
+        for (int q = 0; q < VPT; ++q) {
+            double R = div_by(fi0[q] - FI[(v0 + q) * S::NFI + j * P + i + 1], den0);
+            R = R + div_by(fj0[q] - FJ[(v0 + q) * S::NFJ + (j + 1) * P + i], den1);
+            R = R + div_by(fk0[q] - fk1[q], den2);
+            blk[(size_t)(v0 + q) * NCELL + (size_t)kp * PL + jj * NIP + ii] = u0[q] + hdt * R;
+            u0[q] = u1[q];
+            u1[q] = u2[q];
+            dk[q] = dk1[q];
+            hk0[q] = hk1[q];
+            fk0[q] = fk1[q];
+        }
     }
     if (__syncthreads_or(late)) {
         abort_cta();
