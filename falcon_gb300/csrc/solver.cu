@@ -34,6 +34,7 @@
 #include "../../include/falcon_gb300.h"
 #include "lcc.h"
 #include "solver.h"
+#include "vcycle.cuh"
 
 namespace falcon {
 namespace sv {
@@ -51,13 +52,11 @@ struct HaloList {
     const int32_t* dst;    // padded global offset
     const int32_t* src;    // padded global offset of the base source cell
     const uint8_t* code;   // bit d set: the weight of direction d is not 0
-    const double* w;       // [n][3] (FP64 fills)
-    const float* wf;       // [n][3] (FP32 fills: the V-cycle)
+    const double* w;       // [n][3]
     int32_t sj, sk;        // padded strides of j and k
 };
 
 struct Ops64 { const double *Aii, *Ai, *Aj, *Ak; };
-struct Ops32 { const float *Aii, *Ai, *Aj, *Ak; };
 
 // Launch geometry of the cell kernels: CTAs take chunks of d.chunk cells,
 // block-major (consecutive CTAs stream consecutive memory); a chunk never
@@ -123,12 +122,7 @@ __global__ void k_halo(T* v, HaloList H, const int32_t* cdst, const int32_t* csr
     const size_t s = (size_t)H.src[e];
     const int cd = H.code[e];
     const int a = (cd & 1) ? 1 : 0, bq = (cd & 2) ? H.sj : 0, c = (cd & 4) ? H.sk : 0;
-    T wi, wj, wk;
-    if constexpr (sizeof(T) == 4) {
-        wi = H.wf[3 * e]; wj = H.wf[3 * e + 1]; wk = H.wf[3 * e + 2];
-    } else {
-        wi = H.w[3 * e]; wj = H.w[3 * e + 1]; wk = H.w[3 * e + 2];
-    }
+    const T wi = H.w[3 * e], wj = H.w[3 * e + 1], wk = H.w[3 * e + 2];
     const T ui = T(1) - wi, uj = T(1) - wj, uk = T(1) - wk;
     const T* f = v + s;
     v[H.dst[e]] = f[0] * ui * uj * uk + f[a] * wi * uj * uk + f[bq] * ui * wj * uk + f[c] * ui * uj * wk +
@@ -137,48 +131,20 @@ __global__ void k_halo(T* v, HaloList H, const int32_t* cdst, const int32_t* csr
 
 // ---- FP64 outer iteration ----------------------------------------------------
 struct Dots {
-    double *pAp, *pr, *zAp, *rr, *bb, *ab;   // ab: sum of (|b| + sum_j |A_ij x_j|)^2
+    double *pAp, *zw, *zAp, *rr, *bb, *ab;   // ab: sum of (|b| + sum_j |A_ij x_j|)^2
+    double *pw, *zr;
     const int32_t* active;
     const int32_t* bprob;
 };
 
-// Ap = A p; pAp += p.Ap; pr += p.r (per problem)
-__global__ void k_spmv_dots(Ops64 A, LevelDims d, const double* p, double* Ap, const double* r, Dots D) {
+// y = A x
+__global__ void k_spmv(Ops64 A, LevelDims d, const double* x, double* y) {
     const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    double pa = 0, pr = 0;
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
         int i, j, k;
         cell_ijk(d, c, i, j, k);
-        const double y = apply_A<double>(A, d, p, b, c, i, j, k);
-        const size_t q = (size_t)b * d.nint + c;
-        Ap[q] = y;
-        const double pv = p[pidx(d, b, i, j, k)];
-        pa += pv * y;
-        pr += pv * r[q];
+        y[(size_t)b * d.nint + c] = apply_A<double>(A, d, x, b, c, i, j, k);
     }
-    const int pb = D.bprob[b];
-    block_sum_atomic(pa, &D.pAp[pb]);
-    block_sum_atomic(pr, &D.pr[pb]);
-}
-
-// alpha = p.r / p.Ap; x += alpha p; r -= alpha Ap; rr += r.r; rf = (float)r
-__global__ void k_update_xr(LevelDims d, double* x, const double* p, double* r, const double* Ap, float* rf, Dots D) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    const int pb = D.bprob[b];
-    // a problem whose direction vanished (p.Ap == 0) takes no step instead of 0/0
-    const double alpha = (D.active[pb] && D.pAp[pb] != 0.0) ? D.pr[pb] / D.pAp[pb] : 0.0;
-    double rr = 0;
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const size_t P = pidx(d, b, i, j, k), q = (size_t)b * d.nint + c;
-        x[P] = x[P] + alpha * p[P];
-        const double rv = r[q] - alpha * Ap[q];
-        r[q] = rv;
-        rf[q] = (float)rv;
-        rr += rv * rv;
-    }
-    block_sum_atomic(rr, &D.rr[pb]);
 }
 
 // sum_j |A_ij x_j| of one row: the scale of the rounding error of b - A x
@@ -215,38 +181,6 @@ __global__ void k_residual64(Ops64 A, LevelDims d, const double* x, const double
     block_sum_atomic(rr, &D.rr[pb]);
     block_sum_atomic(ab, &D.ab[pb]);
     if (want_bb) block_sum_atomic(bb, &D.bb[pb]);
-}
-
-// z (FP64, interior) from the preconditioner (FP32 padded z or the residual);
-// zAp += z.Ap
-__global__ void k_take_z(LevelDims d, const float* zf, const double* r, int use_r, double* z, const double* Ap, Dots D,
-                         int want_zAp) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    double za = 0;
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const size_t q = (size_t)b * d.nint + c;
-        const double zv = use_r ? r[q] : (double)zf[pidx(d, b, i, j, k)];
-        z[q] = zv;
-        if (want_zAp) za += zv * Ap[q];
-    }
-    if (want_zAp) block_sum_atomic(za, &D.zAp[D.bprob[b]]);
-}
-
-// p = z + beta p, beta = -z.Ap / p.Ap (flexible CG, one-term A-orthogonalisation);
-// restart (beta = 0) when `restart`
-__global__ void k_update_p(LevelDims d, double* p, const double* z, Dots D, int restart) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        const int pb = D.bprob[b];
-        if (!D.active[pb]) continue;
-        const double beta = (restart || D.pAp[pb] == 0.0) ? 0.0 : -D.zAp[pb] / D.pAp[pb];
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const size_t P = pidx(d, b, i, j, k);
-        p[P] = z[(size_t)b * d.nint + c] + beta * p[P];
-    }
 }
 
 // ---- float-float inner iteration -------------------------------------------------
@@ -292,142 +226,189 @@ __device__ __forceinline__ float2 ff_from(double v) {   // a few FP64 operations
 }
 __device__ __forceinline__ double ff_to(float2 a) { return (double)a.x + (double)a.y; }
 
-// per-problem FF sums -> one FP64 atomic per CTA (FP64 work once per warp)
+__device__ __forceinline__ float2 ff_shfl_xor(float2 v, int o) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+// per-problem FF sums -> one FP64 atomic per CTA and sum. FP64 instructions are
+// the scarce ones (16 cycles each per SM), so the sums stay FF across the warps and only the
+// CTA's totals are converted, one lane each.
 __device__ __forceinline__ void block_sum_atomic_ff(float2 v, double* slot) {
-    for (int o = 16; o > 0; o >>= 1)
-        v = ff_add(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
-    __shared__ double ws[32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = ff_to(v);
+    for (int o = 16; o > 0; o >>= 1) v = ff_add(v, ff_shfl_xor(v, o));
+    __shared__ float2 ws[32];
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
-        atomicAdd(slot, t);
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = ff_add(v, ws[w]);
+        atomicAdd(slot, ff_to(v));
     }
+}
+// four sums at once: each exchange of the first two folds two sums into one
+// (the lanes of either half keep their own), 6 FF additions instead of 20
+__device__ __forceinline__ void block_sum4_atomic_ff(const float2 (&v)[4], double* const (&slot)[4]) {
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 16, top = lane & 8;
+    const float2 a = ff_add(hi ? v[1] : v[0], ff_shfl_xor(hi ? v[0] : v[1], 16));
+    const float2 b = ff_add(hi ? v[3] : v[2], ff_shfl_xor(hi ? v[2] : v[3], 16));
+    float2 s = ff_add(top ? b : a, ff_shfl_xor(top ? a : b, 8));
+    for (int o = 4; o > 0; o >>= 1) s = ff_add(s, ff_shfl_xor(s, o));
+    __shared__ float2 ws[32][4];
+    if ((lane & 7) == 0) ws[threadIdx.x >> 5][(hi ? 1 : 0) + (top ? 2 : 0)] = s;
     __syncthreads();
-}
-
-// y = A' x over the interior, the reference's operand order
-__device__ __forceinline__ float2 apply_A_ff(const Ops2& A, const LevelDims& d, const float2* x, int b, int c, int i,
-                                             int j, int k, float* absrow) {
-    const size_t P = pidx(d, b, i, j, k);
-    const size_t sj = d.p0, sk = (size_t)d.p0 * d.p1;
-    const size_t fi = ((size_t)b * d.m2 * d.m1 + (size_t)(k - 1) * d.m1 + (j - 1)) * (d.m0 + 1) + (i - 1);
-    const size_t fj = ((size_t)b * d.m2 * (d.m1 + 1) + (size_t)(k - 1) * (d.m1 + 1) + (j - 1)) * d.m0 + (i - 1);
-    const size_t fk = ((size_t)b * (d.m2 + 1) * d.m1 + (size_t)(k - 1) * d.m1 + (j - 1)) * d.m0 + (i - 1);
-    const float2 c7[7] = {A.Aii[(size_t)b * d.nint + c], A.Ai[fi], A.Ai[fi + 1], A.Aj[fj], A.Aj[fj + d.m0], A.Ak[fk],
-                          A.Ak[fk + (size_t)d.m0 * d.m1]};
-    const float2 x7[7] = {x[P], x[P - 1], x[P + 1], x[P - sj], x[P + sj], x[P - sk], x[P + sk]};
-    float2 y = ff_mul(c7[0], x7[0]);
-    float ar = fabsf(c7[0].x * x7[0].x);
-#pragma unroll
-    for (int t = 1; t < 7; ++t) {
-        y = ff_add(y, ff_mul(c7[t], x7[t]));
-        ar += fabsf(c7[t].x * x7[t].x);
-    }
-    if (absrow) *absrow = ar;
-    return y;
-}
-
-// Ap = A' p; pAp += p.Ap; pr += p.r
-__global__ void k_spmv_dots_ff(Ops2 A, LevelDims d, const float2* p, float2* Ap, const float2* r, Dots D) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    float2 pa = make_float2(0.f, 0.f), pr = make_float2(0.f, 0.f);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const float2 y = apply_A_ff(A, d, p, b, c, i, j, k, nullptr);
-        const size_t q = (size_t)b * d.nint + c;
-        Ap[q] = y;
-        const float2 pv = p[pidx(d, b, i, j, k)];
-        pa = ff_add(pa, ff_mul(pv, y));
-        pr = ff_add(pr, ff_mul(pv, r[q]));
-    }
-    const int pb = D.bprob[b];
-    block_sum_atomic_ff(pa, &D.pAp[pb]);
-    block_sum_atomic_ff(pr, &D.pr[pb]);
-}
-
-// alpha = p.r / p.Ap; x += alpha p; r -= alpha Ap; rr += r.r; rf = hi(r) (the V-cycle's input)
-__global__ void k_update_xr_ff(LevelDims d, float2* x, const float2* p, float2* r, const float2* Ap, float* rf, Dots D) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    const int pb = D.bprob[b];
-    const double alpha = (D.active[pb] && D.pAp[pb] != 0.0) ? D.pr[pb] / D.pAp[pb] : 0.0;
-    const float2 al = ff_from(alpha), nal = ff_neg(al);
-    float2 rr = make_float2(0.f, 0.f);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const size_t P = pidx(d, b, i, j, k), q = (size_t)b * d.nint + c;
-        x[P] = ff_add(x[P], ff_mul(al, p[P]));
-        const float2 rv = ff_add(r[q], ff_mul(nal, Ap[q]));
-        r[q] = rv;
-        rf[q] = rv.x;
-        rr = ff_add(rr, ff_mul(rv, rv));
-    }
-    block_sum_atomic_ff(rr, &D.rr[pb]);
-}
-
-// z = the preconditioner's FP32 output scaled by sA (it inverts the unscaled
-// FP32 operator), or r; zAp += z.Ap
-__global__ void k_take_z_ff(LevelDims d, const float* zf, const float* sA, const float2* r, int use_r, float2* z,
-                            const float2* Ap, Dots D, int want_zAp) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    const float s = sA[D.bprob[b]];
-    float2 za = make_float2(0.f, 0.f);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const size_t q = (size_t)b * d.nint + c;
-        const float2 zv = use_r ? r[q] : make_float2(zf[pidx(d, b, i, j, k)] * s, 0.f);
-        z[q] = zv;
-        if (want_zAp) za = ff_add(za, ff_mul(zv, Ap[q]));
-    }
-    if (want_zAp) block_sum_atomic_ff(za, &D.zAp[D.bprob[b]]);
-}
-
-// p = z + beta p, beta = -z.Ap / p.Ap; restart (beta = 0) when `restart`
-__global__ void k_update_p_ff(LevelDims d, float2* p, const float2* z, Dots D, int restart) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    const int pb = D.bprob[b];
-    if (!D.active[pb]) return;
-    const double beta = (restart || D.pAp[pb] == 0.0) ? 0.0 : -D.zAp[pb] / D.pAp[pb];
-    const float2 be = ff_from(beta);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const size_t P = pidx(d, b, i, j, k);
-        p[P] = ff_add(z[(size_t)b * d.nint + c], ff_mul(be, p[P]));
+    if (threadIdx.x < 4) {
+        s = ws[0][threadIdx.x];
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) s = ff_add(s, ws[w][threadIdx.x]);
+        double* p = threadIdx.x == 0 ? slot[0] : threadIdx.x == 1 ? slot[1] : threadIdx.x == 2 ? slot[2] : slot[3];
+        atomicAdd(p, ff_to(s));
     }
 }
 
-// halo of an FF vector: the trilinear sum with the 8 corner weights
-// precomputed in FP64 on the host and stored as FF pairs
-struct HaloListFF {
-    int64_t n;
-    const int32_t* dst;
-    const int32_t* src;
-    const uint8_t* code;   // as HaloList
-    const float2* w8;      // [n][8] corner weights
-    int32_t sj, sk;
+// Sums of products of FF numbers in compensated form (Ogita, Rump and Oishi's
+// Dot2 with the low parts added to the error): s the running sum, e the rounding
+// errors of the sums and products, about 2^-46 of the summed magnitudes in a
+// third of the instructions of an FF addition per term.
+struct FFSum {
+    float s = 0.f, e = 0.f;
+    __device__ __forceinline__ void add(float2 a, float2 b) {
+        const float p = a.x * b.x;
+        const float t = s + p, bb = t - s;
+        e += ((s - (t - bb)) + (p - bb)) + fmaf(a.y, b.x, fmaf(a.x, b.y, fmaf(a.x, b.x, -p)));
+        s = t;
+    }
+    __device__ __forceinline__ float2 value() const { return ff_quick(s, e); }
 };
-__global__ void k_halo_ff(float2* v, HaloListFF H, const int32_t* cdst, const int32_t* csrc, int64_t nc) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < nc) {
-        v[cdst[e]] = v[csrc[e]];
+
+// Ghosts of z (FP32, scaled by the problem's sA) at the finest level as FF
+// values, one slot per ghost in the layout of VLevel::ghost. A copied cell's map
+// weights are 0 or 1 up to eps (about 1e-14, see kSnapFF): the ghost is z0 + sum of eps_d
+// (z_d - z0) over the three directions, z_d one cell on (eps > 0) or back (eps
+// < 0); second-order terms are below 2^-64. Other ghosts sum eight cells with
+// FF weights.
+struct GhostFF {
+    const int32_t* ghost;   // [slot] >= 0 source cell, -1 none, <= -2 entry -(v + 2)
+    const float* eps;       // [slot][3]
+    const int32_t* src;     // entry: base source cell
+    const uint8_t* code;    // bit d set: the weight of direction d is not 0
+    const float2* w8;       // [entry][8] corner weights
+    int m;
+    int64_t n;              // slots
+};
+__global__ void k_ghost_ff(GhostFF H, const float* z, const float* scale, const int32_t* bprob, float2* G) {
+    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= H.n) return;
+    const int d = H.ghost[x];
+    if (d == -1) return;   // stays 0
+    const int m = H.m, mm = m * m;
+    const float s = scale ? scale[bprob[x / (6 * mm)]] : 1.f;
+    if (d >= 0) {
+        const float z0 = z[d] * s;
+        float lo = 0.f;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const float ep = H.eps[3 * x + q];
+            const int st = q == 0 ? 1 : q == 1 ? m : mm;
+            if (ep != 0.f) lo = fmaf(fabsf(ep), z[ep > 0.f ? d + st : d - st] * s - z0, lo);
+        }
+        G[x] = ff_two_sum(z0, lo);
         return;
     }
-    e -= nc;
-    if (e >= H.n) return;
-    const int cd = H.code[e];
-    const int a = (cd & 1) ? 1 : 0, bq = (cd & 2) ? H.sj : 0, c = (cd & 4) ? H.sk : 0;
-    const int off[8] = {0, a, bq, c, a + bq, bq + c, a + c, a + bq + c};
-    const float2* f = v + H.src[e];
-    const float2* w = H.w8 + 8 * e;
-    float2 s = ff_mul(w[0], f[0]);
+    const int e = -(d + 2), cd = H.code[e];
+    const int a = (cd & 1) ? 1 : 0, b = (cd & 2) ? m : 0, c = (cd & 4) ? mm : 0;
+    const int off[8] = {0, a, b, c, a + b, b + c, a + c, a + b + c};
+    const float* f = z + H.src[e];
+    const float4* w = reinterpret_cast<const float4*>(H.w8 + 8 * (size_t)e);
+    FFSum y;
 #pragma unroll
-    for (int t = 1; t < 8; ++t) s = ff_add(s, ff_mul(w[t], f[off[t]]));
-    v[H.dst[e]] = s;
+    for (int t = 0; t < 4; ++t) {
+        const float4 w2 = w[t];
+        y.add(make_float2(w2.x, w2.y), make_float2(f[off[2 * t]] * s, 0.f));
+        y.add(make_float2(w2.z, w2.w), make_float2(f[off[2 * t + 1]] * s, 0.f));
+    }
+    G[x] = y.value();
+}
+
+// w = A' z, the reference's operand order, with the four products that the
+// step needs: z.w, z.Ap, p.w, z.r. z is the preconditioner's FP32 output (or
+// the residual's FP32 part): the direction is p' = z + beta p and A' p' = w +
+// beta A' p, so that beta, alpha and the update follow from one pass over the operator
+// and no halo of p is kept.
+template <int M>   // m, or 0
+__global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, const float* z, const float* scale, const float2* G,
+                                                   const float2* p, const float2* r, const float2* Ap, float2* w, Dots D) {
+    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d), pb = D.bprob[b];
+    if (!D.active[pb]) return;
+    const int m = M > 0 ? M : d.m0, mm = m * m;
+    const float s = scale ? scale[pb] : 1.f;
+    const float* zb = z + (size_t)b * d.nint;
+    const float2* Gb = G + (size_t)b * 6 * mm;
+    FFSum zw, za, pw, zr;
+    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
+        const int i = c % m, row = c / m, j = row % m, k = row / m;
+        const size_t fi = ((size_t)b * mm + row) * (m + 1) + i;
+        const size_t fj = ((size_t)b * m * (m + 1) + (size_t)k * (m + 1) + j) * m + i;
+        const size_t fk = ((size_t)b * (m + 1) * m + row) * m + i, q = (size_t)b * d.nint + c;
+        auto inside = [&](int y) { return make_float2(zb[y] * s, 0.f); };
+        const float2 zc = inside(c);
+        FFSum y;
+        y.add(A.Aii[q], zc);
+        y.add(A.Ai[fi], i > 0 ? inside(c - 1) : Gb[row]);
+        y.add(A.Ai[fi + 1], i < m - 1 ? inside(c + 1) : Gb[mm + row]);
+        y.add(A.Aj[fj], j > 0 ? inside(c - m) : Gb[2 * mm + k * m + i]);
+        y.add(A.Aj[fj + m], j < m - 1 ? inside(c + m) : Gb[3 * mm + k * m + i]);
+        y.add(A.Ak[fk], k > 0 ? inside(c - mm) : Gb[4 * mm + j * m + i]);
+        y.add(A.Ak[fk + mm], k < m - 1 ? inside(c + mm) : Gb[5 * mm + j * m + i]);
+        const float2 wv = y.value();
+        w[q] = wv;
+        zw.add(zc, wv);
+        za.add(zc, Ap[q]);
+        pw.add(p[q], wv);
+        zr.add(zc, r[q]);
+    }
+    block_sum4_atomic_ff({zw.value(), za.value(), pw.value(), zr.value()}, {&D.zw[pb], &D.zAp[pb], &D.pw[pb], &D.zr[pb]});
+}
+
+// The step's scalars of a problem from k_spmv_z_ff's products: beta = -z.Ap / p.Ap
+// (flexible CG, one-term A-orthogonalisation; 0 to restart), p'.Ap' and alpha =
+// p'.r / p'.Ap' (p.r = 0 after the step that made r). A direction that vanished
+// takes no step.
+struct StepFF { double alpha, beta, pAp; };
+__device__ __forceinline__ StepFF step_ff(const Dots& D, int pb, int restart) {
+    const double pAp = D.pAp[pb], zAp = D.zAp[pb];
+    StepFF s;
+    s.beta = restart || pAp == 0.0 ? 0.0 : -zAp / pAp;
+    s.pAp = D.zw[pb] + s.beta * (zAp + D.pw[pb] + s.beta * pAp);
+    s.alpha = s.pAp != 0.0 ? D.zr[pb] / s.pAp : 0.0;
+    return s;
+}
+
+// p = z + beta p; Ap = w + beta Ap; x += alpha p; r -= alpha Ap; rr += r.r; rf =
+// hi(r), the V-cycle's input
+__global__ void __launch_bounds__(512) k_step_ff(LevelDims d, const float* z, const float* scale, const float2* w, float2* x,
+                                                 float2* p, float2* r, float2* Ap, float* rf, Dots D, int restart) {
+    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d), pb = D.bprob[b];
+    if (!D.active[pb]) return;
+    __shared__ float2 ab[2];   // the scalars' FP64 work once per CTA
+    if (threadIdx.x == 0) {
+        const StepFF s = step_ff(D, pb, restart);
+        ab[0] = ff_from(s.alpha);
+        ab[1] = ff_from(s.beta);
+    }
+    __syncthreads();
+    const float2 al = ab[0], be = ab[1], nal = ff_neg(al);
+    const float s = scale ? scale[pb] : 1.f;
+    FFSum rr;
+    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
+        const size_t q = (size_t)b * d.nint + c;
+        const float2 pv = ff_add(make_float2(z[q] * s, 0.f), ff_mul(be, p[q]));
+        const float2 av = ff_add(w[q], ff_mul(be, Ap[q]));
+        const float2 rv = ff_add(r[q], ff_mul(nal, av));
+        p[q] = pv;
+        Ap[q] = av;
+        x[q] = ff_add(x[q], ff_mul(al, pv));
+        r[q] = rv;
+        rf[q] = rv.x;
+        rr.add(rv, rv);
+    }
+    block_sum_atomic_ff(rr.value(), &D.rr[pb]);
 }
 
 // ---- the inner solve's loop control on the device -----------------------------
@@ -450,7 +431,7 @@ constexpr int32_t kInnerCap = 100000;
 // h = sqrt(r.r / r0.r0); a problem at or below its eta leaves the iteration
 // (active = 0: no further update). One CTA of 256 threads, problem per thread
 // (nproblems <= 256). With `set_cond`, sets the WHILE node's condition.
-__global__ void __launch_bounds__(256) k_inner_check(int np, const double* rr, const double* rr0, const double* eta,
+__global__ void __launch_bounds__(256) k_inner_check(int np, Dots D, int restart, const double* rr0, const double* eta,
                                                      int32_t* active, InnerCtl* ctl, cudaGraphConditionalHandle h,
                                                      int set_cond) {
     __shared__ double smax[256];
@@ -459,7 +440,9 @@ __global__ void __launch_bounds__(256) k_inner_check(int np, const double* rr, c
     double hq = 0.0;
     int still = 0, bad = 0;
     if (q < np && active[q]) {
-        hq = sqrt(rr[q] / rr0[q]);
+        hq = sqrt(D.rr[q] / rr0[q]);
+        D.pAp[q] = step_ff(D, q, restart).pAp;   // of the direction just taken
+        D.zw[q] = D.zAp[q] = D.pw[q] = D.zr[q] = D.rr[q] = 0.0;   // for the next iteration's sums
         if (!(hq == hq) || hq > 1e300) {
             bad = 1;
         } else if (hq <= eta[q]) {
@@ -526,98 +509,7 @@ __global__ void k_ir_accum(LevelDims d, const float2* x2, const double* fac, con
         int i, j, k;
         cell_ijk(d, c, i, j, k);
         const size_t P = pidx(d, b, i, j, k);
-        x[P] = x[P] + ff_to(x2[P]) * f;
-    }
-}
-
-// ---- FP32 V-cycle ------------------------------------------------------------
-__global__ void k_zero_f(float* v, size_t n) {
-    for (size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (size_t)gridDim.x * blockDim.x) v[x] = 0.f;
-}
-
-// red-black Gauss-Seidel half sweep: z = (r - sum_nb A z_nb) / Aii on cells of one colour
-// (The smoother's rounding is free -- the outer CG is flexible -- so it uses
-// explicit FMAs and a fast division; this file is otherwise compiled without
-// contraction.) With an even row length that divides the chunk a thread takes
-// only cells of the colour: m0/2 cells of each colour per row.
-__device__ __forceinline__ void rbgs_cell(const Ops32& A, const LevelDims& d, const float* r, float* z, int b, int c,
-                                          int i, int j, int k) {
-    const size_t P = pidx(d, b, i, j, k);
-    const size_t sj = d.p0, sk = (size_t)d.p0 * d.p1;
-    const size_t fi = ((size_t)b * d.m2 * d.m1 + (size_t)(k - 1) * d.m1 + (j - 1)) * (d.m0 + 1) + (i - 1);
-    const size_t fj = ((size_t)b * d.m2 * (d.m1 + 1) + (size_t)(k - 1) * (d.m1 + 1) + (j - 1)) * d.m0 + (i - 1);
-    const size_t fk = ((size_t)b * (d.m2 + 1) * d.m1 + (size_t)(k - 1) * d.m1 + (j - 1)) * d.m0 + (i - 1);
-    float off = A.Ai[fi] * z[P - 1];
-    off = fmaf(A.Ai[fi + 1], z[P + 1], off);
-    off = fmaf(A.Aj[fj], z[P - sj], off);
-    off = fmaf(A.Aj[fj + d.m0], z[P + sj], off);
-    off = fmaf(A.Ak[fk], z[P - sk], off);
-    off = fmaf(A.Ak[fk + (size_t)d.m0 * d.m1], z[P + sk], off);
-    z[P] = __fdividef(r[(size_t)b * d.nint + c] - off, A.Aii[(size_t)b * d.nint + c]);
-}
-
-__global__ void k_rbgs(Ops32 A, LevelDims d, const float* r, float* z, int colour) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    if ((d.m0 & 1) == 0 && d.chunk % d.m0 == 0) {   // rows whole within a chunk
-        const int half = d.m0 >> 1;
-        for (int h = (c0 >> 1) + threadIdx.x; h < (c1 >> 1); h += blockDim.x) {
-            const int row = h / half, ih = h - row * half;
-            const int j = row % d.m1 + 1, k = row / d.m1 + 1;
-            const int i = (((colour - j - k) & 1) ? 1 : 2) + 2 * ih;
-            rbgs_cell(A, d, r, z, b, row * d.m0 + (i - 1), i, j, k);
-        }
-        return;
-    }
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        if (((i + j + k) & 1) != colour) continue;
-        const size_t P = pidx(d, b, i, j, k);
-        const size_t sj = d.p0, sk = (size_t)d.p0 * d.p1;
-        const size_t fi = ((size_t)b * d.m2 * d.m1 + (size_t)(k - 1) * d.m1 + (j - 1)) * (d.m0 + 1) + (i - 1);
-        const size_t fj = ((size_t)b * d.m2 * (d.m1 + 1) + (size_t)(k - 1) * (d.m1 + 1) + (j - 1)) * d.m0 + (i - 1);
-        const size_t fk = ((size_t)b * (d.m2 + 1) * d.m1 + (size_t)(k - 1) * d.m1 + (j - 1)) * d.m0 + (i - 1);
-        const float off = A.Ai[fi] * z[P - 1] + A.Ai[fi + 1] * z[P + 1] + A.Aj[fj] * z[P - sj] + A.Aj[fj + d.m0] * z[P + sj] +
-                          A.Ak[fk] * z[P - sk] + A.Ak[fk + (size_t)d.m0 * d.m1] * z[P + sk];
-        z[P] = (r[(size_t)b * d.nint + c] - off) / A.Aii[(size_t)b * d.nint + c];
-    }
-}
-
-// res = r - A z
-__global__ void k_resid32(Ops32 A, LevelDims d, const float* r, const float* z, float* res) {
-    const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        const size_t q = (size_t)b * d.nint + c;
-        res[q] = r[q] - apply_A<float>(A, d, z, b, c, i, j, k);
-    }
-}
-
-// r_coarse(I) = sum of the 8 children of res_fine (R = P^T)
-__global__ void k_restrict(LevelDims f, LevelDims cd, const float* res, float* rc) {
-    const int b = cell_block(cd), c0 = cell_first(cd), c1 = cell_end(cd);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        const int I = c % cd.m0, J = (c / cd.m0) % cd.m1, K = c / (cd.m0 * cd.m1);
-        const float* R = res + (size_t)b * f.nint;
-        float s = 0.f;
-    #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int i = 2 * I + (q & 1), j = 2 * J + ((q >> 1) & 1), k = 2 * K + (q >> 2);
-            s += R[((size_t)k * f.m1 + j) * f.m0 + i];
-        }
-        rc[(size_t)b * cd.nint + c] = s;
-    }
-}
-
-// z_fine(child) += z_coarse(I) (injection)
-__global__ void k_prolong_add(LevelDims f, LevelDims cd, const float* zc, float* zf) {
-    const int b = cell_block(f), c0 = cell_first(f), c1 = cell_end(f);
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(f, c, i, j, k);
-        const int I = (i - 1) / 2 + 1, J = (j - 1) / 2 + 1, K = (k - 1) / 2 + 1;
-        zf[pidx(f, b, i, j, k)] += zc[pidx(cd, b, I, J, K)];
+        x[P] = x[P] + ff_to(x2[(size_t)b * d.nint + c]) * f;
     }
 }
 
@@ -669,13 +561,12 @@ __global__ void k_lcc_feat(LevelDims d, const float* r, const float* Aii, const 
     }
 }
 
-// coarse correction z = s * y (padded coarse layout)
+// coarse correction z = s * y
 __global__ void k_lcc_scatter(LevelDims d, const float* y, const int32_t* gmap, const double* sum, int64_t n, float* z) {
     const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d);
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        int i, j, k;
-        cell_ijk(d, c, i, j, k);
-        z[pidx(d, b, i, j, k)] = (float)(lcc_scale(sum, n) * (double)y[gmap[(size_t)b * d.nint + c]]);
+        const size_t q = (size_t)b * d.nint + c;
+        z[q] = (float)(lcc_scale(sum, n) * (double)y[gmap[q]]);
     }
 }
 
@@ -762,24 +653,27 @@ struct SvLevel {
     LevelDims d{};
     double *Aii = nullptr, *Ai = nullptr, *Aj = nullptr, *Ak = nullptr;
     float *fAii = nullptr, *fAi = nullptr, *fAj = nullptr, *fAk = nullptr;
+    // FP64 halo lists: interpolated entries and plain copies (padded offsets)
     int32_t *hdst = nullptr, *hsrc = nullptr;
     uint8_t* hcode = nullptr;
-    float* hwf = nullptr;
     double* hw = nullptr;
     int64_t nh = 0;
-    int32_t *hcdst = nullptr, *hcsrc = nullptr;   // halo entries that are plain copies
+    int32_t *hcdst = nullptr, *hcsrc = nullptr;
     int64_t nhc = 0;
-    // the copies in three runs: ghost and source both of parity 0 (nhc0), of
-    // differing parities (nhcm), both of parity 1 (the rest); parity of i+j+k
-    int64_t nhc0 = 0, nhcm = 0;
-    float *z = nullptr, *r = nullptr, *res = nullptr;
-    // level 0: the scaled operator A / sA and the halo's corner weights as FF pairs
-    float2 *Aii2 = nullptr, *Ai2 = nullptr, *Aj2 = nullptr, *Ak2 = nullptr, *hw8 = nullptr;
-    HaloList halo() const { return HaloList{nh, hdst, hsrc, hcode, hw, hwf, d.p0, d.p0 * d.p1}; }
-    HaloListFF halo_ff() const { return HaloListFF{nh, hdst, hsrc, hcode, hw8, d.p0, d.p0 * d.p1}; }
+    // FP32 V-cycle: ghost descriptors and interpolation entries (VLevel)
+    int32_t *ghost = nullptr, *isrc = nullptr, *nbr = nullptr;
+    uint8_t* icode = nullptr;
+    float* iw = nullptr;
+    // z: where a V-cycle leaves its result; z and zb take turns inside it
+    float *z = nullptr, *zb = nullptr, *r = nullptr, *res = nullptr;
+    // level 0: the scaled operator A / sA as FF pairs
+    float2 *Aii2 = nullptr, *Ai2 = nullptr, *Aj2 = nullptr, *Ak2 = nullptr;
+    HaloList halo() const { return HaloList{nh, hdst, hsrc, hcode, hw, d.p0, d.p0 * d.p1}; }
     Ops2 ops2() const { return Ops2{Aii2, Ai2, Aj2, Ak2}; }
     Ops64 ops64() const { return Ops64{Aii, Ai, Aj, Ak}; }
-    Ops32 ops32() const { return Ops32{fAii, fAi, fAj, fAk}; }
+    VLevel view(int nb) const {
+        return VLevel{d.m0, d.nint, nb, fAii, fAi, fAj, fAk, ghost, isrc, icode, iw, nbr};
+    }
 };
 
 struct falcon_solver {
@@ -789,11 +683,12 @@ struct falcon_solver {
     cudaStream_t st = nullptr;
     std::vector<SvLevel> lv;
     double *x = nullptr, *p = nullptr, *r = nullptr, *Ap = nullptr, *z = nullptr, *bvec = nullptr;
-    // the float-float inner solve (scaled system, see Ops2): padded x2, p2; interior r2, Ap2, z2
-    float2 *x2 = nullptr, *p2 = nullptr, *r2 = nullptr, *Ap2 = nullptr, *z2 = nullptr;
+    // the float-float inner solve (scaled system, see Ops2), interior: w2 = A' z; ghosts of z
+    float2 *x2 = nullptr, *p2 = nullptr, *r2 = nullptr, *Ap2 = nullptr, *w2 = nullptr, *ghosts2 = nullptr;
+    GhostFF gff{};
     std::vector<double> sA;               // per-problem powers of two (the operator's scale)
     float* dsA = nullptr;                 // sA on the device (FP32: powers of two are exact)
-    double* dots = nullptr;       // [6][nproblems]: pAp, pr, zAp, rr, bb, ab
+    double* dots = nullptr;       // [8][nproblems]: see Dots
     double* ir_par = nullptr;     // [2][nproblems]: 1/sr and sr/sA of the refinement pass
     int32_t *active = nullptr, *bprob = nullptr;
     std::vector<void*> allocs;
@@ -822,6 +717,15 @@ struct falcon_solver {
     bool capturing = false;               // enqueueing into a graph: the V-cycle's kernels inline
     InnerCtl* ictl = nullptr;             // device loop control
     double *rr0 = nullptr, *eta = nullptr;   // device, per problem
+    // the coarsest level's sweeps in one launch (k_coarse_sweeps): CTAs per
+    // problem (0: one launch per half sweep) and cells per thread and colour
+    int coarse_cluster = 0, coarse_r = 1;
+    int32_t* first = nullptr;             // [np + 1] first block of each problem
+    uint32_t* cghost = nullptr;           // its ghost table and gathered ghosts (CoarseArgs)
+    uint2* ceat = nullptr;
+    float4* cew = nullptr;
+    int4* clist = nullptr;
+    int coarse_slots = 0;
     // tile shape of the cell kernels (cells per CTA, threads per CTA), tuned at the first solve
     int tile_chunk = 1024, tile_tpb = 256;
     bool tuned = false;
@@ -847,7 +751,8 @@ struct falcon_solver {
     }
     Dots D() const {
         const int n = S.nproblems;
-        return Dots{dots, dots + n, dots + 2 * n, dots + 3 * n, dots + 4 * n, dots + 5 * n, active, bprob};
+        return Dots{dots, dots + n, dots + 2 * n, dots + 3 * n, dots + 4 * n, dots + 5 * n, dots + 6 * n, dots + 7 * n,
+                    active, bprob};
     }
 };
 
@@ -867,33 +772,10 @@ dim3 grid_cells(const LevelDims& d, int nblocks) {
 }
 unsigned tpb(const LevelDims& d) { return (unsigned)std::min(d.tpb, (std::min(d.nint, d.chunk) + 31) / 32 * 32); }
 
-template <class T> cudaError_t halo_fill(falcon_solver* sv, int l, T* v) {
+cudaError_t halo_fill(falcon_solver* sv, int l, double* v) {
     const SvLevel& L = sv->lv[l];
     const int64_t n = L.nhc + L.nh;
-    if (n > 0) k_halo<T><<<(unsigned)((n + 255) / 256), 256, 0, sv->st>>>(v, L.halo(), L.hcdst, L.hcsrc, L.nhc);
-    return cudaGetLastError();
-}
-
-// Before a red-black half sweep of `colour`: only the ghosts of the other
-// parity are read. Copies whose ghost and source share a parity go stale only
-// when that parity's cells change, so the fill refreshes the copies of the
-// other parity, the copies whose parities differ and every interpolated
-// entry; the copies of `colour`'s parity were refreshed after that colour's
-// last sweep (the sweeps alternate).
-template <class T> cudaError_t halo_fill_part(falcon_solver* sv, int l, T* v, int colour) {
-    const SvLevel& L = sv->lv[l];
-    const int p = 1 - colour;
-    const int64_t off = p == 0 ? 0 : L.nhc0;
-    const int64_t nc = p == 0 ? L.nhc0 + L.nhcm : L.nhc - L.nhc0;
-    const int64_t n = nc + L.nh;
-    if (n > 0) k_halo<T><<<(unsigned)((n + 255) / 256), 256, 0, sv->st>>>(v, L.halo(), L.hcdst + off, L.hcsrc + off, nc);
-    return cudaGetLastError();
-}
-
-cudaError_t halo_fill_ff(falcon_solver* sv, float2* v) {
-    const SvLevel& L = sv->lv[0];
-    const int64_t n = L.nhc + L.nh;
-    if (n > 0) k_halo_ff<<<(unsigned)((n + 255) / 256), 256, 0, sv->st>>>(v, L.halo_ff(), L.hcdst, L.hcsrc, L.nhc);
+    if (n > 0) k_halo<double><<<(unsigned)((n + 255) / 256), 256, 0, sv->st>>>(v, L.halo(), L.hcdst, L.hcsrc, L.nhc);
     return cudaGetLastError();
 }
 
@@ -922,38 +804,278 @@ std::vector<float2> to_ff(const std::vector<double>& v, const std::vector<double
     return o;
 }
 
-// z_0 = M r_0: one V-cycle on the FP32 residual stored in lv[0].r
+// ---- launches of the V-cycle kernels ---------------------------------------------
+unsigned vgrid(int64_t threads) { return (unsigned)((threads + kVThreads - 1) / kVThreads); }
+template <int M, int MODE>
+void vsweep_pairs(falcon_solver* sv, int l, const float* zin, const float* zc, float* zout, int colour) {
+    const SvLevel& L = sv->lv[l];
+    const VLevel V = L.view(sv->S.nblocks);
+    k_vsweep<M, MODE><<<vgrid((int64_t)V.nb * V.nint / 2), kVThreads, 0, sv->st>>>(V, L.r, zin, zc, zout, colour);
+}
+template <int MODE>
+cudaError_t vsweep(falcon_solver* sv, int l, const float* zin, const float* zc, float* zout, int colour) {
+    const SvLevel& L = sv->lv[l];
+    switch (L.d.m0) {
+    case 2: vsweep_pairs<2, MODE>(sv, l, zin, zc, zout, colour); break;
+    case 4: vsweep_pairs<4, MODE>(sv, l, zin, zc, zout, colour); break;
+    case 8: vsweep_pairs<8, MODE>(sv, l, zin, zc, zout, colour); break;
+    case 16: vsweep_pairs<16, MODE>(sv, l, zin, zc, zout, colour); break;
+    case 32: vsweep_pairs<32, MODE>(sv, l, zin, zc, zout, colour); break;
+    default: {
+        const VLevel V = L.view(sv->S.nblocks);
+        k_vsweep_any<MODE><<<vgrid((int64_t)V.nb * V.nint), kVThreads, 0, sv->st>>>(V, L.r, zin, zc, zout,
+                                                                                                  colour);
+    }
+    }
+    return cudaGetLastError();
+}
+cudaError_t vresid(falcon_solver* sv, int l, const float* z, float* res) {
+    const SvLevel& L = sv->lv[l];
+    const VLevel V = L.view(sv->S.nblocks);
+    k_vresid<<<vgrid((int64_t)V.nb * V.nint), kVThreads, 0, sv->st>>>(V, L.r, z, res);
+    return cudaGetLastError();
+}
+// rc = R (r - A z)
+template <int M> void vresid_restrict_pairs(falcon_solver* sv, int l, const float* z, float* rc) {
+    const SvLevel& L = sv->lv[l];
+    const VLevel V = L.view(sv->S.nblocks);
+    k_vresid_restrict<M><<<vgrid((int64_t)V.nb * V.nint / 2), kVThreads, 0, sv->st>>>(V, L.r, z, rc);
+}
+cudaError_t vresid_restrict(falcon_solver* sv, int l, const float* z, float* rc) {
+    const SvLevel& L = sv->lv[l];
+    switch (L.d.m0) {
+    case 2: vresid_restrict_pairs<2>(sv, l, z, rc); break;
+    case 4: vresid_restrict_pairs<4>(sv, l, z, rc); break;
+    case 8: vresid_restrict_pairs<8>(sv, l, z, rc); break;
+    case 16: vresid_restrict_pairs<16>(sv, l, z, rc); break;
+    default: {
+        const cudaError_t e = vresid(sv, l, z, L.res);
+        if (e != cudaSuccess) return e;
+        const int64_t nc = (int64_t)sv->S.nblocks * L.d.nint / 8;
+        k_vrestrict<<<vgrid(nc), kVThreads, 0, sv->st>>>(L.d.m0, (int)nc, L.res, rc);
+    }
+    }
+    return cudaGetLastError();
+}
+
+constexpr size_t coarse_smem(int R, int slots) { return ((size_t)2 * R * kCoarseThreads + 1 + slots) * 4; }
+typedef void (*CoarseKernel)(VLevel, CoarseArgs, const float*, float*);
+template <int M> CoarseKernel coarse_kernel_m(int R, bool cluster) {
+    if (cluster) return R == 1 ? k_coarse_sweeps<M, 1, true> : R == 2 ? k_coarse_sweeps<M, 2, true> : k_coarse_sweeps<M, 4, true>;
+    return R == 1 ? k_coarse_sweeps<M, 1, false> : R == 2 ? k_coarse_sweeps<M, 2, false> : k_coarse_sweeps<M, 4, false>;
+}
+CoarseKernel coarse_kernel(int m, int R, bool cluster) {
+    return m == 2 ? coarse_kernel_m<2>(R, cluster) : m == 4 ? coarse_kernel_m<4>(R, cluster) : nullptr;
+}
+void coarse_config(const falcon_solver* sv, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim = dim3((unsigned)(sv->S.nproblems * sv->coarse_cluster));
+    cfg->blockDim = dim3(kCoarseThreads);
+    cfg->dynamicSmemBytes = coarse_smem(sv->coarse_r, sv->coarse_slots);
+    cfg->stream = sv->st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = (unsigned)sv->coarse_cluster;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg->attrs = at;
+    cfg->numAttrs = sv->coarse_cluster > 1 ? 1 : 0;
+}
+cudaError_t coarse_sweeps(falcon_solver* sv, int sweeps, float* zout) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    coarse_config(sv, &cfg, at);
+    const SvLevel& L = sv->lv.back();
+    return cudaLaunchKernelEx(&cfg, coarse_kernel(L.d.m0, sv->coarse_r, sv->coarse_cluster > 1), L.view(sv->S.nblocks),
+                              CoarseArgs{sv->first, sv->cghost, sv->ceat, sv->cew, sv->clist, sweeps, sv->coarse_cluster,
+                                         sv->coarse_slots},
+                              (const float*)L.r, zout);
+}
+// Whether the coarsest level's sweeps run as one launch, and with how many CTAs
+// per problem: the smallest cluster that holds the largest problem at two
+// cells per thread and colour, one cell where that fits too. Batches whose
+// clusters would take more than three waves of SMs keep a launch per half
+// sweep, which advances all problems at once. Builds the neighbour words.
+int plan_coarse(falcon_solver* sv, const std::vector<int32_t>& ghost, const std::vector<int32_t>& isrc,
+                const std::vector<uint8_t>& icode, const std::vector<float>& iw) {
+    const SolverProblemSet& S = sv->S;
+    sv->coarse_cluster = 0;
+    const SvLevel& L = sv->lv.back();
+    const int m = L.d.m0, nint = L.d.nint, mm = m * m;
+    if (S.nlevels < 2 || !coarse_kernel(m, 1, false)) return FALCON_OK;
+    int most = 0;
+    for (int p = 0; p < S.nproblems; ++p) most = std::max(most, S.problem_first_block[p + 1] - S.problem_first_block[p]);
+    // the cluster with the shortest estimated half sweep, waves of clusters counted
+    int cl = 0, R = 1;
+    double best = 1e30;
+    for (int c = 1; c <= 16; c *= 2) {
+        const int64_t cells = (int64_t)((most + c - 1) / c) * nint;
+        if (cells > 8 * kCoarseThreads) continue;
+        const int r = cells <= 2 * kCoarseThreads ? 1 : cells <= 4 * kCoarseThreads ? 2 : 4;
+        sv->coarse_cluster = c;
+        const CoarseKernel kern = coarse_kernel(m, r, c > 1);
+        int n = 152;
+        if (c > 1) {
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute at[1];
+            coarse_config(sv, &cfg, at);
+            cfg.dynamicSmemBytes = coarse_smem(r, 4 * kCoarseThreads);
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+            if (e == cudaSuccess && c > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
+            if (e != cudaSuccess || n < 1) {
+                cudaGetLastError();
+                continue;
+            }
+        }
+        const double t = ((S.nproblems + n - 1) / n) * ((c == 1 ? 0.35 : 1.0) + 0.25 * r);
+        if (t < best) {
+            best = t;
+            cl = c;
+            R = r;
+        }
+    }
+    sv->coarse_cluster = 0;
+    if (cl == 0 || best > 4.0) return FALCON_OK;
+    // owner CTA of a block, and the word of a cell
+    auto cta = [&](int b) {
+        const int p = S.block_problem[b], pb0 = S.problem_first_block[p];
+        const int bpc = (S.problem_first_block[p + 1] - pb0 + cl - 1) / cl;
+        return p * cl + (b - pb0) / bpc;
+    };
+    auto colour = [&](int c) { return (c % m + (c / m) % m + c / mm + 1) & 1; };
+    auto word = [&](int cell) -> uint32_t {
+        const int b = cell / nint, c = cell - b * nint, p = S.block_problem[b], pb0 = S.problem_first_block[p];
+        const int bpc = (S.problem_first_block[p + 1] - pb0 + cl - 1) / cl, own = (b - pb0) / bpc;
+        return (uint32_t)own << 24 | (uint32_t)((b - pb0 - own * bpc) * nint + c);
+    };
+    // ghosts by (CTA, colour of the cell inside the face): local copies of the other
+    // colour are read in place, the rest gathered
+    std::vector<uint32_t> g(ghost.size(), kNone);
+    std::vector<uint2> eat;
+    std::vector<float4> ew;
+    std::vector<int4> list;
+    int slots = 0, b = 0;
+    for (int c = 0; c < S.nproblems * cl; ++c) {
+        int be = b;
+        while (be < S.nblocks && cta(be) == c) ++be;
+        for (int col = 0; col < 2; ++col) {
+            const int start = (int)eat.size();
+            std::vector<size_t> place[2];   // ghosts of one entry and of two
+            std::vector<CoarseEntry> one[2], two;
+            for (int bb = b; bb < be; ++bb)
+                for (int f = 0; f < 6; ++f)
+                    for (int t = 0; t < mm; ++t) {
+                        const int u = t % m, v = t / m, in = (f & 1) ? m - 1 : 0;
+                        const int i = f < 2 ? in : u, j = f < 2 ? u : f < 4 ? in : v, k = f < 4 ? v : in;
+                        if (((i + j + k + 1) & 1) != col) continue;
+                        const size_t q = ((size_t)bb * 6 + f) * mm + t;
+                        const int32_t d = ghost[q];
+                        if (d == -1) continue;
+                        if (d >= 0 && cta(d / nint) == c && colour(d % nint) != col) {
+                            g[q] = word(d) & 0xffffu;
+                            continue;
+                        }
+                        CoarseEntry E{make_uint2(0, 0), make_float4(1.f, 0.f, 0.f, 0.f)};
+                        bool eight = false;
+                        if (d >= 0) {
+                            E.at.x = word(d);
+                        } else {
+                            const size_t e = (size_t)(-2 - d);
+                            const float wi = iw[3 * e], wj = iw[3 * e + 1], wk = iw[3 * e + 2], ui = 1.f - wi;
+                            const float p[4] = {(1.f - wj) * (1.f - wk), wj * (1.f - wk), (1.f - wj) * wk, wj * wk};
+                            E.at.x = word(isrc[e]);
+                            if (icode[e] == 1) {
+                                E.at.y = 1;
+                                E.w = make_float4(ui, wi, 0.f, 0.f);
+                            } else {   // offsets whose weight is 0 are never used
+                                eight = icode[e] & 1;
+                                E.at.y = (uint32_t)(m | mm << 8 | (m + mm) << 16);
+                                E.w = make_float4(ui * p[0], ui * p[1], ui * p[2], ui * p[3]);
+                                CoarseEntry H = E;
+                                H.at.x += 1;
+                                H.w = make_float4(wi * p[0], wi * p[1], wi * p[2], wi * p[3]);
+                                if (eight) two.push_back(H);
+                            }
+                        }
+                        place[eight].push_back(q);
+                        one[eight].push_back(E);
+                    }
+            int n = 0;
+            for (int e = 0; e < 2; ++e)
+                for (size_t x = 0; x < place[e].size(); ++x) {
+                    g[place[e][x]] = kSlot | (uint32_t)n++;
+                    eat.push_back(one[e][x].at);
+                    ew.push_back(one[e][x].w);
+                }
+            for (const CoarseEntry& H : two) {
+                eat.push_back(H.at);
+                ew.push_back(H.w);
+            }
+            slots = std::max(slots, n);
+            list.push_back(make_int4(start, n, (int)two.size(), 0));
+        }
+        b = be;
+    }
+    sv->coarse_cluster = cl;
+    sv->coarse_r = R;
+    sv->coarse_slots = slots;
+    const CoarseKernel kern = coarse_kernel(m, R, cl > 1);
+    cudaError_t e = coarse_smem(R, slots) > 232448 || 2 * R * kCoarseThreads + 1 + slots > 65536 ? cudaErrorInvalidValue
+                                                   : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                                          (int)coarse_smem(R, slots));
+    if (e == cudaSuccess && cl > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    int n = 1;
+    if (e == cudaSuccess && cl > 1) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[1];
+        coarse_config(sv, &cfg, at);
+        e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
+    }
+    if (e != cudaSuccess || n < 1) {   // the device does not take this cluster
+        cudaGetLastError();
+        sv->coarse_cluster = 0;
+        return FALCON_OK;
+    }
+    SCK(sv->alloc(&sv->cghost, g.size() * 4), "coarse words");
+    SCK(sv->alloc(&sv->ceat, eat.size() * sizeof(uint2)), "coarse words");
+    SCK(sv->alloc(&sv->cew, ew.size() * sizeof(float4)), "coarse words");
+    SCK(sv->alloc(&sv->clist, list.size() * sizeof(int4)), "coarse words");
+    SCK(cudaMemcpy(sv->cghost, g.data(), g.size() * 4, cudaMemcpyHostToDevice), "coarse words");
+    SCK(cudaMemcpy(sv->clist, list.data(), list.size() * sizeof(int4), cudaMemcpyHostToDevice), "coarse words");
+    if (!eat.empty()) {
+        SCK(cudaMemcpy(sv->ceat, eat.data(), eat.size() * sizeof(uint2), cudaMemcpyHostToDevice), "coarse words");
+        SCK(cudaMemcpy(sv->cew, ew.data(), ew.size() * sizeof(float4), cudaMemcpyHostToDevice), "coarse words");
+    }
+    return FALCON_OK;
+}
+
+// z_0 = M r_0: one V-cycle on the FP32 residual stored in lv[0].r, into lv[0].z
 cudaError_t vcycle_body(falcon_solver* sv) {
     const int nl = (int)sv->lv.size(), nb = sv->S.nblocks;
     cudaError_t e = cudaSuccess;
-    // smooth(): `zero` when z (ghosts included) was just zeroed, so the first
-    // sweep needs no fill; otherwise z changed everywhere and the first fill is
-    // whole. Returns the colour of the last half sweep (-1 if none).
-    auto smooth = [&](int l, int sweeps, bool reverse, bool zero) -> int {
-        SvLevel& L = sv->lv[l];
-        int last = -1;
-        for (int s = 0; s < sweeps && e == cudaSuccess; ++s)
-            for (int h = 0; h < 2 && e == cudaSuccess; ++h) {
-                const int colour = reverse ? 1 - h : h;
-                if (last >= 0) e = halo_fill_part<float>(sv, l, L.z, colour);
-                else if (!zero) e = halo_fill<float>(sv, l, L.z);
-                if (e != cudaSuccess) break;
-                k_rbgs<<<grid_cells(L.d, nb), tpb(L.d), 0, sv->st>>>(L.ops32(), L.d, L.r, L.z, colour);
-                e = cudaGetLastError();
-                last = colour;
-            }
-        return last;
+    // the sweeps are out of place: a level's buffers take turns so that its last write lands in z
+    std::vector<int> left(nl);
+    std::vector<float*> zc(nl, nullptr);
+    auto next = [&](int l) { return --left[l] & 1 ? sv->lv[l].zb : sv->lv[l].z; };
+    auto plain = [&](int l, int colour) {
+        if (e != cudaSuccess) return;
+        float* out = next(l);
+        e = vsweep<V_PLAIN>(sv, l, zc[l], nullptr, out, colour);
+        zc[l] = out;
     };
-    int last = -1;
     for (int l = 0; l < nl && e == cudaSuccess; ++l) {
         SvLevel& L = sv->lv[l];
-        k_zero_f<<<1216, 256, 0, sv->st>>>(L.z, (size_t)nb * L.d.npad);
-        e = cudaGetLastError();
-        const bool coarsest = l == nl - 1 && nl > 1;
-        if (coarsest && sv->rec && sv->rec_n < sv->rec_max && e == cudaSuccess)
+        const bool coarsest = l == nl - 1 && nl > 1, net = coarsest && sv->use_net;
+        const int sweeps = net ? sv->net_sweeps : l == nl - 1 ? sv->nu_coarse : sv->nu_pre;
+        // the whole smoothing of a small coarsest level in one launch where several launches are saved
+        const bool one = coarsest && !net && sv->coarse_cluster > 0 && sweeps > 2;
+        left[l] = (net ? 1 + 2 * sweeps : one || sweeps == 0 ? 1 : 2 * sweeps - 1) +
+                  (l < nl - 1 ? std::max(1, 2 * sv->nu_post) : 0);
+        if (coarsest && sv->rec && sv->rec_n < sv->rec_max)
             e = cudaMemcpyAsync(sv->rec + (size_t)sv->rec_n++ * nb * L.d.nint, L.r, (size_t)nb * L.d.nint * 4,
                                 cudaMemcpyDeviceToDevice, sv->st);
-        if (coarsest && sv->use_net && e == cudaSuccess) {
+        if (e != cudaSuccess) break;
+        zc[l] = next(l);
+        if (net) {
             // z_c = s * net(r_c / diag / s, operator) then a few sweeps
             const int64_t N = (int64_t)nb * L.d.nint;
             e = cudaMemsetAsync(sv->csum, 0, 8, sv->st);
@@ -963,34 +1085,30 @@ cudaError_t vcycle_body(falcon_solver* sv) {
                 e = lcc::forward_device(sv->net, sv->feat, 2, sv->cD, sv->cH, sv->cW, sv->yout, sv->st);
             }
             if (e == cudaSuccess) {
-                k_lcc_scatter<<<grid_cells(L.d, nb), tpb(L.d), 0, sv->st>>>(L.d, sv->yout, sv->gmap, sv->csum, N, L.z);
+                k_lcc_scatter<<<grid_cells(L.d, nb), tpb(L.d), 0, sv->st>>>(L.d, sv->yout, sv->gmap, sv->csum, N, zc[l]);
                 e = cudaGetLastError();
             }
-            last = smooth(l, sv->net_sweeps, false, false);
+            for (int s = 0; s < 2 * sweeps; ++s) plain(l, s & 1);
+        } else if (sweeps == 0) {
+            e = cudaMemsetAsync(zc[l], 0, (size_t)nb * L.d.nint * 4, sv->st);
+        } else if (one) {
+            e = coarse_sweeps(sv, sweeps, zc[l]);
         } else {
-            last = smooth(l, l == nl - 1 ? sv->nu_coarse : sv->nu_pre, false, true);
+            e = vsweep<V_FIRST>(sv, l, nullptr, nullptr, zc[l], 1);
+            for (int s = 2; s < 2 * sweeps; ++s) plain(l, s & 1);
         }
-        if (l + 1 < nl && e == cudaSuccess) {
-            // the residual reads every ghost: refresh those of the last sweep's parity
-            e = last >= 0 ? halo_fill_part<float>(sv, l, L.z, 1 - last) : halo_fill<float>(sv, l, L.z);
-            if (e != cudaSuccess) break;
-            k_resid32<<<grid_cells(L.d, nb), tpb(L.d), 0, sv->st>>>(L.ops32(), L.d, L.r, L.z, L.res);
-            SvLevel& C = sv->lv[l + 1];
-            k_restrict<<<grid_cells(C.d, nb), tpb(C.d), 0, sv->st>>>(L.d, C.d, L.res, C.r);
-            e = cudaGetLastError();
-        }
+        if (l + 1 < nl && e == cudaSuccess) e = vresid_restrict(sv, l, zc[l], sv->lv[l + 1].r);
     }
     for (int l = nl - 2; l >= 0 && e == cudaSuccess; --l) {
-        SvLevel& L = sv->lv[l];
-        SvLevel& C = sv->lv[l + 1];
-        k_prolong_add<<<grid_cells(L.d, nb), tpb(L.d), 0, sv->st>>>(L.d, C.d, C.z, L.z);
-        e = cudaGetLastError();
-        smooth(l, sv->nu_post, true, false);
+        float* out = next(l);
+        e = vsweep<V_PROLONG>(sv, l, zc[l], zc[l + 1], out, sv->nu_post ? 1 : -1);
+        zc[l] = out;
+        for (int s = 1; s < 2 * sv->nu_post; ++s) plain(l, 1 - (s & 1));
     }
     return e;
 }
 
-// z_0 = M r_0 as one CUDA graph launch: the V-cycle's ~100 launches are
+// z_0 = M r_0 as one CUDA graph launch: the V-cycle's launches are
 // captured once per shape and replayed (recording calls run eagerly: their
 // destination changes from call to call)
 cudaError_t vcycle(falcon_solver* sv) {
@@ -1013,6 +1131,18 @@ cudaError_t vcycle(falcon_solver* sv) {
         it = sv->vgraphs.emplace(key, x).first;
     }
     return cudaGraphLaunch(it->second, sv->st);
+}
+
+// The tile shape of every cell kernel (all levels); launch shapes are baked
+// into the captured graphs, so they go.
+void apply_tile(falcon_solver* sv, int chunk, int tpb_) {
+    sv->tile_chunk = chunk;
+    sv->tile_tpb = tpb_;
+    for (SvLevel& L : sv->lv) {
+        L.d.chunk = chunk;
+        L.d.tpb = tpb_;
+    }
+    sv->clear_graphs();
 }
 
 int setup(falcon_solver* sv) {
@@ -1051,116 +1181,190 @@ int setup(falcon_solver* sv) {
         SCK(up32(&L.fAi, H.Ai), "operator");
         SCK(up32(&L.fAj, H.Aj), "operator");
         SCK(up32(&L.fAk, H.Ak), "operator");
-        // halo entries -> padded offsets and strides
-        // halo entries -> padded offsets; entries with all weights zero are
-        // plain copies (a separate list: 8 bytes of index per entry)
-        std::vector<int32_t> dst, src, stv, cdst, csrc;
-        std::vector<double> w;
-        const int32_t strides[3] = {1, L.d.p0, L.d.p0 * L.d.p1};
-        for (const HaloEntry& h : H.halo) {
+        // halo entries: the FP64 lists (padded offsets; entries with all
+        // weights zero are plain copies, a separate list of 8 bytes each), and
+        // the FP32 V-cycle's ghost descriptors (interior cell indices). The
+        // map's weights at aligned neighbours are 0 or 1 up to rounding (about
+        // 1e-14), seldom exactly: in FP32 a weight within 2^-24 of 0 or 1 changes
+        // nothing but the last bit, so those ghosts become copies (one read
+        // instead of eight; all but the Yin-Yang seam's).
+        const size_t nent = H.halo.size();
+        const int m = H.m[0];
+        constexpr double kSnap = 1.0 / (1 << 24);
+        auto snapped = [](double x) { return x < kSnap ? 0.0 : x > 1.0 - kSnap ? 1.0 : x; };
+        std::vector<int32_t> ent(nent), ent32(nent);   // index of an interpolated entry, or -1 - (index of a copy)
+        int32_t ni = 0, ncp = 0, ni32 = 0;
+        for (size_t q = 0; q < nent; ++q) {
+            const double* w = H.halo[q].w;
+            ent[q] = w[0] == 0.0 && w[1] == 0.0 && w[2] == 0.0 ? -1 - ncp++ : ni++;
+            bool copy = true;
+            for (int dd = 0; dd < 3; ++dd) {
+                const double x = snapped(w[dd]);
+                copy = copy && (x == 0.0 || x == 1.0);
+            }
+            ent32[q] = copy ? -1 : ni32++;
+        }
+        const size_t n = (size_t)ni, nc = (size_t)ncp, n32 = (size_t)ni32;
+        std::vector<int32_t> dst(n), src(n), cdst(nc), csrc(nc), isrc(n32), ghost((size_t)nb * 6 * m * m, -1);
+        std::vector<double> w(3 * n);
+        std::vector<uint8_t> code(n), icode(n32);
+        std::vector<float> iw(3 * n32);
+        std::vector<size_t> slot_of(nent);   // a halo entry's place in the ghost tables
+#pragma omp parallel for schedule(static)
+        for (int64_t qq = 0; qq < (int64_t)nent; ++qq) {
+            const size_t q = (size_t)qq;
+            const HaloEntry& h = H.halo[q];
             const int32_t t = (int32_t)(h.tb * (int64_t)L.d.npad + ((int64_t)h.tk * L.d.p1 + h.tj) * L.d.p0 + h.ti);
             const int32_t f = (int32_t)(h.sb * (int64_t)L.d.npad + ((int64_t)h.k0 * L.d.p1 + h.j0) * L.d.p0 + h.i0);
-            if (h.w[0] == 0.0 && h.w[1] == 0.0 && h.w[2] == 0.0) {
-                cdst.push_back(t);
-                csrc.push_back(f);
-                continue;
-            }
-            dst.push_back(t);
-            src.push_back(f);
-            for (int dd = 0; dd < 3; ++dd) {
-                w.push_back(h.w[dd]);
-                stv.push_back(h.w[dd] != 0.0 ? strides[dd] : 0);
-            }
-        }
-        {   // target order: a warp's stores write neighbouring ghost cells
-            // (measured faster than source order, most for the PFSS batch)
-            std::vector<size_t> ord(dst.size());
-            for (size_t q = 0; q < ord.size(); ++q) ord[q] = q;
-            std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return dst[a] < dst[b]; });
-            std::vector<int32_t> d2(ord.size()), s2(ord.size()), st2(3 * ord.size());
-            std::vector<double> w2(3 * ord.size());
-            for (size_t q = 0; q < ord.size(); ++q) {
-                d2[q] = dst[ord[q]];
-                s2[q] = src[ord[q]];
-                for (int t = 0; t < 3; ++t) {
-                    st2[3 * q + t] = stv[3 * ord[q] + t];
-                    w2[3 * q + t] = w[3 * ord[q] + t];
+            if (ent[q] < 0) {
+                const size_t c = (size_t)(-1 - ent[q]);
+                cdst[c] = t;
+                csrc[c] = f;
+            } else {
+                const size_t e = (size_t)ent[q];
+                dst[e] = t;
+                src[e] = f;
+                code[e] = 0;
+                for (int dd = 0; dd < 3; ++dd) {
+                    w[3 * e + dd] = h.w[dd];
+                    if (h.w[dd] != 0.0) code[e] |= (uint8_t)(1 << dd);
                 }
             }
-            dst.swap(d2);
-            src.swap(s2);
-            stv.swap(st2);
-            w.swap(w2);
-            std::vector<size_t> oc(cdst.size());
-            for (size_t q = 0; q < oc.size(); ++q) oc[q] = q;
-            std::stable_sort(oc.begin(), oc.end(), [&](size_t a, size_t b) { return cdst[a] < cdst[b]; });
-            // runs by parity (each run keeps the target order), see SvLevel
-            auto par = [&](int32_t o) {
-                const int64_t r = (int64_t)o % L.d.npad;
-                return (int)((r % L.d.p0 + (r / L.d.p0) % L.d.p1 + r / ((int64_t)L.d.p0 * L.d.p1)) & 1);
-            };
-            auto run = [&](size_t q) {
-                const int a = par(cdst[q]), b2 = par(csrc[q]);
-                return a != b2 ? 1 : (a == 0 ? 0 : 2);
-            };
-            std::stable_sort(oc.begin(), oc.end(), [&](size_t a, size_t b) { return run(a) < run(b); });
-            std::vector<int32_t> cd2(oc.size()), cs2(oc.size());
-            int64_t n0 = 0, nm = 0;
-            for (size_t q = 0; q < oc.size(); ++q) {
-                cd2[q] = cdst[oc[q]];
-                cs2[q] = csrc[oc[q]];
-                const int rq = run(oc[q]);
-                n0 += rq == 0;
-                nm += rq == 1;
+            const int32_t step[3] = {1, m, m * m};
+            int32_t base = (int32_t)(h.sb * (int64_t)L.d.nint + ((int64_t)(h.k0 - 1) * m + h.j0 - 1) * m + h.i0 - 1);
+            uint8_t cd = 0;
+            float w3[3];
+            for (int dd = 0; dd < 3; ++dd) {
+                double x = snapped(h.w[dd]);
+                if (x == 1.0) {
+                    base += step[dd];
+                    x = 0.0;
+                }
+                w3[dd] = (float)x;
+                if (x != 0.0) cd |= (uint8_t)(1 << dd);
             }
-            cdst.swap(cd2);
-            csrc.swap(cs2);
-            L.nhc0 = n0;
-            L.nhcm = nm;
+            const int axis = h.ti < 1 || h.ti > m ? 0 : h.tj < 1 || h.tj > m ? 1 : 2;
+            const int tt[3] = {h.ti, h.tj, h.tk}, hi = tt[axis] > m;
+            const int pos = axis == 0 ? (h.tk - 1) * m + h.tj - 1 : axis == 1 ? (h.tk - 1) * m + h.ti - 1 : (h.tj - 1) * m + h.ti - 1;
+            const int32_t e32 = ent32[q];
+            slot_of[q] = (size_t)h.tb * 6 * m * m + (size_t)(2 * axis + hi) * m * m + pos;
+            ghost[slot_of[q]] = e32 < 0 ? base : -2 - e32;
+            if (e32 < 0) continue;
+            isrc[e32] = base;
+            icode[e32] = cd;
+            for (int dd = 0; dd < 3; ++dd) iw[3 * (size_t)e32 + dd] = w3[dd];
         }
-        const size_t n = dst.size(), nc = cdst.size();
         L.nh = (int64_t)n;
         L.nhc = (int64_t)nc;
-        SCK(sv->alloc(&L.hdst, n * 4), "halo");
-        SCK(sv->alloc(&L.hsrc, n * 4), "halo");
-        std::vector<uint8_t> code(n);
-        std::vector<float> wf(3 * n);
-        for (size_t q = 0; q < n; ++q) {
-            code[q] = (uint8_t)((stv[3 * q] ? 1 : 0) | (stv[3 * q + 1] ? 2 : 0) | (stv[3 * q + 2] ? 4 : 0));
-            for (int t = 0; t < 3; ++t) wf[3 * q + t] = (float)w[3 * q + t];
+        auto up = [&](auto** dp, const auto& v) -> cudaError_t {
+            cudaError_t e = sv->alloc(dp, v.size() * sizeof(v[0]));
+            if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*dp, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice);
+            return e;
+        };
+        SCK(up(&L.hdst, dst), "halo");
+        SCK(up(&L.hsrc, src), "halo");
+        SCK(up(&L.hcode, code), "halo");
+        SCK(up(&L.hw, w), "halo");
+        SCK(up(&L.hcdst, cdst), "halo");
+        SCK(up(&L.hcsrc, csrc), "halo");
+        SCK(up(&L.ghost, ghost), "halo");
+        SCK(up(&L.isrc, isrc), "halo");
+        SCK(up(&L.icode, icode), "halo");
+        SCK(up(&L.iw, iw), "halo");
+        // faces whose ghosts come from one block, position by position (VLevel::nbr)
+        std::vector<int32_t> nbr((size_t)nb * 12, -2);
+#pragma omp parallel for schedule(static)
+        for (int gb = 0; gb < nb; ++gb)
+            for (int f = 0; f < 6; ++f) {
+                const int32_t* gf = &ghost[((size_t)gb * 6 + f) * m * m];
+                // the entry's base cell and its weight along i; other directions disqualify
+                auto base = [&](int t, float& wi) -> int32_t {
+                    wi = 0.f;
+                    if (gf[t] >= -1) return gf[t];
+                    const size_t e = (size_t)(-2 - gf[t]);
+                    if (f > 1 || icode[e] != 1) return -1;
+                    wi = iw[3 * e];
+                    return isrc[e];
+                };
+                float w0 = 0.f, wt = 0.f;
+                const int32_t b0 = base(0, w0);
+                const int own = b0 >= 0 ? b0 / L.d.nint : -1, i0 = f < 2 ? b0 % m : 0;
+                bool none = true, same = own >= 0;
+                for (int t = 0; t < m * m; ++t) {
+                    const int u = t % m, v = t / m, in = (f & 1) ? 0 : m - 1;
+                    const int i = f < 2 ? i0 : u, j = f < 2 ? u : f < 4 ? in : v, k = f < 4 ? v : in;
+                    none = none && gf[t] == -1;
+                    same = same && base(t, wt) == own * L.d.nint + (k * m + j) * m + i && wt == w0;
+                }
+                int32_t* o = &nbr[(size_t)gb * 12];
+                o[f] = none ? -2 : same ? own : -1;
+                if (f > 1) continue;
+                o[6 + f] = i0;
+                std::memcpy(&o[8 + f], &w0, 4);
+            }
+        SCK(up(&L.nbr, nbr), "halo");
+        if (l == S.nlevels - 1) {
+            const int rc = plan_coarse(sv, ghost, isrc, icode, iw);
+            if (rc) return rc;
         }
-        SCK(sv->alloc(&L.hcode, n), "halo");
-        SCK(sv->alloc(&L.hwf, 3 * n * 4), "halo");
-        SCK(sv->alloc(&L.hw, 3 * n * 8), "halo");
-        SCK(sv->alloc(&L.hcdst, nc * 4), "halo");
-        SCK(sv->alloc(&L.hcsrc, nc * 4), "halo");
-        if (n) {
-            SCK(cudaMemcpy(L.hdst, dst.data(), n * 4, cudaMemcpyHostToDevice), "halo");
-            SCK(cudaMemcpy(L.hsrc, src.data(), n * 4, cudaMemcpyHostToDevice), "halo");
-            SCK(cudaMemcpy(L.hcode, code.data(), n, cudaMemcpyHostToDevice), "halo");
-            SCK(cudaMemcpy(L.hwf, wf.data(), 3 * n * 4, cudaMemcpyHostToDevice), "halo");
-            SCK(cudaMemcpy(L.hw, w.data(), 3 * n * 8, cudaMemcpyHostToDevice), "halo");
-        }
-        if (nc) {
-            SCK(cudaMemcpy(L.hcdst, cdst.data(), nc * 4, cudaMemcpyHostToDevice), "halo");
-            SCK(cudaMemcpy(L.hcsrc, csrc.data(), nc * 4, cudaMemcpyHostToDevice), "halo");
-        }
-        if (l == 0) {   // the 8 corner weights of each interpolated halo entry, FF pairs
-            std::vector<float2> w8(8 * n);
-            for (size_t q = 0; q < n; ++q) {
-                const double wi = w[3 * q], wj = w[3 * q + 1], wk = w[3 * q + 2];
+        if (l == 0) {   // the ghosts of the float-float iteration (GhostFF)
+            constexpr double kSnapFF = 1.0 / (1LL << 32);
+            const size_t ns = ghost.size();
+            std::vector<int32_t> gd(ns, -1), esrc;
+            std::vector<float> eps(3 * ns, 0.f);
+            std::vector<size_t> two;   // halo entries that stay interpolations
+            for (size_t q = 0; q < nent; ++q) {
+                const HaloEntry& h = H.halo[q];
+                const int32_t st[3] = {1, m, m * m};
+                const size_t slot = slot_of[q];
+                int32_t base = (int32_t)(h.sb * (int64_t)L.d.nint + ((int64_t)(h.k0 - 1) * m + h.j0 - 1) * m + h.i0 - 1);
+                bool copy = true;
+                for (int dd = 0; dd < 3; ++dd) copy = copy && (h.w[dd] < kSnapFF || h.w[dd] > 1.0 - kSnapFF);
+                if (!copy) {
+                    gd[slot] = -2 - (int32_t)two.size();
+                    two.push_back(q);
+                    esrc.push_back(base);
+                    continue;
+                }
+                for (int dd = 0; dd < 3; ++dd) {
+                    if (h.w[dd] > 0.5) {
+                        base += st[dd];
+                        eps[3 * slot + dd] = -(float)(1.0 - h.w[dd]);
+                    } else {
+                        eps[3 * slot + dd] = (float)h.w[dd];
+                    }
+                }
+                gd[slot] = base;
+            }
+            std::vector<float2> w8(8 * two.size());
+            std::vector<uint8_t> ecode(two.size());
+#pragma omp parallel for schedule(static)
+            for (int64_t e = 0; e < (int64_t)two.size(); ++e) {
+                const double* hw = H.halo[two[(size_t)e]].w;
+                const double wi = hw[0], wj = hw[1], wk = hw[2];
                 const double ui = 1.0 - wi, uj = 1.0 - wj, uk = 1.0 - wk;
                 const double c8[8] = {ui * uj * uk, wi * uj * uk, ui * wj * uk, ui * uj * wk,
                                       wi * wj * uk, ui * wj * wk, wi * uj * wk, wi * wj * wk};
                 for (int t = 0; t < 8; ++t) {
                     const float h = (float)c8[t];
-                    w8[8 * q + t] = make_float2(h, (float)(c8[t] - (double)h));
+                    w8[8 * (size_t)e + t] = make_float2(h, (float)(c8[t] - (double)h));
                 }
+                ecode[(size_t)e] = (uint8_t)((wi != 0.0 ? 1 : 0) | (wj != 0.0 ? 2 : 0) | (wk != 0.0 ? 4 : 0));
             }
-            SCK(sv->alloc(&L.hw8, w8.size() * sizeof(float2)), "halo");
-            if (n) SCK(cudaMemcpy(L.hw8, w8.data(), w8.size() * sizeof(float2), cudaMemcpyHostToDevice), "halo");
+            int32_t *dg, *ds;
+            float* de;
+            uint8_t* dc;
+            float2* dw;
+            SCK(up(&dg, gd), "halo");
+            SCK(up(&de, eps), "halo");
+            SCK(up(&ds, esrc), "halo");
+            SCK(up(&dc, ecode), "halo");
+            SCK(up(&dw, w8), "halo");
+            SCK(sv->alloc(&sv->ghosts2, ns * sizeof(float2)), "halo");
+            sv->gff = GhostFF{dg, de, ds, dc, dw, m, (int64_t)ns};
         }
-        SCK(sv->alloc(&L.z, (size_t)nb * L.d.npad * 4), "vectors");
+        SCK(sv->alloc(&L.z, (size_t)nb * L.d.nint * 4), "vectors");
+        SCK(sv->alloc(&L.zb, (size_t)nb * L.d.nint * 4), "vectors");
         SCK(sv->alloc(&L.r, (size_t)nb * L.d.nint * 4), "vectors");
         SCK(sv->alloc(&L.res, (size_t)nb * L.d.nint * 4), "vectors");
     }
@@ -1171,7 +1375,7 @@ int setup(falcon_solver* sv) {
     SCK(sv->alloc(&sv->Ap, (size_t)nb * d0.nint * 8), "vectors");
     SCK(sv->alloc(&sv->z, (size_t)nb * d0.nint * 8), "vectors");
     SCK(sv->alloc(&sv->bvec, (size_t)nb * d0.nint * 8), "vectors");
-    SCK(sv->alloc(&sv->dots, (size_t)6 * S.nproblems * 8), "scalars");
+    SCK(sv->alloc(&sv->dots, (size_t)8 * S.nproblems * 8), "scalars");
     SCK(sv->alloc(&sv->ir_par, (size_t)2 * S.nproblems * 8), "scalars");
     SCK(sv->alloc(&sv->rr0, (size_t)S.nproblems * 8), "scalars");
     SCK(sv->alloc(&sv->eta, (size_t)S.nproblems * 8), "scalars");
@@ -1200,13 +1404,15 @@ int setup(falcon_solver* sv) {
         SCK(upff(&L0.Ai2, H.Ai), "operator");
         SCK(upff(&L0.Aj2, H.Aj), "operator");
         SCK(upff(&L0.Ak2, H.Ak), "operator");
-        for (float2** v : {&sv->x2, &sv->p2}) SCK(sv->alloc(v, (size_t)nb * d0.npad * sizeof(float2)), "vectors");
-        for (float2** v : {&sv->r2, &sv->Ap2, &sv->z2})
+        for (float2** v : {&sv->x2, &sv->p2, &sv->r2, &sv->Ap2, &sv->w2})
             SCK(sv->alloc(v, (size_t)nb * d0.nint * sizeof(float2)), "vectors");
         std::vector<float> fa(sv->sA.begin(), sv->sA.end());
         SCK(sv->alloc(&sv->dsA, fa.size() * 4), "scalars");
         SCK(cudaMemcpy(sv->dsA, fa.data(), fa.size() * 4, cudaMemcpyHostToDevice), "scalars");
     }
+    SCK(sv->alloc(&sv->first, (size_t)(S.nproblems + 1) * 4), "scalars");
+    SCK(cudaMemcpy(sv->first, S.problem_first_block.data(), (size_t)(S.nproblems + 1) * 4, cudaMemcpyHostToDevice), "scalars");
+    apply_tile(sv, sv->tile_chunk, sv->tile_tpb);
     SCK(cudaStreamSynchronize(sv->st), "setup");
     return FALCON_OK;
 }
@@ -1326,7 +1532,7 @@ int coarse_solve(falcon_solver* sv, const float* rc) {
     const double rr0 = h[2];
     if (!(rr0 > 0)) return FALCON_OK;
     for (int it = 0; it < 50000; ++it) {
-        SCK(halo_fill<double>(sv, lc, sv->p), "coarse cg");
+        SCK(halo_fill(sv, lc, sv->p), "coarse cg");
         SCK(cudaMemsetAsync(dots + 1, 0, 8, sv->st), "coarse cg");
         SCK(cudaMemsetAsync(dots + 3, 0, 3 * 8, sv->st), "coarse cg");
         k_ccg_spmv<<<g, tpb(L.d), 0, sv->st>>>(L.ops64(), L.d, sv->p, sv->Ap, dots);
@@ -1396,11 +1602,13 @@ bool all_finite(const double* v, size_t n) {
 }
 
 // ---- the inner solve: one FCG iteration, as a graph or eagerly ----------------
-// One iteration unit on the stream. `first`: z = M r, p = z (restart); else
-// z = M r, beta = -z.Ap / p.Ap, p = z + beta p. Then the halo of p, q = A p
-// with p.q and p.r, alpha, x += alpha p, r -= alpha q with r.r, and the
-// device-side check (k_inner_check), which sets the WHILE condition when
-// `set_cond`. Inactive problems take no step.
+// One iteration unit on the stream: z = M r (the residual's FP32 part without
+// a preconditioner), its ghosts, w = A z with the products that give beta
+// (`first`: 0, a restart) and alpha, the update of p, A p, x and r with r.r, and
+// the device-side check (k_inner_check), which sets the WHILE condition when
+// `set_cond`. Inactive problems take no step. (Forming p first, with its own
+// FF halo of eight weighted reads per ghost, took five kernels and 340 us per
+// iteration at 6.3M cells in 16^3 blocks; this takes three.)
 cudaError_t enqueue_iteration(falcon_solver* sv, int pc, bool first, cudaGraphConditionalHandle h, int set_cond) {
     const int nb = sv->S.nblocks, np = sv->S.nproblems;
     const LevelDims& d = sv->lv[0].d;
@@ -1412,16 +1620,16 @@ cudaError_t enqueue_iteration(falcon_solver* sv, int pc, bool first, cudaGraphCo
         sv->use_net = false;
         if (e != cudaSuccess) return e;
     }
-    k_take_z_ff<<<g, tpb(d), 0, sv->st>>>(d, sv->lv[0].z, sv->dsA, sv->r2, pc == FALCON_PRECOND_NONE, sv->z2, sv->Ap2,
-                                          sv->D(), first ? 0 : 1);
-    k_update_p_ff<<<g, tpb(d), 0, sv->st>>>(d, sv->p2, sv->z2, sv->D(), first ? 1 : 0);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = halo_fill_ff(sv, sv->p2);
-    if (e == cudaSuccess) e = cudaMemsetAsync(sv->dots, 0, (size_t)4 * np * 8, sv->st);
-    if (e != cudaSuccess) return e;
-    k_spmv_dots_ff<<<g, tpb(d), 0, sv->st>>>(sv->lv[0].ops2(), d, sv->p2, sv->Ap2, sv->r2, sv->D());
-    k_update_xr_ff<<<g, tpb(d), 0, sv->st>>>(d, sv->x2, sv->p2, sv->r2, sv->Ap2, sv->lv[0].r, sv->D());
-    k_inner_check<<<1, 256, 0, sv->st>>>(np, sv->dots + 3 * np, sv->rr0, sv->eta, sv->active, sv->ictl, h, set_cond);
+    const bool none = pc == FALCON_PRECOND_NONE;
+    const float* z = none ? sv->lv[0].r : sv->lv[0].z;
+    const float* scale = none ? nullptr : sv->dsA;   // the V-cycle inverts the unscaled FP32 operator
+    k_ghost_ff<<<(unsigned)((sv->gff.n + 255) / 256), 256, 0, sv->st>>>(sv->gff, z, scale, sv->bprob, sv->ghosts2);
+    const auto spmv = d.m0 == 8 ? k_spmv_z_ff<8> : d.m0 == 16 ? k_spmv_z_ff<16> : k_spmv_z_ff<0>;
+    spmv<<<g, std::min(tpb(d), 512u), 0, sv->st>>>(sv->lv[0].ops2(), d, z, scale, sv->ghosts2, sv->p2, sv->r2, sv->Ap2,
+                                                   sv->w2, sv->D());
+    k_step_ff<<<g, std::min(tpb(d), 512u), 0, sv->st>>>(d, z, scale, sv->w2, sv->x2, sv->p2, sv->r2, sv->Ap2, sv->lv[0].r,
+                                                        sv->D(), first ? 1 : 0);
+    k_inner_check<<<1, 256, 0, sv->st>>>(np, sv->D(), first ? 1 : 0, sv->rr0, sv->eta, sv->active, sv->ictl, h, set_cond);
     return cudaGetLastError();
 }
 
@@ -1510,18 +1718,6 @@ cudaError_t run_inner(falcon_solver* sv, int pc, int max_it, InnerCtl* ctl) {
     }
 }
 
-// The tile shape of every cell kernel (all levels); launch shapes are baked
-// into the captured graphs, so they go.
-void apply_tile(falcon_solver* sv, int chunk, int tpb_) {
-    sv->tile_chunk = chunk;
-    sv->tile_tpb = tpb_;
-    for (SvLevel& L : sv->lv) {
-        L.d.chunk = chunk;
-        L.d.tpb = tpb_;
-    }
-    sv->clear_graphs();
-}
-
 // The solver's autotuner: times one eager FCG iteration (V-cycle with the
 // solver's smoothing, the float-float kernels, halo fills) for each candidate
 // tile -- cells per CTA in {512, 1024, 2048, 4096} (a multiple of the row
@@ -1534,10 +1730,11 @@ int autotune_tile(falcon_solver* sv) {
     const int np = sv->S.nproblems;
     const int m0 = sv->lv[0].d.m0;
     std::vector<int32_t> act(np, 1);
-    std::vector<double> ones(np, 1.0), zeros(np, 0.0);
+    std::vector<double> ones(np, 1.0), never(np, -1.0);   // no residual is at or below eta: every problem stays active
     SCK(cudaMemcpyAsync(sv->active, act.data(), np * 4, cudaMemcpyHostToDevice, sv->st), "tune");
     SCK(cudaMemcpyAsync(sv->rr0, ones.data(), np * 8, cudaMemcpyHostToDevice, sv->st), "tune");
-    SCK(cudaMemcpyAsync(sv->eta, zeros.data(), np * 8, cudaMemcpyHostToDevice, sv->st), "tune");
+    SCK(cudaMemcpyAsync(sv->eta, never.data(), np * 8, cudaMemcpyHostToDevice, sv->st), "tune");
+    SCK(cudaMemsetAsync(sv->dots, 0, (size_t)8 * np * 8, sv->st), "tune");
     SCK(cudaStreamSynchronize(sv->st), "tune");
     const int pc = sv->S.nlevels > 1 ? FALCON_PRECOND_MG : FALCON_PRECOND_NONE;
     cudaEvent_t a, b;
@@ -1627,44 +1824,26 @@ int falcon_solver_vcycle_op(falcon_solver* sv, int32_t op, int32_t level, const 
         return sv->fail(FALCON_ERR_INVALID_ARG, "falcon_solver_vcycle_op: bad operation, level or input");
     cudaSetDevice(sv->device);
     SvLevel& L = sv->lv[level];
-    const size_t nf = (size_t)nb * L.d.nint;
-    const dim3 gf = grid_cells(L.d, nb);
+    const size_t nf = (size_t)nb * L.d.nint * 4;
     SCK(cudaStreamSynchronize(sv->st), "vcycle op");
-    if (op == FALCON_VCYCLE_RESTRICT) {
+    if (op == FALCON_VCYCLE_RESTRICT) {   // the residual of r = in0 at z = 0, restricted
         SvLevel& Cl = sv->lv[level + 1];
-        SCK(cudaMemcpyAsync(L.res, in0, nf * 4, cudaMemcpyHostToDevice, sv->st), "vcycle op");
-        k_restrict<<<grid_cells(Cl.d, nb), tpb(Cl.d), 0, sv->st>>>(L.d, Cl.d, L.res, Cl.r);
-        SCK(cudaGetLastError(), "vcycle op");
+        SCK(cudaMemcpyAsync(L.r, in0, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(cudaMemsetAsync(L.z, 0, nf, sv->st), "vcycle op");
+        SCK(vresid_restrict(sv, level, L.z, Cl.r), "vcycle op");
         SCK(cudaMemcpyAsync(out, Cl.r, (size_t)nb * Cl.d.nint * 4, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
     } else if (op == FALCON_VCYCLE_PROLONG_ADD) {
         SvLevel& Cl = sv->lv[level + 1];
-        const size_t nc = (size_t)nb * Cl.d.nint;
-        SCK(cudaMemsetAsync(Cl.z, 0, (size_t)nb * Cl.d.npad * 4, sv->st), "vcycle op");
-        SCK(cudaMemsetAsync(L.z, 0, (size_t)nb * L.d.npad * 4, sv->st), "vcycle op");
-        SCK(cudaMemcpyAsync(Cl.r, in0, nc * 4, cudaMemcpyHostToDevice, sv->st), "vcycle op");
-        SCK(cudaMemcpyAsync(L.res, in1, nf * 4, cudaMemcpyHostToDevice, sv->st), "vcycle op");
-        k_scatter_pad<float><<<grid_cells(Cl.d, nb), tpb(Cl.d), 0, sv->st>>>(Cl.d, Cl.r, Cl.z);
-        k_scatter_pad<float><<<gf, tpb(L.d), 0, sv->st>>>(L.d, L.res, L.z);
-        k_prolong_add<<<gf, tpb(L.d), 0, sv->st>>>(L.d, Cl.d, Cl.z, L.z);
-        k_gather_pad<float><<<gf, tpb(L.d), 0, sv->st>>>(L.d, L.z, L.res);
-        SCK(cudaGetLastError(), "vcycle op");
-        SCK(cudaMemcpyAsync(out, L.res, nf * 4, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
-    } else {
-        // z (interior) into the padded z, its halo filled, then one red-black
-        // half sweep of a colour or the residual r - A z
-        SCK(cudaMemsetAsync(L.z, 0, (size_t)nb * L.d.npad * 4, sv->st), "vcycle op");
-        SCK(cudaMemcpyAsync(L.r, in0, nf * 4, cudaMemcpyHostToDevice, sv->st), "vcycle op");
-        SCK(cudaMemcpyAsync(L.res, in1, nf * 4, cudaMemcpyHostToDevice, sv->st), "vcycle op");
-        k_scatter_pad<float><<<gf, tpb(L.d), 0, sv->st>>>(L.d, L.res, L.z);
-        SCK(halo_fill<float>(sv, level, L.z), "vcycle op");
-        if (op == FALCON_VCYCLE_RESIDUAL) {
-            k_resid32<<<gf, tpb(L.d), 0, sv->st>>>(L.ops32(), L.d, L.r, L.z, L.res);
-        } else {
-            k_rbgs<<<gf, tpb(L.d), 0, sv->st>>>(L.ops32(), L.d, L.r, L.z, op == FALCON_VCYCLE_SMOOTH_RED ? 0 : 1);
-            k_gather_pad<float><<<gf, tpb(L.d), 0, sv->st>>>(L.d, L.z, L.res);
-        }
-        SCK(cudaGetLastError(), "vcycle op");
-        SCK(cudaMemcpyAsync(out, L.res, nf * 4, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
+        SCK(cudaMemcpyAsync(Cl.z, in0, (size_t)nb * Cl.d.nint * 4, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(cudaMemcpyAsync(L.z, in1, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(vsweep<V_PROLONG>(sv, level, L.z, Cl.z, L.zb, -1), "vcycle op");
+        SCK(cudaMemcpyAsync(out, L.zb, nf, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
+    } else {   // one red-black half sweep of a colour from z = in1, or the residual r - A z
+        SCK(cudaMemcpyAsync(L.r, in0, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(cudaMemcpyAsync(L.z, in1, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        if (op == FALCON_VCYCLE_RESIDUAL) SCK(vresid(sv, level, L.z, L.res), "vcycle op");
+        else SCK(vsweep<V_PLAIN>(sv, level, L.z, nullptr, L.zb, op == FALCON_VCYCLE_SMOOTH_RED ? 0 : 1), "vcycle op");
+        SCK(cudaMemcpyAsync(out, op == FALCON_VCYCLE_RESIDUAL ? L.res : L.zb, nf, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
     }
     SCK(cudaStreamSynchronize(sv->st), "vcycle op");
     return FALCON_OK;
@@ -1901,9 +2080,8 @@ int falcon_solver_apply(falcon_solver* sv, const double* x, double* y) {
     SCK(cudaMemcpyAsync(sv->z, x, (size_t)nb * d.nint * 8, cudaMemcpyHostToDevice, sv->st), "apply");
     SCK(cudaMemsetAsync(sv->p, 0, (size_t)nb * d.npad * 8, sv->st), "apply");
     k_scatter_pad<double><<<grid_cells(d, nb), tpb(d), 0, sv->st>>>(d, sv->z, sv->p);
-    SCK(halo_fill<double>(sv, 0, sv->p), "apply halo");
-    SCK(cudaMemsetAsync(sv->dots, 0, (size_t)6 * sv->S.nproblems * 8, sv->st), "apply");
-    k_spmv_dots<<<grid_cells(d, nb), tpb(d), 0, sv->st>>>(sv->lv[0].ops64(), d, sv->p, sv->Ap, sv->r, sv->D());
+    SCK(halo_fill(sv, 0, sv->p), "apply halo");
+    k_spmv<<<grid_cells(d, nb), tpb(d), 0, sv->st>>>(sv->lv[0].ops64(), d, sv->p, sv->Ap);
     SCK(cudaGetLastError(), "apply");
     SCK(cudaMemcpyAsync(y, sv->Ap, (size_t)nb * d.nint * 8, cudaMemcpyDeviceToHost, sv->st), "apply");
     SCK(cudaStreamSynchronize(sv->st), "apply");
@@ -1967,7 +2145,7 @@ int falcon_solver_solve(falcon_solver* sv, double tol, int32_t max_iter, int32_t
         // FP64 true residual of every problem
         SCK(cudaMemsetAsync(sv->dots + 3 * np, 0, (size_t)(first ? 3 : 1) * np * 8, sv->st), "dots");
         SCK(cudaMemsetAsync(sv->dots + 5 * np, 0, (size_t)np * 8, sv->st), "dots");
-        SCK(halo_fill<double>(sv, 0, sv->x), "halo");
+        SCK(halo_fill(sv, 0, sv->x), "halo");
         k_residual64<<<g, tpb(d), 0, sv->st>>>(sv->lv[0].ops64(), d, sv->x, sv->bvec, sv->r, sv->lv[0].r, sv->D(),
                                                first ? 1 : 0);
         SCK(cudaGetLastError(), "residual");
@@ -2010,12 +2188,13 @@ int falcon_solver_solve(falcon_solver* sv, double tol, int32_t max_iter, int32_t
         SCK(cudaMemcpyAsync(sv->active, act.data(), np * 4, cudaMemcpyHostToDevice, sv->st), "active");
         SCK(cudaMemcpyAsync(sv->ir_par, inv_sr.data(), np * 8, cudaMemcpyHostToDevice, sv->st), "scale");
         SCK(cudaMemcpyAsync(sv->ir_par + np, fac.data(), np * 8, cudaMemcpyHostToDevice, sv->st), "scale");
-        SCK(cudaMemsetAsync(sv->x2, 0, (size_t)nb * d.npad * sizeof(float2), sv->st), "init");
-        SCK(cudaMemsetAsync(sv->p2, 0, (size_t)nb * d.npad * sizeof(float2), sv->st), "init");
-        SCK(cudaMemsetAsync(sv->dots, 0, (size_t)5 * np * 8, sv->st), "dots");
+        for (float2* v : {sv->x2, sv->p2, sv->Ap2})
+            SCK(cudaMemsetAsync(v, 0, (size_t)nb * d.nint * sizeof(float2), sv->st), "init");
+        SCK(cudaMemsetAsync(sv->dots, 0, (size_t)8 * np * 8, sv->st), "dots");
         k_ir_start<<<g, tpb(d), 0, sv->st>>>(d, sv->r, sv->ir_par, sv->r2, sv->lv[0].r, sv->D());
         SCK(cudaGetLastError(), "inner start");
         SCK(cudaMemcpyAsync(rr0.data(), sv->dots + 3 * np, np * 8, cudaMemcpyDeviceToHost, sv->st), "rr");
+        SCK(cudaMemsetAsync(sv->dots + 3 * np, 0, (size_t)np * 8, sv->st), "dots");
         SCK(cudaStreamSynchronize(sv->st), "rr");
         for (int q = 0; q < np; ++q) if (!(rr0[q] > 0)) { rr0[q] = 1.0; act[q] = 0; }
         SCK(cudaMemcpyAsync(sv->active, act.data(), np * 4, cudaMemcpyHostToDevice, sv->st), "active");
@@ -2102,7 +2281,7 @@ int falcon_solver_problem_residuals(falcon_solver* sv, double* rel) {
     const int np = sv->S.nproblems, nb = sv->S.nblocks;
     const LevelDims& d = sv->lv[0].d;
     SCK(cudaMemsetAsync(sv->dots, 0, (size_t)6 * np * 8, sv->st), "residuals");
-    SCK(halo_fill<double>(sv, 0, sv->x), "residuals");
+    SCK(halo_fill(sv, 0, sv->x), "residuals");
     k_residual64<<<grid_cells(d, nb), tpb(d), 0, sv->st>>>(sv->lv[0].ops64(), d, sv->x, sv->bvec, sv->r, sv->lv[0].r,
                                                         sv->D(), 1);
     std::vector<double> rr(np), bb(np);
