@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -203,9 +204,9 @@ cudaError_t stage(falcon_ctx* ctx, int s, void* in, void* out, const PushTable& 
     cudaError_t e = timed(ctx, KN_STAGE, [&] {
         return ctx->mixed()
                    ? launch_stage_mixed(ctx->dims, ctx->geom(), (const float*)in, (const float*)ctx->U, (float*)out,
-                                        ctx->Ulo, push, ps, s, 1, ctx->sc, 1, ctx->kpar_stage, ctx->st)
+                                        ctx->Ulo, push, ps, s, 1, ctx->sc, ctx->kpar_stage, ctx->st)
                    : launch_stage_fp64(ctx->dims, ctx->geom(), (const double*)in, (const double*)ctx->U, (double*)out,
-                                       ps, s, 1, ctx->sc, 1, ctx->kpar_stage, ctx->st);
+                                       ps, s, 1, ctx->sc, ctx->kpar_stage, ctx->st);
     });
     if (e != cudaSuccess) return e;
     return psi_after_stage(ctx, s);
@@ -227,7 +228,7 @@ cudaError_t diffusion(falcon_ctx* ctx, void* out, const PushTable& push, int cfl
     e = timed(ctx, KN_DIFF, [&] {
         return ctx->mixed() ? launch_diffusion_mixed(ctx->dims, ctx->geom(), (const float*)ctx->U, (float*)out,
                                                      ctx->Ulo, push, ctx->sc, ctx->kpar_diff, ctx->st, cfl_next)
-                            : launch_diffusion_fp64(ctx->dims, ctx->geom(), (double*)ctx->U, ctx->sc, ctx->kpar_diff, ctx->st);
+                            : launch_diffusion_fp64(ctx->dims, ctx->geom(), (double*)ctx->U, ctx->sc, ctx->st);
     });
     if (e != cudaSuccess || !ctx->P) return e;
     e = cudaMemcpyAsync(ctx->P, ctx->P2, (size_t)ctx->dims.nblocks * ctx->dims.ncell * ctx->elem,
@@ -371,14 +372,14 @@ int autotune(falcon_ctx* ctx) {
                 if (which == 0)
                     e = ctx->mixed() ? launch_stage_mixed(ctx->dims, ctx->geom(), (const float*)ctx->RK, (const float*)ctx->U,
                                                           (float*)ctx->R2, nullptr, ctx->push, psi_args(ctx, 2),
-                                                          2, 1, ctx->sc, 1, kp, ctx->st)
+                                                          2, 1, ctx->sc, kp, ctx->st)
                                      : launch_stage_fp64(ctx->dims, ctx->geom(), (const double*)ctx->RK, (const double*)ctx->U,
                                                          (double*)ctx->RK, psi_args(ctx, 2), 2, 1,
-                                                         ctx->sc, 1, kp, ctx->st);
+                                                         ctx->sc, kp, ctx->st);
                 else
                     e = ctx->mixed() ? launch_diffusion_mixed(ctx->dims, ctx->geom(), (const float*)ctx->RK,
                                                               (float*)ctx->RK, nullptr, PushTable{}, ctx->sc, kp, ctx->st)
-                                     : launch_diffusion_fp64(ctx->dims, ctx->geom(), (double*)ctx->RK, ctx->sc, kp, ctx->st);
+                                     : launch_diffusion_fp64(ctx->dims, ctx->geom(), (double*)ctx->RK, ctx->sc, ctx->st);
                 cudaEventRecord(b, ctx->st);
                 if (e != cudaSuccess || cudaEventSynchronize(b) != cudaSuccess) { ok[q][which] = false; cudaGetLastError(); continue; }
                 float ms = 0.f;
@@ -431,8 +432,10 @@ int check_nan(falcon_ctx* ctx) {
 }
 
 // global element offset of var 0 of padded cell (i,j,k) (Fortran indices) of block b
-inline int64_t cell_off(const Grid& g, int b, int i, int j, int k) {
-    return (int64_t)b * NV * g.ncell + ((int64_t)(k + 1) * g.njp + (j + 1)) * g.nip + (i + 1);
+// element of variable 0 at Fortran cell (i, j, k) of block b; cs: elements from a
+// cell to the next (Layout)
+inline int64_t cell_off(const Grid& g, int b, int i, int j, int k, int cs) {
+    return (int64_t)b * NV * g.ncell + (((int64_t)(k + 1) * g.njp + (j + 1)) * g.nip + (i + 1)) * cs;
 }
 
 // ---- block sharding ------------------------------------------------------------
@@ -471,8 +474,8 @@ cudaError_t upload_interp_list(falcon_ctx* ctx, const std::vector<int64_t>& ks, 
     std::vector<uint8_t> kind(n);
     for (size_t q = 0; q < n; ++q) {
         const GhostMapEntry& e = g.ghosts[ks[q]];
-        dst[q] = (int32_t)cell_off(g, e.e.tblock, e.e.ti, e.e.tj, e.e.tk);
-        src[q] = (int32_t)cell_off(g, e.e.sblock, e.i0, e.j0, e.k0);
+        dst[q] = (int32_t)cell_off(g, e.e.tblock, e.e.ti, e.e.tj, e.e.tk, Layout<double>::cell);
+        src[q] = (int32_t)cell_off(g, e.e.sblock, e.i0, e.j0, e.k0, Layout<double>::cell);
         const int nz = (e.w[0] != 0.0) + (e.w[1] != 0.0) + (e.w[2] != 0.0);
         for (int t = 0; t < 3; ++t) w[3 * q + t] = e.w[t];
         rot[2 * q] = e.rotate ? e.rot[0] : 0.0;
@@ -628,6 +631,7 @@ int setup_device(falcon_ctx* ctx) {
     // Two sets: every ghost cell (the exchange that ends a step) and the face
     // ghosts the stage kernel does not push (the exchanges between stages).
     const bool snap = ctx->mixed();
+    const int cs = ctx->mixed() ? Layout<float>::cell : Layout<double>::cell;
     const int n3[3] = {g.ni, g.nj, g.nk};
     struct GE {
         int32_t d, src;
@@ -653,8 +657,8 @@ int setup_device(falcon_ctx* ctx) {
         q.nz = (q.w[0] != 0.0) + (q.w[1] != 0.0) + (q.w[2] != 0.0);
         q.tb = e.e.tblock; q.sb = e.e.sblock;
         q.t[0] = e.e.ti; q.t[1] = e.e.tj; q.t[2] = e.e.tk;
-        q.d = (int32_t)cell_off(g, q.tb, q.t[0], q.t[1], q.t[2]);
-        q.src = (int32_t)cell_off(g, q.sb, q.base[0], q.base[1], q.base[2]);
+        q.d = (int32_t)cell_off(g, q.tb, q.t[0], q.t[1], q.t[2], cs);
+        q.src = (int32_t)cell_off(g, q.sb, q.base[0], q.base[1], q.base[2], cs);
         q.rotate = e.rotate;
         q.rot[0] = e.rotate ? e.rot[0] : 0.0;
         q.rot[1] = e.rotate ? e.rot[1] : 0.0;
@@ -740,7 +744,7 @@ int setup_device(falcon_ctx* ctx) {
         if (e == cudaSuccess && !vec.empty()) e = cudaMemcpy(*dptr, vec.data(), vec.size() * sizeof(E), cudaMemcpyHostToDevice);
         return e;
     };
-    const int32_t strides[3] = {1, g.nip, g.nip * g.njp};
+    const int32_t strides[3] = {cs, cs * g.nip, cs * g.nip * g.njp};
     // build and upload one set of lists over the entries `keep` selects
     auto build_lists = [&](auto keep, GhostLists& out, int64_t* counts) -> cudaError_t {
         struct Lin { int32_t d, s, st; float w; };
@@ -1377,11 +1381,11 @@ int shard_phase(falcon_ctx* ctx, int phase) {
         double* in = s == 1 ? U : RK;
         double* out = s < 4 ? RK : U;
         if (dl.nblocks > 0)
-            e = launch_stage_fp64(dl, gl, in + off, U + off, out + off, none, s, 1, ctx->sc, 1, ctx->kpar_stage, ctx->st);
+            e = launch_stage_fp64(dl, gl, in + off, U + off, out + off, none, s, 1, ctx->sc, ctx->kpar_stage, ctx->st);
         if (e == cudaSuccess) e = launch_ghost_fp64(ctx->dims, S.local, out, ctx->st);
         S.last_out = out;
     } else {
-        if (dl.nblocks > 0) e = launch_diffusion_fp64(dl, gl, U + off, ctx->sc, ctx->kpar_diff, ctx->st);
+        if (dl.nblocks > 0) e = launch_diffusion_fp64(dl, gl, U + off, ctx->sc, ctx->st);
         if (e == cudaSuccess) e = launch_ghost_fp64(ctx->dims, S.local, U, ctx->st);
         S.last_out = U;
         ++ctx->steps_done;
@@ -1502,6 +1506,41 @@ RestartHeader restart_header(const falcon_ctx* ctx) {
     return h;
 }
 constexpr size_t kIoChunk = 64u << 20;
+
+// Restart files hold the state as [block][var][cell] and the correction as
+// [block][var][interior cell]; the mixed device arrays hold a cell's variables
+// side by side (Layout). Whole blocks of either, in host memory, from one
+// order to the other: n values of `item` bytes per variable and block, `group`
+// variables side by side on the device.
+void reorder_blocks(const unsigned char* src, unsigned char* dst, size_t nblocks, size_t n, int item, int group, bool to_file) {
+    const size_t block = n * NV * (size_t)item;
+#pragma omp parallel for schedule(static)
+    for (long b = 0; b < (long)nblocks; ++b)
+        for (int v = 0; v < NV; ++v)
+            for (size_t c = 0; c < n; ++c) {
+                const size_t file = (size_t)b * block + ((size_t)v * n + c) * item;
+                const size_t dev = (size_t)b * block + (((size_t)(v / group) * n + c) * group + v % group) * item;
+                std::memcpy(dst + (to_file ? file : dev), src + (to_file ? dev : file), (size_t)item);
+            }
+}
+// The restart file's arrays: device pointer, bytes, and for the mixed state and
+// correction the values per variable and block (0: stored as on the device)
+struct RestartPart {
+    void* dev;
+    uint64_t bytes;
+    size_t n;
+    int item, group;
+    size_t chunk() const {   // whole blocks, about kIoChunk
+        const size_t block = n * NV * (size_t)item;
+        return n ? std::max<size_t>(1, kIoChunk / block) * block : kIoChunk;
+    }
+};
+std::array<RestartPart, 3> restart_parts(falcon_ctx* ctx, const RestartHeader& h) {
+    const bool m = ctx->mixed();
+    const size_t nint = (size_t)ctx->dims.ni * ctx->dims.nj * ctx->dims.nk;
+    return {RestartPart{ctx->U, h.bytes_state, m ? (size_t)ctx->dims.ncell : 0, 4, 4},
+            RestartPart{ctx->Ulo, h.bytes_lo, nint, 1, NV}, RestartPart{ctx->P, h.bytes_psi, 0, 0, 0}};
+}
 }  // namespace
 
 int falcon_save_allcells(falcon_ctx* ctx, const char* directory, int32_t step) {
@@ -1606,15 +1645,19 @@ int falcon_save_restart(falcon_ctx* ctx, const char* path) {
     FILE* f = std::fopen(path, "wb");
     if (!f) return ctx->fail(FALCON_ERR_INVALID_ARG, std::string("cannot write ") + path);
     bool ok = std::fwrite(&h, sizeof h, 1, f) == 1;
-    std::vector<unsigned char> buf(kIoChunk);
-    const void* src[3] = {ctx->U, ctx->Ulo, ctx->P};
-    const uint64_t len[3] = {h.bytes_state, h.bytes_lo, h.bytes_psi};
+    std::vector<unsigned char> buf, file;
     cudaError_t e = cudaSuccess;
-    for (int a = 0; a < 3 && ok; ++a)
-        for (uint64_t off = 0; off < len[a] && ok; off += kIoChunk) {
-            const size_t n = (size_t)std::min<uint64_t>(kIoChunk, len[a] - off);
-            e = cudaMemcpy(buf.data(), (const unsigned char*)src[a] + off, n, cudaMemcpyDeviceToHost);
-            ok = e == cudaSuccess && std::fwrite(buf.data(), 1, n, f) == n;
+    for (const RestartPart& p : restart_parts(ctx, h))
+        for (uint64_t off = 0; off < p.bytes && ok; off += p.chunk()) {
+            const size_t n = (size_t)std::min<uint64_t>(p.chunk(), p.bytes - off);
+            buf.resize(n);
+            e = cudaMemcpy(buf.data(), (const unsigned char*)p.dev + off, n, cudaMemcpyDeviceToHost);
+            ok = e == cudaSuccess;
+            if (ok && p.n) {
+                file.resize(n);
+                reorder_blocks(buf.data(), file.data(), n / (p.n * NV * (size_t)p.item), p.n, p.item, p.group, true);
+            }
+            ok = ok && std::fwrite(p.n ? file.data() : buf.data(), 1, n, f) == n;
         }
     ok = (std::fclose(f) == 0) && ok;
     if (e != cudaSuccess) return ctx->cuda_fail(e, "restart");
@@ -1654,16 +1697,20 @@ int falcon_load_restart(falcon_ctx* ctx, const char* path) {
         return ctx->fail(FALCON_ERR_INVALID_ARG, std::string("restart ") + path + ": " + why);
     }
     CK(cudaStreamSynchronize(ctx->st), "restart");
-    std::vector<unsigned char> buf(kIoChunk);
-    void* dst[3] = {ctx->U, ctx->Ulo, ctx->P};
-    const uint64_t len[3] = {h.bytes_state, h.bytes_lo, h.bytes_psi};
+    std::vector<unsigned char> buf, file;
     cudaError_t e = cudaSuccess;
     bool ok = true;
-    for (int a = 0; a < 3 && ok; ++a)
-        for (uint64_t off = 0; off < len[a] && ok; off += kIoChunk) {
-            const size_t n = (size_t)std::min<uint64_t>(kIoChunk, len[a] - off);
+    for (const RestartPart& p : restart_parts(ctx, h))
+        for (uint64_t off = 0; off < p.bytes && ok; off += p.chunk()) {
+            const size_t n = (size_t)std::min<uint64_t>(p.chunk(), p.bytes - off);
+            buf.resize(n);
             ok = std::fread(buf.data(), 1, n, f) == n;
-            if (ok) e = cudaMemcpy((unsigned char*)dst[a] + off, buf.data(), n, cudaMemcpyHostToDevice);
+            if (ok && p.n) {
+                file.swap(buf);
+                buf.resize(n);
+                reorder_blocks(file.data(), buf.data(), n / (p.n * NV * (size_t)p.item), p.n, p.item, p.group, false);
+            }
+            if (ok) e = cudaMemcpy((unsigned char*)p.dev + off, buf.data(), n, cudaMemcpyHostToDevice);
             ok = ok && e == cudaSuccess;
         }
     std::fclose(f);

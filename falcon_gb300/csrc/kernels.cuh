@@ -5,10 +5,19 @@
 //                reference's order, bit-comparable with the CPU oracle;
 //   mhd_mixed.cu (T = float): FP32 state and stencil RHS, p1 assembled in FP64.
 //
-// Data layout in HBM (one state buffer):
-//   u[b][v][kp][jp][ip], ip fastest, padded extents nip=ni+4 etc. This is the
-//   reference's per-block Fortran array primitive(i,j,k,var) laid end to end
-//   (3_6/ModBlock.f90:275-277), so a block uploads/downloads with one memcpy.
+// Data layout in HBM (one state buffer), cells kp, jp, ip with ip fastest, padded
+// extents nip = ni + 4 etc.:
+//   FP64   u[b][v][cell]: the reference's per-block Fortran array
+//          primitive(i,j,k,var) laid end to end (3_6/ModBlock.f90:275-277), so
+//          a block uploads/downloads with one memcpy;
+//   mixed  u[b][half][cell][4]: half 0 holds rho1, vr, vt, vp of a cell side by
+//          side, half 1 br, bt, bp, s1. A cell's four values are one 16-byte
+//          access, and with two ghost cells on either side every piece that a
+//          kernel writes alone -- a row's interior, a pair of radial ghost
+//          cells, a ghost row -- is whole 32-byte sectors (in [v][cell] order a
+//          row of 16 floats starts 8 bytes into a sector: each write of an
+//          interior row touched two sectors in part, and a ghost cell's eight
+//          values lay in eight).
 //
 // Stencil kernels run one CTA per block. The CTA owns an (i,j) interior column
 // per thread (KPAR columns deep in k) and marches in k with a ring of KPAR+4
@@ -22,6 +31,18 @@
 namespace falcon {
 
 enum { V_RHO1 = 0, V_VR = 1, V_VT = 2, V_VP = 3, V_BR = 4, V_BT = 5, V_BP = 6, V_S1 = 7, NV = 8 };
+
+// Element offsets of the state layouts above: variable v's from variable 0's of
+// the same cell, and from a cell to the next.
+template <class T> struct Layout {
+    static constexpr int cell = sizeof(T) == 4 ? 4 : 1;
+    __host__ __device__ static constexpr size_t var(int v, size_t ncell) {
+        return sizeof(T) == 4 ? (size_t)(v >> 2) * 4 * ncell + (size_t)(v & 3) : (size_t)v * ncell;
+    }
+    __host__ __device__ static constexpr size_t at(size_t b, int v, size_t c, size_t ncell) {
+        return b * NV * ncell + var(v, ncell) + c * cell;
+    }
+};
 
 // ---- compensated FP32 state of the mixed path --------------------------------
 // u^n is held as an FP32 value hi plus an 8-bit correction q (a second array
@@ -170,15 +191,13 @@ struct StepDims {
 };
 
 // The u^n correction of the mixed path is stored for interior cells only,
-// [block][var][k][j][i] with the interior extents (1 byte per value, no
-// padding: its rows are whole 16-byte runs for 16^3 blocks). Index of state
-// element e (the state's padded layout), or -1 for a ghost cell.
-__host__ __device__ __forceinline__ int64_t lo_index(int64_t e, const StepDims& d) {
-    const int64_t bv = e / d.ncell;
-    const int c = (int)(e - bv * d.ncell);
+// [block][k][j][i][var] with the interior extents (a byte per value, a cell's
+// eight in one 8-byte access). Index of variable v at padded cell c of block b,
+// or -1 for a ghost cell.
+__host__ __device__ __forceinline__ int64_t lo_index(int64_t b, int v, int c, const StepDims& d) {
     const int ip = c % d.nip, jp = (c / d.nip) % d.njp, kp = c / (d.nip * d.njp);
     if (ip < 2 || ip >= d.nip - 2 || jp < 2 || jp >= d.njp - 2 || kp < 2 || kp >= d.nkp - 2) return -1;
-    return ((bv * d.nk + (kp - 2)) * d.nj + (jp - 2)) * d.ni + (ip - 2);
+    return (((b * d.nk + (kp - 2)) * d.nj + (jp - 2)) * d.ni + (ip - 2)) * NV + v;
 }
 inline size_t lo_elems(const StepDims& d) { return (size_t)d.nblocks * NV * d.ni * d.nj * d.nk; }
 
@@ -201,13 +220,12 @@ struct DivBArgs {
 // (3_6/ModAdvance.f90:101-108)
 cudaError_t launch_stage_fp64(const StepDims& d, const Geometry& g, const double* in, const double* un,
                               double* out, const DivBArgs& psi, int stage, int bc_writeback, StepScalars* sc,
-                              int heat_on, int kpar, cudaStream_t st);
+                              int kpar, cudaStream_t st);
 // GLM: psi's artificial diffusion (into psi_out) and psi's ghost fill
 cudaError_t launch_psi_diffusion_fp64(const StepDims& d, const Geometry& g, const double* u, const double* psi,
                                       double* psi_out, StepScalars* sc, cudaStream_t st);
 cudaError_t launch_psi_ghost_fp64(const StepDims& d, const GhostLists& gl, double* psi, cudaStream_t st);
-cudaError_t launch_diffusion_fp64(const StepDims& d, const Geometry& g, double* u, StepScalars* sc,
-                                  int kpar, cudaStream_t st);
+cudaError_t launch_diffusion_fp64(const StepDims& d, const Geometry& g, double* u, StepScalars* sc, cudaStream_t st);
 cudaError_t launch_cfl_fp64(const StepDims& d, const Geometry& g, const double* u, StepScalars* sc,
                             cudaStream_t st);
 cudaError_t launch_ghost_fp64(const StepDims& d, const GhostLists& gl, double* u, cudaStream_t st);
@@ -223,7 +241,7 @@ cudaError_t launch_shard_unpack_fp64(const StepDims& d, const int32_t* dst, int6
 // pushing needs out != in, since a target block may still be reading `in`.
 cudaError_t launch_stage_mixed(const StepDims& d, const Geometry& g, const float* in, const float* un,
                                float* out, int8_t* lo, const PushTable& push, const DivBArgs& psi, int stage,
-                               int bc_writeback, StepScalars* sc, int heat_on, int kpar, cudaStream_t st);
+                               int bc_writeback, StepScalars* sc, int kpar, cudaStream_t st);
 cudaError_t launch_psi_diffusion_mixed(const StepDims& d, const Geometry& g, const float* u, const float* psi,
                                        float* psi_out, StepScalars* sc, cudaStream_t st);
 cudaError_t launch_psi_ghost_mixed(const StepDims& d, const GhostLists& gl, float* psi, cudaStream_t st);

@@ -4,15 +4,62 @@
 #include "launch_impl.cuh"
 
 namespace falcon {
-using impl::stage_any;
-using impl::diff_any;
 using impl::cfl_any;
 using impl::ghost_any;
 
+namespace impl {
+namespace {
+// k-chunk depths (KPAR) instantiated per block size; the context's autotuner
+// times them on its own grid and keeps the fastest.
+template <int N, int KP, int DIVB>
+cudaError_t stage_nd(const StepDims& d, const Geometry& g, const double* in, const double* un, double* out,
+                     const DivBArgs& psi, int stage, int bcw, StepScalars* sc, cudaStream_t st) {
+    using S = Shape<double, N, N, N, KP>;
+    static const cudaError_t attr = allow_smem(k_stage<N, N, N, KP, DIVB>, S::smem_stage);
+    if (attr != cudaSuccess) return attr;
+    k_stage<N, N, N, KP, DIVB><<<d.nblocks, S::NT, S::smem_stage, st>>>(in, un, out, psi, g, sc, stage, bcw);
+    return cudaGetLastError();
+}
+// The div-B mode is a template parameter: the plain stage keeps its register
+// allocation free of the GLM/Powell terms.
+template <int N, int KP>
+cudaError_t stage_n(const StepDims& d, const Geometry& g, const double* in, const double* un, double* out,
+                    const DivBArgs& psi, int stage, int bcw, StepScalars* sc, cudaStream_t st) {
+    switch (psi.mode) {
+    case 0: return stage_nd<N, KP, 0>(d, g, in, un, out, psi, stage, bcw, sc, st);
+    case 1:
+        if (!psi.in || !psi.un || !psi.out) return cudaErrorInvalidValue;
+        return stage_nd<N, KP, 1>(d, g, in, un, out, psi, stage, bcw, sc, st);
+    case 2: return stage_nd<N, KP, 2>(d, g, in, un, out, psi, stage, bcw, sc, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+// the k march, in place
+template <int N, int VPT>
+cudaError_t diff_march64(const StepDims& d, const Geometry& g, double* u, StepScalars* sc, cudaStream_t st) {
+    using S = M64Shape<N, N, N, VPT>;
+    static const cudaError_t attr = allow_smem(k_diffusion_march64<N, N, N, VPT>, S::smem);
+    if (attr != cudaSuccess) return attr;
+    k_diffusion_march64<N, N, N, VPT><<<d.nblocks, S::NT, S::smem, st>>>(u, g, sc);
+    return cudaGetLastError();
+}
+}  // namespace
+}  // namespace impl
+
 cudaError_t launch_stage_fp64(const StepDims& d, const Geometry& g, const double* in, const double* un, double* out,
-                              const DivBArgs& psi, int stage, int bcw, StepScalars* sc, int heat, int kpar,
-                              cudaStream_t st) {
-    return stage_any<double>(d, g, in, un, out, nullptr, PushTable{}, psi, stage, bcw, sc, heat, kpar, st);
+                              const DivBArgs& psi, int stage, int bcw, StepScalars* sc, int kpar, cudaStream_t st) {
+    if (d.ni != d.nj || d.ni != d.nk) return cudaErrorInvalidValue;
+    if (d.ni == 8 && kpar == 2) return impl::stage_n<8, 2>(d, g, in, un, out, psi, stage, bcw, sc, st);
+    if (d.ni == 8 && kpar == 4) return impl::stage_n<8, 4>(d, g, in, un, out, psi, stage, bcw, sc, st);
+    if (d.ni == 16 && kpar == 1) return impl::stage_n<16, 1>(d, g, in, un, out, psi, stage, bcw, sc, st);
+    return cudaErrorInvalidValue;
+}
+// (any k-chunk depth asked for: the march has one form)
+cudaError_t launch_diffusion_fp64(const StepDims& d, const Geometry& g, double* u, StepScalars* sc, cudaStream_t st) {
+    if (d.ni != d.nj || d.ni != d.nk) return cudaErrorInvalidValue;
+    if (d.ni == 8) return impl::diff_march64<8, 1>(d, g, u, sc, st);
+    if (d.ni == 16) return impl::diff_march64<16, 4>(d, g, u, sc, st);
+    return cudaErrorInvalidValue;
 }
 cudaError_t launch_psi_diffusion_fp64(const StepDims& d, const Geometry& g, const double* u, const double* psi,
                                       double* psi_out, StepScalars* sc, cudaStream_t st) {
@@ -20,10 +67,6 @@ cudaError_t launch_psi_diffusion_fp64(const StepDims& d, const Geometry& g, cons
 }
 cudaError_t launch_psi_ghost_fp64(const StepDims& d, const GhostLists& gl, double* psi, cudaStream_t st) {
     return impl::psi_ghost_any<double>(d, gl, psi, st);
-}
-cudaError_t launch_diffusion_fp64(const StepDims& d, const Geometry& g, double* u, StepScalars* sc,
-                                  int kpar, cudaStream_t st) {
-    return diff_any<double>(d, g, u, u, nullptr, PushTable{}, sc, kpar, st);
 }
 cudaError_t launch_cfl_fp64(const StepDims& d, const Geometry& g, const double* u, StepScalars* sc, cudaStream_t st) {
     return cfl_any<double>(d, g, u, sc, st);
@@ -53,25 +96,28 @@ cudaError_t launch_finalize_dt(StepScalars* sc, cudaStream_t st) {
 }
 
 // Host block arrays carry FALCON_NVAR = 9 variables ([b][9][cell], psi last);
-// the device state carries the 8 evolved ones ([b][8][cell]) and, with GLM,
-// psi in an array of its own ([b][cell]).
-__device__ __forceinline__ int64_t host_index(int64_t x, int64_t ncell) {   // device state element -> host element
+// the device state the 8 evolved ones (see Layout) and, with GLM, psi in an
+// array of its own ([b][cell]). x counts (block, variable, cell) with the cell fastest.
+__device__ __forceinline__ int64_t host_index(int64_t x, int64_t ncell) {   // -> host element
     const int64_t b = x / (NV * ncell);
     return x + b * ncell;
 }
 
 // FP64 host array -> compensated FP32 state: hi = RN(u); interior cells get
 // the correction of u - hi, ghost cells q = 0
-__global__ void k_narrow(const double* s, float* d, int8_t* lo, int64_t n, StepDims dm) {
-    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
-        const double u = s[host_index(x, dm.ncell)];
-        const float hi = (float)u;
-        d[x] = hi;
-        if (lo) {
-            const int64_t q = lo_index(x, dm);
-            if (q >= 0) lo[q] = lo_encode64(hi, u - (double)hi);
-        }
+__device__ __forceinline__ void narrow_one(double u, int64_t x, float* d, int8_t* lo, const StepDims& dm) {
+    const float hi = (float)u;
+    const int64_t bv = x / dm.ncell, b = bv / NV;
+    const int v = (int)(bv - b * NV), c = (int)(x - bv * dm.ncell);
+    d[Layout<float>::at((size_t)b, v, (size_t)c, (size_t)dm.ncell)] = hi;
+    if (lo) {
+        const int64_t q = lo_index(b, v, c, dm);
+        if (q >= 0) lo[q] = lo_encode64(hi, u - (double)hi);
     }
+}
+__global__ void k_narrow(const double* s, float* d, int8_t* lo, int64_t n, StepDims dm) {
+    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x)
+        narrow_one(s[host_index(x, dm.ncell)], x, d, lo, dm);
 }
 // psi plane of the host array -> FP32 psi array (mixed GLM)
 __global__ void k_narrow_psi(const double* s, float* psi, int64_t nb, int64_t ncell) {
@@ -90,29 +136,6 @@ __global__ void k_psi_nonzero(const double* s, int64_t nb, int64_t ncell, int32_
     }
     if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) *flag = 1;
 }
-// host elements [first, first + count) as FP64 from the device state (FP32
-// with its correction, or FP64) and psi (nullptr: psi = 0)
-template <class T>
-__global__ void k_gather_host(const T* U, const int8_t* lo, const T* psi, StepDims dm, int64_t first, int64_t count,
-                              int64_t ncell, double* out) {
-    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < count; x += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t h = first + x;
-        const int64_t b = h / ((NV + 1) * ncell), r = h - b * (NV + 1) * ncell;
-        double v;
-        if (r < NV * ncell) {
-            const int64_t e = b * NV * ncell + r;
-            const T hi = U[e];
-            v = (double)hi;
-            if constexpr (sizeof(T) == 4) {
-                const int64_t q = lo ? lo_index(e, dm) : -1;
-                if (q >= 0) v += (double)lo[q] * (double)lo_unit((float)hi);
-            }
-        } else {
-            v = psi ? (double)psi[b * ncell + (r - NV * ncell)] : 0.0;
-        }
-        out[x] = v;
-    }
-}
 // Wide forms of the transfer kernels: each thread moves kWide elements per
 // pass as kWide/2 16-byte accesses, all issued before any is used (a warp's
 // access q covers 512 contiguous bytes), so that many bytes are in flight when
@@ -120,14 +143,6 @@ __global__ void k_gather_host(const T* U, const int8_t* lo, const T* psi, StepDi
 // arrays, an even cell count and even ranges (pairs never straddle a
 // variable); the launchers fall back to the one-element kernels otherwise.
 constexpr int kWide = 8;
-__device__ __forceinline__ void narrow_one(double u, int64_t x, float* d, int8_t* lo, const StepDims& dm) {
-    const float hi = (float)u;
-    d[x] = hi;
-    if (lo) {
-        const int64_t q = lo_index(x, dm);
-        if (q >= 0) lo[q] = lo_encode64(hi, u - (double)hi);
-    }
-}
 __global__ void k_narrow_wide(const double* s, float* d, int8_t* lo, int64_t n, StepDims dm) {
     const int64_t lane2 = 2 * (threadIdx.x & 31);
     for (int64_t w0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32 * kWide; w0 < n;
@@ -181,21 +196,29 @@ __global__ void k_psi_nonzero_wide(const double* s, int64_t nb, int64_t ncell, i
     }
     if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) *flag = 1;
 }
+// host element h as FP64 from the device state (FP32 with its correction, or
+// FP64) and psi (nullptr: psi = 0)
 template <class T>
 __device__ __forceinline__ double gather_one(const T* U, const int8_t* lo, const T* psi, int64_t h, int64_t ncell,
                                              const StepDims& dm) {
     const int64_t b = h / ((NV + 1) * ncell), r = h - b * (NV + 1) * ncell;
     if (r < NV * ncell) {
-        const int64_t e = b * NV * ncell + r;
-        const T hi = U[e];
-        double v = (double)hi;
+        const int v = (int)(r / ncell), c = (int)(r - v * ncell);
+        const T hi = U[Layout<T>::at((size_t)b, v, (size_t)c, (size_t)ncell)];
+        double x = (double)hi;
         if constexpr (sizeof(T) == 4) {
-            const int64_t q = lo ? lo_index(e, dm) : -1;
-            if (q >= 0) v += (double)lo[q] * (double)lo_unit((float)hi);
+            const int64_t q = lo ? lo_index(b, v, c, dm) : -1;
+            if (q >= 0) x += (double)lo[q] * (double)lo_unit((float)hi);
         }
-        return v;
+        return x;
     }
     return psi ? (double)psi[b * ncell + (r - NV * ncell)] : 0.0;
+}
+template <class T>
+__global__ void k_gather_host(const T* U, const int8_t* lo, const T* psi, StepDims dm, int64_t first, int64_t count,
+                              int64_t ncell, double* out) {
+    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < count; x += (int64_t)gridDim.x * blockDim.x)
+        out[x] = gather_one(U, lo, psi, first + x, ncell, dm);
 }
 template <class T>
 __global__ void k_gather_host_wide(const T* U, const int8_t* lo, const T* psi, StepDims dm, int64_t first,
@@ -221,72 +244,93 @@ bool wide_ok(const void* p, int64_t ncell) { return ((uintptr_t)p % 16) == 0 && 
 // psi last), the interior planes and within them the interior rows, each
 // row whole (its radial ghost columns, which hold the radial boundary
 // condition, included). The interior rows of one plane are one contiguous
-// run of (NJP-4)*NIP host elements: a warp moves one run at a time, block,
-// variable and plane from the run number, the cell from the offset in the
-// run, so no element pays a 64-bit division; each lane's 16-byte host
-// accesses of a pass (kRunVec, a whole 16^3 run of 320 elements) are issued
-// before any is used. Offsets are even and NIP is even, so a pair (ip, ip+1)
-// is either two radial ghost columns or two interior cells, and its device
-// side is one 8-byte (FP32) or 16-byte (FP64) access and one 2-byte access
-// of the correction.
-constexpr int kRunVec = 5;
-struct CoreRun {
-    int64_t host;   // host element of the run's first cell
-    int64_t dev;    // state element of that cell ((b NV + v) ncell + cell0), v < NV
-    int64_t psi;    // psi element of that cell (b ncell + cell0)
-    int64_t lo0;    // correction element of the run's first interior row
-    int v;          // 0..NV-1 state, NV psi
+// run of (NJP-4)*NIP host elements. A warp takes the runs of one plane of one
+// group of a block's variables at a time -- four that the mixed state holds side
+// by side (FP64: one), or psi -- so no element pays a 64-bit division and the
+// mixed state's side is whole 16-byte cells; each lane's 16-byte host accesses of
+// a pass (two cells of every variable, kPass passes) are issued before any is
+// used. Offsets are even and NIP is even, so a pair (ip, ip+1) is either two
+// radial ghost columns or two interior cells.
+template <class T> struct CoreRun {
+    static constexpr int G = sizeof(T) == 4 ? 4 : 1;    // variables of a group
+    static constexpr int NG = NV / G + 1;               // groups, psi last
+    static constexpr int kPass = sizeof(T) == 4 ? 2 : 5;
+    int64_t b, cell0;   // block, padded cell of the run's first element
+    int g;
+    int kp;
+    __device__ CoreRun(int64_t r, const StepDims& dm) {
+        const int nkc = dm.nkp - 4;
+        const int64_t bg = r / nkc;
+        b = bg / NG;
+        g = (int)(bg - b * NG);
+        kp = 2 + (int)(r - bg * nkc);
+        cell0 = (int64_t)kp * dm.nip * dm.njp + 2 * dm.nip;
+    }
+    __device__ bool psi() const { return g == NG - 1; }
+    __device__ int vars() const { return psi() ? 1 : G; }
+    // host element of variable q of the group at offset o of the run
+    __device__ int64_t host(int q, int o, const StepDims& dm) const { return (b * (NV + 1) + g * G + q) * dm.ncell + cell0 + o; }
+    // correction of the cells at offset o (mixed): interior cells of the plane's interior rows
+    __device__ int64_t lo(int o, const StepDims& dm) const {
+        const int jr = o / dm.nip;
+        return (((b * dm.nk + (kp - 2)) * dm.nj + jr) * dm.ni + (o - jr * dm.nip - 2)) * NV + g * G;
+    }
+    __device__ bool interior(int o, const StepDims& dm) const {
+        const int ip = o % dm.nip;
+        return ip >= 2 && ip < dm.nip - 2;
+    }
 };
-__device__ __forceinline__ CoreRun core_run(int64_t r, const StepDims& dm) {
-    const int nkc = dm.nkp - 4;
-    const int64_t bv = r / nkc, b = bv / (NV + 1);
-    const int kp = 2 + (int)(r - bv * nkc);
-    const int64_t cell0 = (int64_t)kp * dm.nip * dm.njp + 2 * dm.nip;
-    CoreRun c;
-    c.v = (int)(bv - b * (NV + 1));
-    c.host = bv * dm.ncell + cell0;
-    c.dev = (b * NV + c.v) * dm.ncell + cell0;
-    c.psi = b * dm.ncell + cell0;
-    c.lo0 = ((b * NV + c.v) * dm.nk + (kp - 2)) * (int64_t)dm.nj * dm.ni;
-    return c;
-}
 // host core -> device: state cells narrowed (FP32 with its correction) or
 // copied (FP64); psi converted into P, or, without P, tested for 0 (flag)
 template <class T>
 __global__ void k_core_up(const double* s, T* U, int8_t* lo, T* P, int32_t* flag, int64_t nruns, StepDims dm) {
+    using R = CoreRun<T>;
     const int lane2 = 2 * (threadIdx.x & 31), len = (dm.njp - 4) * dm.nip;
     int any = 0;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nruns;
          r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        const CoreRun c = core_run(r, dm);
-        for (int o0 = 0; o0 < len; o0 += 64 * kRunVec) {
-            double2 v[kRunVec];
+        const R c(r, dm);
+        const int nv = c.vars();
+        for (int o0 = 0; o0 < len; o0 += 64 * R::kPass) {
+            double2 v[R::kPass][R::G];
 #pragma unroll
-            for (int q = 0; q < kRunVec; ++q)
-                if (o0 + 64 * q + lane2 < len) v[q] = *reinterpret_cast<const double2*>(s + c.host + o0 + 64 * q + lane2);
+            for (int q = 0; q < R::kPass; ++q)
 #pragma unroll
-            for (int q = 0; q < kRunVec; ++q) {
+                for (int g = 0; g < R::G; ++g)
+                    if (o0 + 64 * q + lane2 < len && g < nv)
+                        v[q][g] = *reinterpret_cast<const double2*>(s + c.host(g, o0 + 64 * q + lane2, dm));
+#pragma unroll
+            for (int q = 0; q < R::kPass; ++q) {
                 const int o = o0 + 64 * q + lane2;
                 if (o >= len) continue;
-                if (c.v < NV) {
-                    if constexpr (sizeof(T) == 4) {
-                        const float h0 = (float)v[q].x, h1 = (float)v[q].y;
-                        *reinterpret_cast<float2*>(U + c.dev + o) = make_float2(h0, h1);
-                        const int jr = o / dm.nip, ip = o - jr * dm.nip;
-                        if (lo && ip >= 2 && ip < dm.nip - 2) {
-                            char2 q2;
-                            q2.x = lo_encode64(h0, v[q].x - (double)h0);
-                            q2.y = lo_encode64(h1, v[q].y - (double)h1);
-                            *reinterpret_cast<char2*>(lo + c.lo0 + jr * dm.ni + (ip - 2)) = q2;
-                        }
+                const int64_t pc = c.b * dm.ncell + c.cell0 + o;   // the cells in a [b][cell] array
+                if (c.psi()) {
+                    if (!P) {
+                        any |= (v[q][0].x != 0.0) | (v[q][0].y != 0.0);
+                    } else if constexpr (sizeof(T) == 4) {
+                        *reinterpret_cast<float2*>(P + pc) = make_float2((float)v[q][0].x, (float)v[q][0].y);
                     } else {
-                        *reinterpret_cast<double2*>(U + c.dev + o) = v[q];
+                        *reinterpret_cast<double2*>(P + pc) = v[q][0];
                     }
-                } else if (P) {
-                    if constexpr (sizeof(T) == 4) *reinterpret_cast<float2*>(P + c.psi + o) = make_float2((float)v[q].x, (float)v[q].y);
-                    else *reinterpret_cast<double2*>(P + c.psi + o) = v[q];
+                    continue;
+                }
+                if constexpr (sizeof(T) == 4) {
+                    float4* out = reinterpret_cast<float4*>(U) + (c.b * 2 + c.g) * dm.ncell + c.cell0 + o;
+                    const float4 a = make_float4((float)v[q][0].x, (float)v[q][1].x, (float)v[q][2].x, (float)v[q][3].x);
+                    const float4 e = make_float4((float)v[q][0].y, (float)v[q][1].y, (float)v[q][2].y, (float)v[q][3].y);
+                    out[0] = a;
+                    out[1] = e;
+                    if (lo && c.interior(o, dm)) {
+                        int8_t* l = lo + c.lo(o, dm);
+                        *reinterpret_cast<char4*>(l) =
+                            make_char4(lo_encode64(a.x, v[q][0].x - (double)a.x), lo_encode64(a.y, v[q][1].x - (double)a.y),
+                                       lo_encode64(a.z, v[q][2].x - (double)a.z), lo_encode64(a.w, v[q][3].x - (double)a.w));
+                        *reinterpret_cast<char4*>(l + NV) =
+                            make_char4(lo_encode64(e.x, v[q][0].y - (double)e.x), lo_encode64(e.y, v[q][1].y - (double)e.y),
+                                       lo_encode64(e.z, v[q][2].y - (double)e.z), lo_encode64(e.w, v[q][3].y - (double)e.w));
+                    }
                 } else {
-                    any |= (v[q].x != 0.0) | (v[q].y != 0.0);
+                    *reinterpret_cast<double2*>(U + Layout<T>::at((size_t)c.b, c.g, (size_t)(c.cell0 + o), (size_t)dm.ncell)) = v[q][0];
                 }
             }
         }
@@ -296,47 +340,58 @@ __global__ void k_core_up(const double* s, T* U, int8_t* lo, T* P, int32_t* flag
 // device -> host core (psi 0 without P)
 template <class T>
 __global__ void k_core_down(const T* U, const int8_t* lo, const T* P, double* out, int64_t nruns, StepDims dm) {
+    using R = CoreRun<T>;
     const int lane2 = 2 * (threadIdx.x & 31), len = (dm.njp - 4) * dm.nip;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nruns;
          r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        const CoreRun c = core_run(r, dm);
-        for (int o0 = 0; o0 < len; o0 += 64 * kRunVec) {
-            double2 v[kRunVec];
+        const R c(r, dm);
+        const int nv = c.vars();
+        for (int o0 = 0; o0 < len; o0 += 64 * R::kPass) {
+            double2 v[R::kPass][R::G];
 #pragma unroll
-            for (int q = 0; q < kRunVec; ++q) {
+            for (int q = 0; q < R::kPass; ++q) {
                 const int o = o0 + 64 * q + lane2;
                 if (o >= len) continue;
-                if (c.v < NV) {
-                    if constexpr (sizeof(T) == 4) {
-                        const float2 h = *reinterpret_cast<const float2*>(U + c.dev + o);
-                        v[q] = make_double2((double)h.x, (double)h.y);
-                        const int jr = o / dm.nip, ip = o - jr * dm.nip;
-                        if (lo && ip >= 2 && ip < dm.nip - 2) {
-                            const char2 q2 = *reinterpret_cast<const char2*>(lo + c.lo0 + jr * dm.ni + (ip - 2));
-                            v[q].x += (double)q2.x * (double)lo_unit(h.x);
-                            v[q].y += (double)q2.y * (double)lo_unit(h.y);
-                        }
-                    } else {
-                        v[q] = *reinterpret_cast<const double2*>(U + c.dev + o);
+                const int64_t pc = c.b * dm.ncell + c.cell0 + o;
+                if (c.psi()) {
+                    v[q][0] = make_double2(0.0, 0.0);
+                    if (P) v[q][0] = make_double2((double)P[pc], (double)P[pc + 1]);
+                    continue;
+                }
+                if constexpr (sizeof(T) == 4) {
+                    const float4* in = reinterpret_cast<const float4*>(U) + (c.b * 2 + c.g) * dm.ncell + c.cell0 + o;
+                    const float4 a = in[0], e = in[1];
+                    const float h0[4] = {a.x, a.y, a.z, a.w}, h1[4] = {e.x, e.y, e.z, e.w};
+                    char4 l0 = make_char4(0, 0, 0, 0), l1 = l0;
+                    const bool add = lo && c.interior(o, dm);
+                    if (add) {
+                        const int8_t* l = lo + c.lo(o, dm);
+                        l0 = *reinterpret_cast<const char4*>(l);
+                        l1 = *reinterpret_cast<const char4*>(l + NV);
                     }
-                } else if (P) {
-                    if constexpr (sizeof(T) == 4) {
-                        const float2 h = *reinterpret_cast<const float2*>(P + c.psi + o);
-                        v[q] = make_double2((double)h.x, (double)h.y);
-                    } else {
-                        v[q] = *reinterpret_cast<const double2*>(P + c.psi + o);
+                    const int8_t q0[4] = {l0.x, l0.y, l0.z, l0.w}, q1[4] = {l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+                    for (int g = 0; g < R::G; ++g) {
+                        v[q][g] = make_double2((double)h0[g], (double)h1[g]);
+                        if (add) {
+                            v[q][g].x += (double)q0[g] * (double)lo_unit(h0[g]);
+                            v[q][g].y += (double)q1[g] * (double)lo_unit(h1[g]);
+                        }
                     }
                 } else {
-                    v[q] = make_double2(0.0, 0.0);
+                    v[q][0] = *reinterpret_cast<const double2*>(U + Layout<T>::at((size_t)c.b, c.g, (size_t)(c.cell0 + o), (size_t)dm.ncell));
                 }
             }
 #pragma unroll
-            for (int q = 0; q < kRunVec; ++q)
-                if (o0 + 64 * q + lane2 < len) *reinterpret_cast<double2*>(out + c.host + o0 + 64 * q + lane2) = v[q];
+            for (int q = 0; q < R::kPass; ++q)
+#pragma unroll
+                for (int g = 0; g < R::G; ++g)
+                    if (o0 + 64 * q + lane2 < len && g < nv)
+                        *reinterpret_cast<double2*>(out + c.host(g, o0 + 64 * q + lane2, dm)) = v[q][g];
         }
     }
 }
-int64_t core_runs(const StepDims& dm) { return (int64_t)dm.nblocks * (NV + 1) * (dm.nkp - 4); }
+template <class T> int64_t core_runs(const StepDims& dm) { return (int64_t)dm.nblocks * CoreRun<T>::NG * (dm.nkp - 4); }
 bool core_ok(const void* host, const StepDims& dm) {
     return ((uintptr_t)host % 16) == 0 && dm.ncell % 2 == 0 && dm.nip % 2 == 0;
 }
@@ -381,24 +436,26 @@ cudaError_t launch_gather_host(const void* U, const int8_t* lo, const void* psi,
 cudaError_t launch_core_up(const double* host, void* U, int8_t* lo, void* P, int32_t* flag, bool fp32, const StepDims& dm,
                            cudaStream_t st) {
     if (!core_ok(host, dm)) return cudaErrorInvalidValue;
-    const int64_t n = core_runs(dm);
     if (flag) {
         cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int32_t), st);
         if (e != cudaSuccess) return e;
     }
-    if (fp32) k_core_up<float><<<1216, 256, 0, st>>>(host, (float*)U, lo, (float*)P, flag, n, dm);
-    else k_core_up<double><<<1216, 256, 0, st>>>(host, (double*)U, nullptr, (double*)P, flag, n, dm);
+    if (fp32) k_core_up<float><<<1216, 256, 0, st>>>(host, (float*)U, lo, (float*)P, flag, core_runs<float>(dm), dm);
+    else k_core_up<double><<<1216, 256, 0, st>>>(host, (double*)U, nullptr, (double*)P, flag, core_runs<double>(dm), dm);
     return cudaGetLastError();
 }
 cudaError_t launch_core_down(const void* U, const int8_t* lo, const void* P, bool fp32, double* host, const StepDims& dm,
                              cudaStream_t st) {
     if (!core_ok(host, dm)) return cudaErrorInvalidValue;
-    const int64_t n = core_runs(dm);
-    if (fp32) k_core_down<float><<<1216, 256, 0, st>>>((const float*)U, lo, (const float*)P, host, n, dm);
-    else k_core_down<double><<<1216, 256, 0, st>>>((const double*)U, nullptr, (const double*)P, host, n, dm);
+    if (fp32) k_core_down<float><<<1216, 256, 0, st>>>((const float*)U, lo, (const float*)P, host, core_runs<float>(dm), dm);
+    else k_core_down<double><<<1216, 256, 0, st>>>((const double*)U, nullptr, (const double*)P, host, core_runs<double>(dm), dm);
     return cudaGetLastError();
 }
 
-int kpar_candidates_fp64(const StepDims& d, int* out) { return impl::candidates<double>(d, out); }
+int kpar_candidates_fp64(const StepDims& d, int* out) {
+    if (d.ni == 16) { out[0] = 1; return 1; }
+    if (d.ni == 8) { out[0] = 2; out[1] = 4; return 2; }
+    return 0;
+}
 
 }  // namespace falcon

@@ -410,14 +410,6 @@ __device__ __forceinline__ void apply_bc(T* tile, int lo, int hi, int fl, T* wb)
 __device__ __forceinline__ float blend(float a, float b, float uw, float w) { return __fmaf_rn(a, uw, __fmul_rn(b, w)); }
 __device__ __forceinline__ double blend(double a, double b, double uw, double w) { return a * uw + b * w; }
 
-// Write this cell's new values into the ghost cells of the neighbours whose
-// faces are pushed (PushTable). (ii, jj, kp): padded indices of the cell; o:
-// its 8 new values. Theta/phi faces: the two interior layers next to the side
-// are copied to the target's opposite ghost layers (a shift of one block
-// extent). Radial faces: the thread at the first source cell of a ghost layer
-// blends it with the next cell along i, taken from the next lane (i is the
-// fastest thread index, and the second cell is never beyond the row). Every
-// thread of the CTA calls this (the shuffle needs the full warp).
 // The push-table entries of one block, staged in shared memory before the
 // kernel's first barrier: they are read at the end of every k-chunk, and as
 // global loads their latency held every warp at the chunk's end.
@@ -437,74 +429,6 @@ __device__ __forceinline__ void load_push_block(const PushTable& P, int b, PushB
         s->dst[q] = P.rad_dst[4 * b + q];
         s->w[q] = P.rad_w[4 * b + q];
     }
-}
-
-template <class T, class S, int VN>
-__device__ __forceinline__ void push_faces_part(T* out, const PushBlock& P, int ii, int jj, int kp,
-                                                const T (&o)[VN], int v0) {
-    constexpr int NJ = S::NJP - 4, NK = S::NKP - 4;
-    const int32_t* tg = P.tgt;
-    auto put = [&](int tb, int kt, int jt, int it, const T (&val)[VN]) {
-        T* dst = out + ((size_t)tb * NV + v0) * S::NCELL + ((size_t)kt * S::NJP + jt) * S::NIP + it;
-#pragma unroll
-        for (int v = 0; v < VN; ++v) dst[(size_t)v * S::NCELL] = val[v];
-    };
-    if (jj <= 3 && tg[2] >= 0) put(tg[2], kp, jj + NJ, ii, o);
-    if (jj >= NJ && tg[3] >= 0) put(tg[3], kp, jj - NJ, ii, o);
-    if (kp <= 3 && tg[4] >= 0) put(tg[4], kp + NK, jj, ii, o);
-    if (kp >= NK && tg[5] >= 0) put(tg[5], kp - NK, jj, ii, o);
-    if (tg[0] >= 0 || tg[1] >= 0) {   // uniform over the CTA
-        if constexpr (S::NIP == 20 && 2 * VN <= 16) {
-            // 16-wide rows: every half-warp holds one full row (i = lane % 16).
-            // Lane (v, layer) = (lh / 2, lh % 2) of the half gathers its value
-            // from the row's source lanes, so a side takes one store per row
-            // instead of a divergent store per variable and layer.
-            const int lane = threadIdx.x & 31, lh = lane & 15, hb = lane & 16;
-            const int v = lh >> 1, layer = lh & 1;
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                if (tg[side] < 0) continue;
-                const int q = side * 2 + layer;
-                const int s0 = hb + P.src[q] - 2;
-                const bool two = P.w[side * 2] != 0.f || P.w[side * 2 + 1] != 0.f;   // uniform
-                T a = T(0), c = T(0);
-#pragma unroll
-                for (int u = 0; u < VN; ++u) {
-                    const T x0 = __shfl_sync(0xffffffffu, o[u], s0);
-                    T x1 = T(0);
-                    if (two) x1 = __shfl_sync(0xffffffffu, o[u], s0 + 1);
-                    if (u == v) { a = x0; c = x1; }
-                }
-                if (v < VN) {
-                    const T w = (T)P.w[q];
-                    const T val = w == T(0) ? a : blend(a, c, T(1) - w, w);
-                    out[((size_t)tg[side] * NV + v0 + v) * S::NCELL + ((size_t)kp * S::NJP + jj) * S::NIP + P.dst[q]] = val;
-                }
-            }
-            return;
-        }
-        T nx[VN];
-#pragma unroll
-        for (int v = 0; v < VN; ++v) nx[v] = __shfl_down_sync(0xffffffffu, o[v], 1);
-#pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            if (tg[side] < 0) continue;
-#pragma unroll
-            for (int layer = 0; layer < 2; ++layer) {
-                const int q = side * 2 + layer;
-                if (ii != P.src[q]) continue;
-                const T w = (T)P.w[q], uw = T(1) - w;
-                T val[VN];
-#pragma unroll
-                for (int v = 0; v < VN; ++v) val[v] = w == T(0) ? o[v] : blend(o[v], nx[v], uw, w);
-                put(tg[side], kp, jj, P.dst[q], val);
-            }
-        }
-    }
-}
-template <class T, class S>
-__device__ __forceinline__ void push_faces(T* out, const PushBlock& P, int ii, int jj, int kp, const T (&o)[NV]) {
-    push_faces_part<T, S, NV>(out, P, ii, jj, kp, o, 0);
 }
 
 // Cell (i, j, kq) of a thread in a k-chunk. With 16-wide rows and an even
@@ -576,13 +500,14 @@ __device__ __forceinline__ float2 ff_add2(float2 hi, int8_t q0, int8_t q1, float
 // ---------------------------------------------------------------------------
 // One RK stage of one block: boundary -> RHS (3_6/ModEquation.f90:24-162) ->
 // u_out = u^n + dt*R/(5-s) (3_6/ModAdvance.f90:87-93).
-// The body runs block b with the CTA's threads (NI*NJ*KPAR of them): k_stage
-// calls it for blockIdx.x, the persistent step for each block it takes.
-template <class T, int NI, int NJ, int NK, int KPAR, int DIVB>
-__device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* out, int8_t* ulo, PushTable push,
-                                           DivBArgs psi, Geometry g, StepScalars* sc, int stage, int bc_writeback,
-                                           int heat_on) {
+// FP64 (the mixed stage: stage_quads).
+template <int NI, int NJ, int NK, int KPAR, int DIVB>
+__global__ void __launch_bounds__(NI* NJ* KPAR)
+k_stage(const double* in, const double* un, double* out, DivBArgs psi, Geometry g, StepScalars* sc, int stage,
+        int bc_writeback) {
+    using T = double;
     using S = Shape<T, NI, NJ, NK, KPAR>;
+    const int b = blockIdx.x;
     constexpr int NIP = S::NIP, PL = S::PL, W = S::W, WP = S::WP, NCELL = S::NCELL;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
@@ -600,8 +525,6 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
     const int fl = g.flags[b];
     const T* blk_in = in + (size_t)b * NV * NCELL;
     T* wb = bc_writeback ? const_cast<T*>(blk_in) : nullptr;
-    __shared__ PushBlock pb;
-    load_push_block(push, b, &pb);
     if (threadIdx.x == 0) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
@@ -609,10 +532,9 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
     }
     __syncthreads();
     if (threadIdx.x == 0) issue_planes<T, S>(blk_in, tile, 0, KPAR + 4, &bars[0]);
-    // u^n (and its int8 correction at stage 4) is read with plain loads at
-    // stages 2-4: warm L2 with the planes of the first chunk, then one chunk ahead
+    // u^n is read with plain loads at stages 2-4: warm L2 with the planes of the
+    // first chunk, then one chunk ahead
     const T* blk_un = un + (size_t)b * NV * NCELL;
-    const int8_t* blk_lo = ulo != nullptr ? ulo + (size_t)b * NV * S::NINT : nullptr;
     T* blk_out = out + (size_t)b * NV * NCELL;
     auto prefetch_un = [&](int kp_first) {
         if (threadIdx.x >= NV) return;
@@ -625,8 +547,6 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
 #pragma unroll
         for (int q = 0; q < KPAR; ++q)
             prefetch_l2(blk_un + ((size_t)v * S::NKP + kp_first + q) * PL + 2 * NIP, (uint32_t)(NJ * NIP * sizeof(T)));
-        if (blk_lo != nullptr && stage == 4)
-            prefetch_l2(blk_lo + ((size_t)v * NK + (kp_first - 2)) * S::PLI, KPAR * S::PLI);
     };
     prefetch_un(2);
     load_geometry<T, S>(g, b, gi, gj, gs, a12);
@@ -643,8 +563,7 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
     const T* GSIN = gj + GJ_SIN * S::NJP;
     const T rinv = gi[GI_RINV * NIP + ii], r2inv = gi[GI_R2INV * NIP + ii];
     const T sinv = gj[GJ_SININV * S::NJP + jj], cot = gj[GJ_COT * S::NJP + jj];
-    const T sin_c = GSIN[jj];
-    const T rho0c = GRHO0[ii], rho0inv = gi[GI_RHO0INV * NIP + ii];
+    const T rho0c = GRHO0[ii];
     const T gor0 = gi[GI_GOR0 * NIP + ii], heat = gi[GI_HEAT * NIP + ii], xi2inv = gi[GI_XI2INV * NIP + ii];
     const double dt = sc->dt;
     // (dt R) / (5 - stage): for 4, 2, 1 (stages 1, 3, 4) the division is exact
@@ -655,13 +574,8 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         const double x = dts * R;
         return stage == 2 ? div_by(x, three) : x;
     };
-    Divisor by_rho0{1.0, 1.0, 0u};   // FP64: quotients by the cell's rho0
-    if constexpr (Pol<T>::exact) by_rho0 = divisor((double)rho0c);
-    auto over_rho0 = [&](T x) -> T {
-        if constexpr (Pol<T>::exact) return (T)div_by((double)x, by_rho0);
-        else return Pol<T>::dv(x, rho0c, rho0inv);
-    };
-    const float dtk = sc->dt_stage_f[stage - 1];
+    const Divisor by_rho0 = divisor(rho0c);   // quotients by the cell's rho0
+    auto over_rho0 = [&](T x) { return div_by(x, by_rho0); };
 
     constexpr int nchunk = NK / KPAR;
     const int polls = sc->wait_polls;
@@ -703,39 +617,31 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         for (int x = tid; x < (hi - lo) * PL; x += S::NT) {
             const int kp = lo + x / PL, c = x % PL, ic = c % NIP;
             const int slot = kp % W;
-            if constexpr (Pol<T>::exact) {
-                const double r1 = (double)tile[(V_RHO1 * W + slot) * PL + c];
-                const double s1v = (double)tile[(V_S1 * W + slot) * PL + c];
-                tp1[(kp % WP) * PL + c] = (T)(a12[ic] * r1 + a12[NIP + ic] * s1v);
-                const int jc = c / NIP;
-                if (jc >= 2 && jc < NJ + 2) {   // the k-neighbours of interior cells, and E_theta's i-neighbours
-                    auto at = [&](int v) { return tile[(v * W + slot) * PL + c]; };
-                    const T vr = at(V_VR), vp = at(V_VP), br = at(V_BR), bp = at(V_BP);
-                    te2[((kp % WP) * NJ + jc - 2) * NIP + ic] = vp * br - vr * bp;
-                    if (ic >= 2 && ic < NI + 2) {
-                        const Divisor by_sin{gj[GJ_SIN * S::NJP + jc], gj[GJ_SININV * S::NJP + jc], 1000u};
-                        T* xs = txs + (kp % WP) * S::PLI + (jc - 2) * NI + ic - 2;
-                        xs[0] = div_by(br, by_sin);
-                        xs[WP * S::PLI] = div_by(at(V_VT) * bp - vp * at(V_BT), by_sin);
-                    }
+            const double r1 = tile[(V_RHO1 * W + slot) * PL + c];
+            const double s1v = tile[(V_S1 * W + slot) * PL + c];
+            tp1[(kp % WP) * PL + c] = a12[ic] * r1 + a12[NIP + ic] * s1v;
+            const int jc = c / NIP;
+            if (jc >= 2 && jc < NJ + 2) {   // the k-neighbours of interior cells, and E_theta's i-neighbours
+                auto at = [&](int v) { return tile[(v * W + slot) * PL + c]; };
+                const T vr = at(V_VR), vp = at(V_VP), br = at(V_BR), bp = at(V_BP);
+                te2[((kp % WP) * NJ + jc - 2) * NIP + ic] = vp * br - vr * bp;
+                if (ic >= 2 && ic < NI + 2) {
+                    const Divisor by_sin{gj[GJ_SIN * S::NJP + jc], gj[GJ_SININV * S::NJP + jc], 1000u};
+                    T* xs = txs + (kp % WP) * S::PLI + (jc - 2) * NI + ic - 2;
+                    xs[0] = div_by(br, by_sin);
+                    xs[WP * S::PLI] = div_by(at(V_VT) * bp - vp * at(V_BT), by_sin);
                 }
-            } else {
-                const float* f = reinterpret_cast<const float*>(a12);
-                tp1[(kp % WP) * PL + c] = p1_ff(f[ic], f[NIP + ic], f[2 * NIP + ic], f[3 * NIP + ic],
-                                                (float)tile[(V_RHO1 * W + slot) * PL + c],
-                                                (float)tile[(V_S1 * W + slot) * PL + c]);
             }
         }
-        if constexpr (Pol<T>::exact) {   // E_r and E_phi of the chunk's planes
-            for (int x = tid; x < KPAR * PL; x += S::NT) {
-                const int q = x / PL, c = x % PL, ic = c % NIP, jc = c / NIP, slot = (k0 + 1 + q) % W;
-                const bool in_i = ic >= 2 && ic < NI + 2, in_j = jc >= 2 && jc < NJ + 2;
-                if (!in_i && !in_j) continue;
-                auto at = [&](int v) { return tile[(v * W + slot) * PL + c]; };
-                const T vt = at(V_VT), bt = at(V_BT);
-                te3[q * PL + c] = at(V_VR) * bt - vt * at(V_BR);
-                if (in_i) te1[(q * S::NJP + jc) * NI + ic - 2] = vt * at(V_BP) - at(V_VP) * bt;
-            }
+        // E_r and E_phi of the chunk's planes
+        for (int x = tid; x < KPAR * PL; x += S::NT) {
+            const int q = x / PL, c = x % PL, ic = c % NIP, jc = c / NIP, slot = (k0 + 1 + q) % W;
+            const bool in_i = ic >= 2 && ic < NI + 2, in_j = jc >= 2 && jc < NJ + 2;
+            if (!in_i && !in_j) continue;
+            auto at = [&](int v) { return tile[(v * W + slot) * PL + c]; };
+            const T vt = at(V_VT), bt = at(V_BT);
+            te3[q * PL + c] = at(V_VR) * bt - vt * at(V_BR);
+            if (in_i) te1[(q * S::NJP + jc) * NI + ic - 2] = vt * at(V_BP) - at(V_VP) * bt;
         }
         __syncthreads();
 
@@ -748,9 +654,8 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         auto P = [&](int di, int dj, int dk) -> T { return tp1[sp[dk + 2] * PL + (jj + dj) * NIP + ii + di]; };
         // ModDerivative_1st_O4_3D (3_6/ModDerivative.f90:16-32)
         auto D = [&](T c, auto f) -> T {
-            // 8 f is exact, so the FP64 FMAs round where the reference's sums do
-            if constexpr (Pol<T>::exact) return c * (fma(-8.0, f(-1), fma(8.0, f(1), -f(2))) + f(-2));
-            else return c * (((-f(2) + T(8) * f(1)) - T(8) * f(-1)) + f(-2));
+            // 8 f is exact, so the FMAs round where the reference's sums do
+            return c * (fma(-8.0, f(-1), fma(8.0, f(1), -f(2))) + f(-2));
         };
         const T vr = A(V_VR, 0, 0, 0), vt = A(V_VT, 0, 0, 0), vp = A(V_VP, 0, 0, 0);
         const T br = A(V_BR, 0, 0, 0), bt = A(V_BT, 0, 0, 0), bp = A(V_BP, 0, 0, 0);
@@ -814,10 +719,8 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         {
             T k1 = D(c2, [&](int m) { return A(V_BP, 0, m, 0) * GSIN[jj + m]; }) -
                    D(c3, [&](int m) { return A(V_BT, 0, 0, m); });
-            auto brs = [&](int m) -> T {   // Br / sin(theta) at the k-neighbour m
-                if constexpr (Pol<T>::exact) return txs[sp[m + 2] * S::PLI + j * NI + i];
-                else return Pol<T>::dv(A(V_BR, 0, 0, m), sin_c, sinv);
-            };
+            // Br / sin(theta) at the k-neighbour m
+            auto brs = [&](int m) -> T { return txs[sp[m + 2] * S::PLI + j * NI + i]; };
             T k2 = D(c3, brs) -
                    D(c1, [&](int m) { return A(V_BP, m, 0, 0) * GR[ii + m]; });
             T k3 = D(c1, [&](int m) { return A(V_BT, m, 0, 0) * GR[ii + m]; }) -
@@ -836,28 +739,16 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         // Entropy advection and heating (3_6/ModEquation.f90:132-151)
         T Rs = -adg(V_S1);
         Rs = Rs + heat;
-        (void)heat_on;
         // Induction curl(v x B) (3_6/ModEquation.f90:154-162)
         T RBr, RBt, RBp;
         {
-            // FP64: from the point arrays (E1 along j, E2 along i and k, E3 along i and j)
-            auto E1 = [&](int a, int bq, int c) -> T {
-                if constexpr (Pol<T>::exact) return te1[(kq * S::NJP + jj + bq) * NI + i];
-                else return A(V_VT, a, bq, c) * A(V_BP, a, bq, c) - A(V_VP, a, bq, c) * A(V_BT, a, bq, c);
-            };
-            auto E2 = [&](int a, int bq, int c) -> T {
-                if constexpr (Pol<T>::exact) return te2[(sp[c + 2] * NJ + j) * NIP + ii + a];
-                else return A(V_VP, a, bq, c) * A(V_BR, a, bq, c) - A(V_VR, a, bq, c) * A(V_BP, a, bq, c);
-            };
-            auto E3 = [&](int a, int bq, int c) -> T {
-                if constexpr (Pol<T>::exact) return te3[kq * PL + (jj + bq) * NIP + ii + a];
-                else return A(V_VR, a, bq, c) * A(V_BT, a, bq, c) - A(V_VT, a, bq, c) * A(V_BR, a, bq, c);
-            };
+            // from the point arrays: E1 along j, E2 along i and k, E3 along i and j
+            auto E1 = [&](int, int bq, int) -> T { return te1[(kq * S::NJP + jj + bq) * NI + i]; };
+            auto E2 = [&](int a, int, int c) -> T { return te2[(sp[c + 2] * NJ + j) * NIP + ii + a]; };
+            auto E3 = [&](int a, int bq, int) -> T { return te3[kq * PL + (jj + bq) * NIP + ii + a]; };
             T q1 = D(c2, [&](int m) { return E3(0, m, 0) * GSIN[jj + m]; }) - D(c3, [&](int m) { return E2(0, 0, m); });
-            auto e1s = [&](int m) -> T {   // E1 / sin(theta) at the k-neighbour m
-                if constexpr (Pol<T>::exact) return txs[(WP + sp[m + 2]) * S::PLI + j * NI + i];
-                else return Pol<T>::dv(E1(0, 0, m), sin_c, sinv);
-            };
+            // E1 / sin(theta) at the k-neighbour m
+            auto e1s = [&](int m) -> T { return txs[(WP + sp[m + 2]) * S::PLI + j * NI + i]; };
             T q2 = D(c3, e1s) -
                    D(c1, [&](int m) { return E3(m, 0, 0) * GR[ii + m]; });
             T q3 = D(c1, [&](int m) { return E2(m, 0, 0) * GR[ii + m]; }) - D(c2, [&](int m) { return E1(0, m, 0); });
@@ -905,47 +796,17 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
                   sqrt(u0s[V_VR] * u0s[V_VR] + u0s[V_VT] * u0s[V_VT] + u0s[V_VP] * u0s[V_VP]);
             w = w + sqrt(u0s[V_BR] * u0s[V_BR] + u0s[V_BT] * u0s[V_BT] + u0s[V_BP] * u0s[V_BP]) / sqrt(rho0c);
             const T rcell = GR[ii];
-            const T h = fmin(fmin(gs[GS_DXI], rcell * gs[GS_DXJ]), rcell * sin_c * gs[GS_DXK]);
+            const T h = fmin(fmin(gs[GS_DXI], rcell * gs[GS_DXJ]), rcell * GSIN[jj] * gs[GS_DXK]);
             const T Rpsi = -(w * w * divB) - w / h * Q(0, 0, 0);
             const size_t pc = (size_t)b * NCELL + (size_t)kp * PL + jj * NIP + ii;
             const T pn = static_cast<const T*>(psi.un)[pc];
-            T po;
-            if constexpr (Pol<T>::exact) po = (T)((double)pn + advance((double)Rpsi));
-            else po = fmaf((float)dtk, (float)Rpsi, (float)pn);
-            static_cast<T*>(psi.out)[pc] = po;
+            static_cast<T*>(psi.out)[pc] = pn + advance(Rpsi);
         }
 
         // stage update
         const T R[NV] = {Rrho, Rvr, Rvt, Rvp, RBr, RBt, RBp, Rs};
-        T o[NV];
-        if constexpr (Pol<T>::exact) {
 #pragma unroll
-            for (int v = 0; v < NV; ++v) o[v] = (T)((double)u0s[v] + advance((double)R[v]));
-        } else if (ulo != nullptr && stage == 4) {
-            // u^{n+1} = u^n + dt*R with u^n and u^{n+1} compensated
-            int8_t* ql = ulo + (size_t)b * NV * S::NINT + ((size_t)(kp - 2) * NJ + (jj - 2)) * NI + (ii - 2);
-            int8_t q0[NV];
-#pragma unroll
-            for (int v = 0; v < NV; ++v) q0[v] = ql[(size_t)v * S::NINT];
-#pragma unroll
-            for (int v = 0; v < NV; v += 2) {   // pairs of variables: ff_add2 gives ff_add's bits
-                int8_t qa, qb;
-                const float2 ov = ff_add2(f2((float)u0s[v], (float)u0s[v + 1]), q0[v], q0[v + 1],
-                                          __fmul2_rn(f2(dtk), f2((float)R[v], (float)R[v + 1])), qa, qb);
-                o[v] = ov.x;
-                o[v + 1] = ov.y;
-                ql[(size_t)v * S::NINT] = qa;
-                ql[(size_t)(v + 1) * S::NINT] = qb;
-            }
-        } else {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) o[v] = fmaf((float)dtk, (float)R[v], (float)u0s[v]);
-        }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) out[base + (size_t)v * NCELL] = o[v];
-        if constexpr (!Pol<T>::exact) {
-            if (push.tgt != nullptr) push_faces<T, S>(out, pb, ii, jj, kp, o);
-        }
+        for (int v = 0; v < NV; ++v) out[base + (size_t)v * NCELL] = u0s[v] + advance(R[v]);
     }
     if (__syncthreads_or(late)) {
         copy_wait_abort(sc, bars, nchunk - 1, nchunk - 1);
@@ -956,76 +817,7 @@ __device__ __forceinline__ void stage_body(int b, const T* in, const T* un, T* o
         mbar_inval(&bars[1]);
     }
 }
-template <class T, int NI, int NJ, int NK, int KPAR, int DIVB>
-__global__ void __launch_bounds__(NI* NJ* KPAR, (Shape<T, NI, NJ, NK, KPAR>::min_blocks))
-k_stage(const T* in, const T* un, T* out, int8_t* ulo, PushTable push, DivBArgs psi, Geometry g, StepScalars* sc,
-        int stage, int bc_writeback, int heat_on) {
-    stage_body<T, NI, NJ, NK, KPAR, DIVB>(blockIdx.x, in, un, out, ulo, push, psi, g, sc, stage, bc_writeback, heat_on);
-}
-
 // ---------------------------------------------------------------------------
-// Artificial diffusion with h=2 (3_6/ModDiffusion.f90:9-150) and the update
-// u += 0.5*dt*R (3_6/ModAdvance.f90:101-108), in place.
-//
-// The reference evaluates, for every cell and direction, the limited fluxes
-// through its two faces, so every face flux (and the minmod slopes under it)
-// is formed twice. Here each face flux is formed once per chunk of KPAR
-// planes into shared memory: i and j faces of the chunk's planes, and the k
-// faces in a ring of KPAR+1 face planes (the last face of a chunk is the
-// first of the next). A flux is the same function of the same four values as
-// the reference's, so sharing it changes no bit. Then each cell sums
-// (F_left - F_right)/den over the three directions, in the reference's order.
-template <class T, int NI, int NJ, int NK, int KPAR>
-struct DShape : Shape<T, NI, NJ, NK, KPAR> {
-    using B = Shape<T, NI, NJ, NK, KPAR>;
-    static constexpr int NCELLS = NI * NJ * KPAR;        // interior cells of a chunk
-    // threads per cell in the sum (variables split): one in FP32, two for a
-    // 256-cell FP64 chunk
-    static constexpr int TPC = (NCELLS >= 512 || sizeof(T) == 4) ? 1 : 2;
-    static constexpr int NT = NCELLS * TPC;
-    static constexpr int VPT = NV / TPC;
-    static constexpr int KS = KPAR + 1;                  // k-face ring slots
-    // FP32, 16-wide rows: a warp takes rows j and j+4 of a plane (80 floats,
-    // 16 banks apart) so that its two halves touch disjoint banks in every
-    // tile access (rows j and j+1, 20 floats apart, share 4 banks). The i-face
-    // rows get a pitch of 20 for the same reason, and the j- and k-face rows
-    // are stored in the order rpos() that puts the two rows of a warp side by side.
-    static constexpr bool R4 = sizeof(T) == 4 && NI == 16 && NJ % 8 == 0;
-    static constexpr int FIP = R4 ? 20 : NI + 1;         // i-face row pitch
-    __device__ static __forceinline__ void cell(int c, int& i, int& j, int& kq) {
-        kq = c / (NI * NJ);
-        const int cc = c % (NI * NJ);
-        i = cc % NI;
-        if constexpr (R4) {
-            const int w = cc / 32;
-            j = (w % 4) + 8 * (w / 4) + 4 * ((cc / 16) % 2);
-        } else {
-            j = cc / NI;
-        }
-    }
-    __device__ static __forceinline__ int rpos(int j) {   // j in [0, NJ]; NJ maps to itself
-        if constexpr (R4) return j >= NJ ? NJ : 2 * ((j % 4) + 4 * (j / 8)) + ((j / 4) % 2);
-        else return j;
-    }
-    static constexpr int NFI = NV * KPAR * NJ * FIP;
-    static constexpr int NFJ = NV * KPAR * (NJ + 1) * NI;
-    static constexpr int NFK = KS * NV * NJ * NI;
-    // shared memory: mbarriers | tile[NV][W][PL] | FI | FJ | FK | gi | gj | gs
-    static constexpr size_t off_tile = 16;
-    static constexpr size_t off_fi = off_tile + (size_t)NV * B::W * B::PL * sizeof(T);
-    static constexpr size_t off_fj = off_fi + (size_t)NFI * sizeof(T);
-    static constexpr size_t off_fk = off_fj + (size_t)NFJ * sizeof(T);
-    static constexpr size_t off_gi = off_fk + (size_t)NFK * sizeof(T);
-    static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * B::NIP * sizeof(T);
-    static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * B::NJP * sizeof(T);
-    static constexpr size_t smem = off_gs + GS_COUNT * sizeof(T);
-    static constexpr bool fits = smem <= 232448;         // 227 KB of opt-in shared memory per CTA
-    static constexpr int by_smem = (int)(233472 / (smem + 1024));
-    static constexpr int reg_cap = 2048 / NT;
-    static constexpr int min_blocks =
-        sizeof(T) != 4 || by_smem < 2 ? 1 : (by_smem < reg_cap ? by_smem : (reg_cap < 1 ? 1 : reg_cap));
-};
-
 // Limited flux through the face between cells L and R along one direction
 // (3_6/ModDiffusion.f90:40-60 for one side): values at L-1, L, R, R+1 and
 // the speeds |v_dir| + c_s at L and R.
@@ -1054,647 +846,6 @@ __device__ __forceinline__ T face_flux_s(T fl, T fr, T dL, T dR, T cL, T cR) {
 template <class T>
 __device__ __forceinline__ T face_flux(T fm, T fl, T fr, T fp, T cL, T cR) {
     return face_flux_s(fl, fr, face_slope(fm, fl, fr), face_slope(fl, fr, fp), cL, cR);
-}
-
-//
-// In place (out == u), or out of place into `out` (mixed step): then the
-// kernel also writes the regular ghost faces of its neighbours in `out`
-// (push, as the stage kernel does) and copies the radial physical-boundary
-// ghost columns (set by the boundary condition at stage 1) from u to out, so
-// that with an exchange of the remaining ghost entries `out` holds the whole
-// updated state.
-//
-// cfl_next (mixed): the outputs are the next step's u^n, so the kernel also
-// forms the next step's CFL minimum and NaN flag from them (k_cfl's formula,
-// cfl_ratio_f), and that step skips k_cfl.
-template <class T, int NI, int NJ, int NK, int KPAR>
-__global__ void __launch_bounds__(DShape<T, NI, NJ, NK, KPAR>::NT, (DShape<T, NI, NJ, NK, KPAR>::min_blocks))
-k_diffusion(const T* u, T* out, int8_t* ulo, PushTable push, Geometry g, StepScalars* sc, int cfl_next) {
-    using S = DShape<T, NI, NJ, NK, KPAR>;
-    static_assert(S::fits, "diffusion shared memory above 227 KB");
-    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, KS = S::KS;
-    extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-    T* tile = reinterpret_cast<T*>(smem + S::off_tile);
-    T* FI = reinterpret_cast<T*>(smem + S::off_fi);
-    T* FJ = reinterpret_cast<T*>(smem + S::off_fj);
-    T* FK = reinterpret_cast<T*>(smem + S::off_fk);
-    T* gi = reinterpret_cast<T*>(smem + S::off_gi);
-    T* gj = reinterpret_cast<T*>(smem + S::off_gj);
-    T* gs = reinterpret_cast<T*>(smem + S::off_gs);
-    const int b = blockIdx.x;
-    const T* blk = u + (size_t)b * NV * NCELL;
-    T* oblk = out + (size_t)b * NV * NCELL;
-    const int flb = g.flags[b];
-    const bool copy_bc = out != u && (flb & 6);
-    __shared__ PushBlock pb;
-    load_push_block(push, b, &pb);
-    if (threadIdx.x == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) issue_planes<T, S>(blk, tile, 0, KPAR + 4, &bars[0]);
-    // the int8 corrections of u^n are read with plain loads: warm L2 with the
-    // first chunk's planes, then one chunk ahead
-    const int8_t* blk_lo = ulo != nullptr ? ulo + (size_t)b * NV * S::NINT : nullptr;
-    auto prefetch_lo = [&](int kp_first) {
-        if (threadIdx.x >= NV) return;
-        if (blk_lo != nullptr) prefetch_l2(blk_lo + ((size_t)threadIdx.x * NK + (kp_first - 2)) * S::PLI, KPAR * S::PLI);
-    };
-    prefetch_lo(2);
-    load_geometry<T, S>(g, b, gi, gj, gs, nullptr);
-    __syncthreads();   // the geometry tables are read by every thread below
-    const int tid = threadIdx.x;
-    const T* GCS = gi + GI_CS * NIP;
-    // the cell and variables this thread sums and updates
-    const int c = tid % S::NCELLS, v0 = (tid / S::NCELLS) * S::VPT;
-    int i, j, kq;
-    S::cell(c, i, j, kq);
-    const int ii = i + 2, jj = j + 2, jr = S::rpos(j), jr1 = S::rpos(j + 1);
-    const T rc = gi[GI_R * NIP + ii];
-    const T den[3] = {gs[GS_DXI], gs[GS_DXJ] * rc, gs[GS_DXK] * rc * gj[GJ_SIN * S::NJP + jj]};
-    const T dinv[3] = {T(1) / den[0], T(1) / den[1], T(1) / den[2]};
-    const double hdt = 0.5 * sc->dt;
-    const float hdt_f = sc->dt_half_f;
-    T sk[S::VPT];            // k slopes carried to the next chunk (one plane per chunk)
-#pragma unroll
-    for (int t = 0; t < S::VPT; ++t) sk[t] = T(0);
-    float cmin = INFINITY;   // next step's CFL ratio minimum over this thread's cells
-    int cnan = 0;
-    __shared__ float sb2[S::TPC == 2 ? S::NCELLS : 1];   // |B|^2 from the thread holding B
-    constexpr int nchunk = NK / KPAR;
-    const int polls = sc->wait_polls;
-    int late = 0;   // a wait of this thread for a chunk's planes ran out
-    for (int ch = 0; ch < nchunk; ++ch) {
-        const int k0 = 1 + ch * KPAR;
-        const int hi = k0 + KPAR + 3;
-        // ring slots and face arrays of the previous chunk are free; a wait of
-        // chunk ch-1 that ran out ends the CTA here (chunks ch-1 and ch in flight)
-        if (__syncthreads_or(late)) {
-            copy_wait_abort(sc, bars, ch - 1, ch);
-            return;
-        }
-        if (threadIdx.x == 0 && ch + 1 < nchunk) issue_planes<T, S>(blk, tile, hi, hi + KPAR, &bars[(ch + 1) & 1]);
-        if (ch + 1 < nchunk) prefetch_lo(k0 + KPAR + 1);
-        // this thread's int8 corrections, loaded now so that their latency
-        // overlaps the copy wait and the face phase
-        int8_t qlo[S::VPT];
-        if constexpr (!Pol<T>::exact) {
-            if (ulo != nullptr) {
-                const int8_t* q = ulo + ((size_t)b * NV + v0) * S::NINT +
-                                  ((size_t)(k0 - 1 + kq) * NJ + j) * NI + i;
-#pragma unroll
-                for (int t = 0; t < S::VPT; ++t) qlo[t] = q[(size_t)t * S::NINT];
-            }
-        }
-        // as in the stage kernel: a wait that runs out finishes the chunk on
-        // whatever the slots hold; the step is flagged and discarded
-        late |= mbar_wait(&bars[ch & 1], (uint32_t)((ch >> 1) & 1), polls) ? 0 : 1;
-        const int kp0 = k0 + 1;   // padded index of the chunk's first plane
-        const int kp = kp0 + kq;
-        if (copy_bc) {   // radial boundary ghost columns of the planes new to this chunk
-            const int plo = ch == 0 ? 0 : k0 + 3, phi = k0 + KPAR + 3, fl = flb;
-            const int total = (phi - plo) * S::NJP * NV * 4;
-            for (int x = tid; x < total; x += S::NT) {
-                const int c4 = x & 3, r = x >> 2;
-                const int v = r % NV, r2 = r / NV;
-                const int y = r2 % S::NJP, z = plo + r2 / S::NJP;
-                if (!((c4 < 2) ? (fl & 4) : (fl & 2))) continue;
-                const int xi = c4 < 2 ? c4 : NI + c4;   // 0, 1 (bottom) or NI+2, NI+3 (top)
-                oblk[((size_t)v * S::NKP + z) * PL + y * NIP + xi] = tile[(v * W + z % W) * PL + y * NIP + xi];
-            }
-        }
-        // ring offsets of planes kp-2 .. kp+2
-        int so[5];
-        so[0] = ((kp - 2) % W) * PL;
-#pragma unroll
-        for (int d = 1; d < 5; ++d) so[d] = so[d - 1] + PL >= W * PL ? so[d - 1] + PL - W * PL : so[d - 1] + PL;
-        const T* t0 = tile + jj * NIP + ii;   // this cell's column in every plane
-        // this cell's left i and j faces and right k face, for its variables
-        {
-            const T* tc = t0 + so[2];
-            const T cLi = fabs(tc[V_VR * W * PL - 1]) + GCS[ii - 1], cRi = fabs(tc[V_VR * W * PL]) + GCS[ii];
-            const T cs = GCS[ii];
-            const T cLj = fabs(tc[V_VT * W * PL - NIP]) + cs, cRj = fabs(tc[V_VT * W * PL]) + cs;
-            const T cLk = fabs(t0[V_VP * W * PL + so[2]]) + cs, cRk = fabs(t0[V_VP * W * PL + so[3]]) + cs;
-            T* fkw = FK + ((size_t)((kp - 1) % KS) * NV) * NJ * NI + jr * NI + i;
-#pragma unroll
-            for (int t = 0; t < S::VPT; ++t) {
-                const int v = v0 + t;
-                const T* a = tc + v * W * PL;
-                FI[((v * KPAR + kq) * NJ + j) * S::FIP + i] = face_flux(a[-2], a[-1], a[0], a[1], cLi, cRi);
-                FJ[((v * KPAR + kq) * (NJ + 1) + jr) * NI + i] =
-                    face_flux(a[-2 * NIP], a[-NIP], a[0], a[NIP], cLj, cRj);
-                // the k face's slopes: with one plane per chunk the lower one
-                // is the upper one of the previous chunk (same values, same bits)
-                const T* ak = t0 + v * W * PL;
-                const T dRk = face_slope(ak[so[2]], ak[so[3]], ak[so[4]]);
-                T dLk;
-                if constexpr (KPAR == 1) {
-                    dLk = ch == 0 ? face_slope(ak[so[1]], ak[so[2]], ak[so[3]]) : sk[t];
-                    sk[t] = dRk;
-                } else {
-                    dLk = face_slope(ak[so[1]], ak[so[2]], ak[so[3]]);
-                }
-                fkw[v * NJ * NI] = face_flux_s(ak[so[2]], ak[so[3]], dLk, dRk, cLk, cRk);
-            }
-        }
-        // the right faces of the last cells of i rows and j columns
-        constexpr int NXI = NV * KPAR * NJ, NXJ = NV * KPAR * NI;
-        for (int x = tid; x < NXI + NXJ; x += S::NT) {
-            if (x < NXI) {
-                const int y = x % NJ + 2, q = (x / NJ) % KPAR, v = x / (NJ * KPAR);
-                const T* a = tile + (v * W + (kp0 + q) % W) * PL + y * NIP + NI + 1;   // last interior cell
-                const T* vr = tile + (V_VR * W + (kp0 + q) % W) * PL + y * NIP + NI + 1;
-                const T cL = fabs(vr[0]) + GCS[NI + 1], cR = fabs(vr[1]) + GCS[NI + 2];
-                FI[((v * KPAR + q) * NJ + (y - 2)) * S::FIP + NI] = face_flux(a[-1], a[0], a[1], a[2], cL, cR);
-            } else {
-                const int z = x - NXI;
-                const int xx = z % NI + 2, q = (z / NI) % KPAR, v = z / (NI * KPAR);
-                const T* a = tile + (v * W + (kp0 + q) % W) * PL + (NJ + 1) * NIP + xx;
-                const T* vt = tile + (V_VT * W + (kp0 + q) % W) * PL + (NJ + 1) * NIP + xx;
-                const T cs = GCS[xx];
-                const T cL = fabs(vt[0]) + cs, cR = fabs(vt[NIP]) + cs;
-                FJ[((v * KPAR + q) * (NJ + 1) + NJ) * NI + (xx - 2)] =
-                    face_flux(a[-NIP], a[0], a[NIP], a[2 * NIP], cL, cR);
-            }
-        }
-        // first chunk: the k faces below the first plane (between padded planes 1 and 2)
-        if (ch == 0) {
-            for (int x = tid; x < NV * NJ * NI; x += S::NT) {
-                const int xx = x % NI + 2, y = (x / NI) % NJ + 2, v = x / (NI * NJ);
-                const T* a = tile + (size_t)v * W * PL + y * NIP + xx;
-                const T* vp = tile + (size_t)V_VP * W * PL + y * NIP + xx;
-                const T cs = GCS[xx];
-                const T cL = fabs(vp[PL]) + cs, cR = fabs(vp[2 * PL]) + cs;
-                FK[((0 * NV + v) * NJ + S::rpos(y - 2)) * NI + (xx - 2)] =
-                    face_flux(a[0], a[PL], a[2 * PL], a[3 * PL], cL, cR);
-            }
-        }
-        __syncthreads();
-        const size_t base = (size_t)kp * PL + jj * NIP + ii;
-        const T* fk_l = FK + ((size_t)((kp - 2) % KS) * NV) * NJ * NI + jr * NI + i;
-        const T* fk_r = FK + ((size_t)((kp - 1) % KS) * NV) * NJ * NI + jr * NI + i;
-        T o[S::VPT];
-#pragma unroll
-        for (int t = 0; t < S::VPT; ++t) {
-            const int v = v0 + t;
-            const T* fi = FI + ((v * KPAR + kq) * NJ + j) * S::FIP + i;
-            const T* fj = FJ + ((v * KPAR + kq) * (NJ + 1)) * NI + i;
-            T R = T(0);
-            R = R + Pol<T>::dv(fi[0] - fi[1], den[0], dinv[0]);
-            R = R + Pol<T>::dv(fj[jr * NI] - fj[jr1 * NI], den[1], dinv[1]);
-            R = R + Pol<T>::dv(fk_l[v * NJ * NI] - fk_r[v * NJ * NI], den[2], dinv[2]);
-            const T u0 = t0[v * W * PL + so[2]];
-            if constexpr (Pol<T>::exact) {
-                o[t] = (T)((double)u0 + hdt * (double)R);
-            } else if (ulo != nullptr) {
-                int8_t q1;
-                o[t] = ff_add((float)u0, qlo[t], __fmul_rn(hdt_f, (float)R), q1);
-                ulo[((size_t)b * NV + v) * S::NINT + ((size_t)(kp - 2) * NJ + j) * NI + i] = q1;
-            } else {
-                o[t] = fmaf(hdt_f, (float)R, (float)u0);
-            }
-            oblk[(size_t)v * NCELL + base] = o[t];
-        }
-        if constexpr (!Pol<T>::exact) {
-            if (push.tgt != nullptr) push_faces_part<T, S, S::VPT>(out, pb, ii, jj, kp, o, v0);
-            if (cfl_next) {   // uniform over the CTA
-#pragma unroll
-                for (int t = 0; t < S::VPT; ++t) cnan |= (o[t] != o[t]);
-                float v2 = 0.f, b2 = 0.f;
-                if constexpr (S::TPC == 1) {
-                    v2 = cfl_sq3(o[V_VR], o[V_VT], o[V_VP]);
-                    b2 = cfl_sq3(o[V_BR], o[V_BT], o[V_BP]);
-                } else {
-                    if (v0 != 0) sb2[c] = cfl_sq3(o[V_BR - 4], o[V_BT - 4], o[V_BP - 4]);
-                    __syncthreads();
-                    if (v0 == 0) {
-                        v2 = cfl_sq3(o[V_VR], o[V_VT], o[V_VP]);
-                        b2 = sb2[c];
-                    }
-                }
-                if (v0 == 0) {
-                    float ratio = cfl_ratio_f(v2, b2, GCS[ii], gi[GI_RHO0 * NIP + ii], rc, gj[GJ_SIN * S::NJP + jj],
-                                              gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]);
-                    if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
-                    cmin = fminf(cmin, ratio);
-                }
-            }
-        }
-    }
-    if (__syncthreads_or(late)) {
-        copy_wait_abort(sc, bars, nchunk - 1, nchunk - 1);
-        return;
-    }
-    if constexpr (!Pol<T>::exact) {
-        if (cfl_next) cfl_commit(cmin, cnan, sc);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// FP32 artificial diffusion of one 16^3 block as a march along k (the mixed
-// step's diffusion pass; same arguments and results as k_diffusion).
-//
-// One thread per (i, j) column of the block (256 threads), marching k over the
-// 16 interior planes. Along k everything stays in registers: the column's
-// values at planes kp and kp+1, its k slope at kp and the flux through the
-// face below kp; per plane the thread reads one new value per variable (plane
-// kp+2, from the ring), forms one k slope and one k face. Across the plane,
-// every i and j slope is formed once (phase A, into shared memory, ghost
-// columns and rows by the same threads), then every i and j face flux once
-// (phase B), then each cell sums its six faces and updates (phase C). Per
-// cell and variable that is 3 slopes and 3 fluxes, the minimum; the face
-// fluxes are the same functions of the same values as k_diffusion's, summed
-// in the same order. The arithmetic runs on pairs of variables (packed FP32
-// instructions, above), and the slope and face arrays hold the pairs side by
-// side, so their shared-memory accesses are 64-bit.
-//
-// Planes arrive by bulk copy into a ring of 5 slots, one mbarrier each: the
-// column window needs planes kp..kp+2, and the slot of plane kp is refilled
-// with plane kp+5 once phase B of plane kp has passed its barrier (planes
-// kp+3 and kp+4 are in flight meanwhile). A warp takes rows j and j+4
-// (half-warps of 16 cells), so a half-warp holds one row, as the pushed
-// radial faces need.
-template <int NI, int NJ, int NK, int TPC>
-struct MShape {
-    static constexpr int NG = 2, NIP = NI + 4, NJP = NJ + 4, NKP = NK + 4;
-    static constexpr int PL = NIP * NJP, NCELL = PL * NKP;
-    static constexpr int NCOL = NI * NJ, NT = NCOL * TPC;   // columns; threads (TPC per column)
-    static constexpr int W = 5;                          // plane ring slots
-    static constexpr int PLI = NI * NJ, NINT = PLI * NK;
-    static constexpr int NP = NV / 2, PPT = NP / TPC;    // variable pairs; pairs per thread
-    static constexpr uint32_t PLB = PL * 4u;
-    static constexpr int P = 20;                         // row pitch (pairs) of the slope and face arrays
-    // per pair (float2): SI[NJ][P] slopes along i of cells i = -1..NI at i + 1;
-    // SJ[NJ + 2][P] slopes along j of rows j = -1..NJ at row j + 1;
-    // FI[NJ][P] fluxes through faces i - 1/2, i = 0..NI; FJ[NJ + 1][P] likewise along j
-    static constexpr int NSI = NJ * P, NSJ = (NJ + 2) * P, NFI = NJ * P, NFJ = (NJ + 1) * P;
-    // shared memory: mbarriers | tile[NV][W][PL] | SI | SJ | FI | FJ | gi | gj | gs
-    static constexpr size_t off_tile = 64;
-    static constexpr size_t off_si = off_tile + (size_t)NV * W * PL * 4;
-    static constexpr size_t off_sj = off_si + (size_t)NP * NSI * 8;
-    static constexpr size_t off_fi = off_sj + (size_t)NP * NSJ * 8;
-    static constexpr size_t off_fj = off_fi + (size_t)NP * NFI * 8;
-    static constexpr size_t off_gi = off_fj + (size_t)NP * NFJ * 8;
-    static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * NIP * 4;
-    static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * NJP * 4;
-    // two threads per column: |B|^2 of the second half, [plane parity][column]
-    static constexpr size_t off_sb2 = off_gs + GS_COUNT * 4;
-    static constexpr size_t smem = off_sb2 + (TPC == 2 ? 2 * NCOL * 4 : 0);
-    static_assert(W * 8 <= (int)off_tile, "mbarriers");
-    static_assert(off_si % 8 == 0, "float2 arrays");
-    static_assert(TPC == 1 || TPC == 2, "one or two threads per column");
-};
-
-// TPC threads per column: with two, thread half h = tid / 256 takes the
-// variable pairs 2h, 2h+1 (warps never mix halves), doubling the warps per SM
-// at half the registers; the CFL ratio, which needs v (first half) and B
-// (second half), takes |B|^2 through shared memory one plane later.
-template <int NI, int NJ, int NK, int TPC>
-__device__ __forceinline__ void march_body(int b, const float* u, float* out, int8_t* ulo, PushTable push, Geometry g,
-                                           StepScalars* sc, int cfl_next) {
-    using S = MShape<NI, NJ, NK, TPC>;
-    static_assert(NI == 16 && NJ == 16, "rows of 16 cells: one half-warp per row");
-    static_assert(2 * (S::smem + 1024) <= 233472, "two CTAs per SM");
-    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, P = S::P, PPT = S::PPT;
-    extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-    float* tile = reinterpret_cast<float*>(smem + S::off_tile);
-    float2* SI = reinterpret_cast<float2*>(smem + S::off_si);
-    float2* SJ = reinterpret_cast<float2*>(smem + S::off_sj);
-    float2* FI = reinterpret_cast<float2*>(smem + S::off_fi);
-    float2* FJ = reinterpret_cast<float2*>(smem + S::off_fj);
-    float* gi = reinterpret_cast<float*>(smem + S::off_gi);
-    float* gj = reinterpret_cast<float*>(smem + S::off_gj);
-    float* gs = reinterpret_cast<float*>(smem + S::off_gs);
-    float* sb2 = reinterpret_cast<float*>(smem + S::off_sb2);   // |B|^2 of the second half, by plane parity
-    const int tid = threadIdx.x;
-    const float* blk = u + (size_t)b * NV * NCELL;
-    float* oblk = out + (size_t)b * NV * NCELL;
-    const int flb = g.flags[b];
-    const bool copy_bc = out != u && (flb & 6);
-    __shared__ PushBlock pb;
-    load_push_block(push, b, &pb);
-    if (tid == 0) {
-        for (int s = 0; s < W; ++s) mbar_init(&bars[s], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    int issued = 0;   // thread 0: planes [0, issued) have been requested
-    if (tid == 0) {
-        for (int p = 0; p < W; ++p) issue_planes<float, S>(blk, tile, p, p + 1, &bars[p]);
-        issued = W;
-    }
-    const int8_t* blk_lo = ulo != nullptr ? ulo + (size_t)b * NV * S::NINT : nullptr;
-    if (blk_lo != nullptr && tid < NV) prefetch_l2(blk_lo + (size_t)tid * S::NINT, 2 * S::PLI);
-    load_geometry<float, S>(g, b, gi, gj, gs, nullptr);
-    __syncthreads();   // the geometry tables are read by every thread below
-    // this thread's column: warp w takes rows (w % 4) + 8 (w / 4) and that + 4;
-    // its pairs p0 .. p0 + PPT - 1
-    const int c = tid % S::NCOL, half = tid / S::NCOL, p0 = half * PPT, v0 = 2 * p0;
-    const int wq = c >> 5, i = c & 15;
-    const int j = (wq & 3) + 8 * (wq >> 2) + 4 * ((c >> 4) & 1);
-    const int ii = i + 2, jj = j + 2;
-    const float* GCS = gi + GI_CS * NIP;
-    const float cs = GCS[ii];
-    const float rc = gi[GI_R * NIP + ii];
-    const float den[3] = {gs[GS_DXI], gs[GS_DXJ] * rc, gs[GS_DXK] * rc * gj[GJ_SIN * S::NJP + jj]};
-    const float2 dinv0 = f2(1.f / den[0]), dinv1 = f2(1.f / den[1]), dinv2 = f2(1.f / den[2]);
-    const float2 hdt2 = f2(sc->dt_half_f);
-    const int polls = sc->wait_polls;
-    int late = 0;   // a wait of this thread for a plane ran out
-    auto abort_cta = [&]() {   // after a uniform decision: flag, drain the copies in flight
-        if (tid != 0) return;
-        atomicOr(&sc->nan_flag, 2);
-        for (int p = issued - W < 0 ? 0 : issued - W; p < issued; ++p)
-            mbar_wait(&bars[p % W], (uint32_t)((p / W) & 1), kWaitPolls);
-        for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
-    };
-    // radial boundary ghost columns of planes [plo, phi), u -> out
-    auto copy_cols = [&](int plo, int phi) {
-        const int total = (phi - plo) * S::NJP * NV * 4;
-        for (int x = tid; x < total; x += S::NT) {
-            const int c4 = x & 3, r = x >> 2;
-            const int v = r % NV, r2 = r / NV;
-            const int y = r2 % S::NJP, z = plo + r2 / S::NJP;
-            if (!((c4 < 2) ? (flb & 4) : (flb & 2))) continue;
-            const int xi = c4 < 2 ? c4 : NI + c4;   // 0, 1 (bottom) or NI+2, NI+3 (top)
-            oblk[((size_t)v * S::NKP + z) * PL + y * NIP + xi] = tile[(v * W + z % W) * PL + y * NIP + xi];
-        }
-    };
-    // the pair (v, v+1) of a tile value, p = v / 2, at offset o from variable 0's
-    auto tv = [&](const float* base, int p) { return f2(base[2 * p * W * PL], base[(2 * p + 1) * W * PL]); };
-    // the column window from planes 0..3: u at kp = 2 and 3, the k slope at 2,
-    // the flux through the face between planes 1 and 2
-    for (int p = 0; p < 4; ++p) late |= mbar_wait(&bars[p], 0u, polls) ? 0 : 1;
-    if (copy_bc) copy_cols(0, 4);
-    const float* col = tile + jj * NIP + ii;
-    const float* colvp = col + V_VP * W * PL;
-    float2 u0[PPT], u1[PPT], dk0[PPT], fk0[PPT];
-    {
-        const float2 cc = f2(-0.25f * ((fabsf(colvp[2 * PL]) + cs) + (fabsf(colvp[PL]) + cs)));
-#pragma unroll
-        for (int q = 0; q < PPT; ++q) {
-            const int p = p0 + q;
-            const float2 a0 = tv(col, p), a1 = tv(col + PL, p), a2 = tv(col + 2 * PL, p), a3 = tv(col + 3 * PL, p);
-            const float2 d1 = minmod_sel2(a0, a1, a2), d2 = minmod_sel2(a1, a2, a3);
-            u0[q] = a2;
-            u1[q] = a3;
-            dk0[q] = d2;
-            fk0[q] = face_flux2(a1, a2, d1, d2, cc);
-        }
-    }
-    float cmin = INFINITY;   // next step's CFL ratio minimum over this column
-    int cnan = 0;
-    float v2_prev = 0.f;     // two threads per column: the first half's |v|^2 of the previous plane
-    const float rho0c = gi[GI_RHO0 * NIP + ii], sin_c = gj[GJ_SIN * S::NJP + jj];
-    auto cfl_point = [&](float v2, float b2) {
-        float ratio = cfl_ratio_f(v2, b2, cs, rho0c, rc, sin_c, gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]);
-        if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
-        cmin = fminf(cmin, ratio);
-    };
-    for (int kp = 2; kp < NK + 2; ++kp) {
-        const int p2 = kp + 2;
-        if (blk_lo != nullptr && tid < NV && kp < NK) prefetch_l2(blk_lo + (size_t)tid * S::NINT + (size_t)kp * S::PLI, S::PLI);
-        // this cell's int8 corrections, loaded before the wait
-        int8_t qlo[2 * PPT];
-        if (ulo != nullptr) {
-            const int8_t* q = blk_lo + (size_t)v0 * S::NINT + ((size_t)(kp - 2) * NJ + j) * NI + i;
-#pragma unroll
-            for (int v = 0; v < 2 * PPT; ++v) qlo[v] = q[(size_t)v * S::NINT];
-        }
-        // a wait that runs out finishes the plane on whatever the slot holds;
-        // the step is flagged and discarded
-        late |= mbar_wait(&bars[p2 % W], (uint32_t)((p2 / W) & 1), polls) ? 0 : 1;
-        if (copy_bc) copy_cols(p2, p2 + 1);
-        const int s0 = (kp % W) * PL, s1 = ((kp + 1) % W) * PL, s2 = (p2 % W) * PL;
-        const float* tc = tile + s0 + jj * NIP + ii;   // this cell in plane kp (+ v W PL)
-        // ---- phase A: k slope and k face from the window; i and j slopes
-        float2 u2[PPT], dk1[PPT], fk1[PPT];
-        {
-            const float2 cc = f2(-0.25f * ((fabsf(colvp[s1]) + cs) + (fabsf(colvp[s0]) + cs)));
-#pragma unroll
-            for (int q = 0; q < PPT; ++q) {
-                const int p = p0 + q;
-                u2[q] = tv(col + s2, p);
-                dk1[q] = minmod_sel2(u0[q], u1[q], u2[q]);
-                fk1[q] = face_flux2(u0[q], u1[q], dk0[q], dk1[q], cc);
-                SI[p * S::NSI + j * P + i + 1] = minmod_sel2(tv(tc - 1, p), u0[q], tv(tc + 1, p));
-                SJ[p * S::NSJ + (j + 1) * P + i] = minmod_sel2(tv(tc - NIP, p), u0[q], tv(tc + NIP, p));
-            }
-        }
-        // slopes of the ghost cells next to the block: i = -1, NI of every row
-        // (items 0..255) and j = -1, NJ of every column (items 256..511)
-#pragma unroll
-        for (int x = tid; x < 512; x += S::NT) {
-            const int side = x & 1, r = (x >> 1) & 15, v = (x >> 5) & 7;
-            const float* a = tile + v * W * PL + s0;
-            float* dst;
-            float val;
-            if (x < 256) {
-                const float* q = a + (r + 2) * NIP + (side ? NI + 2 : 1);
-                val = face_slope(q[-1], q[0], q[1]);
-                dst = reinterpret_cast<float*>(SI + (v >> 1) * S::NSI + r * P + (side ? NI + 1 : 0));
-            } else {
-                const float* q = a + (side ? NJ + 2 : 1) * NIP + r + 2;
-                val = face_slope(q[-NIP], q[0], q[NIP]);
-                dst = reinterpret_cast<float*>(SJ + (v >> 1) * S::NSJ + (side ? NJ + 1 : 0) * P + r);
-            }
-            dst[v & 1] = val;
-        }
-        if (__syncthreads_or(late)) {
-            abort_cta();
-            return;
-        }
-        // ---- phase B: the faces i - 1/2 and j - 1/2 of this cell, and the
-        // last faces of the rows (items 0..127) and columns (128..255)
-        float2 fi0[PPT], fj0[PPT];
-        {
-            const float cLi = fabsf(tc[V_VR * W * PL - 1]) + GCS[ii - 1], cRi = fabsf(tc[V_VR * W * PL]) + cs;
-            const float cLj = fabsf(tc[V_VT * W * PL - NIP]) + cs, cRj = fabsf(tc[V_VT * W * PL]) + cs;
-            const float2 cci = f2(-0.25f * (cRi + cLi)), ccj = f2(-0.25f * (cRj + cLj));
-#pragma unroll
-            for (int q = 0; q < PPT; ++q) {
-                const int p = p0 + q;
-                const float2* si = SI + p * S::NSI + j * P + i;
-                const float2* sj = SJ + p * S::NSJ + j * P + i;
-                fi0[q] = face_flux2(tv(tc - 1, p), u0[q], si[0], si[1], cci);
-                fj0[q] = face_flux2(tv(tc - NIP, p), u0[q], sj[0], sj[P], ccj);
-                FI[p * S::NFI + j * P + i] = fi0[q];
-                FJ[p * S::NFJ + j * P + i] = fj0[q];
-            }
-        }
-        if (tid < 256) {
-            const int x = tid, r = x & 15, v = (x >> 4) & 7;
-            const float* sl = reinterpret_cast<const float*>(x < 128 ? SI + (v >> 1) * S::NSI + r * P + NI
-                                                                     : SJ + (v >> 1) * S::NSJ + NJ * P + r);
-            if (x < 128) {
-                const float* a = tile + v * W * PL + s0 + (r + 2) * NIP + NI + 1;   // last interior cell of row r
-                const float* vr = tile + V_VR * W * PL + s0 + (r + 2) * NIP + NI + 1;
-                const float cL = fabsf(vr[0]) + GCS[NI + 1], cR = fabsf(vr[1]) + GCS[NI + 2];
-                reinterpret_cast<float*>(FI + (v >> 1) * S::NFI + r * P + NI)[v & 1] =
-                    face_flux_s(a[0], a[1], sl[v & 1], sl[2 + (v & 1)], cL, cR);
-            } else {
-                const float* a = tile + v * W * PL + s0 + (NJ + 1) * NIP + r + 2;   // last interior row, column r
-                const float* vt = tile + V_VT * W * PL + s0 + (NJ + 1) * NIP + r + 2;
-                const float c2 = GCS[r + 2];
-                const float cL = fabsf(vt[0]) + c2, cR = fabsf(vt[NIP]) + c2;
-                reinterpret_cast<float*>(FJ + (v >> 1) * S::NFJ + NJ * P + r)[v & 1] =
-                    face_flux_s(a[0], a[NIP], sl[v & 1], sl[2 * P + (v & 1)], cL, cR);
-            }
-        }
-        __syncthreads();
-        // planes below kp + 1 are done with: refill their slots, up to plane
-        // kp + W (at kp = 2 that is planes 5, 6, 7; then one plane a step)
-        if (tid == 0) {
-            for (; issued < S::NKP && issued <= kp + W; ++issued)
-                issue_planes<float, S>(blk, tile, issued, issued + 1, &bars[issued % W]);
-        }
-        // ---- phase C: sum the six faces in the reference's order, update
-        const size_t base = (size_t)kp * PL + jj * NIP + ii;
-        float o[2 * PPT];
-#pragma unroll
-        for (int q = 0; q < PPT; ++q) {
-            const int p = p0 + q;
-            float2 R = __fmul2_rn(sub2(fi0[q], FI[p * S::NFI + j * P + i + 1]), dinv0);
-            R = __ffma2_rn(sub2(fj0[q], FJ[p * S::NFJ + (j + 1) * P + i]), dinv1, R);
-            R = __ffma2_rn(sub2(fk0[q], fk1[q]), dinv2, R);
-            float2 ov;
-            if (ulo != nullptr) {
-                int8_t q0, q1;
-                ov = ff_add2(u0[q], qlo[2 * q], qlo[2 * q + 1], __fmul2_rn(hdt2, R), q0, q1);
-                int8_t* qo = ulo + ((size_t)b * NV + 2 * p) * S::NINT + ((size_t)(kp - 2) * NJ + j) * NI + i;
-                qo[0] = q0;
-                qo[S::NINT] = q1;
-            } else {
-                ov = __ffma2_rn(hdt2, R, u0[q]);
-            }
-            o[2 * q] = ov.x;
-            o[2 * q + 1] = ov.y;
-            oblk[(size_t)(2 * p) * NCELL + base] = ov.x;
-            oblk[(size_t)(2 * p + 1) * NCELL + base] = ov.y;
-        }
-        if (push.tgt != nullptr) push_faces_part<float, S, 2 * PPT>(out, pb, ii, jj, kp, o, v0);
-        if (cfl_next) {   // uniform over the CTA
-#pragma unroll
-            for (int v = 0; v < 2 * PPT; ++v) cnan |= (o[v] != o[v]);
-            if constexpr (TPC == 1) {
-                cfl_point(cfl_sq3(o[V_VR], o[V_VT], o[V_VP]), cfl_sq3(o[V_BR], o[V_BT], o[V_BP]));
-            } else if (half == 0) {
-                if (kp > 2) cfl_point(v2_prev, sb2[((kp - 1) & 1) * S::NCOL + c]);
-                v2_prev = cfl_sq3(o[V_VR], o[V_VT], o[V_VP]);
-            } else {
-                sb2[(kp & 1) * S::NCOL + c] = cfl_sq3(o[V_BR - 4], o[V_BT - 4], o[V_BP - 4]);
-            }
-        }
-        // the window moves up one plane
-#pragma unroll
-        for (int q = 0; q < PPT; ++q) {
-            u0[q] = u1[q];
-            u1[q] = u2[q];
-            dk0[q] = dk1[q];
-            fk0[q] = fk1[q];
-        }
-    }
-    if (__syncthreads_or(late)) {
-        abort_cta();
-        return;
-    }
-    if constexpr (TPC == 2) {
-        if (cfl_next && half == 0) cfl_point(v2_prev, sb2[((NK + 1) & 1) * S::NCOL + c]);
-    }
-    if (tid == 0)   // every copy has been waited for
-        for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
-    if (cfl_next) cfl_commit(cmin, cnan, sc);
-}
-template <int NI, int NJ, int NK, int TPC>
-__global__ void __launch_bounds__(NI * NJ * TPC, 2)
-k_diffusion_march(const float* u, float* out, int8_t* ulo, PushTable push, Geometry g, StepScalars* sc, int cfl_next) {
-    march_body<NI, NJ, NK, TPC>(blockIdx.x, u, out, ulo, push, g, sc, cfl_next);
-}
-
-// ---------------------------------------------------------------------------
-// Every cell outside the core of each block and variable set to 0 (the k ghost
-// planes and, in the interior planes, the j ghost rows: per block and
-// variable, (NJP-4)*NIP-wide gaps between the core runs). A core upload clears
-// them before its exchange refills the listed ones: the mixed interpolations
-// read some ghost cells of their source blocks with weight 0, which is
-// harmless for finite values only, and the buffer may hold an earlier state
-// with NaNs there. Cleared, the uploaded state's ghost cells are the same
-// whatever the buffer held (a new context starts with zeros too).
-template <class T>
-__global__ void __launch_bounds__(256) k_clear_outside_core(T* u, int64_t nbv, StepDims d) {
-    const int pl = d.nip * d.njp, lead = 2 * pl + 2 * d.nip, gap = 4 * d.nip;
-    const int per = 2 * lead + (d.nkp - 5) * gap;   // non-core cells per block and variable
-    for (int64_t bv = blockIdx.x; bv < nbv; bv += gridDim.x) {
-        T* base = u + bv * d.ncell;
-        for (int x = threadIdx.x; x < per; x += blockDim.x) {
-            int c;
-            if (x < lead) {
-                c = x;                                   // planes 0, 1 and rows 0, 1 of plane 2
-            } else if (x < per - lead) {
-                const int q = (x - lead) / gap, r = (x - lead) - q * gap;
-                c = (2 + q) * pl + (d.njp - 2) * d.nip + r;   // rows NJP-2, NJP-1 of plane 2+q, rows 0, 1 of the next
-            } else {
-                c = d.ncell - lead + (x - (per - lead));   // rows NJP-2, NJP-1 of the last interior plane, 2 ghost planes
-            }
-            base[c] = T(0);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// After the core of a mixed state has been replaced from the host (the core
-// upload), what the diffusion pass closing a mixed step leaves besides
-// u^{n+1} itself: the regular faces pushed into the neighbours' ghost layers
-// (the face entries left to the final exchange follow as a separate launch),
-// and the next step's CFL minimum with the NaN scan, each cell's ratio the
-// one k_cfl forms. One CTA per block and a thread per (i, j) column marching
-// k; a row of NI cells lies in consecutive lanes, as the pushed radial faces
-// need.
-template <int NI, int NJ, int NK>
-__global__ void __launch_bounds__(NI * NJ) k_push_state(float* u, PushTable push, Geometry g, StepScalars* sc) {
-    using S = MShape<NI, NJ, NK, 1>;
-    constexpr int NIP = S::NIP, NJP = S::NJP;
-    static_assert((NI * NJ) % 32 == 0 && 32 % NI == 0, "whole rows in every warp");
-    __shared__ PushBlock pb;
-    const int b = blockIdx.x, tid = threadIdx.x;
-    load_push_block(push, b, &pb);
-    __syncthreads();
-    const int ii = tid % NI + 2, jj = tid / NI + 2;
-    const float* Gi = gi_ptr<float>(g) + (size_t)b * GI_COUNT * NIP;
-    const float* Gj = gj_ptr<float>(g) + (size_t)b * GJ_COUNT * NJP;
-    const float* Gs = gs_ptr<float>(g) + (size_t)b * GS_COUNT;
-    const float cs = Gi[GI_CS * NIP + ii], rho0 = Gi[GI_RHO0 * NIP + ii], r = Gi[GI_R * NIP + ii];
-    const float sin_t = Gj[GJ_SIN * NJP + jj], dxi = Gs[GS_DXI], dxj = Gs[GS_DXJ], dxk = Gs[GS_DXK];
-    const float* blk = u + (size_t)b * NV * S::NCELL;
-    float cmin = INFINITY;
-    int cnan = 0;
-    constexpr int G = 4;   // planes whose loads are all issued before the first push
-    static_assert(NK % G == 0, "whole plane groups");
-    for (int k0 = 2; k0 < NK + 2; k0 += G) {
-        float o[G][NV];
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            const size_t base = ((size_t)(k0 + q) * NJP + jj) * NIP + ii;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) o[q][v] = blk[(size_t)v * S::NCELL + base];
-        }
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            if (push.tgt != nullptr) push_faces_part<float, S, NV>(u, pb, ii, jj, k0 + q, o[q], 0);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) cnan |= (o[q][v] != o[q][v]);
-            float ratio = cfl_ratio_f(cfl_sq3(o[q][V_VR], o[q][V_VT], o[q][V_VP]),
-                                      cfl_sq3(o[q][V_BR], o[q][V_BT], o[q][V_BP]), cs, rho0, r, sin_t, dxi, dxj, dxk);
-            if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
-            cmin = fminf(cmin, ratio);
-        }
-    }
-    cfl_commit(cmin, cnan, sc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1933,6 +1084,32 @@ __device__ __forceinline__ void finalize_dt_body(StepScalars* sc) {
     sc->step_counter += 1;
 }
 
+// The eight values of a cell, p its variable 0 (Layout): FP32 as two 16-byte
+// accesses. CG: ld.global.cg (L2 only) -- in the persistent step another SM wrote
+// the source cells in the phase before, after this SM may have cached the
+// same lines in its L1.
+template <bool CG>
+__device__ __forceinline__ void load_cell(const double* p, size_t ncell, double (&v)[NV]) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = CG ? __ldcg(p + q * ncell) : p[q * ncell];
+}
+template <bool CG>
+__device__ __forceinline__ void load_cell(const float* p, size_t ncell, float (&v)[NV]) {
+    const float4* f = reinterpret_cast<const float4*>(p);
+    const float4 a = CG ? __ldcg(f) : f[0], b = CG ? __ldcg(f + ncell) : f[ncell];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void store_cell(double* p, size_t ncell, const double (&v)[NV]) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) p[q * ncell] = v[q];
+}
+__device__ __forceinline__ void store_cell(float* p, size_t ncell, const float (&v)[NV]) {
+    float4* f = reinterpret_cast<float4*>(p);
+    f[0] = make_float4(v[0], v[1], v[2], v[3]);
+    f[ncell] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
 // ---------------------------------------------------------------------------
 // Wave speed (3_6/ModWaveSpeed.f90:8-27), h/v_wave min-reduction
 // (3_6/ModTimeStep.f90:10-30) and the NaN scan of 3_6/ModCheck.f90:12-71.
@@ -1948,13 +1125,10 @@ __global__ void __launch_bounds__(256) k_cfl(const T* u, Geometry g, StepScalars
     int nan = 0;
     if (q < nint) {
         const int i = q % d.ni + 2, j = (q / d.ni) % d.nj + 2, k = q / (d.ni * d.nj) + 2;
-        const T* blk = u + (size_t)b * NV * d.ncell + ((size_t)k * d.njp + j) * d.nip + i;
         T x[NV];
+        load_cell<false>(u + Layout<T>::at(b, 0, ((size_t)k * d.njp + j) * d.nip + i, d.ncell), d.ncell, x);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            x[v] = blk[(size_t)v * d.ncell];
-            nan |= (x[v] != x[v]);
-        }
+        for (int v = 0; v < NV; ++v) nan |= (x[v] != x[v]);
         const T* Gi = gi_ptr<T>(g) + (size_t)b * GI_COUNT * d.nip;
         const T* Gj = gj_ptr<T>(g) + (size_t)b * GJ_COUNT * d.njp;
         const T* Gs = gs_ptr<T>(g) + (size_t)b * GS_COUNT;
@@ -1997,227 +1171,97 @@ __global__ void __launch_bounds__(256) k_cfl(const T* u, Geometry g, StepScalars
 // (3_6/ModCommunication.f90:655-795). Exact copies first, then trilinear
 // entries (3_6/ModMath.f90:283-291) with the Yin-Yang vector rotation
 // (3_6/ModYinYang.f90:58-60).
-// Source values are read with ld (CG false) or, in the persistent step,
-// with ld.global.cg (L2 only): there another SM wrote them in the phase
-// before, after this SM may have cached the same lines in its L1.
-template <bool CG, class T>
-__device__ __forceinline__ T ldsrc(const T* p) {
-    if constexpr (CG) return __ldcg(p);
-    else return *p;
-}
 template <class T, bool CG = false>
 __device__ __forceinline__ void ghost_copy_one(T* u, const GhostCopyList& L, int ncell, int64_t e) {
-    const size_t d = (size_t)L.dst[e], s = (size_t)L.src[e];
     T v[NV];
-#pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = ldsrc<CG>(u + s + (size_t)q * ncell);
-#pragma unroll
-    for (int q = 0; q < NV; ++q) u[d + (size_t)q * ncell] = v[q];
+    load_cell<CG>(u + (size_t)L.src[e], ncell, v);
+    store_cell(u + (size_t)L.dst[e], ncell, v);
 }
 
 // one-dimensional linear interpolation (radial neighbours of different
 // spacing: the other two weights snapped to exactly 0), mixed path only
 template <class T, bool CG = false>
 __device__ __forceinline__ void ghost_lin_one(T* u, const GhostLinList& L, int ncell, int64_t e) {
-    const size_t d = (size_t)L.dst[e], s = (size_t)L.src[e], st = (size_t)L.stride[e];
     const T w = (T)L.w[e], uw = T(1) - w;
-    T v[NV];
+    T v[NV], n[NV];
+    load_cell<CG>(u + (size_t)L.src[e], ncell, v);
+    load_cell<CG>(u + (size_t)L.src[e] + (size_t)L.stride[e], ncell, n);
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        const T* f = u + s + (size_t)q * ncell;
-        v[q] = blend(ldsrc<CG>(f), ldsrc<CG>(f + st), uw, w);
-    }
-#pragma unroll
-    for (int q = 0; q < NV; ++q) u[d + (size_t)q * ncell] = v[q];
+    for (int q = 0; q < NV; ++q) v[q] = blend(v[q], n[q], uw, w);
+    store_cell(u + (size_t)L.dst[e], ncell, v);
 }
 
-// The values of one interpolated/rotated ghost entry (into val); the FP64
-// path is the reference's trilinear form and operand order.
+template <class T>
+__device__ __forceinline__ void ghost_rotate(T (&val)[NV], T a, T c) {
+    T x2 = val[V_BT], x3 = val[V_BP];
+    val[V_BT] = -(a * x2) - c * x3;
+    val[V_BP] = -(a * x3) + c * x2;
+    x2 = val[V_VT]; x3 = val[V_VP];
+    val[V_VT] = -(a * x2) - c * x3;
+    val[V_VP] = -(a * x3) + c * x2;
+}
+// The values of one interpolated/rotated ghost entry (into val): the
+// reference's trilinear form and operand order.
 template <class T, bool CG = false>
-__device__ __forceinline__ void ghost_interp_vals(const T* u, const GhostInterpList& L, int ncell, int nip, int pl,
-                                                  int64_t e, T* val);
-
+__device__ __forceinline__ void ghost_interp_vals(const double* u, const GhostInterpList& L, int ncell, int nip, int pl,
+                                                  int64_t e, double (&val)[NV]) {
+    const int kind = L.kind[e];
+    const size_t s = (size_t)L.src[e];
+    if (kind & 1) {
+        const double wi = L.w[3 * e], wj = L.w[3 * e + 1], wk = L.w[3 * e + 2];
+        const double ui = 1.0 - wi, uj = 1.0 - wj, uk = 1.0 - wk;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const double* f = u + s + (size_t)v * ncell;
+            val[v] = f[0] * ui * uj * uk + f[1] * wi * uj * uk + f[nip] * ui * wj * uk + f[pl] * ui * uj * wk +
+                     f[1 + nip] * wi * wj * uk + f[nip + pl] * ui * wj * wk + f[1 + pl] * wi * uj * wk +
+                     f[1 + nip + pl] * wi * wj * wk;
+        }
+    } else {
+        load_cell<CG>(u + s, ncell, val);
+    }
+    if (kind & 2) ghost_rotate(val, L.rot[2 * e], L.rot[2 * e + 1]);
+}
+// FP32 weights; the Yin-Yang seam is aligned in r (wi == 0 after snapping), so
+// most entries are bilinear in (j, k): four source cells. A cell is two 16-byte
+// reads, so an entry's gather touches 8 sectors where [var][cell] order touched 32
+// (21.2M cells, all entries of a stage: 114 -> 62 us).
+template <class T, bool CG = false>
+__device__ __forceinline__ void ghost_interp_vals(const float* u, const GhostInterpList& L, int ncell, int nip, int pl,
+                                                  int64_t e, float (&val)[NV]) {
+    constexpr int CS = Layout<float>::cell;
+    const int kind = L.kind[e];
+    const float* s = u + (size_t)L.src[e];
+    auto at = [&](int off, float (&v)[NV]) { load_cell<CG>(s + (size_t)CS * off, ncell, v); };
+    const float wi = L.wf[3 * e], wj = L.wf[3 * e + 1], wk = L.wf[3 * e + 2];
+    const float ui = 1.f - wi, uj = 1.f - wj, uk = 1.f - wk;
+    if (!(kind & 1)) {
+        at(0, val);
+    } else if (wi == 0.f) {
+        float f0[NV], f1[NV], f2_[NV], f3[NV];
+        at(0, f0); at(nip, f1); at(pl, f2_); at(nip + pl, f3);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) val[v] = f0[v] * uj * uk + f1[v] * wj * uk + f2_[v] * uj * wk + f3[v] * wj * wk;
+    } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const size_t q = Layout<float>::var(v, ncell);
+            auto f = [&](int off) -> float {
+                const float* p = s + q + (size_t)CS * off;
+                return CG ? __ldcg(p) : *p;
+            };
+            val[v] = f(0) * ui * uj * uk + f(1) * wi * uj * uk + f(nip) * ui * wj * uk + f(pl) * ui * uj * wk +
+                     f(1 + nip) * wi * wj * uk + f(nip + pl) * ui * wj * wk + f(1 + pl) * wi * uj * wk +
+                     f(1 + nip + pl) * wi * wj * wk;
+        }
+    }
+    if (kind & 2) ghost_rotate(val, L.rotf[2 * e], L.rotf[2 * e + 1]);
+}
 template <class T, bool CG = false>
 __device__ __forceinline__ void ghost_interp_one(T* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e) {
     T val[NV];
     ghost_interp_vals<T, CG>(u, L, ncell, nip, pl, e, val);
-    const size_t dd = (size_t)L.dst[e];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) u[dd + (size_t)v * ncell] = val[v];
-}
-
-template <class T, bool CG>
-__device__ __forceinline__ void ghost_interp_vals(const T* u, const GhostInterpList& L, int ncell, int nip, int pl,
-                                                  int64_t e, T* val) {
-    const int kind = L.kind[e];
-    const size_t s = (size_t)L.src[e];
-    if constexpr (!Pol<T>::exact) {
-        // FP32 weights; the Yin-Yang seam is aligned in r (wi == 0 after
-        // snapping), so most entries are bilinear in (j, k): 4 source points
-        const float wi = L.wf[3 * e], wj = L.wf[3 * e + 1], wk = L.wf[3 * e + 2];
-        const float ui = 1.f - wi, uj = 1.f - wj, uk = 1.f - wk;
-        if (!(kind & 1)) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) val[v] = ldsrc<CG>(u + s + (size_t)v * ncell);
-        } else if (wi == 0.f) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const T* f = u + s + (size_t)v * ncell;
-                val[v] = ldsrc<CG>(f + (0)) * uj * uk + ldsrc<CG>(f + (nip)) * wj * uk + ldsrc<CG>(f + (pl)) * uj * wk + ldsrc<CG>(f + (nip + pl)) * wj * wk;
-            }
-        } else {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const T* f = u + s + (size_t)v * ncell;
-                val[v] = ldsrc<CG>(f + (0)) * ui * uj * uk + ldsrc<CG>(f + (1)) * wi * uj * uk + ldsrc<CG>(f + (nip)) * ui * wj * uk + ldsrc<CG>(f + (pl)) * ui * uj * wk +
-                         ldsrc<CG>(f + (1 + nip)) * wi * wj * uk + ldsrc<CG>(f + (nip + pl)) * ui * wj * wk + ldsrc<CG>(f + (1 + pl)) * wi * uj * wk +
-                         ldsrc<CG>(f + (1 + nip + pl)) * wi * wj * wk;
-            }
-        }
-        if (kind & 2) {
-            const float a = L.rotf[2 * e], c = L.rotf[2 * e + 1];
-            T x2 = val[V_BT], x3 = val[V_BP];
-            val[V_BT] = -(a * x2) - c * x3;
-            val[V_BP] = -(a * x3) + c * x2;
-            x2 = val[V_VT]; x3 = val[V_VP];
-            val[V_VT] = -(a * x2) - c * x3;
-            val[V_VP] = -(a * x3) + c * x2;
-        }
-        return;
-    }
-    if (kind & 1) {
-        const T wi = (T)L.w[3 * e], wj = (T)L.w[3 * e + 1], wk = (T)L.w[3 * e + 2];
-        const T ui = T(1) - wi, uj = T(1) - wj, uk = T(1) - wk;
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const T* f = u + s + (size_t)v * ncell;
-            val[v] = ldsrc<CG>(f + (0)) * ui * uj * uk + ldsrc<CG>(f + (1)) * wi * uj * uk + ldsrc<CG>(f + (nip)) * ui * wj * uk + ldsrc<CG>(f + (pl)) * ui * uj * wk +
-                     ldsrc<CG>(f + (1 + nip)) * wi * wj * uk + ldsrc<CG>(f + (nip + pl)) * ui * wj * wk + ldsrc<CG>(f + (1 + pl)) * wi * uj * wk +
-                     ldsrc<CG>(f + (1 + nip + pl)) * wi * wj * wk;
-        }
-    } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) val[v] = ldsrc<CG>(u + s + (size_t)v * ncell);
-    }
-    if (kind & 2) {
-        const T a = (T)L.rot[2 * e], c = (T)L.rot[2 * e + 1];
-        T x2 = val[V_BT], x3 = val[V_BP];
-        val[V_BT] = -(a * x2) - c * x3;
-        val[V_BP] = -(a * x3) + c * x2;
-        x2 = val[V_VT]; x3 = val[V_VP];
-        val[V_VT] = -(a * x2) - c * x3;
-        val[V_VP] = -(a * x3) + c * x2;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// A barrier over every CTA of a cooperative launch (all co-resident). Thread
-// 0 of each CTA reads the generation, arrives on the counter; the last one
-// resets the counter and advances the generation, the others poll it, at most
-// `polls` times (a poll that runs out flags the step: bit 1 of nan_flag, the
-// host returns FALCON_ERR_TIMEOUT, and the CTA goes on). Fences on both sides
-// make every CTA's writes before the barrier visible to every CTA after it.
-struct GridBarrier {
-    unsigned int* count;   // 0 between barriers
-    unsigned int* gen;
-    unsigned int* ticket;  // [5]: the next block of each block phase (4 stages, diffusion), 0 at launch
-};
-__device__ __forceinline__ void grid_sync(const GridBarrier& gb, StepScalars* sc, int polls) {
-    // the next phase reads this one's global writes also through bulk copies
-    // (the async proxy): order them across the proxies on both sides
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned int g0 = *(volatile unsigned int*)gb.gen;
-        __threadfence();
-        if (atomicAdd(gb.count, 1u) == gridDim.x - 1) {
-            atomicExch(gb.count, 0u);
-            __threadfence();
-            atomicAdd(gb.gen, 1u);
-        } else {
-            int it = 0;
-            while (*(volatile unsigned int*)gb.gen == g0) {
-                if (++it > polls) {
-                    atomicOr(&sc->nan_flag, 2);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-}
-
-// The pointers of one mixed step: u^n in U, the stage buffer RK, the second
-// state buffer R2 (u^{n+1} is written there, then the host swaps U and R2).
-struct StepBuffers {
-    float* U;
-    float* RK;
-    float* R2;
-    int8_t* ulo;
-};
-
-// One mixed RK4 step of 16^3 blocks in one persistent launch: the CTAs take
-// the blocks (and, in the exchanges, the ghost entries) in turn and meet at a
-// grid barrier between the phases the graph runs as separate launches:
-// dt, then per stage s the stage kernel's body into seq[s] (pushing the
-// regular ghost faces) and the exchange of the rest (face lists), then the
-// diffusion body into R2 (pushes, next step's CFL minimum) and the exchange
-// of the remaining entries. The bodies are the separate kernels' own
-// (KPAR 2 for the stages, two threads per column for the diffusion: 512
-// threads each, and every variant computes the same bits), so the step
-// equals the graph's bit for bit.
-template <int N>
-__global__ void __launch_bounds__(512, 2)
-k_step_persistent(StepBuffers sb, PushTable push, Geometry g, StepScalars* sc, GhostLists gl_stage,
-                  GhostLists gl_final, StepDims d, GridBarrier gb) {
-    static_assert(N == 16, "16^3 blocks");
-    const int polls = sc->wait_polls;
-    if (blockIdx.x == 0 && threadIdx.x == 0) finalize_dt_body(sc);
-    grid_sync(gb, sc, polls);
-    const int64_t tstride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    auto exchange = [&](const GhostLists& G, float* u) {
-        for (int64_t e = t0; e < G.ip.n; e += tstride)
-            ghost_interp_one<float, true>(u, G.ip, d.ncell, d.nip, d.nip * d.njp, e);
-        for (int64_t e = t0; e < G.ln.n; e += tstride) ghost_lin_one<float, true>(u, G.ln, d.ncell, e);
-        for (int64_t e = t0; e < G.cp.n; e += tstride) ghost_copy_one<float, true>(u, G.cp, d.ncell, e);
-    };
-    // between two bodies in one CTA: the generic writes of the one before
-    // are ordered before the bulk copies of the next into the same memory
-    auto next_body = [&]() {
-        fence_proxy_async();
-        __syncthreads();
-    };
-    // blocks are handed out one at a time from a ticket counter per phase, as
-    // the hardware scheduler hands CTAs to SMs: a CTA that finishes early
-    // takes the next block instead of waiting at the barrier
-    __shared__ int next_b;
-    auto take = [&](int phase) -> int {
-        if (threadIdx.x == 0) next_b = (int)atomicAdd(&gb.ticket[phase], 1u);
-        __syncthreads();
-        return next_b;   // read before the next take's write: a body or next_body() barrier lies between
-    };
-    for (int s = 1; s <= 4; ++s) {
-        float* in = s == 1 ? sb.U : (s == 3 ? sb.R2 : sb.RK);
-        float* out = s == 4 ? sb.U : (s == 2 ? sb.R2 : sb.RK);   // U -> RK -> R2 -> RK -> U
-        for (int b = take(s - 1); b < d.nblocks; b = take(s - 1)) {
-            stage_body<float, 16, 16, 16, 2, 0>(b, in, sb.U, out, sb.ulo, push, DivBArgs{nullptr, nullptr, nullptr, 0},
-                                                g, sc, s, 1, 1);
-            next_body();
-        }
-        grid_sync(gb, sc, polls);
-        exchange(gl_stage, out);
-        grid_sync(gb, sc, polls);
-    }
-    for (int b = take(4); b < d.nblocks; b = take(4)) {
-        march_body<16, 16, 16, 2>(b, sb.U, sb.R2, sb.ulo, push, g, sc, 1);
-        next_body();
-    }
-    grid_sync(gb, sc, polls);
-    exchange(gl_final, sb.R2);
+    store_cell(u + (size_t)L.dst[e], ncell, val);
 }
 
 // ---- block sharding: the entries that cross ranks ---------------------------
@@ -2231,7 +1275,7 @@ __global__ void __launch_bounds__(128) k_shard_pack(const T* u, GhostInterpList 
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= L.n) return;
     T val[NV];
-    ghost_interp_vals(u, L, ncell, nip, pl, e, val);
+    ghost_interp_vals<T>(u, L, ncell, nip, pl, e, val);
 #pragma unroll
     for (int v = 0; v < NV; ++v) pack[e * NV + v] = val[v];
 }
@@ -2302,12 +1346,13 @@ __global__ void __launch_bounds__(256) k_psi_diffusion(const T* u, const T* psi,
 #pragma unroll
     for (int dir = 0; dir < 3; ++dir) {
         const size_t s = strides[dir];
-        const T* vd = u + (size_t)b * NV * d.ncell + (size_t)(V_VR + dir) * d.ncell + (c0 - (size_t)b * d.ncell);
+        const T* vd = u + Layout<T>::at(b, V_VR + dir, c0 - (size_t)b * d.ncell, d.ncell);
+        const ptrdiff_t vs = (ptrdiff_t)(s * Layout<T>::cell);
         auto at = [&](int m) -> T { return psi[(ptrdiff_t)c0 + (ptrdiff_t)m * (ptrdiff_t)s]; };
         const T csm = dir == 0 ? GCS[ii - 1] : GCS[ii];
         const T cs0 = GCS[ii];
         const T csp = dir == 0 ? GCS[ii + 1] : GCS[ii];
-        const T cm = fabs(vd[-(ptrdiff_t)s]) + csm, cz = fabs(vd[0]) + cs0, cp = fabs(vd[s]) + csp;
+        const T cm = fabs(vd[-vs]) + csm, cz = fabs(vd[0]) + cs0, cp = fabs(vd[vs]) + csp;
         const T fm2 = at(-2), fm1 = at(-1), f0 = at(0), fp1 = at(1), fp2 = at(2);
         const T dm1 = minmod(fm2, fm1, f0);
         const T d0 = minmod(fm1, f0, fp1);
@@ -2330,26 +1375,27 @@ __global__ void __launch_bounds__(256) k_psi_diffusion(const T* u, const T* psi,
 }
 
 // GLM psi ghost fill with the state's ghost lists (psi is a scalar: no
-// rotation). List offsets address var 0 of the [b][NV][cell] state; psi's
+// rotation). List offsets address var 0 of a cell of the state (Layout); psi's
 // array is [b][cell].
+template <class T>
 __device__ __forceinline__ size_t psi_off(size_t off, int ncell) {
     const size_t b = off / ((size_t)NV * ncell);
-    return off - b * (size_t)(NV - 1) * ncell;
+    return b * ncell + (off - b * (size_t)NV * ncell) / Layout<T>::cell;
 }
 template <class T>
 __global__ void __launch_bounds__(256) k_psi_ghost(T* psi, GhostLists L, int ncell, int nip, int pl) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t ncp = L.cp.n, nln = L.ln.n, nip_ = L.ip.n;
     if (e < ncp) {
-        psi[psi_off(L.cp.dst[e], ncell)] = psi[psi_off(L.cp.src[e], ncell)];
+        psi[psi_off<T>(L.cp.dst[e], ncell)] = psi[psi_off<T>(L.cp.src[e], ncell)];
     } else if (e < ncp + nln) {
         const int64_t q = e - ncp;
-        const T* f = psi + psi_off(L.ln.src[q], ncell);
+        const T* f = psi + psi_off<T>(L.ln.src[q], ncell);
         const T w = (T)L.ln.w[q];
-        psi[psi_off(L.ln.dst[q], ncell)] = blend(f[0], f[L.ln.stride[q]], T(1) - w, w);
+        psi[psi_off<T>(L.ln.dst[q], ncell)] = blend(f[0], f[L.ln.stride[q] / Layout<T>::cell], T(1) - w, w);
     } else if (e < ncp + nln + nip_) {
         const int64_t q = e - ncp - nln;
-        const T* f = psi + psi_off(L.ip.src[q], ncell);
+        const T* f = psi + psi_off<T>(L.ip.src[q], ncell);
         T val;
         if (!(L.ip.kind[q] & 1)) {
             val = f[0];
@@ -2362,7 +1408,7 @@ __global__ void __launch_bounds__(256) k_psi_ghost(T* psi, GhostLists L, int nce
                   f[1 + nip] * wi * wj * uk + f[nip + pl] * ui * wj * wk + f[1 + pl] * wi * uj * wk +
                   f[1 + nip + pl] * wi * wj * wk;
         }
-        psi[psi_off(L.ip.dst[q], ncell)] = val;
+        psi[psi_off<T>(L.ip.dst[q], ncell)] = val;
     }
 }
 

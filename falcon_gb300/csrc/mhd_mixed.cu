@@ -1,13 +1,86 @@
-// mhd_mixed.cu -- mixed-precision instantiation of the step kernels: FP32
-// state (u^n compensated by an 8-bit correction) and stencil RHS; p1 assembled
-// in FP64; FP64 CFL reduction and dt.
+// mhd_mixed.cu -- launchers of the mixed-precision step kernels: FP32 state
+// (u^n compensated by an 8-bit correction) and stencil RHS; p1 in float-float;
+// FP64 CFL reduction and dt.
 #include "launch_impl.cuh"
+#include "mhd_mixed_impl.cuh"
 
 namespace falcon {
+namespace impl {
+namespace {
+// CTAs per block, each a run of `planes / split` k planes (out of place only: in
+// place, a part would overwrite planes that its neighbours still read). A grid
+// with few blocks leaves SMs idle or unevenly loaded: the split is the power of
+// two that minimises the planes of the busiest SM, counting one more plane per
+// part for the ghost planes it rereads. 108 blocks of 16^3: stage 34.3 us whole,
+// 32.9 in two, 28.9 in four parts (the rule's); diffusion 50, 41, 37. 864 blocks of
+// 8^3: stage 36.3 whole (the rule's), 41.4 in two.
+int split_of(const StepDims& d, int most) {
+    auto cost = [&](int s) { return ((int64_t)d.nblocks * s + 151) / 152 * (d.nk / s + 1); };
+    int best = 1;
+    for (int s = 2; s <= most; s *= 2)
+        if (cost(s) < cost(best)) best = s;
+    return best;
+}
+
+template <int N, int KP, int DIVB>
+cudaError_t stage_nd(const StepDims& d, const Geometry& g, const float* in, const float* un, float* out, int8_t* lo,
+                     const PushTable& push, const DivBArgs& psi, int stage, int bcw, StepScalars* sc, cudaStream_t st) {
+    using S = Shape<float, N, N, N, KP>;
+    static const cudaError_t attr = allow_smem(k_stage_quads<N, N, N, KP, DIVB>, S::smem_stage);
+    if (attr != cudaSuccess) return attr;
+    const int split = in != out ? split_of(d, N / KP) : 1;
+    k_stage_quads<N, N, N, KP, DIVB>
+        <<<d.nblocks * split, S::NT, S::smem_stage, st>>>(in, un, out, lo, push, psi, g, sc, stage, bcw, split);
+    return cudaGetLastError();
+}
+// The div-B mode is a template parameter: the plain stage keeps its register
+// allocation free of the GLM/Powell terms.
+template <int N, int KP>
+cudaError_t stage_n(const StepDims& d, const Geometry& g, const float* in, const float* un, float* out, int8_t* lo,
+                    const PushTable& push, const DivBArgs& psi, int stage, int bcw, StepScalars* sc, cudaStream_t st) {
+    switch (psi.mode) {
+    case 0: return stage_nd<N, KP, 0>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    case 1:
+        if (!psi.in || !psi.un || !psi.out) return cudaErrorInvalidValue;
+        return stage_nd<N, KP, 1>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    case 2: return stage_nd<N, KP, 2>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int N, int KP>
+cudaError_t diff_n(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo, const PushTable& push,
+                   StepScalars* sc, int cfl_next, cudaStream_t st) {
+    using S = DShape<N, N, N, KP>;
+    static const cudaError_t attr = allow_smem(k_diffusion_quads<N, N, N, KP>, S::smem);
+    if (attr != cudaSuccess) return attr;
+    k_diffusion_quads<N, N, N, KP><<<d.nblocks, S::NT, S::smem, st>>>(u, out, lo, push, g, sc, cfl_next);
+    return cudaGetLastError();
+}
+// 16^3 blocks: the k march
+template <int TPC>
+cudaError_t diff_march16(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo,
+                         const PushTable& push, StepScalars* sc, int cfl_next, cudaStream_t st) {
+    using S = MShape<16, 16, 16, TPC>;
+    static const cudaError_t attr = allow_smem(k_march_quads<16, 16, 16, TPC>, S::smem);
+    if (attr != cudaSuccess) return attr;
+    const int split = out != u ? split_of(d, 4) : 1;
+    k_march_quads<16, 16, 16, TPC><<<d.nblocks * split, S::NT, S::smem, st>>>(u, out, lo, push, g, sc, cfl_next, split);
+    return cudaGetLastError();
+}
+}  // namespace
+}  // namespace impl
+
 cudaError_t launch_stage_mixed(const StepDims& d, const Geometry& g, const float* in, const float* un, float* out,
                                int8_t* lo, const PushTable& push, const DivBArgs& psi, int stage, int bcw, StepScalars* sc,
-                               int heat, int kpar, cudaStream_t st) {
-    return impl::stage_any<float>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, heat, kpar, st);
+                               int kpar, cudaStream_t st) {
+#define FALCON_STAGE_CASE(N, K) \
+    if (d.ni == N && kpar == K) return impl::stage_n<N, K>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    if (d.ni != d.nj || d.ni != d.nk) return cudaErrorInvalidValue;
+    FALCON_STAGE_CASE(8, 2) FALCON_STAGE_CASE(8, 4) FALCON_STAGE_CASE(8, 8)
+    FALCON_STAGE_CASE(16, 1) FALCON_STAGE_CASE(16, 2) FALCON_STAGE_CASE(16, 4)
+#undef FALCON_STAGE_CASE
+    return cudaErrorInvalidValue;
 }
 cudaError_t launch_psi_diffusion_mixed(const StepDims& d, const Geometry& g, const float* u, const float* psi,
                                        float* psi_out, StepScalars* sc, cudaStream_t st) {
@@ -16,9 +89,22 @@ cudaError_t launch_psi_diffusion_mixed(const StepDims& d, const Geometry& g, con
 cudaError_t launch_psi_ghost_mixed(const StepDims& d, const GhostLists& gl, float* psi, cudaStream_t st) {
     return impl::psi_ghost_any<float>(d, gl, psi, st);
 }
+// 16^3 blocks: the k-chunk depth asked for selects one thread per column (1) or
+// two (2 and 4); 8^3 blocks: planes per chunk
 cudaError_t launch_diffusion_mixed(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo,
                                    const PushTable& push, StepScalars* sc, int kpar, cudaStream_t st, int cfl_next) {
-    return impl::diff_any<float>(d, g, u, out, lo, push, sc, kpar, st, cfl_next);
+    if (push.tgt != nullptr && out == u) return cudaErrorInvalidValue;   // pushing needs out != u
+    if (d.ni != d.nj || d.ni != d.nk) return cudaErrorInvalidValue;
+    if (d.ni == 16)
+        return kpar == 1 ? impl::diff_march16<1>(d, g, u, out, lo, push, sc, cfl_next, st)
+                         : impl::diff_march16<2>(d, g, u, out, lo, push, sc, cfl_next, st);
+    if (d.ni != 8) return cudaErrorInvalidValue;
+    switch (kpar) {
+    case 2: return impl::diff_n<8, 2>(d, g, u, out, lo, push, sc, cfl_next, st);
+    case 4: return impl::diff_n<8, 4>(d, g, u, out, lo, push, sc, cfl_next, st);
+    case 8: return impl::diff_n<8, 8>(d, g, u, out, lo, push, sc, cfl_next, st);
+    }
+    return cudaErrorInvalidValue;
 }
 cudaError_t launch_cfl_mixed(const StepDims& d, const Geometry& g, const float* u, StepScalars* sc, cudaStream_t st) {
     return impl::cfl_any<float>(d, g, u, sc, st);
@@ -26,10 +112,19 @@ cudaError_t launch_cfl_mixed(const StepDims& d, const Geometry& g, const float* 
 cudaError_t launch_ghost_mixed(const StepDims& d, const GhostLists& gl, float* u, cudaStream_t st) {
     return impl::ghost_any<float>(d, gl, u, st);
 }
-int kpar_candidates_mixed(const StepDims& d, int* out) { return impl::candidates<float>(d, out); }
+// k-chunk depths instantiated per block size; the context's autotuner times
+// them on its own grid and keeps the fastest.
+int kpar_candidates_mixed(const StepDims& d, int* out) {
+    const int first = d.ni == 16 ? 1 : d.ni == 8 ? 2 : 0;
+    for (int q = 0; q < 3 && first; ++q) out[q] = first << q;
+    return first ? 3 : 0;
+}
 cudaError_t launch_clear_outside_core_mixed(const StepDims& d, float* u, int nvar, cudaStream_t st) {
-    const int64_t nbv = (int64_t)d.nblocks * nvar;
-    impl::k_clear_outside_core<float><<<(unsigned)(nbv < 65535 * 4 ? nbv : 65535 * 4), 256, 0, st>>>(u, nbv, d);
+    const int64_t n = nvar == NV ? (int64_t)d.nblocks * 2 : d.nblocks;   // the state's halves, or a [b][cell] array
+    const unsigned grid = (unsigned)(n < 65535 * 4 ? n : 65535 * 4);
+    if (nvar == NV) impl::k_clear_outside_core<float4><<<grid, 256, 0, st>>>(reinterpret_cast<float4*>(u), n, d);
+    else if (nvar == 1) impl::k_clear_outside_core<float><<<grid, 256, 0, st>>>(u, n, d);
+    else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 cudaError_t launch_push_state_mixed(const StepDims& d, const Geometry& g, float* u, const PushTable& push,

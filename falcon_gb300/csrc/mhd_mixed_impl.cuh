@@ -1,0 +1,1219 @@
+// mhd_mixed_impl.cuh -- kernels of the mixed step: FP32 state [b][half][cell][4]
+// (Layout), u^n compensated by an 8-bit correction [b][interior cell][8].
+// Included by mhd_mixed.cu.
+#pragma once
+#include "mhd_impl.cuh"
+
+namespace falcon {
+namespace impl {
+
+// the four values of half `h` of padded cell c of block b
+__device__ __forceinline__ size_t quad(int b, int h, int ncell) { return ((size_t)b * 2 + h) * ncell; }
+__device__ __forceinline__ const float4* quads(const float* u) { return reinterpret_cast<const float4*>(u); }
+__device__ __forceinline__ float4* quads(float* u) { return reinterpret_cast<float4*>(u); }
+__device__ __forceinline__ float4 f4(const float* v) { return make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void split(float4 a, float4 b, float (&v)[NV]) {
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// Thread 0: bulk-copy planes kp in [lo, hi) of both halves of the block into
+// their ring slots (plane kp in slot (kp - p0) % W), completing on `bar`.
+template <class S>
+__device__ __forceinline__ void issue_quads(const float* blk, float4* tile, int lo, int hi, int p0, uint64_t* bar) {
+    mbar_expect_tx(bar, (uint32_t)(2 * (hi - lo)) * S::PL * 16u);
+    for (int h = 0; h < 2; ++h)
+        for (int kp = lo; kp < hi; ++kp)
+            tma_load_1d(tile + ((size_t)h * S::W + (kp - p0) % S::W) * S::PL,
+                        quads(blk) + ((size_t)h * S::NKP + kp) * S::PL, S::PL * 16u, bar);
+}
+
+// Radial mirror boundary (3_6/ModBoundary.f90:10-55) on planes [lo, hi) of the
+// ring, whole rows including their theta ghosts; optionally written back.
+template <class S>
+__device__ __forceinline__ void apply_bc_quads(float4* tile, int lo, int hi, int p0, int fl, float* wb, int nt) {
+    const bool top = fl & 2, bot = fl & 4;
+    if (!top && !bot) return;
+    const int NI = S::NIP - 4;
+    // top mirrors rho1, vt, vp, s1, br and anti-mirrors vr, bt, bp; bottom
+    // mirrors rho1, vt, vp, s1, bt, bp and anti-mirrors vr, br
+    const int total = (hi - lo) * S::NJP * 4;
+    for (int x = threadIdx.x; x < total; x += nt) {
+        const int g = x & 1, h = (x >> 1) & 1, rest = x >> 2, j = rest % S::NJP, kp = lo + rest / S::NJP;
+        float4* row = tile + ((size_t)h * S::W + (kp - p0) % S::W) * S::PL + j * S::NIP;
+        float4* out = wb ? quads(wb) + ((size_t)h * S::NKP + kp) * S::PL + j * S::NIP : nullptr;
+        if (top) {   // Fortran i = ni+1+g <- 2*ni+1-i = ni-g ; padded index = Fortran + 1
+            float4 s = row[NI - g + 1];
+            s = h ? make_float4(s.x, -s.y, -s.z, s.w) : make_float4(s.x, -s.y, s.z, s.w);
+            row[NI + 2 + g] = s;
+            if (out) out[NI + 2 + g] = s;
+        }
+        if (bot) {   // Fortran i = -g <- 1-i = 1+g
+            float4 s = row[2 + g];
+            s = h ? make_float4(-s.x, s.y, s.z, s.w) : make_float4(s.x, -s.y, s.z, s.w);
+            row[1 - g] = s;
+            if (out) out[1 - g] = s;
+        }
+    }
+}
+
+// Write this cell's new values into the ghost cells of the neighbours whose
+// faces are pushed (PushTable): halves [H0, H0 + NH) of the cell, o its values.
+// (ii, jj, kp): padded indices. Theta/phi faces: the two interior layers next to
+// the side are copied to the target's opposite ghost layers (a shift of one
+// block extent). Radial faces: the thread at the first source cell of a ghost
+// layer blends it with the next cell along i, taken from the next lane (i is
+// the fastest thread index, and the second cell is never beyond the row). Every
+// write is whole 16-byte cells, the two layers of a radial face one sector.
+// Every thread of the warp calls this (the shuffle needs it).
+template <class S, int NH, int H0>
+__device__ __forceinline__ void push_quads(float* out, const PushBlock& P, int ii, int jj, int kp, const float (&o)[4 * NH]) {
+    constexpr int NJ = S::NJP - 4, NK = S::NKP - 4;
+    const int32_t* tg = P.tgt;
+    auto put = [&](int tb, int kt, int jt, int it, const float (&val)[4 * NH]) {
+        float4* dst = quads(out) + quad(tb, H0, S::NCELL) + ((size_t)kt * S::NJP + jt) * S::NIP + it;
+#pragma unroll
+        for (int h = 0; h < NH; ++h) dst[(size_t)h * S::NCELL] = f4(val + 4 * h);
+    };
+    if (jj <= 3 && tg[2] >= 0) put(tg[2], kp, jj + NJ, ii, o);
+    if (jj >= NJ && tg[3] >= 0) put(tg[3], kp, jj - NJ, ii, o);
+    if (kp <= 3 && tg[4] >= 0) put(tg[4], kp + NK, jj, ii, o);
+    if (kp >= NK && tg[5] >= 0) put(tg[5], kp - NK, jj, ii, o);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        if (tg[side] < 0) continue;   // uniform over the CTA
+        const float w0 = P.w[2 * side], w1 = P.w[2 * side + 1];
+        const bool l0 = ii == P.src[2 * side], l1 = ii == P.src[2 * side + 1];
+        if (w0 == 0.f && w1 == 0.f) {   // copies
+            if (l0) put(tg[side], kp, jj, P.dst[2 * side], o);
+            if (l1) put(tg[side], kp, jj, P.dst[2 * side + 1], o);
+            continue;
+        }
+        float nx[4 * NH];
+#pragma unroll
+        for (int v = 0; v < 4 * NH; ++v) nx[v] = __shfl_down_sync(0xffffffffu, o[v], 1);
+#pragma unroll
+        for (int layer = 0; layer < 2; ++layer) {
+            if (!(layer ? l1 : l0)) continue;
+            const float w = layer ? w1 : w0, uw = 1.f - w;
+            float val[4 * NH];
+#pragma unroll
+            for (int v = 0; v < 4 * NH; ++v) val[v] = w == 0.f ? o[v] : blend(o[v], nx[v], uw, w);
+            put(tg[side], kp, jj, P.dst[2 * side + layer], val);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// One RK stage of a block, or of planes [ch0, ch1) x KPAR of it: boundary -> RHS
+// (3_6/ModEquation.f90:24-162) -> u_out = u^n + dt*R/(5-s)
+// (3_6/ModAdvance.f90:87-93). A chunk of KPAR planes is a thread per cell; the
+// derivatives are formed direction by direction, each from the four neighbours'
+// eight values read as two 16-byte accesses, so that a cell takes 26
+// shared-memory reads for its 13 points instead of one per value and use.
+// 21.2M cells: 919 -> 877 us per stage (152 B of HBM traffic a cell instead of
+// 236); 442k cells with split blocks: 37 -> 29.8 us.
+template <int NI, int NJ, int NK, int KPAR, int DIVB>
+__device__ __forceinline__ void stage_quads(int b, int ch0, int ch1, const float* in, const float* un, float* out,
+                                            int8_t* ulo, const PushTable& push, const DivBArgs& psi, const Geometry& g,
+                                            StepScalars* sc, int stage, int bc_writeback) {
+    using S = Shape<float, NI, NJ, NK, KPAR>;
+    using T = float;
+    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, WP = S::WP, NCELL = S::NCELL;
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+    double* a12 = reinterpret_cast<double*>(smem + S::off_a12);
+    float4* tile = reinterpret_cast<float4*>(smem + S::off_tile);   // [2][W][PL]
+    T* tp1 = reinterpret_cast<T*>(smem + S::off_p1);
+    T* gi = reinterpret_cast<T*>(smem + S::off_gi);
+    T* gj = reinterpret_cast<T*>(smem + S::off_gj);
+    T* gs = reinterpret_cast<T*>(smem + S::off_gs);
+    static_assert(S::off_tile % 16 == 0, "16-byte cells");
+
+    const int fl = g.flags[b];
+    const float* blk_in = in + (size_t)b * NV * NCELL;
+    float* wb = bc_writeback ? const_cast<float*>(blk_in) : nullptr;
+    __shared__ PushBlock pb;
+    load_push_block(push, b, &pb);
+    if (threadIdx.x == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) issue_quads<S>(blk_in, tile, ch0 * KPAR, ch0 * KPAR + KPAR + 4, 0, &bars[0]);
+    // u^n (and its int8 correction at stage 4) is read with plain loads at
+    // stages 2-4: warm L2 with the rows of the first chunk, then one chunk ahead
+    auto prefetch_un = [&](int kp_first) {
+        if (stage == 1) return;
+        for (int x = threadIdx.x; x < 2 * KPAR * NJ; x += S::NT) {   // a row of one half: NI cells of 16 bytes
+            const int h = x & 1, r = x >> 1, j = r % NJ, q = r / NJ;
+            prefetch_l2(quads(un) + quad(b, h, NCELL) + (size_t)(kp_first + q) * PL + (j + 2) * NIP + 2, NI * 16u);
+        }
+        if (ulo != nullptr && stage == 4 && threadIdx.x == 0)
+            prefetch_l2(ulo + ((size_t)b * S::NINT + (size_t)(kp_first - 2) * S::PLI) * NV, KPAR * S::PLI * NV);
+    };
+    prefetch_un(ch0 * KPAR + 2);
+    load_geometry<T, S>(g, b, gi, gj, gs, a12);
+    __syncthreads();   // the geometry tables are read by every thread below
+
+    const int tid = threadIdx.x;
+    int i, j, kq;
+    cell_of_thread<NI, NJ, KPAR>(tid, i, j, kq);
+    const int ii = i + 2, jj = j + 2;
+    const T c1 = gs[GS_C1], c2 = gs[GS_C2], c3 = gs[GS_C3];
+    const T* GR = gi + GI_R * NIP;
+    const T* GR2 = gi + GI_R2 * NIP;
+    const T* GRHO0 = gi + GI_RHO0 * NIP;
+    const T* GSIN = gj + GJ_SIN * S::NJP;
+    const T rinv = gi[GI_RINV * NIP + ii], r2inv = gi[GI_R2INV * NIP + ii];
+    const T sinv = gj[GJ_SININV * S::NJP + jj], cot = gj[GJ_COT * S::NJP + jj];
+    const T rho0c = GRHO0[ii], rho0inv = gi[GI_RHO0INV * NIP + ii];
+    const T gor0 = gi[GI_GOR0 * NIP + ii], heat = gi[GI_HEAT * NIP + ii], xi2inv = gi[GI_XI2INV * NIP + ii];
+    const float dtk = sc->dt_stage_f[stage - 1];
+    const int polls = sc->wait_polls;
+    int late = 0;   // a wait of this thread for a chunk's planes ran out
+    for (int ch = ch0; ch < ch1; ++ch) {
+        const int n = ch - ch0;
+        const int k0 = 1 + ch * KPAR;  // first Fortran k of the chunk
+        const int lo = n == 0 ? ch * KPAR : k0 + 3;   // first padded plane new to this chunk
+        const int hi = k0 + KPAR + 3;                 // one past the last plane it needs
+        // the chunk before is done with the slots the prefetch below overwrites; a
+        // wait of it that ran out ends the CTA here
+        if (__syncthreads_or(late)) {
+            copy_wait_abort(sc, bars, n - 1, n);
+            return;
+        }
+        if (threadIdx.x == 0 && ch + 1 < ch1) issue_quads<S>(blk_in, tile, hi, hi + KPAR, 0, &bars[(n + 1) & 1]);
+        if (ch + 1 < ch1) prefetch_un(k0 + KPAR + 1);
+        // a wait that runs out does not leave the chunk (its barriers must be
+        // reached by every thread): the chunk computes on whatever the slots
+        // hold, the step is flagged and its results are discarded
+        late |= mbar_wait(&bars[n & 1], (uint32_t)((n >> 1) & 1), polls) ? 0 : 1;
+        // u^n for the update (stages 2-4), loaded here so that the latency of
+        // these plain loads overlaps the boundary and p1 phases below
+        const int kp = k0 + kq + 1;
+        const size_t cell = (size_t)kp * PL + jj * NIP + ii;
+        float4 ua = make_float4(0.f, 0.f, 0.f, 0.f), ub = ua;
+        if (stage != 1) {
+            ua = quads(un)[quad(b, 0, NCELL) + cell];
+            ub = quads(un)[quad(b, 1, NCELL) + cell];
+        }
+        if (fl & 6) {   // radial boundary block (uniform over the CTA)
+            apply_bc_quads<S>(tile, lo, hi, 0, fl, wb, S::NT);
+            fence_proxy_async();   // order these generic writes before later bulk copies into the slots
+            __syncthreads();
+        }
+        // p1 = gamma1*(p0/rho0)*rho1 + (gamma3-1)*(rho0*T0)*s1 (3_6/ModEquation.f90:40-46)
+        for (int x = tid; x < (hi - lo) * PL; x += S::NT) {
+            const int kx = lo + x / PL, c = x % PL, ic = c % NIP, slot = kx % W;
+            const float* f = reinterpret_cast<const float*>(a12);
+            tp1[(kx % WP) * PL + c] = p1_ff(f[ic], f[NIP + ic], f[2 * NIP + ic], f[3 * NIP + ic],
+                                            tile[slot * PL + c].x, tile[(W + slot) * PL + c].w);
+        }
+        __syncthreads();
+
+        int sl[5], sp[5];
+#pragma unroll
+        for (int d = 0; d < 5; ++d) { sl[d] = (kp + d - 2) % W * PL + jj * NIP + ii; sp[d] = (kp + d - 2) % WP * PL + jj * NIP + ii; }
+        const float4* ta = tile;
+        const float4* tb = tile + W * PL;
+        // ModDerivative_1st_O4_3D (3_6/ModDerivative.f90:16-32)
+        auto D = [&](T c, auto f) -> T { return c * (((-f(2) + T(8) * f(1)) - T(8) * f(-1)) + f(-2)); };
+        const float4 ca = ta[sl[2]], cb = tb[sl[2]];
+        const T rho1 = ca.x, vr = ca.y, vt = ca.z, vp = ca.w, br = cb.x, bt = cb.y, bp = cb.z;
+        if (stage == 1) {   // the input is u^n and sits in the ring
+            ua = ca;
+            ub = cb;
+        }
+        T dA, a_vr, a_vt, a_vp, a_s1, g1, d_bpr, d_btr, q_e3r, q_e2r, dB = T(0);
+        {   // along i
+            float4 A[5], B[5];
+            T P[5];
+#pragma unroll
+            for (int m = -2; m <= 2; ++m) {
+                if (m == 0) continue;
+                A[m + 2] = ta[sl[2] + m];
+                B[m + 2] = tb[sl[2] + m];
+                P[m + 2] = tp1[sp[2] + m];
+            }
+            auto E2 = [&](int m) { return A[m + 2].w * B[m + 2].x - A[m + 2].y * B[m + 2].z; };
+            auto E3 = [&](int m) { return A[m + 2].y * B[m + 2].y - A[m + 2].z * B[m + 2].x; };
+            dA = D(c1, [&](int m) { return (GRHO0[ii + m] * A[m + 2].y) * GR2[ii + m]; });
+            dA = dA * r2inv;
+            a_vr = vr * D(c1, [&](int m) { return A[m + 2].y; });
+            a_vt = vr * D(c1, [&](int m) { return A[m + 2].z; });
+            a_vp = vr * D(c1, [&](int m) { return A[m + 2].w; });
+            a_s1 = vr * D(c1, [&](int m) { return B[m + 2].w; });
+            g1 = D(c1, [&](int m) { return P[m + 2]; });
+            d_bpr = D(c1, [&](int m) { return B[m + 2].z * GR[ii + m]; });
+            d_btr = D(c1, [&](int m) { return B[m + 2].y * GR[ii + m]; });
+            q_e3r = D(c1, [&](int m) { return E3(m) * GR[ii + m]; });
+            q_e2r = D(c1, [&](int m) { return E2(m) * GR[ii + m]; });
+            if constexpr (DIVB != 0) dB = D(c1, [&](int m) { return B[m + 2].x * GR2[ii + m]; });
+        }
+        T d23, g2, k1, k3, q1, q3, e23 = T(0);
+        {   // along j
+            float4 A[5], B[5];
+            T P[5];
+#pragma unroll
+            for (int m = -2; m <= 2; ++m) {
+                if (m == 0) continue;
+                A[m + 2] = ta[sl[2] + m * NIP];
+                B[m + 2] = tb[sl[2] + m * NIP];
+                P[m + 2] = tp1[sp[2] + m * NIP];
+            }
+            auto E1 = [&](int m) { return A[m + 2].z * B[m + 2].z - A[m + 2].w * B[m + 2].y; };
+            auto E3 = [&](int m) { return A[m + 2].y * B[m + 2].y - A[m + 2].z * B[m + 2].x; };
+            d23 = D(c2, [&](int m) { return (rho0c * A[m + 2].z) * GSIN[jj + m]; });
+            T t = vt * D(c2, [&](int m) { return A[m + 2].y; });
+            a_vr = a_vr + t * rinv;
+            t = vt * D(c2, [&](int m) { return A[m + 2].z; });
+            a_vt = a_vt + t * rinv;
+            t = vt * D(c2, [&](int m) { return A[m + 2].w; });
+            a_vp = a_vp + t * rinv;
+            t = vt * D(c2, [&](int m) { return B[m + 2].w; });
+            a_s1 = a_s1 + t * rinv;
+            g2 = D(c2, [&](int m) { return P[m + 2]; });
+            k1 = D(c2, [&](int m) { return B[m + 2].z * GSIN[jj + m]; });
+            k3 = d_btr - D(c2, [&](int m) { return B[m + 2].x; });
+            q1 = D(c2, [&](int m) { return E3(m) * GSIN[jj + m]; });
+            q3 = q_e2r - D(c2, [&](int m) { return E1(m); });
+            if constexpr (DIVB != 0) e23 = D(c2, [&](int m) { return B[m + 2].y * GSIN[jj + m]; });
+        }
+        T g3, k2, q2;
+        {   // along k
+            float4 A[5], B[5];
+            T P[5];
+#pragma unroll
+            for (int m = -2; m <= 2; ++m) {
+                if (m == 0) continue;
+                A[m + 2] = ta[sl[m + 2]];
+                B[m + 2] = tb[sl[m + 2]];
+                P[m + 2] = tp1[sp[m + 2]];
+            }
+            auto E1 = [&](int m) { return A[m + 2].z * B[m + 2].z - A[m + 2].w * B[m + 2].y; };
+            auto E2 = [&](int m) { return A[m + 2].w * B[m + 2].x - A[m + 2].y * B[m + 2].z; };
+            d23 = d23 + D(c3, [&](int m) { return rho0c * A[m + 2].w; });
+            T t = vp * D(c3, [&](int m) { return A[m + 2].y; });
+            t = t * rinv;
+            a_vr = a_vr + sinv * t;
+            t = vp * D(c3, [&](int m) { return A[m + 2].z; });
+            t = t * rinv;
+            a_vt = a_vt + sinv * t;
+            t = vp * D(c3, [&](int m) { return A[m + 2].w; });
+            t = t * rinv;
+            a_vp = a_vp + sinv * t;
+            t = vp * D(c3, [&](int m) { return B[m + 2].w; });
+            t = t * rinv;
+            a_s1 = a_s1 + sinv * t;
+            g3 = D(c3, [&](int m) { return P[m + 2]; });
+            k1 = k1 - D(c3, [&](int m) { return B[m + 2].y; });
+            k2 = D(c3, [&](int m) { return B[m + 2].x * sinv; }) - d_bpr;
+            q1 = q1 - D(c3, [&](int m) { return E2(m); });
+            q2 = D(c3, [&](int m) { return E1(m) * sinv; }) - q_e3r;
+            if constexpr (DIVB != 0) e23 = e23 + D(c3, [&](int m) { return B[m + 2].z; });
+        }
+        // Mass conservation: -div(rho0 v)/Xi^2 (3_6/ModEquation.f90:50-61, ModSpherical_div :104-159)
+        d23 = d23 * sinv;
+        d23 = d23 * rinv;
+        const T Rrho = -(xi2inv * (dA + d23));
+        // Inertial force -(v.grad)v with curvature terms (3_6/ModSpherical.f90:281-343)
+        T Rvr, Rvt, Rvp;
+        {
+            T tmp = -(vt * vt) - vp * vp;
+            a_vr = a_vr + tmp * rinv;
+            tmp = -(vp * vp);
+            tmp = tmp * cot;
+            tmp = tmp + vt * vr;
+            a_vt = a_vt + tmp * rinv;
+            tmp = vp * vt;
+            tmp = tmp * cot;
+            tmp = tmp + vp * vr;
+            a_vp = a_vp + tmp * rinv;
+            Rvr = -a_vr; Rvt = -a_vt; Rvp = -a_vp;
+        }
+        // Pressure gradient -grad(p1)/rho0 (3_6/ModEquation.f90:79-92)
+        g2 = g2 * rinv;
+        g3 = g3 * rinv;
+        g3 = g3 * sinv;
+        Rvr = Rvr - g1 * rho0inv;
+        Rvt = Rvt - g2 * rho0inv;
+        Rvp = Rvp - g3 * rho0inv;
+        // Lorentz force (curl B) x B / rho0 (3_6/ModEquation.f90:97-116, curl :38-102)
+        {
+            k1 = k1 * rinv; k2 = k2 * rinv; k3 = k3 * rinv;
+            k1 = k1 * sinv;
+            const T x1 = k2 * bp - k3 * bt;
+            const T x2 = k3 * br - k1 * bp;
+            const T x3 = k1 * bt - k2 * br;
+            Rvr = Rvr + x1 * rho0inv;
+            Rvt = Rvt + x2 * rho0inv;
+            Rvp = Rvp + x3 * rho0inv;
+        }
+        // Buoyancy -(g/rho0) rho1 (3_6/ModEquation.f90:121-127)
+        Rvr = Rvr - gor0 * rho1;
+        // Entropy advection and heating (3_6/ModEquation.f90:132-151)
+        T Rs = -a_s1;
+        Rs = Rs + heat;
+        // Induction curl(v x B) (3_6/ModEquation.f90:154-162)
+        q1 = q1 * rinv; q2 = q2 * rinv; q3 = q3 * rinv;
+        q1 = q1 * sinv;
+        T RBr = q1, RBt = q2, RBp = q3;
+
+        // div-B control. GLM cleaning (3_6/ModDivB.f90:13-38), after the
+        // equation terms as 3_6/ModAdvance.f90:82-84 orders it: dB += -grad(psi);
+        // dpsi = -v_wave^2 div(B) - v_wave/h_LLL psi, v_wave from u^n. Powell
+        // (3_5/ModEquation.f90:169-176): dB += -(div B) v.
+        T divB = T(0);
+        if constexpr (DIVB != 0) {   // ModSpherical_div of B (3_6/ModSpherical.f90:104-159)
+            dB = dB * r2inv;
+            e23 = e23 * sinv;
+            e23 = e23 * rinv;
+            divB = dB + e23;
+        }
+        if constexpr (DIVB == 2) {
+            RBr = RBr - divB * vr;
+            RBt = RBt - divB * vt;
+            RBp = RBp - divB * vp;
+        }
+        if constexpr (DIVB == 1) {
+            const T* P = static_cast<const T*>(psi.in) + (size_t)b * NCELL + cell;
+            auto Q = [&](int di, int dj, int dk) -> T { return P[(ptrdiff_t)dk * PL + dj * NIP + di]; };
+            // ModSpherical_Grad_f (3_6/ModSpherical.f90:201-239)
+            const T h1 = D(c1, [&](int m) { return Q(m, 0, 0); });
+            T h2 = D(c2, [&](int m) { return Q(0, m, 0); });
+            h2 = h2 * rinv;
+            T h3 = D(c3, [&](int m) { return Q(0, 0, m); });
+            h3 = h3 * rinv;
+            h3 = h3 * sinv;
+            RBr = RBr - h1;
+            RBt = RBt - h2;
+            RBp = RBp - h3;
+            // ModWaveSpeed_Dynamo (3_6/ModWaveSpeed.f90:8-27) and h_LLL
+            // (3_6/ModBlock.f90:416-425) at this cell, as the CFL pass forms them
+            T w = gi[GI_CS * NIP + ii] + sqrt(ua.y * ua.y + ua.z * ua.z + ua.w * ua.w);
+            w = w + sqrt(ub.x * ub.x + ub.y * ub.y + ub.z * ub.z) / sqrt(rho0c);
+            const T rcell = GR[ii];
+            const T h = fmin(fmin(gs[GS_DXI], rcell * gs[GS_DXJ]), rcell * GSIN[jj] * gs[GS_DXK]);
+            const T Rpsi = -(w * w * divB) - w / h * Q(0, 0, 0);
+            const size_t pc = (size_t)b * NCELL + cell;
+            const T pn = static_cast<const T*>(psi.un)[pc];
+            static_cast<T*>(psi.out)[pc] = fmaf(dtk, Rpsi, pn);
+        }
+
+        // stage update
+        const T R[NV] = {Rrho, Rvr, Rvt, Rvp, RBr, RBt, RBp, Rs};
+        T u0s[NV], o[NV];
+        split(ua, ub, u0s);
+        if (ulo != nullptr && stage == 4) {
+            // u^{n+1} = u^n + dt*R with u^n and u^{n+1} compensated
+            int2* ql = reinterpret_cast<int2*>(ulo + ((size_t)b * S::NINT + ((size_t)(kp - 2) * NJ + j) * NI + i) * NV);
+            const int2 q8 = *ql;
+            int qn[2] = {0, 0};
+#pragma unroll
+            for (int v = 0; v < NV; v += 2) {   // pairs of variables: ff_add2 gives ff_add's bits
+                const int q = v < 4 ? q8.x : q8.y, sh = 8 * (v & 3);
+                int8_t qa, qb;
+                const float2 ov = ff_add2(f2(u0s[v], u0s[v + 1]), (int8_t)(q >> sh), (int8_t)(q >> (sh + 8)),
+                                          __fmul2_rn(f2(dtk), f2(R[v], R[v + 1])), qa, qb);
+                o[v] = ov.x;
+                o[v + 1] = ov.y;
+                qn[v >> 2] |= ((int)(uint8_t)qa | (int)(uint8_t)qb << 8) << sh;
+            }
+            *ql = make_int2(qn[0], qn[1]);
+        } else {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) o[v] = fmaf(dtk, R[v], u0s[v]);
+        }
+        quads(out)[quad(b, 0, NCELL) + cell] = f4(o);
+        quads(out)[quad(b, 1, NCELL) + cell] = f4(o + 4);
+        if (push.tgt != nullptr) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+    }
+    const int nch = ch1 - ch0;
+    if (__syncthreads_or(late)) {
+        copy_wait_abort(sc, bars, nch - 1, nch - 1);
+        return;
+    }
+    if (threadIdx.x == 0) {   // every copy has been waited for
+        mbar_inval(&bars[0]);
+        mbar_inval(&bars[1]);
+    }
+}
+// split CTAs per block, each a run of whole chunks
+template <int NI, int NJ, int NK, int KPAR, int DIVB>
+__global__ void __launch_bounds__(NI* NJ* KPAR, (Shape<float, NI, NJ, NK, KPAR>::min_blocks))
+k_stage_quads(const float* in, const float* un, float* out, int8_t* ulo, PushTable push, DivBArgs psi, Geometry g,
+              StepScalars* sc, int stage, int bc_writeback, int split) {
+    const int b = blockIdx.x / split, part = blockIdx.x - b * split, n = NK / KPAR / split;
+    stage_quads<NI, NJ, NK, KPAR, DIVB>(b, part * n, (part + 1) * n, in, un, out, ulo, push, psi, g, sc, stage, bc_writeback);
+}
+
+// ---------------------------------------------------------------------------
+// FP32 artificial diffusion (3_6/ModDiffusion.f90:9-150, h = 2) and the update
+// u += 0.5*dt*R (3_6/ModAdvance.f90:101-108) of 8^3 blocks, a chunk of KPAR
+// planes at a time (a thread per cell). Each face flux is formed once per chunk
+// into shared memory: i and j faces of the chunk's planes, and the k faces in a
+// ring of KPAR+1 face planes (the last face of a chunk is the first of the
+// next). Then each cell sums (F_left - F_right)/den over the three directions,
+// in the reference's order. Out of place (out != u) the kernel also writes the
+// regular ghost faces of its neighbours in `out` and copies the radial
+// physical-boundary ghost columns (set by the boundary condition at stage 1);
+// cfl_next: the outputs are the next step's u^n, so it forms the next step's CFL
+// minimum and NaN flag from them (k_cfl's formula, cfl_ratio_f).
+template <int NI, int NJ, int NK, int KPAR>
+struct DShape : Shape<float, NI, NJ, NK, KPAR> {
+    using B = Shape<float, NI, NJ, NK, KPAR>;
+    static constexpr int NT = NI * NJ * KPAR;
+    static constexpr int KS = KPAR + 1;                  // k-face ring slots
+    static constexpr int FIP = NI + 1;                   // i-face row pitch
+    static constexpr int NFI = NV * KPAR * NJ * FIP;
+    static constexpr int NFJ = NV * KPAR * (NJ + 1) * NI;
+    static constexpr int NFK = KS * NV * NJ * NI;
+    // shared memory: mbarriers | tile[2][W][PL] of 16 bytes | FI | FJ | FK | gi | gj | gs
+    static constexpr size_t off_tile = 16;
+    static constexpr size_t off_fi = off_tile + (size_t)NV * B::W * B::PL * 4;
+    static constexpr size_t off_fj = off_fi + (size_t)NFI * 4;
+    static constexpr size_t off_fk = off_fj + (size_t)NFJ * 4;
+    static constexpr size_t off_gi = off_fk + (size_t)NFK * 4;
+    static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * B::NIP * 4;
+    static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * B::NJP * 4;
+    static constexpr size_t smem = off_gs + GS_COUNT * 4;
+    static_assert(smem <= 232448, "227 KB of opt-in shared memory per CTA");
+    static constexpr int by_smem = (int)(233472 / (smem + 1024));
+    static constexpr int reg_cap = 2048 / NT;
+    static constexpr int min_blocks = by_smem < 2 ? 1 : (by_smem < reg_cap ? by_smem : (reg_cap < 1 ? 1 : reg_cap));
+};
+
+// radial boundary ghost columns of planes [plo, phi), tile -> out
+template <class S>
+__device__ __forceinline__ void copy_bc_columns(const float4* tile, int p0, float* out, int b, int fl, int plo, int phi, int nt) {
+    constexpr int NI = S::NIP - 4;
+    const int total = (phi - plo) * S::NJP * 8;
+    for (int x = threadIdx.x; x < total; x += nt) {
+        const int c4 = x & 3, h = (x >> 2) & 1, r = x >> 3, y = r % S::NJP, z = plo + r / S::NJP;
+        if (!((c4 < 2) ? (fl & 4) : (fl & 2))) continue;
+        const int xi = c4 < 2 ? c4 : NI + c4;   // 0, 1 (bottom) or NI+2, NI+3 (top)
+        quads(out)[quad(b, h, S::NCELL) + (size_t)z * S::PL + y * S::NIP + xi] =
+            tile[((size_t)h * S::W + (z - p0) % S::W) * S::PL + y * S::NIP + xi];
+    }
+}
+
+template <int NI, int NJ, int NK, int KPAR>
+__global__ void __launch_bounds__(DShape<NI, NJ, NK, KPAR>::NT, (DShape<NI, NJ, NK, KPAR>::min_blocks))
+k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geometry g, StepScalars* sc, int cfl_next) {
+    using S = DShape<NI, NJ, NK, KPAR>;
+    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, KS = S::KS;
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+    float4* tile = reinterpret_cast<float4*>(smem + S::off_tile);
+    float* FI = reinterpret_cast<float*>(smem + S::off_fi);
+    float* FJ = reinterpret_cast<float*>(smem + S::off_fj);
+    float* FK = reinterpret_cast<float*>(smem + S::off_fk);
+    float* gi = reinterpret_cast<float*>(smem + S::off_gi);
+    float* gj = reinterpret_cast<float*>(smem + S::off_gj);
+    float* gs = reinterpret_cast<float*>(smem + S::off_gs);
+    const int b = blockIdx.x;
+    const float* blk = u + (size_t)b * NV * NCELL;
+    const int flb = g.flags[b];
+    const bool copy_bc = out != u && (flb & 6);
+    __shared__ PushBlock pb;
+    load_push_block(push, b, &pb);
+    if (threadIdx.x == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) issue_quads<S>(blk, tile, 0, KPAR + 4, 0, &bars[0]);
+    // the int8 corrections of u^n are read with plain loads: warm L2 one chunk ahead
+    auto prefetch_lo = [&](int kp_first) {
+        if (ulo != nullptr && threadIdx.x == 0)
+            prefetch_l2(ulo + ((size_t)b * S::NINT + (size_t)(kp_first - 2) * S::PLI) * NV, KPAR * S::PLI * NV);
+    };
+    prefetch_lo(2);
+    load_geometry<float, S>(g, b, gi, gj, gs, nullptr);
+    __syncthreads();   // the geometry tables are read by every thread below
+    const int tid = threadIdx.x;
+    const float* GCS = gi + GI_CS * NIP;
+    const int kq = tid / (NI * NJ), i = tid % NI, j = tid / NI % NJ;
+    const int ii = i + 2, jj = j + 2;
+    const float rc = gi[GI_R * NIP + ii], cs = GCS[ii];
+    const float den[3] = {gs[GS_DXI], gs[GS_DXJ] * rc, gs[GS_DXK] * rc * gj[GJ_SIN * S::NJP + jj]};
+    const float dinv[3] = {1.f / den[0], 1.f / den[1], 1.f / den[2]};
+    const float hdt_f = sc->dt_half_f;
+    float cmin = INFINITY;   // next step's CFL ratio minimum over this thread's cells
+    int cnan = 0;
+    constexpr int nchunk = NK / KPAR;
+    const int polls = sc->wait_polls;
+    int late = 0;   // a wait of this thread for a chunk's planes ran out
+    // variable v of padded cell c in a plane's slot
+    auto val = [&](int v, int slot, int c) -> float {
+        return reinterpret_cast<const float*>(tile + ((v >> 2) * W + slot) * PL + c)[v & 3];
+    };
+    for (int ch = 0; ch < nchunk; ++ch) {
+        const int k0 = 1 + ch * KPAR;
+        const int hi = k0 + KPAR + 3;
+        // ring slots and face arrays of the previous chunk are free; a wait of
+        // chunk ch-1 that ran out ends the CTA here (chunks ch-1 and ch in flight)
+        if (__syncthreads_or(late)) {
+            copy_wait_abort(sc, bars, ch - 1, ch);
+            return;
+        }
+        if (threadIdx.x == 0 && ch + 1 < nchunk) issue_quads<S>(blk, tile, hi, hi + KPAR, 0, &bars[(ch + 1) & 1]);
+        if (ch + 1 < nchunk) prefetch_lo(k0 + KPAR + 1);
+        const int kp0 = k0 + 1, kp = kp0 + kq;   // padded index of the chunk's first plane, this cell's plane
+        // this thread's int8 corrections, loaded now so that their latency
+        // overlaps the copy wait and the face phase
+        int2* ql = reinterpret_cast<int2*>(ulo + ((size_t)b * S::NINT + ((size_t)(kp - 2) * NJ + j) * NI + i) * NV);
+        int2 q8 = make_int2(0, 0);
+        if (ulo != nullptr) q8 = *ql;
+        // as in the stage kernel: a wait that runs out finishes the chunk on
+        // whatever the slots hold; the step is flagged and discarded
+        late |= mbar_wait(&bars[ch & 1], (uint32_t)((ch >> 1) & 1), polls) ? 0 : 1;
+        if (copy_bc)   // the planes new to this chunk
+            copy_bc_columns<S>(tile, 0, out, b, flb, ch == 0 ? 0 : k0 + 3, k0 + KPAR + 3, S::NT);
+        // slots of planes kp-1 .. kp+2
+        int so[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) so[d] = (kp + d - 1) % W * PL;
+        const int c0 = jj * NIP + ii;
+        const float4 ca = tile[so[1] + c0], cb = tile[W * PL + so[1] + c0];   // this cell
+        // this cell's left i and j faces and right k face
+        {
+            const float4* tA = tile + c0;
+            const float cLi = fabsf(tA[so[1] - 1].y) + GCS[ii - 1], cRi = fabsf(ca.y) + cs;
+            const float cLj = fabsf(tA[so[1] - NIP].z) + cs, cRj = fabsf(ca.z) + cs;
+            const float cLk = fabsf(ca.w) + cs, cRk = fabsf(tA[so[2]].w) + cs;
+            float* fkw = FK + (size_t)((kp - 1) % KS) * NV * NJ * NI + j * NI + i;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float4* t = tile + h * W * PL + c0;
+                auto comp = [](const float4& x, int q) { return q == 0 ? x.x : q == 1 ? x.y : q == 2 ? x.z : x.w; };
+                const float4 z = t[so[1]];
+                {
+                    const float4 x2 = t[so[1] - 2], x1 = t[so[1] - 1], y1 = t[so[1] + 1];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        FI[(((4 * h + q) * KPAR + kq) * NJ + j) * S::FIP + i] =
+                            face_flux(comp(x2, q), comp(x1, q), comp(z, q), comp(y1, q), cLi, cRi);
+                }
+                {
+                    const float4 x2 = t[so[1] - 2 * NIP], x1 = t[so[1] - NIP], y1 = t[so[1] + NIP];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        FJ[(((4 * h + q) * KPAR + kq) * (NJ + 1) + j) * NI + i] =
+                            face_flux(comp(x2, q), comp(x1, q), comp(z, q), comp(y1, q), cLj, cRj);
+                }
+                {
+                    const float4 x1 = t[so[0]], y1 = t[so[2]], y2 = t[so[3]];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        fkw[(4 * h + q) * NJ * NI] = face_flux(comp(x1, q), comp(z, q), comp(y1, q), comp(y2, q), cLk, cRk);
+                }
+            }
+        }
+        // the right faces of the last cells of i rows and j columns
+        constexpr int NXI = NV * KPAR * NJ, NXJ = NV * KPAR * NI;
+        for (int x = tid; x < NXI + NXJ; x += S::NT) {
+            const bool on_i = x < NXI;
+            const int y = on_i ? x : x - NXI, n = on_i ? NJ : NI;
+            const int r = y % n + 2, q = (y / n) % KPAR, v = y / (n * KPAR), slot = (kp0 + q) % W;
+            const int c = on_i ? r * NIP + NI + 1 : (NJ + 1) * NIP + r, st = on_i ? 1 : NIP;   // last interior cell
+            const int vd = on_i ? V_VR : V_VT;
+            const float cL = fabsf(val(vd, slot, c)) + GCS[on_i ? NI + 1 : r], cR = fabsf(val(vd, slot, c + st)) + GCS[on_i ? NI + 2 : r];
+            const float f = face_flux(val(v, slot, c - st), val(v, slot, c), val(v, slot, c + st), val(v, slot, c + 2 * st), cL, cR);
+            if (on_i) FI[((v * KPAR + q) * NJ + (r - 2)) * S::FIP + NI] = f;
+            else FJ[((v * KPAR + q) * (NJ + 1) + NJ) * NI + (r - 2)] = f;
+        }
+        // first chunk: the k faces below the first plane (between padded planes 1 and 2)
+        if (ch == 0) {
+            for (int x = tid; x < NV * NJ * NI; x += S::NT) {
+                const int xx = x % NI + 2, y = (x / NI) % NJ + 2, v = x / (NI * NJ), c = y * NIP + xx;
+                const float cL = fabsf(val(V_VP, 1, c)) + GCS[xx], cR = fabsf(val(V_VP, 2, c)) + GCS[xx];
+                FK[(v * NJ + (y - 2)) * NI + (xx - 2)] = face_flux(val(v, 0, c), val(v, 1, c), val(v, 2, c), val(v, 3, c), cL, cR);
+            }
+        }
+        __syncthreads();
+        const size_t cell = (size_t)kp * PL + c0;
+        const float* fk_l = FK + (size_t)((kp - 2) % KS) * NV * NJ * NI + j * NI + i;
+        const float* fk_r = FK + (size_t)((kp - 1) % KS) * NV * NJ * NI + j * NI + i;
+        float o[NV], u0[NV];
+        split(ca, cb, u0);
+        int qn[2] = {0, 0};
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const float* fi = FI + ((v * KPAR + kq) * NJ + j) * S::FIP + i;
+            const float* fj = FJ + ((v * KPAR + kq) * (NJ + 1) + j) * NI + i;
+            float R = 0.f;
+            R = R + (fi[0] - fi[1]) * dinv[0];
+            R = R + (fj[0] - fj[NI]) * dinv[1];
+            R = R + (fk_l[v * NJ * NI] - fk_r[v * NJ * NI]) * dinv[2];
+            if (ulo != nullptr) {
+                const int sh = 8 * (v & 3);
+                int8_t q1;
+                o[v] = ff_add(u0[v], (int8_t)((v < 4 ? q8.x : q8.y) >> sh), __fmul_rn(hdt_f, R), q1);
+                qn[v >> 2] |= (int)(uint8_t)q1 << sh;
+            } else {
+                o[v] = fmaf(hdt_f, R, u0[v]);
+            }
+        }
+        if (ulo != nullptr) *ql = make_int2(qn[0], qn[1]);
+        quads(out)[quad(b, 0, NCELL) + cell] = f4(o);
+        quads(out)[quad(b, 1, NCELL) + cell] = f4(o + 4);
+        if (push.tgt != nullptr) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+        if (cfl_next) {   // uniform over the CTA
+#pragma unroll
+            for (int v = 0; v < NV; ++v) cnan |= (o[v] != o[v]);
+            float ratio = cfl_ratio_f(cfl_sq3(o[V_VR], o[V_VT], o[V_VP]), cfl_sq3(o[V_BR], o[V_BT], o[V_BP]), cs,
+                                      gi[GI_RHO0 * NIP + ii], rc, gj[GJ_SIN * S::NJP + jj], gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]);
+            if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
+            cmin = fminf(cmin, ratio);
+        }
+    }
+    if (__syncthreads_or(late)) {
+        copy_wait_abort(sc, bars, nchunk - 1, nchunk - 1);
+        return;
+    }
+    if (cfl_next) cfl_commit(cmin, cnan, sc);
+}
+
+// ---------------------------------------------------------------------------
+// FP32 artificial diffusion of one 16^3 block, or of planes [ka, kb) of it, as a
+// march along k (same arguments and results as k_diffusion_quads).
+//
+// One thread per (i, j) column of the block (256 threads), marching k over the
+// 16 interior planes. Along k everything stays in registers: the column's
+// values at planes kp and kp+1, its k slope at kp and the flux through the
+// face below kp; per plane the thread reads one new value per variable (plane
+// kp+2, from the ring), forms one k slope and one k face. Across the plane,
+// every i and j slope is formed once (phase A, into shared memory, ghost
+// columns and rows by the same threads), then every i and j face flux once
+// (phase B), then each cell sums its six faces and updates (phase C). Per
+// cell and variable that is 3 slopes and 3 fluxes, the minimum; the face
+// fluxes are the same functions of the same values as k_diffusion's, summed
+// in the same order. The arithmetic runs on pairs of variables (packed FP32
+// instructions, above), and the slope and face arrays hold the pairs side by
+// side, so their shared-memory accesses are 64-bit; a cell's values come from
+// the ring four at a time (128-bit).
+//
+// Planes arrive by bulk copy into a ring of 5 slots, one mbarrier each: the
+// column window needs planes kp..kp+2, and the slot of plane kp is refilled
+// with plane kp+5 once phase B of plane kp has passed its barrier (planes
+// kp+3 and kp+4 are in flight meanwhile). A warp takes rows j and j+4
+// (half-warps of 16 cells), so a half-warp holds one row, as the pushed
+// radial faces need. 21.2M cells: 1,229 -> 1,135 us; 442k cells with split
+// blocks: 60 -> 37 us.
+template <int NI, int NJ, int NK, int TPC>
+struct MShape {
+    static constexpr int NG = 2, NIP = NI + 4, NJP = NJ + 4, NKP = NK + 4;
+    static constexpr int PL = NIP * NJP, NCELL = PL * NKP;
+    static constexpr int NCOL = NI * NJ, NT = NCOL * TPC;   // columns; threads (TPC per column)
+    static constexpr int W = 5;                          // plane ring slots
+    static constexpr int PLI = NI * NJ, NINT = PLI * NK;
+    static constexpr int NP = NV / 2, PPT = NP / TPC;    // variable pairs; pairs per thread
+    static constexpr uint32_t PLB = PL * 4u;
+    static constexpr int P = 20;                         // row pitch (pairs) of the slope and face arrays
+    // per pair (float2): SI[NJ][P] slopes along i of cells i = -1..NI at i + 1;
+    // SJ[NJ + 2][P] slopes along j of rows j = -1..NJ at row j + 1;
+    // FI[NJ][P] fluxes through faces i - 1/2, i = 0..NI; FJ[NJ + 1][P] likewise along j
+    static constexpr int NSI = NJ * P, NSJ = (NJ + 2) * P, NFI = NJ * P, NFJ = (NJ + 1) * P;
+    // shared memory: mbarriers | tile[2][W][PL] of 16 bytes | SI | SJ | FI | FJ | gi | gj | gs
+    static constexpr size_t off_tile = 64;
+    static constexpr size_t off_si = off_tile + (size_t)NV * W * PL * 4;
+    static constexpr size_t off_sj = off_si + (size_t)NP * NSI * 8;
+    static constexpr size_t off_fi = off_sj + (size_t)NP * NSJ * 8;
+    static constexpr size_t off_fj = off_fi + (size_t)NP * NFI * 8;
+    static constexpr size_t off_gi = off_fj + (size_t)NP * NFJ * 8;
+    static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * NIP * 4;
+    static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * NJP * 4;
+    // two threads per column: |B|^2 of the second half, [plane parity][column]
+    static constexpr size_t off_sb2 = off_gs + GS_COUNT * 4;
+    static constexpr size_t smem = off_sb2 + (TPC == 2 ? 2 * NCOL * 4 : 0);
+    static_assert(W * 8 <= (int)off_tile, "mbarriers");
+    static_assert(off_si % 8 == 0, "float2 arrays");
+    static_assert(TPC == 1 || TPC == 2, "one or two threads per column");
+};
+
+// TPC threads per column: with two, thread half h = tid / 256 takes the
+// variable pairs 2h, 2h+1 (warps never mix halves), doubling the warps per SM
+// at half the registers; the CFL ratio, which needs v (first half) and B
+// (second half), takes |B|^2 through shared memory one plane later.
+template <int NI, int NJ, int NK, int TPC>
+__device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* u, float* out, int8_t* ulo,
+                                            const PushTable& push, const Geometry& g, StepScalars* sc, int cfl_next) {
+    using S = MShape<NI, NJ, NK, TPC>;
+    static_assert(NI == 16 && NJ == 16, "rows of 16 cells: one half-warp per row");
+    static_assert(2 * (S::smem + 1024) <= 233472, "two CTAs per SM");
+    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, P = S::P, PPT = S::PPT;
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+    float4* tile = reinterpret_cast<float4*>(smem + S::off_tile);   // [2][W][PL]
+    float2* SI = reinterpret_cast<float2*>(smem + S::off_si);
+    float2* SJ = reinterpret_cast<float2*>(smem + S::off_sj);
+    float2* FI = reinterpret_cast<float2*>(smem + S::off_fi);
+    float2* FJ = reinterpret_cast<float2*>(smem + S::off_fj);
+    float* gi = reinterpret_cast<float*>(smem + S::off_gi);
+    float* gj = reinterpret_cast<float*>(smem + S::off_gj);
+    float* gs = reinterpret_cast<float*>(smem + S::off_gs);
+    float* sb2 = reinterpret_cast<float*>(smem + S::off_sb2);   // |B|^2 of the second half, by plane parity
+    const int tid = threadIdx.x;
+    const float* blk = u + (size_t)b * NV * NCELL;
+    const int flb = g.flags[b];
+    const bool copy_bc = out != u && (flb & 6);
+    __shared__ PushBlock pb;
+    load_push_block(push, b, &pb);
+    if (tid == 0) {
+        for (int s = 0; s < W; ++s) mbar_init(&bars[s], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    // planes are counted from pa, the first that [ka, kb) needs; pe: one past the last
+    const int pa = ka - 2, pe = kb + 2;
+    int issued = pa;   // thread 0: planes [pa, issued) have been requested
+    auto issue = [&]() {
+        issue_quads<S>(blk, tile, issued, issued + 1, pa, &bars[(issued - pa) % W]);
+        ++issued;
+    };
+    if (tid == 0)
+        while (issued < pa + W) issue();
+    int8_t* blk_lo = ulo != nullptr ? ulo + (size_t)b * NV * S::NINT : nullptr;
+    if (blk_lo != nullptr && tid == 0) prefetch_l2(blk_lo + (size_t)(ka - 2) * S::PLI * NV, 2 * S::PLI * NV);
+    load_geometry<float, S>(g, b, gi, gj, gs, nullptr);
+    __syncthreads();   // the geometry tables are read by every thread below
+    // this thread's column: warp w takes rows (w % 4) + 8 (w / 4) and that + 4;
+    // its pairs p0 .. p0 + PPT - 1
+    const int c = tid % S::NCOL, half = tid / S::NCOL, p0 = half * PPT, v0 = 2 * p0;
+    const int wq = c >> 5, i = c & 15;
+    const int j = (wq & 3) + 8 * (wq >> 2) + 4 * ((c >> 4) & 1);
+    const int ii = i + 2, jj = j + 2;
+    const float* GCS = gi + GI_CS * NIP;
+    const float cs = GCS[ii];
+    const float rc = gi[GI_R * NIP + ii];
+    const float den[3] = {gs[GS_DXI], gs[GS_DXJ] * rc, gs[GS_DXK] * rc * gj[GJ_SIN * S::NJP + jj]};
+    const float2 dinv0 = f2(1.f / den[0]), dinv1 = f2(1.f / den[1]), dinv2 = f2(1.f / den[2]);
+    const float2 hdt2 = f2(sc->dt_half_f);
+    const int polls = sc->wait_polls;
+    int late = 0;   // a wait of this thread for a plane ran out
+    auto abort_cta = [&]() {   // after a uniform decision: flag, drain the copies in flight
+        if (tid != 0) return;
+        atomicOr(&sc->nan_flag, 2);
+        for (int p = issued - pa < W ? 0 : issued - pa - W; p < issued - pa; ++p)
+            mbar_wait(&bars[p % W], (uint32_t)((p / W) & 1), kWaitPolls);
+        for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
+    };
+    // this thread's halves of a cell in a plane's slot
+    constexpr int NH = PPT / 2;
+    const float4* mine = tile + (size_t)(p0 / 2) * W * PL;
+    auto quad_of = [&](int slot, int c, int h) { return mine[(size_t)h * W * PL + slot + c]; };
+    auto lo2 = [](const float4& x) { return f2(x.x, x.y); };
+    auto hi2 = [](const float4& x) { return f2(x.z, x.w); };
+    const int c0 = jj * NIP + ii;
+    auto slot_of = [&](int p) { return (p - pa) % W * PL; };
+    // pairs of one quad into two of an array
+    auto pairs = [&](int slot, int c, float2 (&v)[PPT]) {
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            const float4 x = quad_of(slot, c, h);
+            v[2 * h] = lo2(x);
+            v[2 * h + 1] = hi2(x);
+        }
+    };
+    // the column window from planes ka-2 .. ka+1: u at kp = ka and ka + 1, the k
+    // slope at ka, the flux through the face between planes ka-1 and ka
+    for (int p = 0; p < 4; ++p) late |= mbar_wait(&bars[p], 0u, polls) ? 0 : 1;
+    if (copy_bc) copy_bc_columns<S>(tile, pa, out, b, flb, pa, pa + 4, S::NT);
+    float2 u0[PPT], u1[PPT], dk0[PPT], fk0[PPT];
+    {
+        const float2 cc = f2(-0.25f * ((fabsf(tile[2 * PL + c0].w) + cs) + (fabsf(tile[PL + c0].w) + cs)));
+        float2 a0[PPT], a1[PPT];
+        pairs(0, c0, a0);
+        pairs(PL, c0, a1);
+        pairs(2 * PL, c0, u0);
+        pairs(3 * PL, c0, u1);
+#pragma unroll
+        for (int q = 0; q < PPT; ++q) {
+            const float2 d1 = minmod_sel2(a0[q], a1[q], u0[q]);
+            dk0[q] = minmod_sel2(a1[q], u0[q], u1[q]);
+            fk0[q] = face_flux2(a1[q], u0[q], d1, dk0[q], cc);
+        }
+    }
+    float cmin = INFINITY;   // next step's CFL ratio minimum over this column
+    int cnan = 0;
+    float v2_prev = 0.f;     // two threads per column: the first half's |v|^2 of the previous plane
+    const float rho0c = gi[GI_RHO0 * NIP + ii], sin_c = gj[GJ_SIN * S::NJP + jj];
+    auto cfl_point = [&](float v2, float b2) {
+        float ratio = cfl_ratio_f(v2, b2, cs, rho0c, rc, sin_c, gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]);
+        if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
+        cmin = fminf(cmin, ratio);
+    };
+    for (int kp = ka; kp < kb; ++kp) {
+        const int p2 = kp + 2;
+        if (blk_lo != nullptr && tid == 0 && kp + 2 < kb)
+            prefetch_l2(blk_lo + (size_t)kp * S::PLI * NV, S::PLI * NV);
+        // this cell's int8 corrections, loaded before the wait
+        int qlo[NH];
+        int* qp = reinterpret_cast<int*>(blk_lo + (((size_t)(kp - 2) * NJ + j) * NI + i) * NV + v0);
+        if (blk_lo != nullptr) {
+#pragma unroll
+            for (int h = 0; h < NH; ++h) qlo[h] = qp[h];
+        }
+        // a wait that runs out finishes the plane on whatever the slot holds;
+        // the step is flagged and discarded
+        late |= mbar_wait(&bars[(p2 - pa) % W], (uint32_t)(((p2 - pa) / W) & 1), polls) ? 0 : 1;
+        if (copy_bc) copy_bc_columns<S>(tile, pa, out, b, flb, p2, p2 + 1, S::NT);
+        const int s0 = slot_of(kp), s1 = slot_of(kp + 1), s2 = slot_of(p2);
+        // the half with the velocities at this cell
+        const float4 vc = tile[s0 + c0], vl = tile[s0 + c0 - 1], vd = tile[s0 + c0 - NIP];
+        // ---- phase A: k slope and k face from the window; i and j slopes
+        float2 u2[PPT], dk1[PPT], fk1[PPT];
+        {
+            const float2 cc = f2(-0.25f * ((fabsf(tile[s1 + c0].w) + cs) + (fabsf(vc.w) + cs)));
+            pairs(s2, c0, u2);
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) {
+                dk1[q] = minmod_sel2(u0[q], u1[q], u2[q]);
+                fk1[q] = face_flux2(u0[q], u1[q], dk0[q], dk1[q], cc);
+            }
+            float2 l[PPT], r[PPT];
+            pairs(s0, c0 - 1, l);
+            pairs(s0, c0 + 1, r);
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) SI[(p0 + q) * S::NSI + j * P + i + 1] = minmod_sel2(l[q], u0[q], r[q]);
+            pairs(s0, c0 - NIP, l);
+            pairs(s0, c0 + NIP, r);
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) SJ[(p0 + q) * S::NSJ + (j + 1) * P + i] = minmod_sel2(l[q], u0[q], r[q]);
+        }
+        // slopes of the ghost cells next to the block: i = -1, NI of every row
+        // (items 0..255) and j = -1, NJ of every column (items 256..511)
+#pragma unroll
+        for (int x = tid; x < 512; x += S::NT) {
+            const int side = x & 1, r = (x >> 1) & 15, v = (x >> 5) & 7;
+            const float* a = reinterpret_cast<const float*>(tile + (v >> 2) * W * PL + s0) + (v & 3);
+            float* dst;
+            float val;
+            if (x < 256) {
+                const float* q = a + 4 * ((r + 2) * NIP + (side ? NI + 2 : 1));
+                val = face_slope(q[-4], q[0], q[4]);
+                dst = reinterpret_cast<float*>(SI + (v >> 1) * S::NSI + r * P + (side ? NI + 1 : 0));
+            } else {
+                const float* q = a + 4 * ((side ? NJ + 2 : 1) * NIP + r + 2);
+                val = face_slope(q[-4 * NIP], q[0], q[4 * NIP]);
+                dst = reinterpret_cast<float*>(SJ + (v >> 1) * S::NSJ + (side ? NJ + 1 : 0) * P + r);
+            }
+            dst[v & 1] = val;
+        }
+        if (__syncthreads_or(late)) {
+            abort_cta();
+            return;
+        }
+        // ---- phase B: the faces i - 1/2 and j - 1/2 of this cell, and the
+        // last faces of the rows (items 0..127) and columns (128..255)
+        float2 fi0[PPT], fj0[PPT];
+        {
+            const float cLi = fabsf(vl.y) + GCS[ii - 1], cRi = fabsf(vc.y) + cs;
+            const float cLj = fabsf(vd.z) + cs, cRj = fabsf(vc.z) + cs;
+            const float2 cci = f2(-0.25f * (cRi + cLi)), ccj = f2(-0.25f * (cRj + cLj));
+            float2 l[PPT], d[PPT];
+            pairs(s0, c0 - 1, l);
+            pairs(s0, c0 - NIP, d);
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) {
+                const int p = p0 + q;
+                const float2* si = SI + p * S::NSI + j * P + i;
+                const float2* sj = SJ + p * S::NSJ + j * P + i;
+                fi0[q] = face_flux2(l[q], u0[q], si[0], si[1], cci);
+                fj0[q] = face_flux2(d[q], u0[q], sj[0], sj[P], ccj);
+                FI[p * S::NFI + j * P + i] = fi0[q];
+                FJ[p * S::NFJ + j * P + i] = fj0[q];
+            }
+        }
+        if (tid < 256) {
+            const int x = tid, r = x & 15, v = (x >> 4) & 7;
+            const float* sl = reinterpret_cast<const float*>(x < 128 ? SI + (v >> 1) * S::NSI + r * P + NI
+                                                                     : SJ + (v >> 1) * S::NSJ + NJ * P + r);
+            if (x < 128) {
+                const float* a = reinterpret_cast<const float*>(tile + (v >> 2) * W * PL + s0 + (r + 2) * NIP + NI + 1) + (v & 3);
+                const float4* vr = tile + s0 + (r + 2) * NIP + NI + 1;   // last interior cell of row r
+                const float cL = fabsf(vr[0].y) + GCS[NI + 1], cR = fabsf(vr[1].y) + GCS[NI + 2];
+                reinterpret_cast<float*>(FI + (v >> 1) * S::NFI + r * P + NI)[v & 1] =
+                    face_flux_s(a[0], a[4], sl[v & 1], sl[2 + (v & 1)], cL, cR);
+            } else {
+                const float* a = reinterpret_cast<const float*>(tile + (v >> 2) * W * PL + s0 + (NJ + 1) * NIP + r + 2) + (v & 3);
+                const float4* vt = tile + s0 + (NJ + 1) * NIP + r + 2;   // last interior row, column r
+                const float c2 = GCS[r + 2];
+                const float cL = fabsf(vt[0].z) + c2, cR = fabsf(vt[NIP].z) + c2;
+                reinterpret_cast<float*>(FJ + (v >> 1) * S::NFJ + NJ * P + r)[v & 1] =
+                    face_flux_s(a[0], a[4 * NIP], sl[v & 1], sl[2 * P + (v & 1)], cL, cR);
+            }
+        }
+        __syncthreads();
+        // planes below kp + 1 are done with: refill their slots, up to plane
+        // kp + W (at kp = 2 that is planes 5, 6, 7; then one plane a step)
+        if (tid == 0)
+            while (issued < pe && issued <= kp + W) issue();
+        // ---- phase C: sum the six faces in the reference's order, update
+        const size_t cell = (size_t)kp * PL + c0;
+        float o[2 * PPT];
+        int qn[NH] = {};
+#pragma unroll
+        for (int q = 0; q < PPT; ++q) {
+            const int p = p0 + q;
+            float2 R = __fmul2_rn(sub2(fi0[q], FI[p * S::NFI + j * P + i + 1]), dinv0);
+            R = __ffma2_rn(sub2(fj0[q], FJ[p * S::NFJ + (j + 1) * P + i]), dinv1, R);
+            R = __ffma2_rn(sub2(fk0[q], fk1[q]), dinv2, R);
+            float2 ov;
+            if (ulo != nullptr) {
+                int8_t q0, q1;
+                const int sh = 16 * (q & 1);
+                ov = ff_add2(u0[q], (int8_t)(qlo[q >> 1] >> sh), (int8_t)(qlo[q >> 1] >> (sh + 8)), __fmul2_rn(hdt2, R), q0, q1);
+                qn[q >> 1] |= ((int)(uint8_t)q0 | (int)(uint8_t)q1 << 8) << sh;
+            } else {
+                ov = __ffma2_rn(hdt2, R, u0[q]);
+            }
+            o[2 * q] = ov.x;
+            o[2 * q + 1] = ov.y;
+        }
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            if (ulo != nullptr) qp[h] = qn[h];
+            quads(out)[quad(b, p0 / 2 + h, NCELL) + cell] = f4(o + 4 * h);
+        }
+        if (push.tgt != nullptr) {
+            if constexpr (TPC == 1) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+            else if (half == 0) push_quads<S, 1, 0>(out, pb, ii, jj, kp, o);   // warps never mix halves
+            else push_quads<S, 1, 1>(out, pb, ii, jj, kp, o);
+        }
+        if (cfl_next) {   // uniform over the CTA
+#pragma unroll
+            for (int v = 0; v < 2 * PPT; ++v) cnan |= (o[v] != o[v]);
+            if constexpr (TPC == 1) {
+                cfl_point(cfl_sq3(o[V_VR], o[V_VT], o[V_VP]), cfl_sq3(o[V_BR], o[V_BT], o[V_BP]));
+            } else if (half == 0) {
+                if (kp > ka) cfl_point(v2_prev, sb2[((kp - 1) & 1) * S::NCOL + c]);
+                v2_prev = cfl_sq3(o[V_VR], o[V_VT], o[V_VP]);
+            } else {
+                sb2[(kp & 1) * S::NCOL + c] = cfl_sq3(o[V_BR - 4], o[V_BT - 4], o[V_BP - 4]);
+            }
+        }
+        // the window moves up one plane
+#pragma unroll
+        for (int q = 0; q < PPT; ++q) {
+            u0[q] = u1[q];
+            u1[q] = u2[q];
+            dk0[q] = dk1[q];
+            fk0[q] = fk1[q];
+        }
+    }
+    if (__syncthreads_or(late)) {
+        abort_cta();
+        return;
+    }
+    if constexpr (TPC == 2) {
+        if (cfl_next && half == 0) cfl_point(v2_prev, sb2[((kb - 1) & 1) * S::NCOL + c]);
+    }
+    if (tid == 0)   // every copy has been waited for
+        for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
+    if (cfl_next) cfl_commit(cmin, cnan, sc);
+}
+// split CTAs per block, each a run of planes
+template <int NI, int NJ, int NK, int TPC>
+__global__ void __launch_bounds__(NI * NJ * TPC, 2)
+k_march_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geometry g, StepScalars* sc, int cfl_next, int split) {
+    const int b = blockIdx.x / split, part = blockIdx.x - b * split, n = NK / split;
+    march_quads<NI, NJ, NK, TPC>(b, 2 + part * n, 2 + (part + 1) * n, u, out, ulo, push, g, sc, cfl_next);
+}
+
+// ---------------------------------------------------------------------------
+// Every cell outside the core of each block and variable set to 0 (the k ghost
+// planes and, in the interior planes, the j ghost rows: per block and
+// variable, (NJP-4)*NIP-wide gaps between the core runs). A core upload clears
+// them before its exchange refills the listed ones: the mixed interpolations
+// read some ghost cells of their source blocks with weight 0, which is
+// harmless for finite values only, and the buffer may hold an earlier state
+// with NaNs there. Cleared, the uploaded state's ghost cells are the same
+// whatever the buffer held (a new context starts with zeros too).
+// T: float4 for the state's halves, float for psi; nbv arrays of ncell cells.
+template <class T>
+__global__ void __launch_bounds__(256) k_clear_outside_core(T* u, int64_t nbv, StepDims d) {
+    const int pl = d.nip * d.njp, lead = 2 * pl + 2 * d.nip, gap = 4 * d.nip;
+    const int per = 2 * lead + (d.nkp - 5) * gap;   // non-core cells per block and variable
+    for (int64_t bv = blockIdx.x; bv < nbv; bv += gridDim.x) {
+        T* base = u + bv * d.ncell;
+        for (int x = threadIdx.x; x < per; x += blockDim.x) {
+            int c;
+            if (x < lead) {
+                c = x;                                   // planes 0, 1 and rows 0, 1 of plane 2
+            } else if (x < per - lead) {
+                const int q = (x - lead) / gap, r = (x - lead) - q * gap;
+                c = (2 + q) * pl + (d.njp - 2) * d.nip + r;   // rows NJP-2, NJP-1 of plane 2+q, rows 0, 1 of the next
+            } else {
+                c = d.ncell - lead + (x - (per - lead));   // rows NJP-2, NJP-1 of the last interior plane, 2 ghost planes
+            }
+            base[c] = T{};
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// After the core of a mixed state has been replaced from the host (the core
+// upload), what the diffusion pass closing a mixed step leaves besides
+// u^{n+1} itself: the regular faces pushed into the neighbours' ghost layers
+// (the face entries left to the final exchange follow as a separate launch),
+// and the next step's CFL minimum with the NaN scan, each cell's ratio the
+// one k_cfl forms. One CTA per block and a thread per (i, j) column marching
+// k; a row of NI cells lies in consecutive lanes, as the pushed radial faces
+// need.
+template <int NI, int NJ, int NK>
+__global__ void __launch_bounds__(NI * NJ) k_push_state(float* u, PushTable push, Geometry g, StepScalars* sc) {
+    using S = MShape<NI, NJ, NK, 1>;
+    constexpr int NIP = S::NIP, NJP = S::NJP;
+    static_assert((NI * NJ) % 32 == 0 && 32 % NI == 0, "whole rows in every warp");
+    __shared__ PushBlock pb;
+    const int b = blockIdx.x, tid = threadIdx.x;
+    load_push_block(push, b, &pb);
+    __syncthreads();
+    const int ii = tid % NI + 2, jj = tid / NI + 2;
+    const float* Gi = gi_ptr<float>(g) + (size_t)b * GI_COUNT * NIP;
+    const float* Gj = gj_ptr<float>(g) + (size_t)b * GJ_COUNT * NJP;
+    const float* Gs = gs_ptr<float>(g) + (size_t)b * GS_COUNT;
+    const float cs = Gi[GI_CS * NIP + ii], rho0 = Gi[GI_RHO0 * NIP + ii], r = Gi[GI_R * NIP + ii];
+    const float sin_t = Gj[GJ_SIN * NJP + jj], dxi = Gs[GS_DXI], dxj = Gs[GS_DXJ], dxk = Gs[GS_DXK];
+    float cmin = INFINITY;
+    int cnan = 0;
+    constexpr int G = 4;   // planes whose loads are all issued before the first push
+    static_assert(NK % G == 0, "whole plane groups");
+    for (int k0 = 2; k0 < NK + 2; k0 += G) {
+        float o[G][NV];
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            const size_t cell = ((size_t)(k0 + q) * NJP + jj) * NIP + ii;
+            load_cell<false>(u + Layout<float>::at(b, 0, cell, S::NCELL), S::NCELL, o[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            if (push.tgt != nullptr) push_quads<S, 2, 0>(u, pb, ii, jj, k0 + q, o[q]);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) cnan |= (o[q][v] != o[q][v]);
+            float ratio = cfl_ratio_f(cfl_sq3(o[q][V_VR], o[q][V_VT], o[q][V_VP]),
+                                      cfl_sq3(o[q][V_BR], o[q][V_BT], o[q][V_BP]), cs, rho0, r, sin_t, dxi, dxj, dxk);
+            if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
+            cmin = fminf(cmin, ratio);
+        }
+    }
+    cfl_commit(cmin, cnan, sc);
+}
+
+// ---------------------------------------------------------------------------
+// A barrier over every CTA of a cooperative launch (all co-resident). Thread
+// 0 of each CTA reads the generation, arrives on the counter; the last one
+// resets the counter and advances the generation, the others poll it, at most
+// `polls` times (a poll that runs out flags the step: bit 1 of nan_flag, the
+// host returns FALCON_ERR_TIMEOUT, and the CTA goes on). Fences on both sides
+// make every CTA's writes before the barrier visible to every CTA after it.
+struct GridBarrier {
+    unsigned int* count;   // 0 between barriers
+    unsigned int* gen;
+    unsigned int* ticket;  // [5]: the next block of each block phase (4 stages, diffusion), 0 at launch
+};
+__device__ __forceinline__ void grid_sync(const GridBarrier& gb, StepScalars* sc, int polls) {
+    // the next phase reads this one's global writes also through bulk copies
+    // (the async proxy): order them across the proxies on both sides
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned int g0 = *(volatile unsigned int*)gb.gen;
+        __threadfence();
+        if (atomicAdd(gb.count, 1u) == gridDim.x - 1) {
+            atomicExch(gb.count, 0u);
+            __threadfence();
+            atomicAdd(gb.gen, 1u);
+        } else {
+            int it = 0;
+            while (*(volatile unsigned int*)gb.gen == g0) {
+                if (++it > polls) {
+                    atomicOr(&sc->nan_flag, 2);
+                    break;
+                }
+                __nanosleep(64);
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+}
+
+// The pointers of one mixed step: u^n in U, the stage buffer RK, the second
+// state buffer R2 (u^{n+1} is written there, then the host swaps U and R2).
+struct StepBuffers {
+    float* U;
+    float* RK;
+    float* R2;
+    int8_t* ulo;
+};
+
+// One mixed RK4 step of 16^3 blocks in one persistent launch: the CTAs take
+// the blocks (and, in the exchanges, the ghost entries) in turn and meet at a
+// grid barrier between the phases the graph runs as separate launches:
+// dt, then per stage s the stage kernel's body into seq[s] (pushing the
+// regular ghost faces) and the exchange of the rest (face lists), then the
+// diffusion body into R2 (pushes, next step's CFL minimum) and the exchange
+// of the remaining entries. The bodies are the separate kernels' own
+// (KPAR 2 for the stages, two threads per column for the diffusion: 512
+// threads each, and every variant computes the same bits), so the step
+// equals the graph's bit for bit.
+template <int N>
+__global__ void __launch_bounds__(512, 2)
+k_step_persistent(StepBuffers sb, PushTable push, Geometry g, StepScalars* sc, GhostLists gl_stage,
+                  GhostLists gl_final, StepDims d, GridBarrier gb) {
+    static_assert(N == 16, "16^3 blocks");
+    const int polls = sc->wait_polls;
+    if (blockIdx.x == 0 && threadIdx.x == 0) finalize_dt_body(sc);
+    grid_sync(gb, sc, polls);
+    const int64_t tstride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    auto exchange = [&](const GhostLists& G, float* u) {
+        for (int64_t e = t0; e < G.ip.n; e += tstride)
+            ghost_interp_one<float, true>(u, G.ip, d.ncell, d.nip, d.nip * d.njp, e);
+        for (int64_t e = t0; e < G.ln.n; e += tstride) ghost_lin_one<float, true>(u, G.ln, d.ncell, e);
+        for (int64_t e = t0; e < G.cp.n; e += tstride) ghost_copy_one<float, true>(u, G.cp, d.ncell, e);
+    };
+    // between two bodies in one CTA: the generic writes of the one before
+    // are ordered before the bulk copies of the next into the same memory
+    auto next_body = [&]() {
+        fence_proxy_async();
+        __syncthreads();
+    };
+    // blocks are handed out one at a time from a ticket counter per phase, as
+    // the hardware scheduler hands CTAs to SMs: a CTA that finishes early
+    // takes the next block instead of waiting at the barrier
+    __shared__ int next_b;
+    auto take = [&](int phase) -> int {
+        if (threadIdx.x == 0) next_b = (int)atomicAdd(&gb.ticket[phase], 1u);
+        __syncthreads();
+        return next_b;   // read before the next take's write: a body or next_body() barrier lies between
+    };
+    for (int s = 1; s <= 4; ++s) {
+        float* in = s == 1 ? sb.U : (s == 3 ? sb.R2 : sb.RK);
+        float* out = s == 4 ? sb.U : (s == 2 ? sb.R2 : sb.RK);   // U -> RK -> R2 -> RK -> U
+        for (int b = take(s - 1); b < d.nblocks; b = take(s - 1)) {
+            stage_quads<16, 16, 16, 2, 0>(b, 0, 8, in, sb.U, out, sb.ulo, push, DivBArgs{nullptr, nullptr, nullptr, 0}, g, sc, s,
+                                          1);
+            next_body();
+        }
+        grid_sync(gb, sc, polls);
+        exchange(gl_stage, out);
+        grid_sync(gb, sc, polls);
+    }
+    for (int b = take(4); b < d.nblocks; b = take(4)) {
+        march_quads<16, 16, 16, 2>(b, 2, 18, sb.U, sb.R2, sb.ulo, push, g, sc, 1);
+        next_body();
+    }
+    grid_sync(gb, sc, polls);
+    exchange(gl_final, sb.R2);
+}
+
+}  // namespace impl
+}  // namespace falcon

@@ -18,11 +18,10 @@ __device__ __forceinline__ double cell_value(const T* U, const int8_t* lo, const
                                              const StepDims& d) {
     const int64_t ncell = d.ncell;
     if (v == NV) return psi ? (double)psi[b * ncell + c] : 0.0;
-    const int64_t e = (b * NV + v) * ncell + c;
-    const T hi = U[e];
+    const T hi = U[Layout<T>::at((size_t)b, v, (size_t)c, (size_t)ncell)];
     double x = (double)hi;
     if constexpr (sizeof(T) == 4) {
-        const int64_t q = lo ? lo_index(e, d) : -1;
+        const int64_t q = lo ? lo_index(b, v, (int)c, d) : -1;
         if (q >= 0) x += (double)lo[q] * (double)lo_unit((float)hi);
     }
     return x;

@@ -68,13 +68,13 @@ __global__ void k_synth(T* U, const double* xj, const double* xk, Geometry geo, 
         const double qq = (sp.rb / r) * (sp.rb / r) * (sp.rb / r);
         double br = 2.0 * sp.B0 * qq * cos(ty), bt = sp.B0 * qq * sin(ty), bp = 0.0;
         if (!yin) yy_vec_d(ty, py, bt, bp);
-        T* c = U + (size_t)b * NV * d.ncell + q;
-        const size_t n = d.ncell;
-        c[V_RHO1 * n] = T(0);
-        c[V_S1 * n] = (T)s1;
-        c[V_BR * n] = (T)br;
-        c[V_BT * n] = (T)bt;
-        c[V_BP * n] = (T)bp;
+        T* c = U + Layout<T>::at(b, 0, q, d.ncell);
+        auto var = [&](int v) { return Layout<T>::var(v, d.ncell); };
+        c[var(V_RHO1)] = T(0);
+        c[var(V_S1)] = (T)s1;
+        c[var(V_BR)] = (T)br;
+        c[var(V_BT)] = (T)bt;
+        c[var(V_BP)] = (T)bp;
         double vr = 0, vt = 0, vp = 0;
         const bool interior = ip >= 2 && ip < d.nip - 2 && jp >= 2 && jp < d.njp - 2 && kp >= 2 && kp < d.nkp - 2;
         if (sp.with_v && interior) {
@@ -93,9 +93,9 @@ __global__ void k_synth(T* U, const double* xj, const double* xk, Geometry geo, 
             if (!yin) yy_vec_d(ty, py, vt, vp);
             local = vr * vr + vt * vt + vp * vp;
         }
-        c[V_VR * n] = (T)vr;
-        c[V_VT * n] = (T)vt;
-        c[V_VP * n] = (T)vp;
+        c[var(V_VR)] = (T)vr;
+        c[var(V_VT)] = (T)vt;
+        c[var(V_VP)] = (T)vp;
     }
     // the CTA's sum of |v|^2 into its own slot (summed on the host in a fixed
     // order, so the scale and the seeded state are the same on every run)
@@ -120,11 +120,11 @@ __global__ void k_scale_v(T* U, Geometry geo, StepDims d, double scale) {
     // local sound speed c_s = sqrt(gamma1 p0/rho0) = Xi * CS column
     const double A1 = Gi[GI_A1 * d.nip + ip];   // gamma1*p0/rho0
     const double f = scale * sqrt(A1);
-    T* c = U + (size_t)b * NV * d.ncell + q;
-    const size_t n = d.ncell;
-    c[V_VR * n] = (T)((double)c[V_VR * n] * f);
-    c[V_VT * n] = (T)((double)c[V_VT * n] * f);
-    c[V_VP * n] = (T)((double)c[V_VP * n] * f);
+    T* c = U + Layout<T>::at(b, 0, q, d.ncell);
+    for (int v : {V_VR, V_VT, V_VP}) {
+        T& x = c[Layout<T>::var(v, d.ncell)];
+        x = (T)((double)x * f);
+    }
 }
 
 }  // namespace
