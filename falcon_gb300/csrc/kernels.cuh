@@ -19,11 +19,12 @@
 //          interior row touched two sectors in part, and a ghost cell's eight
 //          values lay in eight).
 //
-// Stencil kernels run one CTA per block. The CTA owns an (i,j) interior column
-// per thread (KPAR columns deep in k) and marches in k with a ring of KPAR+4
-// shared-memory planes holding all 8 variables: every padded plane is read
-// from HBM exactly once, and because a plane is only overwritten after the
-// ring has moved past it, stages and the diffusion pass update in place.
+// Stencil kernels run one CTA per block (small mixed grids: several, each a run of
+// k planes). The CTA takes an (i, j) column per thread (or KPAR planes of it at a
+// time) through a ring of shared-memory planes holding all 8 variables: a CTA reads
+// every padded plane from HBM exactly once, and because a plane is only
+// overwritten after the ring has moved past it, a whole block can be updated in
+// place.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

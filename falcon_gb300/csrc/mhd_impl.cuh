@@ -226,6 +226,9 @@ __device__ __forceinline__ void fence_proxy_async() {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // 1-D bulk copy global -> shared, completion counted on `bar` (16-byte aligned, size % 16 == 0)
 // Hint: pull `bytes` (a multiple of 16, 16-byte aligned) of global memory into
 // L2 ahead of plain loads.

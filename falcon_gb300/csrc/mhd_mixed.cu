@@ -11,9 +11,9 @@ namespace {
 // place, a part would overwrite planes that its neighbours still read). A grid
 // with few blocks leaves SMs idle or unevenly loaded: the split is the power of
 // two that minimises the planes of the busiest SM, counting one more plane per
-// part for the ghost planes it rereads. 108 blocks of 16^3: stage 34.3 us whole,
-// 32.9 in two, 28.9 in four parts (the rule's); diffusion 50, 41, 37. 864 blocks of
-// 8^3: stage 36.3 whole (the rule's), 41.4 in two.
+// part for the ghost planes it rereads. 108 blocks of 16^3: diffusion 50 us whole,
+// 41 in two, 37 in four parts (the rule's). 864 blocks of 8^3: stage 36.3 us whole
+// (the rule's), 41.4 in two.
 int split_of(const StepDims& d, int most) {
     auto cost = [&](int s) { return ((int64_t)d.nblocks * s + 151) / 152 * (d.nk / s + 1); };
     int best = 1;
@@ -22,16 +22,19 @@ int split_of(const StepDims& d, int most) {
     return best;
 }
 
+// 8^3 blocks: chunks of KP planes; 16^3 blocks (KP 0): the march
 template <int N, int KP, int DIVB>
 cudaError_t stage_nd(const StepDims& d, const Geometry& g, const float* in, const float* un, float* out, int8_t* lo,
                      const PushTable& push, const DivBArgs& psi, int stage, int bcw, StepScalars* sc, cudaStream_t st) {
-    using S = Shape<float, N, N, N, KP>;
-    static const cudaError_t attr = allow_smem(k_stage_quads<N, N, N, KP, DIVB>, S::smem_stage);
-    if (attr != cudaSuccess) return attr;
-    const int split = in != out ? split_of(d, N / KP) : 1;
-    k_stage_quads<N, N, N, KP, DIVB>
-        <<<d.nblocks * split, S::NT, S::smem_stage, st>>>(in, un, out, lo, push, psi, g, sc, stage, bcw, split);
-    return cudaGetLastError();
+    auto run = [&](auto kernel, size_t smem, int nt, int most) {
+        static const cudaError_t attr = allow_smem(kernel, smem);
+        if (attr != cudaSuccess) return attr;
+        const int split = in != out ? split_of(d, most) : 1;
+        kernel<<<d.nblocks * split, nt, smem, st>>>(in, un, out, lo, push, psi, g, sc, stage, bcw, split);
+        return cudaGetLastError();
+    };
+    if constexpr (KP == 0) return run(k_stage_march<N, N, N, DIVB>, SMarch<N, N, N>::smem, N * N, 8);
+    else return run(k_stage_chunks<N, N, N, KP, DIVB>, QShape<N, N, N, KP>::smem, N * N * KP, N / KP);
 }
 // The div-B mode is a template parameter: the plain stage keeps its register
 // allocation free of the GLM/Powell terms.
@@ -71,15 +74,18 @@ cudaError_t diff_march16(const StepDims& d, const Geometry& g, const float* u, f
 }  // namespace
 }  // namespace impl
 
+// 8^3 blocks: planes per chunk; 16^3 blocks: the march, whatever depth is asked for
 cudaError_t launch_stage_mixed(const StepDims& d, const Geometry& g, const float* in, const float* un, float* out,
                                int8_t* lo, const PushTable& push, const DivBArgs& psi, int stage, int bcw, StepScalars* sc,
                                int kpar, cudaStream_t st) {
-#define FALCON_STAGE_CASE(N, K) \
-    if (d.ni == N && kpar == K) return impl::stage_n<N, K>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
     if (d.ni != d.nj || d.ni != d.nk) return cudaErrorInvalidValue;
-    FALCON_STAGE_CASE(8, 2) FALCON_STAGE_CASE(8, 4) FALCON_STAGE_CASE(8, 8)
-    FALCON_STAGE_CASE(16, 1) FALCON_STAGE_CASE(16, 2) FALCON_STAGE_CASE(16, 4)
-#undef FALCON_STAGE_CASE
+    if (d.ni == 16) return impl::stage_n<16, 0>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    if (d.ni != 8) return cudaErrorInvalidValue;
+    switch (kpar) {
+    case 2: return impl::stage_n<8, 2>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    case 4: return impl::stage_n<8, 4>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    case 8: return impl::stage_n<8, 8>(d, g, in, un, out, lo, push, psi, stage, bcw, sc, st);
+    }
     return cudaErrorInvalidValue;
 }
 cudaError_t launch_psi_diffusion_mixed(const StepDims& d, const Geometry& g, const float* u, const float* psi,
@@ -141,10 +147,10 @@ cudaError_t launch_step_persistent_mixed(const StepDims& d, const Geometry& g, f
                                          const GhostLists& gl_final, StepScalars* sc, unsigned int* bar,
                                          cudaStream_t st) {
     if (d.ni != 16 || d.nj != 16 || d.nk != 16 || !bar) return cudaErrorInvalidValue;
-    using SS = impl::Shape<float, 16, 16, 16, 2>;
-    using SD = impl::MShape<16, 16, 16, 2>;
-    constexpr size_t smem = SS::smem_stage > SD::smem ? SS::smem_stage : SD::smem;
-    // two CTAs of 512 threads per SM, as the separate stage and diffusion
+    using SS = impl::SMarch<16, 16, 16>;
+    using SD = impl::MShape<16, 16, 16, 1>;
+    constexpr size_t smem = SS::smem > SD::smem ? SS::smem : SD::smem;
+    // two CTAs of 256 threads per SM, as the separate stage and diffusion
     // launches run (228 KB per SM, 1 KB of it reserved per CTA, and about
     // 0.5 KB of static shared memory in the bodies)
     static_assert(2 * (smem + 512 + 1024) <= 233472, "two CTAs per SM");
@@ -156,7 +162,7 @@ cudaError_t launch_step_persistent_mixed(const StepDims& d, const Geometry& g, f
     if (dev != dev_cached) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0, nsm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorLaunchOutOfResources;
@@ -168,7 +174,7 @@ cudaError_t launch_step_persistent_mixed(const StepDims& d, const Geometry& g, f
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(512);
+    cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

@@ -105,348 +105,567 @@ __device__ __forceinline__ void push_quads(float* out, const PushBlock& P, int i
 }
 
 // ---------------------------------------------------------------------------
-// One RK stage of a block, or of planes [ch0, ch1) x KPAR of it: boundary -> RHS
-// (3_6/ModEquation.f90:24-162) -> u_out = u^n + dt*R/(5-s)
-// (3_6/ModAdvance.f90:87-93). A chunk of KPAR planes is a thread per cell; the
-// derivatives are formed direction by direction, each from the four neighbours'
-// eight values read as two 16-byte accesses, so that a cell takes 26
-// shared-memory reads for its 13 points instead of one per value and use.
-// 21.2M cells: 919 -> 877 us per stage (152 B of HBM traffic a cell instead of
-// 236); 442k cells with split blocks: 37 -> 29.8 us.
-template <int NI, int NJ, int NK, int KPAR, int DIVB>
-__device__ __forceinline__ void stage_quads(int b, int ch0, int ch1, const float* in, const float* un, float* out,
-                                            int8_t* ulo, const PushTable& push, const DivBArgs& psi, const Geometry& g,
-                                            StepScalars* sc, int stage, int bc_writeback) {
-    using S = Shape<float, NI, NJ, NK, KPAR>;
+// The RK stage: boundary -> RHS (3_6/ModEquation.f90:24-162) ->
+// u_out = u^n + dt*R/(5-s) (3_6/ModAdvance.f90:87-93). Two kernels around one cell
+// update (stage_cell): the march of 16^3 blocks and the chunks of 8^3 blocks.
+//
+// The derivatives need rho1 only through p1, so p1 takes rho1's place in the
+// shared-memory ring as soon as a plane has arrived (its reads come with the
+// velocities'); rho1 of the cells themselves is kept beside it, for the
+// buoyancy. The derivatives are formed direction by direction, each from the
+// four neighbours' eight values read as two 16-byte accesses.
+
+// Geometry of a block in shared memory: a cell's radial factors in 16-byte
+// groups, the theta factors likewise
+enum { TI_P1 = 0, TI_R, TI_INV, TI_SRC, TI_COUNT };
+struct StageTables {
+    float4* ti;   // [TI_COUNT][NIP]: p1 coefficients (hi, lo pairs) | rho0, r^2, r, cs | 1/r, 1/r^2, 1/rho0, 1/Xi^2 | g/rho0, heat
+    float4* tj;   // [NJP]: sin, 1/sin, cot of theta
+    float* gs;    // [GS_COUNT]
+    template <int NIP, int NJP> static constexpr size_t bytes() { return ((size_t)TI_COUNT * NIP + NJP) * 16 + GS_COUNT * 4; }
+    __device__ StageTables(unsigned char* m, int nip, int njp)
+        : ti(reinterpret_cast<float4*>(m)), tj(ti + TI_COUNT * nip), gs(reinterpret_cast<float*>(tj + njp)) {}
+    __device__ void load(const Geometry& g, int b, int nip, int njp, int nt) {
+        const float* Gi = g.gi_f + (size_t)b * GI_COUNT * nip;
+        const float* Gj = g.gj_f + (size_t)b * GJ_COUNT * njp;
+        const double* Gd = g.gi + (size_t)b * GI_COUNT * nip;
+        for (int x = threadIdx.x; x < nip; x += nt) {
+            // p1's coefficients as FP32 pairs, hi + lo to about 2^-48
+            const double a1 = Gd[GI_A1 * nip + x], a2 = Gd[GI_A2 * nip + x];
+            const float h1 = (float)a1, h2 = (float)a2;
+            ti[TI_P1 * nip + x] = make_float4(h1, (float)(a1 - (double)h1), h2, (float)(a2 - (double)h2));
+            ti[TI_R * nip + x] = make_float4(Gi[GI_RHO0 * nip + x], Gi[GI_R2 * nip + x], Gi[GI_R * nip + x], Gi[GI_CS * nip + x]);
+            ti[TI_INV * nip + x] = make_float4(Gi[GI_RINV * nip + x], Gi[GI_R2INV * nip + x], Gi[GI_RHO0INV * nip + x], Gi[GI_XI2INV * nip + x]);
+            ti[TI_SRC * nip + x] = make_float4(Gi[GI_GOR0 * nip + x], Gi[GI_HEAT * nip + x], 0.f, 0.f);
+        }
+        for (int x = threadIdx.x; x < njp; x += nt)
+            tj[x] = make_float4(Gj[GJ_SIN * njp + x], Gj[GJ_SININV * njp + x], Gj[GJ_COT * njp + x], 0.f);
+        if (threadIdx.x < GS_COUNT) gs[threadIdx.x] = g.gs_f[(size_t)b * GS_COUNT + threadIdx.x];
+    }
+    // p1 = gamma1*(p0/rho0)*rho1 + (gamma3-1)*(rho0*T0)*s1 (3_6/ModEquation.f90:40-46)
+    __device__ float p1(int ic, float r1, float s1) const {   // (the p1 group is the first)
+        const float4 t = ti[ic];
+        return p1_ff(t.x, t.y, t.z, t.w, r1, s1);
+    }
+};
+
+// The ghost cells of a plane that its interior cells' differences reach (rows
+// and columns; corners have no reader), by index y in [0, 4 (NI + NJ)): padded
+// cell c and its i. Sizes are powers of two: no divisions.
+template <int NI, int NJ, int NIP>
+__device__ __forceinline__ void reached_ghost(int y, int& c, int& ic) {
+    constexpr int HC = 4 * (NI + NJ);
+    static_assert((HC & (HC - 1)) == 0 && NI == NJ, "by shifts and masks");
+    // s: which of the four lines, m: along it. Columns: neighbouring lanes on the
+    // four lines (the rows of a line lie in two shared-memory banks)
+    const bool row = y < HC / 2;
+    const int s = row ? y / NI % 4 : y % 4, m = (row ? y % NI : y % (HC / 2) / 4) + 2, e = s < 2 ? s : NI + s;
+    c = row ? e * NIP + m : m * NIP + e;
+    ic = row ? m : e;
+}
+
+// -(f(2) - 8 f(1) + 8 f(-1) - f(-2)): the O4 difference's sum for two values at
+// once (packed FP32), negated (every rounding is symmetric)
+__device__ __forceinline__ float2 d4neg2(float2 fp2, float2 fp1, float2 fm1, float2 fm2) {
+    return __ffma2_rn(fm2, f2(-1.f), __ffma2_rn(fm1, f2(8.f), __ffma2_rn(fp1, f2(-8.f), fp2)));
+}
+
+// One cell: (ca, cb) its values with p1 in rho1's place, along_x(h, m) those of
+// the neighbour m in {-2, -1, 1, 2} along x, half h; (ua, ub) its u^n and q8 the
+// correction (u^n set by before_k at the latest; final_stage: compensated update,
+// q8 renewed). o: the new values. No branch between the sums: which products of
+// a sum the compiler contracts, and so the last bits, follows from its basic block.
+template <int NIP, int PL, int NCELL, int DIVB, class FI, class FJ, class FK, class FG, class FS, class FB>
+__device__ __forceinline__ void stage_cell(const StageTables& tab, int b, int ii, int jj, size_t cell, float4 ca, float4 cb,
+                                           float rho1, FI along_i, FJ along_j, FK along_k, FG radial, FS sine, FB before_k, const float4& ua,
+                                           const float4& ub, int2& q8, bool final_stage, float dtk, const DivBArgs& psi,
+                                           float (&o)[NV]) {
     using T = float;
-    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, WP = S::WP, NCELL = S::NCELL;
+    const T c1 = tab.gs[GS_C1], c2 = tab.gs[GS_C2], c3 = tab.gs[GS_C3];
+    const float4 inv = tab.ti[TI_INV * NIP + ii], th = tab.tj[jj];
+    const T rinv = inv.x, r2inv = inv.y, rho0inv = inv.z, xi2inv = inv.w, sinv = th.y, cot = th.z;
+    const T rho0c = tab.ti[TI_R * NIP + ii].x;
+    // ModDerivative_1st_O4_3D (3_6/ModDerivative.f90:16-32)
+    auto D = [&](T c, auto f) -> T { return c * (((-f(2) + T(8) * f(1)) - T(8) * f(-1)) + f(-2)); };
+    const T vr = ca.y, vt = ca.z, vp = ca.w, br = cb.x, bt = cb.y, bp = cb.z;
+    T dA, a_vr, a_vt, a_vp, a_s1, g1, d_bpr, d_btr, q_e3r, q_e2r, dB = T(0);
+    {   // along i
+        float4 A[5], B[5], G[5];
+#pragma unroll
+        for (int m = -2; m <= 2; ++m) {
+            if (m == 0) continue;
+            A[m + 2] = along_i(0, m);
+            B[m + 2] = along_i(1, m);
+            G[m + 2] = radial(m);   // rho0, r^2, r
+        }
+        auto E2 = [&](int m) { return A[m + 2].w * B[m + 2].x - A[m + 2].y * B[m + 2].z; };
+        auto E3 = [&](int m) { return A[m + 2].y * B[m + 2].y - A[m + 2].z * B[m + 2].x; };
+        const float2 d0 = d4neg2(f2(A[4].x, A[4].y), f2(A[3].x, A[3].y), f2(A[1].x, A[1].y), f2(A[0].x, A[0].y));
+        const float2 d1 = d4neg2(f2(A[4].z, A[4].w), f2(A[3].z, A[3].w), f2(A[1].z, A[1].w), f2(A[0].z, A[0].w));
+        dA = D(c1, [&](int m) { return (G[m + 2].x * A[m + 2].y) * G[m + 2].y; });
+        dA = dA * r2inv;
+        a_vr = vr * (-c1 * d0.y);
+        a_vt = vr * (-c1 * d1.x);
+        a_vp = vr * (-c1 * d1.y);
+        a_s1 = vr * D(c1, [&](int m) { return B[m + 2].w; });
+        g1 = -c1 * d0.x;
+        d_bpr = D(c1, [&](int m) { return B[m + 2].z * G[m + 2].z; });
+        d_btr = D(c1, [&](int m) { return B[m + 2].y * G[m + 2].z; });
+        q_e3r = D(c1, [&](int m) { return E3(m) * G[m + 2].z; });
+        q_e2r = D(c1, [&](int m) { return E2(m) * G[m + 2].z; });
+        if constexpr (DIVB != 0) dB = D(c1, [&](int m) { return B[m + 2].x * G[m + 2].y; });
+    }
+    T d23, g2, k1, k3, q1, q3, e23 = T(0);
+    {   // along j
+        float4 A[5], B[5];
+        T sn[5];
+#pragma unroll
+        for (int m = -2; m <= 2; ++m) {
+            if (m == 0) continue;
+            A[m + 2] = along_j(0, m);
+            B[m + 2] = along_j(1, m);
+            sn[m + 2] = sine(m);
+        }
+        auto E1 = [&](int m) { return A[m + 2].z * B[m + 2].z - A[m + 2].w * B[m + 2].y; };
+        auto E3 = [&](int m) { return A[m + 2].y * B[m + 2].y - A[m + 2].z * B[m + 2].x; };
+        const float2 d0 = d4neg2(f2(A[4].x, A[4].y), f2(A[3].x, A[3].y), f2(A[1].x, A[1].y), f2(A[0].x, A[0].y));
+        const float2 d1 = d4neg2(f2(A[4].z, A[4].w), f2(A[3].z, A[3].w), f2(A[1].z, A[1].w), f2(A[0].z, A[0].w));
+        d23 = D(c2, [&](int m) { return (rho0c * A[m + 2].z) * sn[m + 2]; });
+        T t = vt * (-c2 * d0.y);
+        a_vr = a_vr + t * rinv;
+        t = vt * (-c2 * d1.x);
+        a_vt = a_vt + t * rinv;
+        t = vt * (-c2 * d1.y);
+        a_vp = a_vp + t * rinv;
+        t = vt * D(c2, [&](int m) { return B[m + 2].w; });
+        a_s1 = a_s1 + t * rinv;
+        g2 = -c2 * d0.x;
+        k1 = D(c2, [&](int m) { return B[m + 2].z * sn[m + 2]; });
+        k3 = d_btr - D(c2, [&](int m) { return B[m + 2].x; });
+        q1 = D(c2, [&](int m) { return E3(m) * sn[m + 2]; });
+        q3 = q_e2r - D(c2, [&](int m) { return E1(m); });
+        if constexpr (DIVB != 0) e23 = D(c2, [&](int m) { return B[m + 2].y * sn[m + 2]; });
+    }
+    before_k();
+    T g3, k2, q2;
+    {   // along k
+        float4 A[5], B[5];
+#pragma unroll
+        for (int m = -2; m <= 2; ++m) {
+            if (m == 0) continue;
+            A[m + 2] = along_k(0, m);
+            B[m + 2] = along_k(1, m);
+        }
+        auto E1 = [&](int m) { return A[m + 2].z * B[m + 2].z - A[m + 2].w * B[m + 2].y; };
+        auto E2 = [&](int m) { return A[m + 2].w * B[m + 2].x - A[m + 2].y * B[m + 2].z; };
+        const float2 d0 = d4neg2(f2(A[4].x, A[4].y), f2(A[3].x, A[3].y), f2(A[1].x, A[1].y), f2(A[0].x, A[0].y));
+        const float2 d1 = d4neg2(f2(A[4].z, A[4].w), f2(A[3].z, A[3].w), f2(A[1].z, A[1].w), f2(A[0].z, A[0].w));
+        d23 = d23 + D(c3, [&](int m) { return rho0c * A[m + 2].w; });
+        T t = vp * (-c3 * d0.y);
+        t = t * rinv;
+        a_vr = a_vr + sinv * t;
+        t = vp * (-c3 * d1.x);
+        t = t * rinv;
+        a_vt = a_vt + sinv * t;
+        t = vp * (-c3 * d1.y);
+        t = t * rinv;
+        a_vp = a_vp + sinv * t;
+        t = vp * D(c3, [&](int m) { return B[m + 2].w; });
+        t = t * rinv;
+        a_s1 = a_s1 + sinv * t;
+        g3 = -c3 * d0.x;
+        k1 = k1 - D(c3, [&](int m) { return B[m + 2].y; });
+        k2 = D(c3, [&](int m) { return B[m + 2].x * sinv; }) - d_bpr;
+        q1 = q1 - D(c3, [&](int m) { return E2(m); });
+        q2 = D(c3, [&](int m) { return E1(m) * sinv; }) - q_e3r;
+        if constexpr (DIVB != 0) e23 = e23 + D(c3, [&](int m) { return B[m + 2].z; });
+    }
+    const float4 src = tab.ti[TI_SRC * NIP + ii];
+    const T gor0 = src.x, heat = src.y;
+    // Mass conservation: -div(rho0 v)/Xi^2 (3_6/ModEquation.f90:50-61, ModSpherical_div :104-159)
+    d23 = d23 * sinv;
+    d23 = d23 * rinv;
+    const T Rrho = -(xi2inv * (dA + d23));
+    // Inertial force -(v.grad)v with curvature terms (3_6/ModSpherical.f90:281-343)
+    T Rvr, Rvt, Rvp;
+    {
+        T tmp = -(vt * vt) - vp * vp;
+        a_vr = a_vr + tmp * rinv;
+        tmp = -(vp * vp);
+        tmp = tmp * cot;
+        tmp = tmp + vt * vr;
+        a_vt = a_vt + tmp * rinv;
+        tmp = vp * vt;
+        tmp = tmp * cot;
+        tmp = tmp + vp * vr;
+        a_vp = a_vp + tmp * rinv;
+        Rvr = -a_vr; Rvt = -a_vt; Rvp = -a_vp;
+    }
+    // Pressure gradient -grad(p1)/rho0 (3_6/ModEquation.f90:79-92)
+    g2 = g2 * rinv;
+    g3 = g3 * rinv;
+    g3 = g3 * sinv;
+    Rvr = Rvr - g1 * rho0inv;
+    Rvt = Rvt - g2 * rho0inv;
+    Rvp = Rvp - g3 * rho0inv;
+    // Lorentz force (curl B) x B / rho0 (3_6/ModEquation.f90:97-116, curl :38-102)
+    {
+        k1 = k1 * rinv; k2 = k2 * rinv; k3 = k3 * rinv;
+        k1 = k1 * sinv;
+        const T x1 = k2 * bp - k3 * bt;
+        const T x2 = k3 * br - k1 * bp;
+        const T x3 = k1 * bt - k2 * br;
+        Rvr = Rvr + x1 * rho0inv;
+        Rvt = Rvt + x2 * rho0inv;
+        Rvp = Rvp + x3 * rho0inv;
+    }
+    // Buoyancy -(g/rho0) rho1 (3_6/ModEquation.f90:121-127)
+    Rvr = Rvr - gor0 * rho1;
+    // Entropy advection and heating (3_6/ModEquation.f90:132-151)
+    T Rs = -a_s1;
+    Rs = Rs + heat;
+    // Induction curl(v x B) (3_6/ModEquation.f90:154-162)
+    q1 = q1 * rinv; q2 = q2 * rinv; q3 = q3 * rinv;
+    q1 = q1 * sinv;
+    T RBr = q1, RBt = q2, RBp = q3;
+
+    // div-B control. GLM cleaning (3_6/ModDivB.f90:13-38), after the
+    // equation terms as 3_6/ModAdvance.f90:82-84 orders it: dB += -grad(psi);
+    // dpsi = -v_wave^2 div(B) - v_wave/h_LLL psi, v_wave from u^n. Powell
+    // (3_5/ModEquation.f90:169-176): dB += -(div B) v.
+    T divB = T(0);
+    if constexpr (DIVB != 0) {   // ModSpherical_div of B (3_6/ModSpherical.f90:104-159)
+        dB = dB * r2inv;
+        e23 = e23 * sinv;
+        e23 = e23 * rinv;
+        divB = dB + e23;
+    }
+    if constexpr (DIVB == 2) {
+        RBr = RBr - divB * vr;
+        RBt = RBt - divB * vt;
+        RBp = RBp - divB * vp;
+    }
+    if constexpr (DIVB == 1) {
+        const T* P = static_cast<const T*>(psi.in) + (size_t)b * NCELL + cell;
+        auto Q = [&](int di, int dj, int dk) -> T { return P[(ptrdiff_t)dk * PL + dj * NIP + di]; };
+        // ModSpherical_Grad_f (3_6/ModSpherical.f90:201-239)
+        const T h1 = D(c1, [&](int m) { return Q(m, 0, 0); });
+        T h2 = D(c2, [&](int m) { return Q(0, m, 0); });
+        h2 = h2 * rinv;
+        T h3 = D(c3, [&](int m) { return Q(0, 0, m); });
+        h3 = h3 * rinv;
+        h3 = h3 * sinv;
+        RBr = RBr - h1;
+        RBt = RBt - h2;
+        RBp = RBp - h3;
+        // ModWaveSpeed_Dynamo (3_6/ModWaveSpeed.f90:8-27) and h_LLL
+        // (3_6/ModBlock.f90:416-425) at this cell, as the CFL pass forms them
+        T w = tab.ti[TI_R * NIP + ii].w + sqrt(ua.y * ua.y + ua.z * ua.z + ua.w * ua.w);
+        w = w + sqrt(ub.x * ub.x + ub.y * ub.y + ub.z * ub.z) / sqrt(rho0c);
+        const T rcell = tab.ti[TI_R * NIP + ii].z;
+        const T h = fmin(fmin(tab.gs[GS_DXI], rcell * tab.gs[GS_DXJ]), rcell * th.x * tab.gs[GS_DXK]);
+        const T Rpsi = -(w * w * divB) - w / h * Q(0, 0, 0);
+        const size_t pc = (size_t)b * NCELL + cell;
+        const T pn = static_cast<const T*>(psi.un)[pc];
+        static_cast<T*>(psi.out)[pc] = fmaf(dtk, Rpsi, pn);
+    }
+
+    // stage update
+    const T R[NV] = {Rrho, Rvr, Rvt, Rvp, RBr, RBt, RBp, Rs};
+    T u0s[NV];
+    split(ua, ub, u0s);
+    if (final_stage) {
+        // u^{n+1} = u^n + dt*R with u^n and u^{n+1} compensated
+        int qn[2] = {0, 0};
+#pragma unroll
+        for (int v = 0; v < NV; v += 2) {   // pairs of variables: ff_add2 gives ff_add's bits
+            const int q = v < 4 ? q8.x : q8.y, sh = 8 * (v & 3);
+            int8_t qa, qb;
+            const float2 ov = ff_add2(f2(u0s[v], u0s[v + 1]), (int8_t)(q >> sh), (int8_t)(q >> (sh + 8)),
+                                      __fmul2_rn(f2(dtk), f2(R[v], R[v + 1])), qa, qb);
+            o[v] = ov.x;
+            o[v + 1] = ov.y;
+            qn[v >> 2] |= ((int)(uint8_t)qa | (int)(uint8_t)qb << 8) << sh;
+        }
+        q8 = make_int2(qn[0], qn[1]);
+    } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) o[v] = fmaf(dtk, R[v], u0s[v]);
+    }
+}
+
+// Chunks of KPAR planes, a thread per cell: 8^3 blocks. Planes [ch0, ch1) x KPAR of
+// block b. The planes of the next chunk, copied during this one, get their
+// boundary condition and p1 at its end, so a chunk is one barrier.
+// 442k cells (864 blocks): 36.3 -> 34 us per stage.
+template <int NI, int NJ, int NK, int KPAR>
+struct QShape : Shape<float, NI, NJ, NK, KPAR> {
+    using B = Shape<float, NI, NJ, NK, KPAR>;
+    // shared memory: mbarriers | tile[2][W][PL] of 16 bytes | rho1[W][PLI] | tables
+    static constexpr size_t off_tile = 16;
+    static constexpr size_t off_rho = off_tile + (size_t)2 * B::W * B::PL * 16;
+    static constexpr size_t off_tab = off_rho + (size_t)B::W * B::PLI * 4;
+    static constexpr size_t smem = off_tab + StageTables::bytes<B::NIP, B::NJP>();
+    static_assert(off_tab % 16 == 0 && smem <= 232448, "16-byte tables; 227 KB of opt-in shared memory per CTA");
+    // as many CTAs per SM as the shared memory holds (228 KB, 1 KB of it reserved
+    // and about 0.2 KB static per CTA): the registers must fit them too
+    static constexpr int by_smem = (int)(233472 / (smem + 1280));
+    static constexpr int reg_cap = 2048 / B::NT;
+    static constexpr int min_blocks = by_smem < reg_cap ? by_smem : reg_cap;
+};
+template <int NI, int NJ, int NK, int KPAR, int DIVB>
+__device__ __forceinline__ void stage_chunks(int b, int ch0, int ch1, const float* in, const float* un, float* out,
+                                             int8_t* ulo, const PushTable& push, const DivBArgs& psi, const Geometry& g,
+                                             StepScalars* sc, int stage, int bc_writeback) {
+    using S = QShape<NI, NJ, NK, KPAR>;
+    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, HC = 4 * (NI + NJ);
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-    double* a12 = reinterpret_cast<double*>(smem + S::off_a12);
     float4* tile = reinterpret_cast<float4*>(smem + S::off_tile);   // [2][W][PL]
-    T* tp1 = reinterpret_cast<T*>(smem + S::off_p1);
-    T* gi = reinterpret_cast<T*>(smem + S::off_gi);
-    T* gj = reinterpret_cast<T*>(smem + S::off_gj);
-    T* gs = reinterpret_cast<T*>(smem + S::off_gs);
-    static_assert(S::off_tile % 16 == 0, "16-byte cells");
-
+    float* rho = reinterpret_cast<float*>(smem + S::off_rho);       // [W][PLI]
+    StageTables tab(smem + S::off_tab, NIP, S::NJP);
     const int fl = g.flags[b];
     const float* blk_in = in + (size_t)b * NV * NCELL;
     float* wb = bc_writeback ? const_cast<float*>(blk_in) : nullptr;
     __shared__ PushBlock pb;
     load_push_block(push, b, &pb);
-    if (threadIdx.x == 0) {
+    const int tid = threadIdx.x, nch = ch1 - ch0;
+    if (tid == 0) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         fence_mbar_init();
+        issue_quads<S>(blk_in, tile, ch0 * KPAR, ch0 * KPAR + KPAR + 4, 0, &bars[0]);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) issue_quads<S>(blk_in, tile, ch0 * KPAR, ch0 * KPAR + KPAR + 4, 0, &bars[0]);
-    // u^n (and its int8 correction at stage 4) is read with plain loads at
-    // stages 2-4: warm L2 with the rows of the first chunk, then one chunk ahead
-    auto prefetch_un = [&](int kp_first) {
-        if (stage == 1) return;
-        for (int x = threadIdx.x; x < 2 * KPAR * NJ; x += S::NT) {   // a row of one half: NI cells of 16 bytes
-            const int h = x & 1, r = x >> 1, j = r % NJ, q = r / NJ;
-            prefetch_l2(quads(un) + quad(b, h, NCELL) + (size_t)(kp_first + q) * PL + (j + 2) * NIP + 2, NI * 16u);
-        }
-        if (ulo != nullptr && stage == 4 && threadIdx.x == 0)
-            prefetch_l2(ulo + ((size_t)b * S::NINT + (size_t)(kp_first - 2) * S::PLI) * NV, KPAR * S::PLI * NV);
-    };
-    prefetch_un(ch0 * KPAR + 2);
-    load_geometry<T, S>(g, b, gi, gj, gs, a12);
-    __syncthreads();   // the geometry tables are read by every thread below
+    tab.load(g, b, NIP, S::NJP, S::NT);
+    __syncthreads();   // barriers and tables are used by every thread below
 
-    const int tid = threadIdx.x;
     int i, j, kq;
     cell_of_thread<NI, NJ, KPAR>(tid, i, j, kq);
-    const int ii = i + 2, jj = j + 2;
-    const T c1 = gs[GS_C1], c2 = gs[GS_C2], c3 = gs[GS_C3];
-    const T* GR = gi + GI_R * NIP;
-    const T* GR2 = gi + GI_R2 * NIP;
-    const T* GRHO0 = gi + GI_RHO0 * NIP;
-    const T* GSIN = gj + GJ_SIN * S::NJP;
-    const T rinv = gi[GI_RINV * NIP + ii], r2inv = gi[GI_R2INV * NIP + ii];
-    const T sinv = gj[GJ_SININV * S::NJP + jj], cot = gj[GJ_COT * S::NJP + jj];
-    const T rho0c = GRHO0[ii], rho0inv = gi[GI_RHO0INV * NIP + ii];
-    const T gor0 = gi[GI_GOR0 * NIP + ii], heat = gi[GI_HEAT * NIP + ii], xi2inv = gi[GI_XI2INV * NIP + ii];
+    const int ii = i + 2, jj = j + 2, c0 = jj * NIP + ii;
     const float dtk = sc->dt_stage_f[stage - 1];
     const int polls = sc->wait_polls;
+    const bool final_stage = ulo != nullptr && stage == 4;
     int late = 0;   // a wait of this thread for a chunk's planes ran out
-    for (int ch = ch0; ch < ch1; ++ch) {
-        const int n = ch - ch0;
-        const int k0 = 1 + ch * KPAR;  // first Fortran k of the chunk
-        const int lo = n == 0 ? ch * KPAR : k0 + 3;   // first padded plane new to this chunk
-        const int hi = k0 + KPAR + 3;                 // one past the last plane it needs
-        // the chunk before is done with the slots the prefetch below overwrites; a
-        // wait of it that ran out ends the CTA here
-        if (__syncthreads_or(late)) {
-            copy_wait_abort(sc, bars, n - 1, n);
-            return;
-        }
-        if (threadIdx.x == 0 && ch + 1 < ch1) issue_quads<S>(blk_in, tile, hi, hi + KPAR, 0, &bars[(n + 1) & 1]);
-        if (ch + 1 < ch1) prefetch_un(k0 + KPAR + 1);
-        // a wait that runs out does not leave the chunk (its barriers must be
-        // reached by every thread): the chunk computes on whatever the slots
-        // hold, the step is flagged and its results are discarded
-        late |= mbar_wait(&bars[n & 1], (uint32_t)((n >> 1) & 1), polls) ? 0 : 1;
-        // u^n for the update (stages 2-4), loaded here so that the latency of
-        // these plain loads overlaps the boundary and p1 phases below
-        const int kp = k0 + kq + 1;
-        const size_t cell = (size_t)kp * PL + jj * NIP + ii;
-        float4 ua = make_float4(0.f, 0.f, 0.f, 0.f), ub = ua;
-        if (stage != 1) {
-            ua = quads(un)[quad(b, 0, NCELL) + cell];
-            ub = quads(un)[quad(b, 1, NCELL) + cell];
-        }
+
+    // planes [lo, lo + np), just copied: boundary condition, p1 in rho1's place
+    auto prepare = [&](int lo, int np) {
         if (fl & 6) {   // radial boundary block (uniform over the CTA)
-            apply_bc_quads<S>(tile, lo, hi, 0, fl, wb, S::NT);
-            fence_proxy_async();   // order these generic writes before later bulk copies into the slots
+            apply_bc_quads<S>(tile, lo, lo + np, 0, fl, wb, S::NT);
             __syncthreads();
         }
-        // p1 = gamma1*(p0/rho0)*rho1 + (gamma3-1)*(rho0*T0)*s1 (3_6/ModEquation.f90:40-46)
-        for (int x = tid; x < (hi - lo) * PL; x += S::NT) {
-            const int kx = lo + x / PL, c = x % PL, ic = c % NIP, slot = kx % W;
-            const float* f = reinterpret_cast<const float*>(a12);
-            tp1[(kx % WP) * PL + c] = p1_ff(f[ic], f[NIP + ic], f[2 * NIP + ic], f[3 * NIP + ic],
-                                            tile[slot * PL + c].x, tile[(W + slot) * PL + c].w);
+        auto p1_at = [&](int slot, int c, int ic) {
+            float4* a = tile + slot * PL + c;
+            const float r1 = a->x;
+            a->x = tab.p1(ic, r1, tile[(W + slot) * PL + c].w);
+            return r1;
+        };
+        for (int q = kq; q < np; q += KPAR) {
+            const int slot = (lo + q) % W;
+            rho[slot * S::PLI + j * NI + i] = p1_at(slot, c0, ii);
         }
-        __syncthreads();
-
-        int sl[5], sp[5];
+        for (int x = tid; x < np * HC; x += S::NT) {
+            int c, ic;
+            reached_ghost<NI, NJ, NIP>(x % HC, c, ic);
+            p1_at((lo + x / HC) % W, c, ic);
+        }
+        fence_proxy_async();   // order these generic writes before later bulk copies into the slots
+    };
+    late |= mbar_wait(&bars[0], 0u, polls) ? 0 : 1;
+    prepare(ch0 * KPAR, KPAR + 4);
+    for (int n = 0; n < nch; ++n) {
+        const int ch = ch0 + n, next = (ch + 1) * KPAR + 4;   // next: first plane new to the next chunk
+        // this chunk's planes are complete and the slots of the next one's are
+        // free. A wait that ran out does not leave its chunk (its barriers must be
+        // reached by every thread): whatever the slots held was computed on, the
+        // step is flagged here and its results are discarded
+        if (__syncthreads_or(late)) {
+            copy_wait_abort(sc, bars, n, n);
+            return;
+        }
+        if (tid == 0 && n + 1 < nch) issue_quads<S>(blk_in, tile, next, next + KPAR, 0, &bars[(n + 1) & 1]);
+        const int kp = ch * KPAR + kq + 2;
+        const size_t cell = (size_t)kp * PL + c0;
+        int sl[5];
 #pragma unroll
-        for (int d = 0; d < 5; ++d) { sl[d] = (kp + d - 2) % W * PL + jj * NIP + ii; sp[d] = (kp + d - 2) % WP * PL + jj * NIP + ii; }
-        const float4* ta = tile;
-        const float4* tb = tile + W * PL;
-        // ModDerivative_1st_O4_3D (3_6/ModDerivative.f90:16-32)
-        auto D = [&](T c, auto f) -> T { return c * (((-f(2) + T(8) * f(1)) - T(8) * f(-1)) + f(-2)); };
-        const float4 ca = ta[sl[2]], cb = tb[sl[2]];
-        const T rho1 = ca.x, vr = ca.y, vt = ca.z, vp = ca.w, br = cb.x, bt = cb.y, bp = cb.z;
-        if (stage == 1) {   // the input is u^n and sits in the ring
-            ua = ca;
-            ub = cb;
-        }
-        T dA, a_vr, a_vt, a_vp, a_s1, g1, d_bpr, d_btr, q_e3r, q_e2r, dB = T(0);
-        {   // along i
-            float4 A[5], B[5];
-            T P[5];
-#pragma unroll
-            for (int m = -2; m <= 2; ++m) {
-                if (m == 0) continue;
-                A[m + 2] = ta[sl[2] + m];
-                B[m + 2] = tb[sl[2] + m];
-                P[m + 2] = tp1[sp[2] + m];
-            }
-            auto E2 = [&](int m) { return A[m + 2].w * B[m + 2].x - A[m + 2].y * B[m + 2].z; };
-            auto E3 = [&](int m) { return A[m + 2].y * B[m + 2].y - A[m + 2].z * B[m + 2].x; };
-            dA = D(c1, [&](int m) { return (GRHO0[ii + m] * A[m + 2].y) * GR2[ii + m]; });
-            dA = dA * r2inv;
-            a_vr = vr * D(c1, [&](int m) { return A[m + 2].y; });
-            a_vt = vr * D(c1, [&](int m) { return A[m + 2].z; });
-            a_vp = vr * D(c1, [&](int m) { return A[m + 2].w; });
-            a_s1 = vr * D(c1, [&](int m) { return B[m + 2].w; });
-            g1 = D(c1, [&](int m) { return P[m + 2]; });
-            d_bpr = D(c1, [&](int m) { return B[m + 2].z * GR[ii + m]; });
-            d_btr = D(c1, [&](int m) { return B[m + 2].y * GR[ii + m]; });
-            q_e3r = D(c1, [&](int m) { return E3(m) * GR[ii + m]; });
-            q_e2r = D(c1, [&](int m) { return E2(m) * GR[ii + m]; });
-            if constexpr (DIVB != 0) dB = D(c1, [&](int m) { return B[m + 2].x * GR2[ii + m]; });
-        }
-        T d23, g2, k1, k3, q1, q3, e23 = T(0);
-        {   // along j
-            float4 A[5], B[5];
-            T P[5];
-#pragma unroll
-            for (int m = -2; m <= 2; ++m) {
-                if (m == 0) continue;
-                A[m + 2] = ta[sl[2] + m * NIP];
-                B[m + 2] = tb[sl[2] + m * NIP];
-                P[m + 2] = tp1[sp[2] + m * NIP];
-            }
-            auto E1 = [&](int m) { return A[m + 2].z * B[m + 2].z - A[m + 2].w * B[m + 2].y; };
-            auto E3 = [&](int m) { return A[m + 2].y * B[m + 2].y - A[m + 2].z * B[m + 2].x; };
-            d23 = D(c2, [&](int m) { return (rho0c * A[m + 2].z) * GSIN[jj + m]; });
-            T t = vt * D(c2, [&](int m) { return A[m + 2].y; });
-            a_vr = a_vr + t * rinv;
-            t = vt * D(c2, [&](int m) { return A[m + 2].z; });
-            a_vt = a_vt + t * rinv;
-            t = vt * D(c2, [&](int m) { return A[m + 2].w; });
-            a_vp = a_vp + t * rinv;
-            t = vt * D(c2, [&](int m) { return B[m + 2].w; });
-            a_s1 = a_s1 + t * rinv;
-            g2 = D(c2, [&](int m) { return P[m + 2]; });
-            k1 = D(c2, [&](int m) { return B[m + 2].z * GSIN[jj + m]; });
-            k3 = d_btr - D(c2, [&](int m) { return B[m + 2].x; });
-            q1 = D(c2, [&](int m) { return E3(m) * GSIN[jj + m]; });
-            q3 = q_e2r - D(c2, [&](int m) { return E1(m); });
-            if constexpr (DIVB != 0) e23 = D(c2, [&](int m) { return B[m + 2].y * GSIN[jj + m]; });
-        }
-        T g3, k2, q2;
-        {   // along k
-            float4 A[5], B[5];
-            T P[5];
-#pragma unroll
-            for (int m = -2; m <= 2; ++m) {
-                if (m == 0) continue;
-                A[m + 2] = ta[sl[m + 2]];
-                B[m + 2] = tb[sl[m + 2]];
-                P[m + 2] = tp1[sp[m + 2]];
-            }
-            auto E1 = [&](int m) { return A[m + 2].z * B[m + 2].z - A[m + 2].w * B[m + 2].y; };
-            auto E2 = [&](int m) { return A[m + 2].w * B[m + 2].x - A[m + 2].y * B[m + 2].z; };
-            d23 = d23 + D(c3, [&](int m) { return rho0c * A[m + 2].w; });
-            T t = vp * D(c3, [&](int m) { return A[m + 2].y; });
-            t = t * rinv;
-            a_vr = a_vr + sinv * t;
-            t = vp * D(c3, [&](int m) { return A[m + 2].z; });
-            t = t * rinv;
-            a_vt = a_vt + sinv * t;
-            t = vp * D(c3, [&](int m) { return A[m + 2].w; });
-            t = t * rinv;
-            a_vp = a_vp + sinv * t;
-            t = vp * D(c3, [&](int m) { return B[m + 2].w; });
-            t = t * rinv;
-            a_s1 = a_s1 + sinv * t;
-            g3 = D(c3, [&](int m) { return P[m + 2]; });
-            k1 = k1 - D(c3, [&](int m) { return B[m + 2].y; });
-            k2 = D(c3, [&](int m) { return B[m + 2].x * sinv; }) - d_bpr;
-            q1 = q1 - D(c3, [&](int m) { return E2(m); });
-            q2 = D(c3, [&](int m) { return E1(m) * sinv; }) - q_e3r;
-            if constexpr (DIVB != 0) e23 = e23 + D(c3, [&](int m) { return B[m + 2].z; });
-        }
-        // Mass conservation: -div(rho0 v)/Xi^2 (3_6/ModEquation.f90:50-61, ModSpherical_div :104-159)
-        d23 = d23 * sinv;
-        d23 = d23 * rinv;
-        const T Rrho = -(xi2inv * (dA + d23));
-        // Inertial force -(v.grad)v with curvature terms (3_6/ModSpherical.f90:281-343)
-        T Rvr, Rvt, Rvp;
-        {
-            T tmp = -(vt * vt) - vp * vp;
-            a_vr = a_vr + tmp * rinv;
-            tmp = -(vp * vp);
-            tmp = tmp * cot;
-            tmp = tmp + vt * vr;
-            a_vt = a_vt + tmp * rinv;
-            tmp = vp * vt;
-            tmp = tmp * cot;
-            tmp = tmp + vp * vr;
-            a_vp = a_vp + tmp * rinv;
-            Rvr = -a_vr; Rvt = -a_vt; Rvp = -a_vp;
-        }
-        // Pressure gradient -grad(p1)/rho0 (3_6/ModEquation.f90:79-92)
-        g2 = g2 * rinv;
-        g3 = g3 * rinv;
-        g3 = g3 * sinv;
-        Rvr = Rvr - g1 * rho0inv;
-        Rvt = Rvt - g2 * rho0inv;
-        Rvp = Rvp - g3 * rho0inv;
-        // Lorentz force (curl B) x B / rho0 (3_6/ModEquation.f90:97-116, curl :38-102)
-        {
-            k1 = k1 * rinv; k2 = k2 * rinv; k3 = k3 * rinv;
-            k1 = k1 * sinv;
-            const T x1 = k2 * bp - k3 * bt;
-            const T x2 = k3 * br - k1 * bp;
-            const T x3 = k1 * bt - k2 * br;
-            Rvr = Rvr + x1 * rho0inv;
-            Rvt = Rvt + x2 * rho0inv;
-            Rvp = Rvp + x3 * rho0inv;
-        }
-        // Buoyancy -(g/rho0) rho1 (3_6/ModEquation.f90:121-127)
-        Rvr = Rvr - gor0 * rho1;
-        // Entropy advection and heating (3_6/ModEquation.f90:132-151)
-        T Rs = -a_s1;
-        Rs = Rs + heat;
-        // Induction curl(v x B) (3_6/ModEquation.f90:154-162)
-        q1 = q1 * rinv; q2 = q2 * rinv; q3 = q3 * rinv;
-        q1 = q1 * sinv;
-        T RBr = q1, RBt = q2, RBp = q3;
-
-        // div-B control. GLM cleaning (3_6/ModDivB.f90:13-38), after the
-        // equation terms as 3_6/ModAdvance.f90:82-84 orders it: dB += -grad(psi);
-        // dpsi = -v_wave^2 div(B) - v_wave/h_LLL psi, v_wave from u^n. Powell
-        // (3_5/ModEquation.f90:169-176): dB += -(div B) v.
-        T divB = T(0);
-        if constexpr (DIVB != 0) {   // ModSpherical_div of B (3_6/ModSpherical.f90:104-159)
-            dB = dB * r2inv;
-            e23 = e23 * sinv;
-            e23 = e23 * rinv;
-            divB = dB + e23;
-        }
-        if constexpr (DIVB == 2) {
-            RBr = RBr - divB * vr;
-            RBt = RBt - divB * vt;
-            RBp = RBp - divB * vp;
-        }
-        if constexpr (DIVB == 1) {
-            const T* P = static_cast<const T*>(psi.in) + (size_t)b * NCELL + cell;
-            auto Q = [&](int di, int dj, int dk) -> T { return P[(ptrdiff_t)dk * PL + dj * NIP + di]; };
-            // ModSpherical_Grad_f (3_6/ModSpherical.f90:201-239)
-            const T h1 = D(c1, [&](int m) { return Q(m, 0, 0); });
-            T h2 = D(c2, [&](int m) { return Q(0, m, 0); });
-            h2 = h2 * rinv;
-            T h3 = D(c3, [&](int m) { return Q(0, 0, m); });
-            h3 = h3 * rinv;
-            h3 = h3 * sinv;
-            RBr = RBr - h1;
-            RBt = RBt - h2;
-            RBp = RBp - h3;
-            // ModWaveSpeed_Dynamo (3_6/ModWaveSpeed.f90:8-27) and h_LLL
-            // (3_6/ModBlock.f90:416-425) at this cell, as the CFL pass forms them
-            T w = gi[GI_CS * NIP + ii] + sqrt(ua.y * ua.y + ua.z * ua.z + ua.w * ua.w);
-            w = w + sqrt(ub.x * ub.x + ub.y * ub.y + ub.z * ub.z) / sqrt(rho0c);
-            const T rcell = GR[ii];
-            const T h = fmin(fmin(gs[GS_DXI], rcell * gs[GS_DXJ]), rcell * GSIN[jj] * gs[GS_DXK]);
-            const T Rpsi = -(w * w * divB) - w / h * Q(0, 0, 0);
-            const size_t pc = (size_t)b * NCELL + cell;
-            const T pn = static_cast<const T*>(psi.un)[pc];
-            static_cast<T*>(psi.out)[pc] = fmaf(dtk, Rpsi, pn);
-        }
-
-        // stage update
-        const T R[NV] = {Rrho, Rvr, Rvt, Rvp, RBr, RBt, RBp, Rs};
-        T u0s[NV], o[NV];
-        split(ua, ub, u0s);
-        if (ulo != nullptr && stage == 4) {
-            // u^{n+1} = u^n + dt*R with u^n and u^{n+1} compensated
-            int2* ql = reinterpret_cast<int2*>(ulo + ((size_t)b * S::NINT + ((size_t)(kp - 2) * NJ + j) * NI + i) * NV);
-            const int2 q8 = *ql;
-            int qn[2] = {0, 0};
-#pragma unroll
-            for (int v = 0; v < NV; v += 2) {   // pairs of variables: ff_add2 gives ff_add's bits
-                const int q = v < 4 ? q8.x : q8.y, sh = 8 * (v & 3);
-                int8_t qa, qb;
-                const float2 ov = ff_add2(f2(u0s[v], u0s[v + 1]), (int8_t)(q >> sh), (int8_t)(q >> (sh + 8)),
-                                          __fmul2_rn(f2(dtk), f2(R[v], R[v + 1])), qa, qb);
-                o[v] = ov.x;
-                o[v + 1] = ov.y;
-                qn[v >> 2] |= ((int)(uint8_t)qa | (int)(uint8_t)qb << 8) << sh;
-            }
-            *ql = make_int2(qn[0], qn[1]);
-        } else {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) o[v] = fmaf(dtk, R[v], u0s[v]);
-        }
+        for (int d = 0; d < 5; ++d) sl[d] = (kp + d - 2) % W * PL + c0;
+        float4 ua, ub;
+        int2* ql = reinterpret_cast<int2*>(ulo + ((size_t)b * S::NINT + ((size_t)(kp - 2) * NJ + j) * NI + i) * NV);
+        int2 q8 = make_int2(0, 0);
+        if (final_stage) q8 = *ql;
+        float o[NV];
+        stage_cell<NIP, PL, NCELL, DIVB>(
+            tab, b, ii, jj, cell, tile[sl[2]], tile[W * PL + sl[2]], rho[kp % W * S::PLI + j * NI + i],
+            [&](int h, int m) { return tile[h * W * PL + sl[2] + m]; },
+            [&](int h, int m) { return tile[h * W * PL + sl[2] + m * NIP]; },
+            [&](int h, int m) { return tile[h * W * PL + sl[m + 2]]; },
+            [&](int m) { return tab.ti[TI_R * NIP + ii + m]; }, [&](int m) { return tab.tj[jj + m].x; },
+            // u^n (at stage 1 the input: in L2), loaded here so that the latency
+            // overlaps the k derivatives (earlier, the registers spill)
+            [&]() {
+                ua = quads(un)[quad(b, 0, NCELL) + cell];
+                ub = quads(un)[quad(b, 1, NCELL) + cell];
+            },
+            ua, ub, q8, final_stage, dtk, psi, o);
+        if (final_stage) *ql = q8;
         quads(out)[quad(b, 0, NCELL) + cell] = f4(o);
         quads(out)[quad(b, 1, NCELL) + cell] = f4(o + 4);
         if (push.tgt != nullptr) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+        if (n + 1 < nch) {
+            late |= mbar_wait(&bars[(n + 1) & 1], (uint32_t)(((n + 1) >> 1) & 1), polls) ? 0 : 1;
+            prepare(next, KPAR);
+        }
     }
-    const int nch = ch1 - ch0;
-    if (__syncthreads_or(late)) {
-        copy_wait_abort(sc, bars, nch - 1, nch - 1);
-        return;
-    }
-    if (threadIdx.x == 0) {   // every copy has been waited for
-        mbar_inval(&bars[0]);
-        mbar_inval(&bars[1]);
-    }
+    // every copy was waited for before the last chunk's barrier
 }
-// split CTAs per block, each a run of whole chunks
+
+// The march along k: 16^3 blocks, planes [ka, kb) of block b, one thread per (i, j)
+// column (256 threads, two CTAs per SM). Planes arrive by bulk copy into a ring of
+// 7 slots, an mbarrier each; a plane's boundary condition and p1 (each thread its
+// own column, the first 128 a ghost cell as well) are formed one plane before its
+// first use, as the neighbour kp + 2, so a plane is one barrier. u^n is read a
+// plane ahead, and what depends on the column alone (the neighbours' radial and
+// theta factors) stays in registers.
+//
+// What bounds it: the shared-memory reads (70% of that pipe's cycles) and, with
+// 16 warps per SM, the issue (56%). A register window along k spares 8 of the 26
+// reads and costs as much in moves (763 us), unrolled by five to avoid those it
+// loses to the instruction cache (823); chunks of two planes with 64 registers a
+// thread spill (1,006). 21.2M cells: 877 -> 708 us per stage.
+template <int NI, int NJ, int NK>
+struct SMarch {
+    static constexpr int NIP = NI + 4, NJP = NJ + 4, NKP = NK + 4, PL = NIP * NJP, NCELL = PL * NKP, PLI = NI * NJ, NINT = PLI * NK;
+    static constexpr int NT = NI * NJ, W = 7;
+    // shared memory: mbarriers | tile[2][W][PL] of 16 bytes | rho1[4][PLI] | tables
+    static constexpr size_t off_tile = 128, off_rho = off_tile + (size_t)2 * W * PL * 16, off_tab = off_rho + (size_t)4 * PLI * 4;
+    static constexpr size_t smem = off_tab + StageTables::bytes<NIP, NJP>();
+    static_assert(2 * (smem + 1280) <= 233472, "two CTAs per SM");
+};
+template <int NI, int NJ, int NK, int DIVB>
+__device__ __forceinline__ void stage_march(int b, int ka, int kb, const float* in, const float* un, float* out,
+                                            int8_t* ulo, const PushTable& push, const DivBArgs& psi, const Geometry& g,
+                                            StepScalars* sc, int stage, int bc_writeback) {
+    using S = SMarch<NI, NJ, NK>;
+    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, HC = 4 * (NI + NJ);
+    static_assert(NI == 16 && HC <= S::NT, "rows of 16 cells: one half-warp per row; a plane's ghost cells in one pass");
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);   // plane p's: p - p0 counted from the first plane, modulo W
+    float4* tile = reinterpret_cast<float4*>(smem + S::off_tile);   // [2][W][PL]
+    StageTables tab(smem + S::off_tab, NIP, S::NJP);
+    const int fl = g.flags[b];
+    const float* blk_in = in + (size_t)b * NV * NCELL;
+    float* wb = bc_writeback ? const_cast<float*>(blk_in) : nullptr;
+    __shared__ PushBlock pb;
+    load_push_block(push, b, &pb);
+    const int tid = threadIdx.x, p0 = ka - 2, pe = kb + 2;   // planes [p0, pe) are read
+    int issued = p0;                                         // thread 0: planes [p0, issued) have been requested
+    auto issue = [&](int last) {
+        for (; issued <= last && issued < pe; ++issued)
+            issue_quads<S>(blk_in, tile, issued, issued + 1, p0, &bars[(issued - p0) % W]);
+    };
+    if (tid == 0) {
+        for (int q = 0; q < W; ++q) mbar_init(&bars[q], 1);
+        fence_mbar_init();
+        issue(p0 + W - 1);
+    }
+    tab.load(g, b, NIP, S::NJP, S::NT);
+    __syncthreads();   // barriers and tables are used by every thread below
+    const int i = tid % NI, j = tid / NI, ii = i + 2, jj = j + 2, c0 = jj * NIP + ii;
+    const float dtk = sc->dt_stage_f[stage - 1];
+    const int polls = sc->wait_polls;
+    const bool final_stage = ulo != nullptr && stage == 4;
+    // a wait of this thread ran out: it computes on whatever the slots hold (and
+    // waits no more), the step is flagged and its results are discarded
+    int late = 0;
+    auto arrived = [&](int p) {
+        late |= mbar_wait(&bars[(p - p0) % W], (uint32_t)(((p - p0) / W) & 1), late ? 1 : polls) ? 0 : 1;
+    };
+    int gc, gic;   // this thread's ghost cell of a plane (the first HC threads)
+    reached_ghost<NI, NJ, NIP>(tid % HC, gc, gic);
+    float* rho = reinterpret_cast<float*>(smem + S::off_rho) + tid;   // its rho1 of planes kp .. kp + 3, plane p's at p % 4
+    // plane p in slot s, just copied: boundary condition, p1 in rho1's place
+    auto prepare = [&](int p, int s) {
+        if (fl & 6) {   // radial boundary block (uniform over the CTA)
+            apply_bc_quads<S>(tile, p, p + 1, p0, fl, wb, S::NT);
+            __syncthreads();
+        }
+        float4* a = tile + s * PL + c0;
+        const float r1 = a->x;
+        rho[p % 4 * S::PLI] = r1;
+        a->x = tab.p1(ii, r1, a[W * PL].w);
+        if (tid < HC) {
+            a = tile + s * PL + gc;
+            a->x = tab.p1(gic, a->x, a[W * PL].w);
+        }
+        fence_proxy_async();   // order these generic writes before later bulk copies into the slot
+    };
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+        arrived(p0 + m);
+        prepare(p0 + m, m);
+    }
+    __syncthreads();
+    const float4* un_b = quads(un) + quad(b, 0, NCELL);
+    float4* out_b = quads(out) + quad(b, 0, NCELL);
+    int2* lo_b = reinterpret_cast<int2*>(ulo + ((size_t)b * S::NINT + tid) * NV);
+    // the neighbours' radial and theta factors
+    float4 gr[5];
+    float sn[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) { gr[m] = tab.ti[TI_R * NIP + ii + m - 2]; sn[m] = tab.tj[jj + m - 2].x; }
+    float4 na = un_b[ka * PL + c0], nb = un_b[NCELL + ka * PL + c0];
+    int s = 2;   // slot of plane kp
+    for (int kp = ka; kp < kb; ++kp) {
+        // everyone is through with the cells of plane kp - 1: plane kp - 3's slot is free
+        if (tid == 0 && !late) issue(kp + W - 3);
+        const int cell = kp * PL + c0;
+        int2* ql = lo_b + (kp - 2) * S::PLI;
+        const float4 ua = na, ub = nb;   // u^n (at stage 1 the input itself, in L2)
+        if (kp + 1 < kb) { na = un_b[cell + PL]; nb = un_b[NCELL + cell + PL]; }
+        int2 q8 = make_int2(0, 0);
+        if (final_stage) q8 = *ql;
+        const float4* a = tile + s * PL + c0;
+        int sk[5];
+#pragma unroll
+        for (int d = 0; d < 5; ++d) { const int z = s + d - 2; sk[d] = (z < 0 ? z + W : z >= W ? z - W : z) * PL + c0; }
+        float o[NV];
+        stage_cell<NIP, PL, NCELL, DIVB>(
+            tab, b, ii, jj, cell, a[0], a[W * PL], rho[kp % 4 * S::PLI], [&](int h, int m) { return a[h * W * PL + m]; },
+            [&](int h, int m) { return a[h * W * PL + m * NIP]; }, [&](int h, int m) { return tile[h * W * PL + sk[m + 2]]; },
+            [&](int m) { return make_float4(gr[m + 2].x, gr[m + 2].y, gr[m + 2].z, 0.f); }, [&](int m) { return sn[m + 2]; },
+            []() {}, ua, ub, q8, final_stage, dtk, psi, o);
+        if (final_stage) *ql = q8;
+        out_b[cell] = f4(o);
+        out_b[NCELL + cell] = f4(o + 4);
+        if (push.tgt != nullptr) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+        if (kp + 1 < kb) {
+            arrived(kp + 3);
+            prepare(kp + 3, s + 3 < W ? s + 3 : s + 3 - W);
+            s = s + 1 < W ? s + 1 : 0;
+            __syncthreads();
+        }
+    }
+    if (__syncthreads_or(late) && tid == 0) {
+        atomicOr(&sc->nan_flag, 2);
+        for (int p = issued - p0 < W ? p0 : issued - W; p < issued; ++p)   // the copies in flight
+            mbar_wait(&bars[(p - p0) % W], (uint32_t)(((p - p0) / W) & 1), kWaitPolls);
+    }
+    if (tid == 0)
+        for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
+}
+// split CTAs per block, each a run of planes
 template <int NI, int NJ, int NK, int KPAR, int DIVB>
-__global__ void __launch_bounds__(NI* NJ* KPAR, (Shape<float, NI, NJ, NK, KPAR>::min_blocks))
-k_stage_quads(const float* in, const float* un, float* out, int8_t* ulo, PushTable push, DivBArgs psi, Geometry g,
-              StepScalars* sc, int stage, int bc_writeback, int split) {
+__global__ void __launch_bounds__(NI* NJ* KPAR, (QShape<NI, NJ, NK, KPAR>::min_blocks))
+k_stage_chunks(const float* in, const float* un, float* out, int8_t* ulo, PushTable push, DivBArgs psi, Geometry g,
+               StepScalars* sc, int stage, int bc_writeback, int split) {
     const int b = blockIdx.x / split, part = blockIdx.x - b * split, n = NK / KPAR / split;
-    stage_quads<NI, NJ, NK, KPAR, DIVB>(b, part * n, (part + 1) * n, in, un, out, ulo, push, psi, g, sc, stage, bc_writeback);
+    stage_chunks<NI, NJ, NK, KPAR, DIVB>(b, part * n, (part + 1) * n, in, un, out, ulo, push, psi, g, sc, stage, bc_writeback);
+}
+template <int NI, int NJ, int NK, int DIVB>
+__global__ void __launch_bounds__(NI* NJ, 2)
+k_stage_march(const float* in, const float* un, float* out, int8_t* ulo, PushTable push, DivBArgs psi, Geometry g,
+              StepScalars* sc, int stage, int bc_writeback, int split) {
+    const int b = blockIdx.x / split, part = blockIdx.x - b * split, n = NK / split;
+    stage_march<NI, NJ, NK, DIVB>(b, 2 + part * n, 2 + (part + 1) * n, in, un, out, ulo, push, psi, g, sc, stage, bc_writeback);
 }
 
 // ---------------------------------------------------------------------------
@@ -1161,11 +1380,10 @@ struct StepBuffers {
 // regular ghost faces) and the exchange of the rest (face lists), then the
 // diffusion body into R2 (pushes, next step's CFL minimum) and the exchange
 // of the remaining entries. The bodies are the separate kernels' own
-// (KPAR 2 for the stages, two threads per column for the diffusion: 512
-// threads each, and every variant computes the same bits), so the step
-// equals the graph's bit for bit.
+// (a thread per column: 256 each; every variant computes the same bits), so the
+// step equals the graph's bit for bit.
 template <int N>
-__global__ void __launch_bounds__(512, 2)
+__global__ void __launch_bounds__(256, 2)
 k_step_persistent(StepBuffers sb, PushTable push, Geometry g, StepScalars* sc, GhostLists gl_stage,
                   GhostLists gl_final, StepDims d, GridBarrier gb) {
     static_assert(N == 16, "16^3 blocks");
@@ -1199,7 +1417,7 @@ k_step_persistent(StepBuffers sb, PushTable push, Geometry g, StepScalars* sc, G
         float* in = s == 1 ? sb.U : (s == 3 ? sb.R2 : sb.RK);
         float* out = s == 4 ? sb.U : (s == 2 ? sb.R2 : sb.RK);   // U -> RK -> R2 -> RK -> U
         for (int b = take(s - 1); b < d.nblocks; b = take(s - 1)) {
-            stage_quads<16, 16, 16, 2, 0>(b, 0, 8, in, sb.U, out, sb.ulo, push, DivBArgs{nullptr, nullptr, nullptr, 0}, g, sc, s,
+            stage_march<16, 16, 16, 0>(b, 2, 18, in, sb.U, out, sb.ulo, push, DivBArgs{nullptr, nullptr, nullptr, 0}, g, sc, s,
                                           1);
             next_body();
         }
@@ -1208,7 +1426,7 @@ k_step_persistent(StepBuffers sb, PushTable push, Geometry g, StepScalars* sc, G
         grid_sync(gb, sc, polls);
     }
     for (int b = take(4); b < d.nblocks; b = take(4)) {
-        march_quads<16, 16, 16, 2>(b, 2, 18, sb.U, sb.R2, sb.ulo, push, g, sc, 1);
+        march_quads<16, 16, 16, 1>(b, 2, 18, sb.U, sb.R2, sb.ulo, push, g, sc, 1);
         next_body();
     }
     grid_sync(gb, sc, polls);
