@@ -352,8 +352,9 @@ cudaError_t mirror_state(falcon_ctx* ctx, bool stage = false) {
 int autotune(falcon_ctx* ctx) {
     if (ctx->kpar_stage && ctx->kpar_diff) return FALCON_OK;
     int cand[8];
-    const int n = ctx->mixed() ? kpar_candidates_mixed(ctx->dims, cand) : kpar_candidates_fp64(ctx->dims, cand);
+    int n = ctx->mixed() ? kpar_candidates_mixed(ctx->dims, cand) : kpar_candidates_fp64(ctx->dims, cand);
     if (n == 0) return ctx->fail(FALCON_ERR_INVALID_ARG, "no kernel instantiation for this block size");
+    if (ctx->mixed() && ctx->dims.ni == 16) n = 1;   // one kernel each, whatever the depth
     // the candidates take turns within each round of launches, so that a drift
     // of the clocks over the tuning touches every candidate alike; the first
     // round pays for set-up and is not counted

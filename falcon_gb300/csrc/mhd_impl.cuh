@@ -115,7 +115,7 @@ __device__ __forceinline__ double half_minmod(double dl, double dr, double da) {
     if (!same || E < -132) m = 0ull;
     return with_sign_of(m, da);
 }
-// The limited flux through a face (face_flux_s below) from the cell values fl,
+// The limited flux through a face (3_6/ModDiffusion.f90:40-60) from the cell values fl,
 // fr, their difference den = fr - fl, the half slopes and the sum of the two
 // cells' speeds. phi = max(0, 1 + 2 (num/den - 1)) is 0 unless num/den > 1/2 --
 // decided by sign and magnitude, and 0/0 counts as 0 -- and 1 for num = den
@@ -142,23 +142,6 @@ __device__ __forceinline__ double face_flux_h(double fl, double fr, double den, 
         q = -fma(0.5, num / den - 1.0, 0.25);   // num/den > 1/2: not negative
     }
     return q * num * speed;
-}
-
-// FP32 minmod with the reference's selector written as a compare: the
-// reference forms t = max(0,ab)max(0,bc)*1e10 - 1e-30 and returns
-// (sign(t)/2 + 1/2) * sign(a) min(|a|,|b|,|c|), which is min(...) with a's
-// sign when t >= 0 and zero otherwise
-__device__ __forceinline__ float minmod_sel(float ul, float u, float ur) {
-    const float a = (ur - ul) * 0.5f;
-    const float b = 2.f * (ur - u);
-    const float c = 2.f * (u - ul);
-    // max(0, ab) 1e10 max(0, bc) >= 1e-30 is the same test as ab > 0 and
-    // (ab 1e10) bc >= 1e-30: with ab > 0 the first max is ab, and with bc <= 0
-    // or NaN both products are <= 0 or NaN (0 or -0 times an infinity)
-    const float ab = a * b;
-    const float x = (ab * 1.e10f) * (b * c);
-    const float m = fminf(fminf(fabsf(a), fabsf(b)), fabsf(c));
-    return ab > 0.f && x >= 1.e-30f ? copysignf(m, a) : 0.f;
 }
 
 // The per-cell CFL ratio h_LLL / v_wave of the mixed path, shared by k_cfl and
@@ -452,52 +435,6 @@ __device__ __forceinline__ void cell_of_thread(int tid, int& i, int& j, int& kq)
         j = (tid / NI) % NJ;
         kq = tid / (NI * NJ);
     }
-}
-
-// ---------------------------------------------------------------------------
-// Packed FP32 pairs (Blackwell's two-lane FFMA2/FADD2/FMUL2): the diffusion
-// march runs its slopes, fluxes and update on variables v and v+1 at once,
-// the stage its stage-4 update. Each helper gives bit for bit what its scalar counterpart gives (a
-// difference a - b is formed as fma(b, -1, a), one rounding of the exact
-// difference, as FADD does).
-__device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
-__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
-__device__ __forceinline__ float2 max02(float2 a) { return f2(fmaxf(0.f, a.x), fmaxf(0.f, a.y)); }
-// minmod_sel for two variables
-__device__ __forceinline__ float2 minmod_sel2(float2 ul, float2 u, float2 ur) {
-    const float2 a = __fmul2_rn(sub2(ur, ul), f2(0.5f));
-    const float2 b = __fmul2_rn(sub2(ur, u), f2(2.f));
-    const float2 c = __fmul2_rn(sub2(u, ul), f2(2.f));
-    const float2 ab = __fmul2_rn(a, b);   // the test of minmod_sel
-    const float2 x = __fmul2_rn(__fmul2_rn(ab, f2(1.e10f)), __fmul2_rn(b, c));
-    const float mx = fminf(fminf(fabsf(a.x), fabsf(b.x)), fabsf(c.x));
-    const float my = fminf(fminf(fabsf(a.y), fabsf(b.y)), fabsf(c.y));
-    return f2(ab.x > 0.f && x.x >= 1.e-30f ? copysignf(mx, a.x) : 0.f,
-              ab.y > 0.f && x.y >= 1.e-30f ? copysignf(my, a.y) : 0.f);
-}
-// face_flux_s<float> for two variables; cc = -0.25 (cR + cL), the face's
-// speed factor (the same for every variable; -0.25 scales exactly, so
-// (phi num) cc is the scalar form's ((-0.25 phi) num)(cR + cL) bit for bit)
-__device__ __forceinline__ float2 face_flux2(float2 fl, float2 fr, float2 dL, float2 dR, float2 cc) {
-    const float2 num = __ffma2_rn(dL, f2(-0.5f), sub2(__ffma2_rn(dR, f2(-0.5f), fr), fl));
-    const float2 den = sub2(fr, fl);
-    const float2 r = __ffma2_rn(f2(__fdividef(num.x, den.x), __fdividef(num.y, den.y)), f2(2.f), f2(-1.f));
-    return __fmul2_rn(__fmul2_rn(max02(r), num), cc);
-}
-// ff_add for two variables
-__device__ __forceinline__ float2 ff_add2(float2 hi, int8_t q0, int8_t q1, float2 d, int8_t& o0, int8_t& o1) {
-    const float2 l = __fmul2_rn(f2(lo_decode(q0), lo_decode(q1)), f2(lo_unit(hi.x), lo_unit(hi.y)));
-    const float2 s = __fadd2_rn(hi, d);
-    const float2 bs = sub2(s, hi);
-    const float2 es = __fadd2_rn(sub2(hi, sub2(s, bs)), sub2(d, bs));
-    const float2 t = __fadd2_rn(es, l);
-    const float2 h = __fadd2_rn(s, t);
-    const float2 bh = sub2(h, s);
-    const float2 r = __fadd2_rn(sub2(s, sub2(h, bh)), sub2(t, bh));
-    o0 = lo_encode(h.x, r.x);
-    o1 = lo_encode(h.y, r.y);
-    return h;
 }
 
 // ---------------------------------------------------------------------------
@@ -820,37 +757,6 @@ k_stage(const double* in, const double* un, double* out, DivBArgs psi, Geometry 
         mbar_inval(&bars[1]);
     }
 }
-// ---------------------------------------------------------------------------
-// Limited flux through the face between cells L and R along one direction
-// (3_6/ModDiffusion.f90:40-60 for one side): values at L-1, L, R, R+1 and
-// the speeds |v_dir| + c_s at L and R.
-// The limited slope of a cell from its two neighbours along one direction.
-template <class T>
-__device__ __forceinline__ T face_slope(T ul, T u, T ur) {
-    if constexpr (Pol<T>::exact) return minmod(ul, u, ur);
-    else return minmod_sel(ul, u, ur);   // the minmod selector as a compare
-}
-// The flux from the face's two cell values and their slopes.
-template <class T>
-__device__ __forceinline__ T face_flux_s(T fl, T fr, T dL, T dR, T cL, T cR) {
-    if constexpr (Pol<T>::exact) {
-        const T num = ((fr - dR * T(0.5)) - fl) - dL * T(0.5);
-        const T phi = fmax(T(0), T(1) + T(2) * (Pol<T>::ratio(num, fr - fl) - T(1)));
-        const T f = -(T(0.5) * phi * num);
-        return f * (cR + cL) * T(0.5);
-    } else {
-        // the same limiter in fewer FP32 operations: 1 + 2(r - 1) as 2r - 1,
-        // the two halves folded
-        const float num = fmaf(-0.5f, dL, fmaf(-0.5f, dR, fr) - fl);
-        const float phi = fmaxf(0.f, fmaf(2.f, __fdividef(num, fr - fl), -1.f));
-        return (-0.25f * phi) * num * (cR + cL);
-    }
-}
-template <class T>
-__device__ __forceinline__ T face_flux(T fm, T fl, T fr, T fp, T cL, T cR) {
-    return face_flux_s(fl, fr, face_slope(fm, fl, fr), face_slope(fl, fr, fp), cL, cR);
-}
-
 // ---------------------------------------------------------------------------
 // FP64 artificial diffusion (3_6/ModDiffusion.f90:9-150) of one block as a k
 // march, in place (the exact path: no pushes, no fused CFL minimum, no u^n

@@ -12,7 +12,7 @@ namespace {
 // with few blocks leaves SMs idle or unevenly loaded: the split is the power of
 // two that minimises the planes of the busiest SM, counting one more plane per
 // part for the ghost planes it rereads. 108 blocks of 16^3: diffusion 50 us whole,
-// 41 in two, 37 in four parts (the rule's). 864 blocks of 8^3: stage 36.3 us whole
+// 41 in two, 37 in four parts (the rule's; 34 now). 864 blocks of 8^3: stage 36.3 us whole
 // (the rule's), 41.4 in two.
 int split_of(const StepDims& d, int most) {
     auto cost = [&](int s) { return ((int64_t)d.nblocks * s + 151) / 152 * (d.nk / s + 1); };
@@ -61,14 +61,13 @@ cudaError_t diff_n(const StepDims& d, const Geometry& g, const float* u, float* 
     return cudaGetLastError();
 }
 // 16^3 blocks: the k march
-template <int TPC>
 cudaError_t diff_march16(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo,
                          const PushTable& push, StepScalars* sc, int cfl_next, cudaStream_t st) {
-    using S = MShape<16, 16, 16, TPC>;
-    static const cudaError_t attr = allow_smem(k_march_quads<16, 16, 16, TPC>, S::smem);
+    using S = MShape<16, 16, 16>;
+    static const cudaError_t attr = allow_smem(k_march_quads<16, 16, 16>, S::smem);
     if (attr != cudaSuccess) return attr;
     const int split = out != u ? split_of(d, 4) : 1;
-    k_march_quads<16, 16, 16, TPC><<<d.nblocks * split, S::NT, S::smem, st>>>(u, out, lo, push, g, sc, cfl_next, split);
+    k_march_quads<16, 16, 16><<<d.nblocks * split, S::NT, S::smem, st>>>(u, out, lo, push, g, sc, cfl_next, split);
     return cudaGetLastError();
 }
 }  // namespace
@@ -95,15 +94,12 @@ cudaError_t launch_psi_diffusion_mixed(const StepDims& d, const Geometry& g, con
 cudaError_t launch_psi_ghost_mixed(const StepDims& d, const GhostLists& gl, float* psi, cudaStream_t st) {
     return impl::psi_ghost_any<float>(d, gl, psi, st);
 }
-// 16^3 blocks: the k-chunk depth asked for selects one thread per column (1) or
-// two (2 and 4); 8^3 blocks: planes per chunk
+// 8^3 blocks: planes per chunk; 16^3 blocks: the march, whatever depth is asked for
 cudaError_t launch_diffusion_mixed(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo,
                                    const PushTable& push, StepScalars* sc, int kpar, cudaStream_t st, int cfl_next) {
     if (push.tgt != nullptr && out == u) return cudaErrorInvalidValue;   // pushing needs out != u
     if (d.ni != d.nj || d.ni != d.nk) return cudaErrorInvalidValue;
-    if (d.ni == 16)
-        return kpar == 1 ? impl::diff_march16<1>(d, g, u, out, lo, push, sc, cfl_next, st)
-                         : impl::diff_march16<2>(d, g, u, out, lo, push, sc, cfl_next, st);
+    if (d.ni == 16) return impl::diff_march16(d, g, u, out, lo, push, sc, cfl_next, st);
     if (d.ni != 8) return cudaErrorInvalidValue;
     switch (kpar) {
     case 2: return impl::diff_n<8, 2>(d, g, u, out, lo, push, sc, cfl_next, st);
@@ -148,7 +144,7 @@ cudaError_t launch_step_persistent_mixed(const StepDims& d, const Geometry& g, f
                                          cudaStream_t st) {
     if (d.ni != 16 || d.nj != 16 || d.nk != 16 || !bar) return cudaErrorInvalidValue;
     using SS = impl::SMarch<16, 16, 16>;
-    using SD = impl::MShape<16, 16, 16, 1>;
+    using SD = impl::MShape<16, 16, 16>;
     constexpr size_t smem = SS::smem > SD::smem ? SS::smem : SD::smem;
     // two CTAs of 256 threads per SM, as the separate stage and diffusion
     // launches run (228 KB per SM, 1 KB of it reserved per CTA, and about

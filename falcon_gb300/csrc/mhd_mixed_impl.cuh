@@ -17,6 +17,113 @@ __device__ __forceinline__ void split(float4 a, float4 b, float (&v)[NV]) {
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+// ---------------------------------------------------------------------------
+// FP32 arithmetic of the mixed step, on pairs of values where it can be (Blackwell's
+// two-lane FFMA2/FADD2/FMUL2). The scalar forms give the pairs' bits (a difference
+// a - b is formed as fma(b, -1, a), one rounding of the exact difference, as FADD does).
+__device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+
+// Half the minmod slope of a cell (3_6/ModLinReconstruct.f90:44-48, halved: the
+// fluxes use it so). With da = ur - ul, dr = ur - u, dl = u - ul the reference's
+// a = da/2, b = 2 dr, c = 2 dl and its selector max(0, ab) 1e10 max(0, bc) >= 1e-30
+// is (|da dr| 1e10) (dr dl) >= 2.5e-31: ab = da dr and bc = 4 dr dl, and of products
+// large enough to pass, ab is positive where bc is. The minimum of |a|, |b|, |c| is
+// halved likewise, all by powers of two.
+__device__ __forceinline__ float half_slope_of(float da, float dr, float dl, float qa, float t, float p) {
+    const float m = fminf(fminf(fabsf(qa), fabsf(dr)), fabsf(dl));
+    return __fmul_rn(fabsf(t), p) >= 0.25f * 1.e-30f ? copysignf(m, da) : 0.f;
+}
+__device__ __forceinline__ float half_slope(float ul, float u, float ur) {
+    const float da = __fsub_rn(ur, ul), dr = __fsub_rn(ur, u), dl = __fsub_rn(u, ul);
+    return half_slope_of(da, dr, dl, __fmul_rn(da, 0.25f), __fmul_rn(__fmul_rn(da, dr), 1.e10f), __fmul_rn(dr, dl));
+}
+__device__ __forceinline__ float2 half_slope2(float2 ul, float2 u, float2 ur) {
+    const float2 da = sub2(ur, ul), dr = sub2(ur, u), dl = sub2(u, ul);
+    const float2 qa = __fmul2_rn(da, f2(0.25f)), t = __fmul2_rn(__fmul2_rn(da, dr), f2(1.e10f)), p = __fmul2_rn(dr, dl);
+    return f2(half_slope_of(da.x, dr.x, dl.x, qa.x, t.x, p.x), half_slope_of(da.y, dr.y, dl.y, qa.y, t.y, p.y));
+}
+
+// The limited flux through a face (3_6/ModDiffusion.f90:40-60) from its two cells'
+// values and half slopes: -(phi/2 num) speed/2 with phi = max(0, 1 + 2 (num/den - 1)),
+// den = fr - fl, num the jump left between the reconstructions; cc = -2 speed, speed
+// the sum of the cells' |v_dir| + c_s. The slopes limit num/den to [-1, 3], so phi/8
+// saturates to [0, 1] without clipping phi from above; one saturating FMA forms it,
+// 0/0 as 0. The quotient is num times the approximate reciprocal of den, which flushes
+// a denormal den: there the saturated phi keeps the flux as small as num.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float eighth_phi(float r) { return __saturatef(__fmaf_rn(r, 0.25f, -0.125f)); }
+__device__ __forceinline__ float face_flux(float fl, float fr, float hL, float hR, float cc) {
+    const float num = __fsub_rn(__fsub_rn(__fsub_rn(fr, hR), fl), hL);
+    return __fmul_rn(__fmul_rn(eighth_phi(__fmul_rn(num, rcp_approx(__fsub_rn(fr, fl)))), num), cc);
+}
+__device__ __forceinline__ float2 face_flux2(float2 fl, float2 fr, float2 hL, float2 hR, float2 cc) {
+    const float2 num = sub2(sub2(sub2(fr, hR), fl), hL), den = sub2(fr, fl);
+    const float2 r = __fmul2_rn(num, f2(rcp_approx(den.x), rcp_approx(den.y)));
+    return __fmul2_rn(__fmul2_rn(f2(eighth_phi(r.x), eighth_phi(r.y)), num), cc);
+}
+// cc of a face: uL, uR the velocity across it, csL, csR the sound speeds of its cells
+__device__ __forceinline__ float face_speed(float uL, float csL, float uR, float csR) {
+    return -2.f * ((fabsf(uR) + csR) + (fabsf(uL) + csL));
+}
+
+// (hi + q*unit(hi)) + d for four values, rounded to the nearest (hi', q') pairs: two
+// error-free FP32 sums (Knuth's TwoSum), no contraction. q: four corrections in a
+// word, renewed. A correction q is q + 128 in the low bits of 2^23's float; the
+// rounding to the nearest integer, ties to even, is the add of 1.5 * 2^23, whose ulp
+// is 1 and whose low byte is then q (the clamp comes first, NaN residuals give -127).
+__device__ __forceinline__ float2 ff_add2(float2 hi, float2 q, float2 d, float2& lo) {
+    auto unit = [](float x) { return __int_as_float(max((__float_as_int(x) & 0x7f800000) - (31 << 23), 0)); };   // lo_unit
+    auto inv_unit = [](float x) {   // lo_inv_unit
+        const unsigned t = (unsigned)__float_as_int(x) & 0x7f800000u;
+        return __int_as_float((int)(t >= (32u << 23) ? (285u << 23) - t : 0u));
+    };
+    const float2 l = __fmul2_rn(__fadd2_rn(q, f2(-8388736.f)), f2(unit(hi.x), unit(hi.y)));   // exact
+    const float2 s = __fadd2_rn(hi, d);
+    const float2 bs = sub2(s, hi);
+    const float2 es = __fadd2_rn(sub2(hi, sub2(s, bs)), sub2(d, bs));
+    const float2 t = __fadd2_rn(es, l);
+    const float2 h = __fadd2_rn(s, t);
+    const float2 bh = sub2(h, s);
+    const float2 r = __fmul2_rn(__fadd2_rn(sub2(s, sub2(h, bh)), sub2(t, bh)), f2(inv_unit(h.x), inv_unit(h.y)));
+    lo = __fadd2_rn(f2(fminf(fmaxf(r.x, -127.f), 127.f), fminf(fmaxf(r.y, -127.f), 127.f)), f2(12582912.f));
+    return h;
+}
+__device__ __forceinline__ void ff_add4(const float* hi, int& q, const float2 (&d)[2], float* o) {
+    const unsigned w = (unsigned)q ^ 0x80808080u;
+    auto byte = [&](int k) { return __int_as_float((int)__byte_perm(w, 0x4B000000u, 0x7440 + k)); };
+    float2 la, lb;
+    const float2 a = ff_add2(f2(hi[0], hi[1]), f2(byte(0), byte(1)), d[0], la);
+    const float2 b = ff_add2(f2(hi[2], hi[3]), f2(byte(2), byte(3)), d[1], lb);
+    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+    auto bits = [](float x) { return (unsigned)__float_as_int(x); };
+    q = (int)__byte_perm(__byte_perm(bits(la.x), bits(la.y), 0x40), __byte_perm(bits(lb.x), bits(lb.y), 0x40), 0x5410);
+}
+
+// v_wave of the CFL ratio (cfl_ratio_f's) at a cell of a column with c_s = cs and
+// sqrt(rho0) = d, y = RN(1/d): the quotient sqrt(b2)/d through the reciprocal (P.
+// Markstein, IBM J. R&D 34 (1990) 111; the first correction brings q within an ulp).
+// RN(h / w) falls as w grows and h is the column's, so its minimum over a column is
+// h / max(w): one division a column.
+__device__ __forceinline__ float cfl_speed(float v2, float b2, float cs, float d, float y) {
+    const float a = __fsqrt_rn(b2);
+    float q = __fmul_rn(a, y);
+    if (q < INFINITY) {
+        q = __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
+        q = __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
+    }
+    return __fadd_rn(__fadd_rn(cs, __fsqrt_rn(v2)), q);
+}
+// The column's minimum ratio, from its largest speed
+__device__ __forceinline__ float cfl_column(float wmax, float r, float sin_t, float dxi, float dxj, float dxk) {
+    return __fdiv_rn(fminf(fminf(dxi, __fmul_rn(r, dxj)), __fmul_rn(__fmul_rn(r, sin_t), dxk)), wmax);
+}
+
 // Thread 0: bulk-copy planes kp in [lo, hi) of both halves of the block into
 // their ring slots (plane kp in slot (kp - p0) % W), completing on `bar`.
 template <class S>
@@ -58,7 +165,7 @@ __device__ __forceinline__ void apply_bc_quads(float4* tile, int lo, int hi, int
 }
 
 // Write this cell's new values into the ghost cells of the neighbours whose
-// faces are pushed (PushTable): halves [H0, H0 + NH) of the cell, o its values.
+// faces are pushed (PushTable), o its values.
 // (ii, jj, kp): padded indices. Theta/phi faces: the two interior layers next to
 // the side are copied to the target's opposite ghost layers (a shift of one
 // block extent). Radial faces: the thread at the first source cell of a ghost
@@ -66,14 +173,14 @@ __device__ __forceinline__ void apply_bc_quads(float4* tile, int lo, int hi, int
 // the fastest thread index, and the second cell is never beyond the row). Every
 // write is whole 16-byte cells, the two layers of a radial face one sector.
 // Every thread of the warp calls this (the shuffle needs it).
-template <class S, int NH, int H0>
-__device__ __forceinline__ void push_quads(float* out, const PushBlock& P, int ii, int jj, int kp, const float (&o)[4 * NH]) {
+template <class S>
+__device__ __forceinline__ void push_quads(float* out, const PushBlock& P, int ii, int jj, int kp, const float (&o)[NV]) {
     constexpr int NJ = S::NJP - 4, NK = S::NKP - 4;
     const int32_t* tg = P.tgt;
-    auto put = [&](int tb, int kt, int jt, int it, const float (&val)[4 * NH]) {
-        float4* dst = quads(out) + quad(tb, H0, S::NCELL) + ((size_t)kt * S::NJP + jt) * S::NIP + it;
-#pragma unroll
-        for (int h = 0; h < NH; ++h) dst[(size_t)h * S::NCELL] = f4(val + 4 * h);
+    auto put = [&](int tb, int kt, int jt, int it, const float (&val)[NV]) {
+        float4* dst = quads(out) + quad(tb, 0, S::NCELL) + ((size_t)kt * S::NJP + jt) * S::NIP + it;
+        dst[0] = f4(val);
+        dst[S::NCELL] = f4(val + 4);
     };
     if (jj <= 3 && tg[2] >= 0) put(tg[2], kp, jj + NJ, ii, o);
     if (jj >= NJ && tg[3] >= 0) put(tg[3], kp, jj - NJ, ii, o);
@@ -89,16 +196,16 @@ __device__ __forceinline__ void push_quads(float* out, const PushBlock& P, int i
             if (l1) put(tg[side], kp, jj, P.dst[2 * side + 1], o);
             continue;
         }
-        float nx[4 * NH];
+        float nx[NV];
 #pragma unroll
-        for (int v = 0; v < 4 * NH; ++v) nx[v] = __shfl_down_sync(0xffffffffu, o[v], 1);
+        for (int v = 0; v < NV; ++v) nx[v] = __shfl_down_sync(0xffffffffu, o[v], 1);
 #pragma unroll
         for (int layer = 0; layer < 2; ++layer) {
             if (!(layer ? l1 : l0)) continue;
             const float w = layer ? w1 : w0, uw = 1.f - w;
-            float val[4 * NH];
+            float val[NV];
 #pragma unroll
-            for (int v = 0; v < 4 * NH; ++v) val[v] = w == 0.f ? o[v] : blend(o[v], nx[v], uw, w);
+            for (int v = 0; v < NV; ++v) val[v] = w == 0.f ? o[v] : blend(o[v], nx[v], uw, w);
             put(tg[side], kp, jj, P.dst[2 * side + layer], val);
         }
     }
@@ -376,18 +483,9 @@ __device__ __forceinline__ void stage_cell(const StageTables& tab, int b, int ii
     split(ua, ub, u0s);
     if (final_stage) {
         // u^{n+1} = u^n + dt*R with u^n and u^{n+1} compensated
-        int qn[2] = {0, 0};
-#pragma unroll
-        for (int v = 0; v < NV; v += 2) {   // pairs of variables: ff_add2 gives ff_add's bits
-            const int q = v < 4 ? q8.x : q8.y, sh = 8 * (v & 3);
-            int8_t qa, qb;
-            const float2 ov = ff_add2(f2(u0s[v], u0s[v + 1]), (int8_t)(q >> sh), (int8_t)(q >> (sh + 8)),
-                                      __fmul2_rn(f2(dtk), f2(R[v], R[v + 1])), qa, qb);
-            o[v] = ov.x;
-            o[v + 1] = ov.y;
-            qn[v >> 2] |= ((int)(uint8_t)qa | (int)(uint8_t)qb << 8) << sh;
-        }
-        q8 = make_int2(qn[0], qn[1]);
+        auto dt2 = [&](int v) { return __fmul2_rn(f2(dtk), f2(R[v], R[v + 1])); };
+        ff_add4(u0s, q8.x, {dt2(0), dt2(2)}, o);
+        ff_add4(u0s + 4, q8.y, {dt2(4), dt2(6)}, o + 4);
     } else {
 #pragma unroll
         for (int v = 0; v < NV; ++v) o[v] = fmaf(dtk, R[v], u0s[v]);
@@ -509,7 +607,7 @@ __device__ __forceinline__ void stage_chunks(int b, int ch0, int ch1, const floa
         if (final_stage) *ql = q8;
         quads(out)[quad(b, 0, NCELL) + cell] = f4(o);
         quads(out)[quad(b, 1, NCELL) + cell] = f4(o + 4);
-        if (push.tgt != nullptr) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+        if (push.tgt != nullptr) push_quads<S>(out, pb, ii, jj, kp, o);
         if (n + 1 < nch) {
             late |= mbar_wait(&bars[(n + 1) & 1], (uint32_t)(((n + 1) >> 1) & 1), polls) ? 0 : 1;
             prepare(next, KPAR);
@@ -530,7 +628,7 @@ __device__ __forceinline__ void stage_chunks(int b, int ch0, int ch1, const floa
 // 16 warps per SM, the issue (56%). A register window along k spares 8 of the 26
 // reads and costs as much in moves (763 us), unrolled by five to avoid those it
 // loses to the instruction cache (823); chunks of two planes with 64 registers a
-// thread spill (1,006). 21.2M cells: 877 -> 708 us per stage.
+// thread spill (1,006). 21.2M cells: 877 -> 685 us per stage.
 template <int NI, int NJ, int NK>
 struct SMarch {
     static constexpr int NIP = NI + 4, NJP = NJ + 4, NKP = NK + 4, PL = NIP * NJP, NCELL = PL * NKP, PLI = NI * NJ, NINT = PLI * NK;
@@ -636,7 +734,7 @@ __device__ __forceinline__ void stage_march(int b, int ka, int kb, const float* 
         if (final_stage) *ql = q8;
         out_b[cell] = f4(o);
         out_b[NCELL + cell] = f4(o + 4);
-        if (push.tgt != nullptr) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+        if (push.tgt != nullptr) push_quads<S>(out, pb, ii, jj, kp, o);
         if (kp + 1 < kb) {
             arrived(kp + 3);
             prepare(kp + 3, s + 3 < W ? s + 3 : s + 3 - W);
@@ -761,8 +859,9 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
     const float den[3] = {gs[GS_DXI], gs[GS_DXJ] * rc, gs[GS_DXK] * rc * gj[GJ_SIN * S::NJP + jj]};
     const float dinv[3] = {1.f / den[0], 1.f / den[1], 1.f / den[2]};
     const float hdt_f = sc->dt_half_f;
-    float cmin = INFINITY;   // next step's CFL ratio minimum over this thread's cells
+    float wmax = 0.f;   // the largest wave speed of this thread's cells, for the next step's CFL minimum
     int cnan = 0;
+    const float srho = __fsqrt_rn(gi[GI_RHO0 * NIP + ii]), srho_inv = __frcp_rn(srho);
     constexpr int nchunk = NK / KPAR;
     const int polls = sc->wait_polls;
     int late = 0;   // a wait of this thread for a chunk's planes ran out
@@ -801,37 +900,32 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
         // this cell's left i and j faces and right k face
         {
             const float4* tA = tile + c0;
-            const float cLi = fabsf(tA[so[1] - 1].y) + GCS[ii - 1], cRi = fabsf(ca.y) + cs;
-            const float cLj = fabsf(tA[so[1] - NIP].z) + cs, cRj = fabsf(ca.z) + cs;
-            const float cLk = fabsf(ca.w) + cs, cRk = fabsf(tA[so[2]].w) + cs;
+            const float cci = face_speed(tA[so[1] - 1].y, GCS[ii - 1], ca.y, cs);
+            const float ccj = face_speed(tA[so[1] - NIP].z, cs, ca.z, cs);
+            const float cck = face_speed(ca.w, cs, tA[so[2]].w, cs);
             float* fkw = FK + (size_t)((kp - 1) % KS) * NV * NJ * NI + j * NI + i;
+            auto lo2 = [](const float4& x) { return f2(x.x, x.y); };
+            auto hi2 = [](const float4& x) { return f2(x.z, x.w); };
+            // the fluxes of a half's four values through a face: arrays pitch apart
+            auto face4 = [&](const float4& fm, const float4& fl, const float4& fr, const float4& fp, float cc, float* to, int pitch) {
+                const float2 a = face_flux2(lo2(fl), lo2(fr), half_slope2(lo2(fm), lo2(fl), lo2(fr)), half_slope2(lo2(fl), lo2(fr), lo2(fp)), f2(cc));
+                const float2 b = face_flux2(hi2(fl), hi2(fr), half_slope2(hi2(fm), hi2(fl), hi2(fr)), half_slope2(hi2(fl), hi2(fr), hi2(fp)), f2(cc));
+                to[0] = a.x; to[pitch] = a.y; to[2 * pitch] = b.x; to[3 * pitch] = b.y;
+            };
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float4* t = tile + h * W * PL + c0;
-                auto comp = [](const float4& x, int q) { return q == 0 ? x.x : q == 1 ? x.y : q == 2 ? x.z : x.w; };
                 const float4 z = t[so[1]];
-                {
-                    const float4 x2 = t[so[1] - 2], x1 = t[so[1] - 1], y1 = t[so[1] + 1];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        FI[(((4 * h + q) * KPAR + kq) * NJ + j) * S::FIP + i] =
-                            face_flux(comp(x2, q), comp(x1, q), comp(z, q), comp(y1, q), cLi, cRi);
-                }
-                {
-                    const float4 x2 = t[so[1] - 2 * NIP], x1 = t[so[1] - NIP], y1 = t[so[1] + NIP];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        FJ[(((4 * h + q) * KPAR + kq) * (NJ + 1) + j) * NI + i] =
-                            face_flux(comp(x2, q), comp(x1, q), comp(z, q), comp(y1, q), cLj, cRj);
-                }
-                {
-                    const float4 x1 = t[so[0]], y1 = t[so[2]], y2 = t[so[3]];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        fkw[(4 * h + q) * NJ * NI] = face_flux(comp(x1, q), comp(z, q), comp(y1, q), comp(y2, q), cLk, cRk);
-                }
+                face4(t[so[1] - 2], t[so[1] - 1], z, t[so[1] + 1], cci, FI + ((4 * h * KPAR + kq) * NJ + j) * S::FIP + i, KPAR * NJ * S::FIP);
+                face4(t[so[1] - 2 * NIP], t[so[1] - NIP], z, t[so[1] + NIP], ccj, FJ + ((4 * h * KPAR + kq) * (NJ + 1) + j) * NI + i,
+                      KPAR * (NJ + 1) * NI);
+                face4(t[so[0]], z, t[so[2]], t[so[3]], cck, fkw + 4 * h * NJ * NI, NJ * NI);
             }
         }
+        // one value's flux from the four around the face
+        auto face1 = [&](float fm, float fl, float fr, float fp, float cc) {
+            return face_flux(fl, fr, half_slope(fm, fl, fr), half_slope(fl, fr, fp), cc);
+        };
         // the right faces of the last cells of i rows and j columns
         constexpr int NXI = NV * KPAR * NJ, NXJ = NV * KPAR * NI;
         for (int x = tid; x < NXI + NXJ; x += S::NT) {
@@ -840,8 +934,8 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
             const int r = y % n + 2, q = (y / n) % KPAR, v = y / (n * KPAR), slot = (kp0 + q) % W;
             const int c = on_i ? r * NIP + NI + 1 : (NJ + 1) * NIP + r, st = on_i ? 1 : NIP;   // last interior cell
             const int vd = on_i ? V_VR : V_VT;
-            const float cL = fabsf(val(vd, slot, c)) + GCS[on_i ? NI + 1 : r], cR = fabsf(val(vd, slot, c + st)) + GCS[on_i ? NI + 2 : r];
-            const float f = face_flux(val(v, slot, c - st), val(v, slot, c), val(v, slot, c + st), val(v, slot, c + 2 * st), cL, cR);
+            const float cc = face_speed(val(vd, slot, c), GCS[on_i ? NI + 1 : r], val(vd, slot, c + st), GCS[on_i ? NI + 2 : r]);
+            const float f = face1(val(v, slot, c - st), val(v, slot, c), val(v, slot, c + st), val(v, slot, c + 2 * st), cc);
             if (on_i) FI[((v * KPAR + q) * NJ + (r - 2)) * S::FIP + NI] = f;
             else FJ[((v * KPAR + q) * (NJ + 1) + NJ) * NI + (r - 2)] = f;
         }
@@ -849,52 +943,47 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
         if (ch == 0) {
             for (int x = tid; x < NV * NJ * NI; x += S::NT) {
                 const int xx = x % NI + 2, y = (x / NI) % NJ + 2, v = x / (NI * NJ), c = y * NIP + xx;
-                const float cL = fabsf(val(V_VP, 1, c)) + GCS[xx], cR = fabsf(val(V_VP, 2, c)) + GCS[xx];
-                FK[(v * NJ + (y - 2)) * NI + (xx - 2)] = face_flux(val(v, 0, c), val(v, 1, c), val(v, 2, c), val(v, 3, c), cL, cR);
+                const float cc = face_speed(val(V_VP, 1, c), GCS[xx], val(V_VP, 2, c), GCS[xx]);
+                FK[(v * NJ + (y - 2)) * NI + (xx - 2)] = face1(val(v, 0, c), val(v, 1, c), val(v, 2, c), val(v, 3, c), cc);
             }
         }
         __syncthreads();
         const size_t cell = (size_t)kp * PL + c0;
         const float* fk_l = FK + (size_t)((kp - 2) % KS) * NV * NJ * NI + j * NI + i;
         const float* fk_r = FK + (size_t)((kp - 1) % KS) * NV * NJ * NI + j * NI + i;
-        float o[NV], u0[NV];
+        float o[NV], u0[NV], R[NV];
         split(ca, cb, u0);
-        int qn[2] = {0, 0};
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             const float* fi = FI + ((v * KPAR + kq) * NJ + j) * S::FIP + i;
             const float* fj = FJ + ((v * KPAR + kq) * (NJ + 1) + j) * NI + i;
-            float R = 0.f;
-            R = R + (fi[0] - fi[1]) * dinv[0];
-            R = R + (fj[0] - fj[NI]) * dinv[1];
-            R = R + (fk_l[v * NJ * NI] - fk_r[v * NJ * NI]) * dinv[2];
-            if (ulo != nullptr) {
-                const int sh = 8 * (v & 3);
-                int8_t q1;
-                o[v] = ff_add(u0[v], (int8_t)((v < 4 ? q8.x : q8.y) >> sh), __fmul_rn(hdt_f, R), q1);
-                qn[v >> 2] |= (int)(uint8_t)q1 << sh;
-            } else {
-                o[v] = fmaf(hdt_f, R, u0[v]);
-            }
+            R[v] = __fmul_rn(fi[0] - fi[1], dinv[0]);
+            R[v] = __fmaf_rn(fj[0] - fj[NI], dinv[1], R[v]);
+            R[v] = __fmaf_rn(fk_l[v * NJ * NI] - fk_r[v * NJ * NI], dinv[2], R[v]);
         }
-        if (ulo != nullptr) *ql = make_int2(qn[0], qn[1]);
+        if (ulo != nullptr) {
+            auto dt2 = [&](int v) { return __fmul2_rn(f2(hdt_f), f2(R[v], R[v + 1])); };
+            ff_add4(u0, q8.x, {dt2(0), dt2(2)}, o);
+            ff_add4(u0 + 4, q8.y, {dt2(4), dt2(6)}, o + 4);
+            *ql = q8;
+        } else {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) o[v] = __fmaf_rn(hdt_f, R[v], u0[v]);
+        }
         quads(out)[quad(b, 0, NCELL) + cell] = f4(o);
         quads(out)[quad(b, 1, NCELL) + cell] = f4(o + 4);
-        if (push.tgt != nullptr) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
+        if (push.tgt != nullptr) push_quads<S>(out, pb, ii, jj, kp, o);
         if (cfl_next) {   // uniform over the CTA
 #pragma unroll
             for (int v = 0; v < NV; ++v) cnan |= (o[v] != o[v]);
-            float ratio = cfl_ratio_f(cfl_sq3(o[V_VR], o[V_VT], o[V_VP]), cfl_sq3(o[V_BR], o[V_BT], o[V_BP]), cs,
-                                      gi[GI_RHO0 * NIP + ii], rc, gj[GJ_SIN * S::NJP + jj], gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]);
-            if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
-            cmin = fminf(cmin, ratio);
+            wmax = fmaxf(wmax, cfl_speed(cfl_sq3(o[V_VR], o[V_VT], o[V_VP]), cfl_sq3(o[V_BR], o[V_BT], o[V_BP]), cs, srho, srho_inv));
         }
     }
     if (__syncthreads_or(late)) {
         copy_wait_abort(sc, bars, nchunk - 1, nchunk - 1);
         return;
     }
-    if (cfl_next) cfl_commit(cmin, cnan, sc);
+    if (cfl_next) cfl_commit(cfl_column(wmax, rc, gj[GJ_SIN * S::NJP + jj], gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]), cnan, sc);
 }
 
 // ---------------------------------------------------------------------------
@@ -910,7 +999,7 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
 // columns and rows by the same threads), then every i and j face flux once
 // (phase B), then each cell sums its six faces and updates (phase C). Per
 // cell and variable that is 3 slopes and 3 fluxes, the minimum; the face
-// fluxes are the same functions of the same values as k_diffusion's, summed
+// fluxes are the same functions of the same values as k_diffusion_quads', summed
 // in the same order. The arithmetic runs on pairs of variables (packed FP32
 // instructions, above), and the slope and face arrays hold the pairs side by
 // side, so their shared-memory accesses are 64-bit; a cell's values come from
@@ -921,16 +1010,20 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
 // with plane kp+5 once phase B of plane kp has passed its barrier (planes
 // kp+3 and kp+4 are in flight meanwhile). A warp takes rows j and j+4
 // (half-warps of 16 cells), so a half-warp holds one row, as the pushed
-// radial faces need. 21.2M cells: 1,229 -> 1,135 us; 442k cells with split
-// blocks: 60 -> 37 us.
-template <int NI, int NJ, int NK, int TPC>
+// radial faces need.
+//
+// What bounds it is the issue (16 warps per SM, 128 registers a thread): 1,124 warp
+// instructions per 32 cells, issued in 58% of the cycles. 21.2M cells: 1,229 ->
+// 1,022 us; 442k cells with split blocks: 60 -> 34 us. Two threads per column with
+// 64 registers each: 1,367 us (of 1,135 then).
+template <int NI, int NJ, int NK>
 struct MShape {
     static constexpr int NG = 2, NIP = NI + 4, NJP = NJ + 4, NKP = NK + 4;
     static constexpr int PL = NIP * NJP, NCELL = PL * NKP;
-    static constexpr int NCOL = NI * NJ, NT = NCOL * TPC;   // columns; threads (TPC per column)
+    static constexpr int NT = NI * NJ;
     static constexpr int W = 5;                          // plane ring slots
     static constexpr int PLI = NI * NJ, NINT = PLI * NK;
-    static constexpr int NP = NV / 2, PPT = NP / TPC;    // variable pairs; pairs per thread
+    static constexpr int NP = NV / 2;                    // variable pairs
     static constexpr uint32_t PLB = PL * 4u;
     static constexpr int P = 20;                         // row pitch (pairs) of the slope and face arrays
     // per pair (float2): SI[NJ][P] slopes along i of cells i = -1..NI at i + 1;
@@ -946,25 +1039,18 @@ struct MShape {
     static constexpr size_t off_gi = off_fj + (size_t)NP * NFJ * 8;
     static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * NIP * 4;
     static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * NJP * 4;
-    // two threads per column: |B|^2 of the second half, [plane parity][column]
-    static constexpr size_t off_sb2 = off_gs + GS_COUNT * 4;
-    static constexpr size_t smem = off_sb2 + (TPC == 2 ? 2 * NCOL * 4 : 0);
+    static constexpr size_t smem = off_gs + GS_COUNT * 4;
     static_assert(W * 8 <= (int)off_tile, "mbarriers");
     static_assert(off_si % 8 == 0, "float2 arrays");
-    static_assert(TPC == 1 || TPC == 2, "one or two threads per column");
 };
 
-// TPC threads per column: with two, thread half h = tid / 256 takes the
-// variable pairs 2h, 2h+1 (warps never mix halves), doubling the warps per SM
-// at half the registers; the CFL ratio, which needs v (first half) and B
-// (second half), takes |B|^2 through shared memory one plane later.
-template <int NI, int NJ, int NK, int TPC>
+template <int NI, int NJ, int NK>
 __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* u, float* out, int8_t* ulo,
                                             const PushTable& push, const Geometry& g, StepScalars* sc, int cfl_next) {
-    using S = MShape<NI, NJ, NK, TPC>;
+    using S = MShape<NI, NJ, NK>;
     static_assert(NI == 16 && NJ == 16, "rows of 16 cells: one half-warp per row");
     static_assert(2 * (S::smem + 1024) <= 233472, "two CTAs per SM");
-    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, P = S::P, PPT = S::PPT;
+    constexpr int NIP = S::NIP, PL = S::PL, W = S::W, NCELL = S::NCELL, P = S::P, NP = S::NP;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     float4* tile = reinterpret_cast<float4*>(smem + S::off_tile);   // [2][W][PL]
@@ -975,7 +1061,6 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
     float* gi = reinterpret_cast<float*>(smem + S::off_gi);
     float* gj = reinterpret_cast<float*>(smem + S::off_gj);
     float* gs = reinterpret_cast<float*>(smem + S::off_gs);
-    float* sb2 = reinterpret_cast<float*>(smem + S::off_sb2);   // |B|^2 of the second half, by plane parity
     const int tid = threadIdx.x;
     const float* blk = u + (size_t)b * NV * NCELL;
     const int flb = g.flags[b];
@@ -1000,11 +1085,9 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
     if (blk_lo != nullptr && tid == 0) prefetch_l2(blk_lo + (size_t)(ka - 2) * S::PLI * NV, 2 * S::PLI * NV);
     load_geometry<float, S>(g, b, gi, gj, gs, nullptr);
     __syncthreads();   // the geometry tables are read by every thread below
-    // this thread's column: warp w takes rows (w % 4) + 8 (w / 4) and that + 4;
-    // its pairs p0 .. p0 + PPT - 1
-    const int c = tid % S::NCOL, half = tid / S::NCOL, p0 = half * PPT, v0 = 2 * p0;
-    const int wq = c >> 5, i = c & 15;
-    const int j = (wq & 3) + 8 * (wq >> 2) + 4 * ((c >> 4) & 1);
+    // this thread's column: warp w takes rows (w % 4) + 8 (w / 4) and that + 4
+    const int wq = tid >> 5, i = tid & 15;
+    const int j = (wq & 3) + 8 * (wq >> 2) + 4 * ((tid >> 4) & 1);
     const int ii = i + 2, jj = j + 2;
     const float* GCS = gi + GI_CS * NIP;
     const float cs = GCS[ii];
@@ -1021,19 +1104,15 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
             mbar_wait(&bars[p % W], (uint32_t)((p / W) & 1), kWaitPolls);
         for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
     };
-    // this thread's halves of a cell in a plane's slot
-    constexpr int NH = PPT / 2;
-    const float4* mine = tile + (size_t)(p0 / 2) * W * PL;
-    auto quad_of = [&](int slot, int c, int h) { return mine[(size_t)h * W * PL + slot + c]; };
     auto lo2 = [](const float4& x) { return f2(x.x, x.y); };
     auto hi2 = [](const float4& x) { return f2(x.z, x.w); };
     const int c0 = jj * NIP + ii;
     auto slot_of = [&](int p) { return (p - pa) % W * PL; };
-    // pairs of one quad into two of an array
-    auto pairs = [&](int slot, int c, float2 (&v)[PPT]) {
+    // the pairs of a cell in a plane's slot
+    auto pairs = [&](int slot, int c, float2 (&v)[NP]) {
 #pragma unroll
-        for (int h = 0; h < NH; ++h) {
-            const float4 x = quad_of(slot, c, h);
+        for (int h = 0; h < 2; ++h) {
+            const float4 x = tile[h * W * PL + slot + c];
             v[2 * h] = lo2(x);
             v[2 * h + 1] = hi2(x);
         }
@@ -1042,41 +1121,32 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
     // slope at ka, the flux through the face between planes ka-1 and ka
     for (int p = 0; p < 4; ++p) late |= mbar_wait(&bars[p], 0u, polls) ? 0 : 1;
     if (copy_bc) copy_bc_columns<S>(tile, pa, out, b, flb, pa, pa + 4, S::NT);
-    float2 u0[PPT], u1[PPT], dk0[PPT], fk0[PPT];
+    float2 u0[NP], u1[NP], dk0[NP], fk0[NP];
     {
-        const float2 cc = f2(-0.25f * ((fabsf(tile[2 * PL + c0].w) + cs) + (fabsf(tile[PL + c0].w) + cs)));
-        float2 a0[PPT], a1[PPT];
+        const float2 cc = f2(face_speed(tile[PL + c0].w, cs, tile[2 * PL + c0].w, cs));
+        float2 a0[NP], a1[NP];
         pairs(0, c0, a0);
         pairs(PL, c0, a1);
         pairs(2 * PL, c0, u0);
         pairs(3 * PL, c0, u1);
 #pragma unroll
-        for (int q = 0; q < PPT; ++q) {
-            const float2 d1 = minmod_sel2(a0[q], a1[q], u0[q]);
-            dk0[q] = minmod_sel2(a1[q], u0[q], u1[q]);
+        for (int q = 0; q < NP; ++q) {
+            const float2 d1 = half_slope2(a0[q], a1[q], u0[q]);
+            dk0[q] = half_slope2(a1[q], u0[q], u1[q]);
             fk0[q] = face_flux2(a1[q], u0[q], d1, dk0[q], cc);
         }
     }
-    float cmin = INFINITY;   // next step's CFL ratio minimum over this column
+    float wmax = 0.f;   // the column's largest wave speed, for the next step's CFL minimum
     int cnan = 0;
-    float v2_prev = 0.f;     // two threads per column: the first half's |v|^2 of the previous plane
-    const float rho0c = gi[GI_RHO0 * NIP + ii], sin_c = gj[GJ_SIN * S::NJP + jj];
-    auto cfl_point = [&](float v2, float b2) {
-        float ratio = cfl_ratio_f(v2, b2, cs, rho0c, rc, sin_c, gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]);
-        if (ratio != ratio) { cnan = 1; ratio = INFINITY; }
-        cmin = fminf(cmin, ratio);
-    };
+    const float srho = __fsqrt_rn(gi[GI_RHO0 * NIP + ii]), srho_inv = __frcp_rn(srho);
     for (int kp = ka; kp < kb; ++kp) {
         const int p2 = kp + 2;
         if (blk_lo != nullptr && tid == 0 && kp + 2 < kb)
             prefetch_l2(blk_lo + (size_t)kp * S::PLI * NV, S::PLI * NV);
         // this cell's int8 corrections, loaded before the wait
-        int qlo[NH];
-        int* qp = reinterpret_cast<int*>(blk_lo + (((size_t)(kp - 2) * NJ + j) * NI + i) * NV + v0);
-        if (blk_lo != nullptr) {
-#pragma unroll
-            for (int h = 0; h < NH; ++h) qlo[h] = qp[h];
-        }
+        int2 q8 = make_int2(0, 0);
+        int2* ql = reinterpret_cast<int2*>(blk_lo + (((size_t)(kp - 2) * NJ + j) * NI + i) * NV);
+        if (blk_lo != nullptr) q8 = *ql;
         // a wait that runs out finishes the plane on whatever the slot holds;
         // the step is flagged and discarded
         late |= mbar_wait(&bars[(p2 - pa) % W], (uint32_t)(((p2 - pa) / W) & 1), polls) ? 0 : 1;
@@ -1085,24 +1155,24 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
         // the half with the velocities at this cell
         const float4 vc = tile[s0 + c0], vl = tile[s0 + c0 - 1], vd = tile[s0 + c0 - NIP];
         // ---- phase A: k slope and k face from the window; i and j slopes
-        float2 u2[PPT], dk1[PPT], fk1[PPT];
+        float2 u2[NP], dk1[NP], fk1[NP];
         {
-            const float2 cc = f2(-0.25f * ((fabsf(tile[s1 + c0].w) + cs) + (fabsf(vc.w) + cs)));
+            const float2 cc = f2(face_speed(vc.w, cs, tile[s1 + c0].w, cs));
             pairs(s2, c0, u2);
 #pragma unroll
-            for (int q = 0; q < PPT; ++q) {
-                dk1[q] = minmod_sel2(u0[q], u1[q], u2[q]);
+            for (int q = 0; q < NP; ++q) {
+                dk1[q] = half_slope2(u0[q], u1[q], u2[q]);
                 fk1[q] = face_flux2(u0[q], u1[q], dk0[q], dk1[q], cc);
             }
-            float2 l[PPT], r[PPT];
+            float2 l[NP], r[NP];
             pairs(s0, c0 - 1, l);
             pairs(s0, c0 + 1, r);
 #pragma unroll
-            for (int q = 0; q < PPT; ++q) SI[(p0 + q) * S::NSI + j * P + i + 1] = minmod_sel2(l[q], u0[q], r[q]);
+            for (int q = 0; q < NP; ++q) SI[q * S::NSI + j * P + i + 1] = half_slope2(l[q], u0[q], r[q]);
             pairs(s0, c0 - NIP, l);
             pairs(s0, c0 + NIP, r);
 #pragma unroll
-            for (int q = 0; q < PPT; ++q) SJ[(p0 + q) * S::NSJ + (j + 1) * P + i] = minmod_sel2(l[q], u0[q], r[q]);
+            for (int q = 0; q < NP; ++q) SJ[q * S::NSJ + (j + 1) * P + i] = half_slope2(l[q], u0[q], r[q]);
         }
         // slopes of the ghost cells next to the block: i = -1, NI of every row
         // (items 0..255) and j = -1, NJ of every column (items 256..511)
@@ -1114,11 +1184,11 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
             float val;
             if (x < 256) {
                 const float* q = a + 4 * ((r + 2) * NIP + (side ? NI + 2 : 1));
-                val = face_slope(q[-4], q[0], q[4]);
+                val = half_slope(q[-4], q[0], q[4]);
                 dst = reinterpret_cast<float*>(SI + (v >> 1) * S::NSI + r * P + (side ? NI + 1 : 0));
             } else {
                 const float* q = a + 4 * ((side ? NJ + 2 : 1) * NIP + r + 2);
-                val = face_slope(q[-4 * NIP], q[0], q[4 * NIP]);
+                val = half_slope(q[-4 * NIP], q[0], q[4 * NIP]);
                 dst = reinterpret_cast<float*>(SJ + (v >> 1) * S::NSJ + (side ? NJ + 1 : 0) * P + r);
             }
             dst[v & 1] = val;
@@ -1129,23 +1199,20 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
         }
         // ---- phase B: the faces i - 1/2 and j - 1/2 of this cell, and the
         // last faces of the rows (items 0..127) and columns (128..255)
-        float2 fi0[PPT], fj0[PPT];
+        float2 fi0[NP], fj0[NP];
         {
-            const float cLi = fabsf(vl.y) + GCS[ii - 1], cRi = fabsf(vc.y) + cs;
-            const float cLj = fabsf(vd.z) + cs, cRj = fabsf(vc.z) + cs;
-            const float2 cci = f2(-0.25f * (cRi + cLi)), ccj = f2(-0.25f * (cRj + cLj));
-            float2 l[PPT], d[PPT];
+            const float2 cci = f2(face_speed(vl.y, GCS[ii - 1], vc.y, cs)), ccj = f2(face_speed(vd.z, cs, vc.z, cs));
+            float2 l[NP], d[NP];
             pairs(s0, c0 - 1, l);
             pairs(s0, c0 - NIP, d);
 #pragma unroll
-            for (int q = 0; q < PPT; ++q) {
-                const int p = p0 + q;
-                const float2* si = SI + p * S::NSI + j * P + i;
-                const float2* sj = SJ + p * S::NSJ + j * P + i;
+            for (int q = 0; q < NP; ++q) {
+                                const float2* si = SI + q * S::NSI + j * P + i;
+                const float2* sj = SJ + q * S::NSJ + j * P + i;
                 fi0[q] = face_flux2(l[q], u0[q], si[0], si[1], cci);
                 fj0[q] = face_flux2(d[q], u0[q], sj[0], sj[P], ccj);
-                FI[p * S::NFI + j * P + i] = fi0[q];
-                FJ[p * S::NFJ + j * P + i] = fj0[q];
+                FI[q * S::NFI + j * P + i] = fi0[q];
+                FJ[q * S::NFJ + j * P + i] = fj0[q];
             }
         }
         if (tid < 256) {
@@ -1155,16 +1222,14 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
             if (x < 128) {
                 const float* a = reinterpret_cast<const float*>(tile + (v >> 2) * W * PL + s0 + (r + 2) * NIP + NI + 1) + (v & 3);
                 const float4* vr = tile + s0 + (r + 2) * NIP + NI + 1;   // last interior cell of row r
-                const float cL = fabsf(vr[0].y) + GCS[NI + 1], cR = fabsf(vr[1].y) + GCS[NI + 2];
                 reinterpret_cast<float*>(FI + (v >> 1) * S::NFI + r * P + NI)[v & 1] =
-                    face_flux_s(a[0], a[4], sl[v & 1], sl[2 + (v & 1)], cL, cR);
+                    face_flux(a[0], a[4], sl[v & 1], sl[2 + (v & 1)], face_speed(vr[0].y, GCS[NI + 1], vr[1].y, GCS[NI + 2]));
             } else {
                 const float* a = reinterpret_cast<const float*>(tile + (v >> 2) * W * PL + s0 + (NJ + 1) * NIP + r + 2) + (v & 3);
                 const float4* vt = tile + s0 + (NJ + 1) * NIP + r + 2;   // last interior row, column r
                 const float c2 = GCS[r + 2];
-                const float cL = fabsf(vt[0].z) + c2, cR = fabsf(vt[NIP].z) + c2;
                 reinterpret_cast<float*>(FJ + (v >> 1) * S::NFJ + NJ * P + r)[v & 1] =
-                    face_flux_s(a[0], a[4 * NIP], sl[v & 1], sl[2 * P + (v & 1)], cL, cR);
+                    face_flux(a[0], a[4 * NIP], sl[v & 1], sl[2 * P + (v & 1)], face_speed(vt[0].z, c2, vt[NIP].z, c2));
             }
         }
         __syncthreads();
@@ -1174,51 +1239,39 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
             while (issued < pe && issued <= kp + W) issue();
         // ---- phase C: sum the six faces in the reference's order, update
         const size_t cell = (size_t)kp * PL + c0;
-        float o[2 * PPT];
-        int qn[NH] = {};
+        float o[NV], u[NV];
+        float2 R[NP];
 #pragma unroll
-        for (int q = 0; q < PPT; ++q) {
-            const int p = p0 + q;
-            float2 R = __fmul2_rn(sub2(fi0[q], FI[p * S::NFI + j * P + i + 1]), dinv0);
-            R = __ffma2_rn(sub2(fj0[q], FJ[p * S::NFJ + (j + 1) * P + i]), dinv1, R);
-            R = __ffma2_rn(sub2(fk0[q], fk1[q]), dinv2, R);
-            float2 ov;
-            if (ulo != nullptr) {
-                int8_t q0, q1;
-                const int sh = 16 * (q & 1);
-                ov = ff_add2(u0[q], (int8_t)(qlo[q >> 1] >> sh), (int8_t)(qlo[q >> 1] >> (sh + 8)), __fmul2_rn(hdt2, R), q0, q1);
-                qn[q >> 1] |= ((int)(uint8_t)q0 | (int)(uint8_t)q1 << 8) << sh;
-            } else {
-                ov = __ffma2_rn(hdt2, R, u0[q]);
+        for (int q = 0; q < NP; ++q) {
+            R[q] = __fmul2_rn(sub2(fi0[q], FI[q * S::NFI + j * P + i + 1]), dinv0);
+            R[q] = __ffma2_rn(sub2(fj0[q], FJ[q * S::NFJ + (j + 1) * P + i]), dinv1, R[q]);
+            R[q] = __ffma2_rn(sub2(fk0[q], fk1[q]), dinv2, R[q]);
+            u[2 * q] = u0[q].x;
+            u[2 * q + 1] = u0[q].y;
+        }
+        if (ulo != nullptr) {
+            ff_add4(u, q8.x, {__fmul2_rn(hdt2, R[0]), __fmul2_rn(hdt2, R[1])}, o);
+            ff_add4(u + 4, q8.y, {__fmul2_rn(hdt2, R[2]), __fmul2_rn(hdt2, R[3])}, o + 4);
+            *ql = q8;
+        } else {
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                const float2 ov = __ffma2_rn(hdt2, R[q], u0[q]);
+                o[2 * q] = ov.x;
+                o[2 * q + 1] = ov.y;
             }
-            o[2 * q] = ov.x;
-            o[2 * q + 1] = ov.y;
         }
-#pragma unroll
-        for (int h = 0; h < NH; ++h) {
-            if (ulo != nullptr) qp[h] = qn[h];
-            quads(out)[quad(b, p0 / 2 + h, NCELL) + cell] = f4(o + 4 * h);
-        }
-        if (push.tgt != nullptr) {
-            if constexpr (TPC == 1) push_quads<S, 2, 0>(out, pb, ii, jj, kp, o);
-            else if (half == 0) push_quads<S, 1, 0>(out, pb, ii, jj, kp, o);   // warps never mix halves
-            else push_quads<S, 1, 1>(out, pb, ii, jj, kp, o);
-        }
+        quads(out)[quad(b, 0, NCELL) + cell] = f4(o);
+        quads(out)[quad(b, 1, NCELL) + cell] = f4(o + 4);
+        if (push.tgt != nullptr) push_quads<S>(out, pb, ii, jj, kp, o);
         if (cfl_next) {   // uniform over the CTA
 #pragma unroll
-            for (int v = 0; v < 2 * PPT; ++v) cnan |= (o[v] != o[v]);
-            if constexpr (TPC == 1) {
-                cfl_point(cfl_sq3(o[V_VR], o[V_VT], o[V_VP]), cfl_sq3(o[V_BR], o[V_BT], o[V_BP]));
-            } else if (half == 0) {
-                if (kp > ka) cfl_point(v2_prev, sb2[((kp - 1) & 1) * S::NCOL + c]);
-                v2_prev = cfl_sq3(o[V_VR], o[V_VT], o[V_VP]);
-            } else {
-                sb2[(kp & 1) * S::NCOL + c] = cfl_sq3(o[V_BR - 4], o[V_BT - 4], o[V_BP - 4]);
-            }
+            for (int v = 0; v < NV; ++v) cnan |= (o[v] != o[v]);
+            wmax = fmaxf(wmax, cfl_speed(cfl_sq3(o[V_VR], o[V_VT], o[V_VP]), cfl_sq3(o[V_BR], o[V_BT], o[V_BP]), cs, srho, srho_inv));
         }
         // the window moves up one plane
 #pragma unroll
-        for (int q = 0; q < PPT; ++q) {
+        for (int q = 0; q < NP; ++q) {
             u0[q] = u1[q];
             u1[q] = u2[q];
             dk0[q] = dk1[q];
@@ -1229,19 +1282,16 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
         abort_cta();
         return;
     }
-    if constexpr (TPC == 2) {
-        if (cfl_next && half == 0) cfl_point(v2_prev, sb2[((kb - 1) & 1) * S::NCOL + c]);
-    }
     if (tid == 0)   // every copy has been waited for
         for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
-    if (cfl_next) cfl_commit(cmin, cnan, sc);
+    if (cfl_next) cfl_commit(cfl_column(wmax, rc, gj[GJ_SIN * S::NJP + jj], gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]), cnan, sc);
 }
 // split CTAs per block, each a run of planes
-template <int NI, int NJ, int NK, int TPC>
-__global__ void __launch_bounds__(NI * NJ * TPC, 2)
+template <int NI, int NJ, int NK>
+__global__ void __launch_bounds__(NI * NJ, 2)
 k_march_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geometry g, StepScalars* sc, int cfl_next, int split) {
     const int b = blockIdx.x / split, part = blockIdx.x - b * split, n = NK / split;
-    march_quads<NI, NJ, NK, TPC>(b, 2 + part * n, 2 + (part + 1) * n, u, out, ulo, push, g, sc, cfl_next);
+    march_quads<NI, NJ, NK>(b, 2 + part * n, 2 + (part + 1) * n, u, out, ulo, push, g, sc, cfl_next);
 }
 
 // ---------------------------------------------------------------------------
@@ -1286,7 +1336,7 @@ __global__ void __launch_bounds__(256) k_clear_outside_core(T* u, int64_t nbv, S
 // need.
 template <int NI, int NJ, int NK>
 __global__ void __launch_bounds__(NI * NJ) k_push_state(float* u, PushTable push, Geometry g, StepScalars* sc) {
-    using S = MShape<NI, NJ, NK, 1>;
+    using S = MShape<NI, NJ, NK>;
     constexpr int NIP = S::NIP, NJP = S::NJP;
     static_assert((NI * NJ) % 32 == 0 && 32 % NI == 0, "whole rows in every warp");
     __shared__ PushBlock pb;
@@ -1312,7 +1362,7 @@ __global__ void __launch_bounds__(NI * NJ) k_push_state(float* u, PushTable push
         }
 #pragma unroll
         for (int q = 0; q < G; ++q) {
-            if (push.tgt != nullptr) push_quads<S, 2, 0>(u, pb, ii, jj, k0 + q, o[q]);
+            if (push.tgt != nullptr) push_quads<S>(u, pb, ii, jj, k0 + q, o[q]);
 #pragma unroll
             for (int v = 0; v < NV; ++v) cnan |= (o[q][v] != o[q][v]);
             float ratio = cfl_ratio_f(cfl_sq3(o[q][V_VR], o[q][V_VT], o[q][V_VP]),
@@ -1426,7 +1476,7 @@ k_step_persistent(StepBuffers sb, PushTable push, Geometry g, StepScalars* sc, G
         grid_sync(gb, sc, polls);
     }
     for (int b = take(4); b < d.nblocks; b = take(4)) {
-        march_quads<16, 16, 16, 1>(b, 2, 18, sb.U, sb.R2, sb.ulo, push, g, sc, 1);
+        march_quads<16, 16, 16>(b, 2, 18, sb.U, sb.R2, sb.ulo, push, g, sc, 1);
         next_body();
     }
     grid_sync(gb, sc, polls);

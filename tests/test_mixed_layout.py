@@ -52,3 +52,23 @@ def test_split_blocks_step_as_whole_ones(tiles):
     ua = a.download_state()
     assert np.isfinite(ua).all()
     assert np.array_equal(ua, b.download_state())
+
+
+@pytest.mark.parametrize("block,tiles", [(8, (1, 2, 6)), (16, (1, 1, 3))])
+def test_denormal_fields_stay_small(block, tiles):
+    """The limiter's quotient flushes a denormal jump: its flux stays of the size of
+    the jumps themselves. A field of noise below the smallest normal number
+    (jumps to 4e-39) takes fluxes of at most 8 times three jumps and the step's
+    CFL number below 1, so it stays below 1e-36."""
+    cfg = config.make_config(block=(block,) * 3, root_tiles=tiles, radial_levels=1, amr=(), precision=config.PREC_MIXED)
+    f = fg.Falcon(cfg)
+    u = synth.initial_state(cfg, f.block_ranges(), f.block_flags(), seed=79)
+    rng = np.random.default_rng(79)
+    u[:, 4:7] = rng.uniform(-2e-39, 2e-39, u[:, 4:7].shape)
+    f.upload_state(u)
+    f.exchange()
+    for _ in range(2):
+        f.advance_rk4()
+    out = f.download_state()
+    assert np.isfinite(out).all()
+    assert np.abs(out[:, 4:7]).max() < 1e-36
