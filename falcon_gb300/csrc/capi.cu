@@ -798,6 +798,19 @@ int setup_device(falcon_ctx* ctx) {
             std::vector<size_t> ord(idst.size());
             for (size_t q = 0; q < ord.size(); ++q) ord[q] = q;
             std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return idst[a] < idst[b]; });
+            if (!snap) {
+                // FP64: entries of one kind together (which axes are near, to which
+                // side: ghost_weights), so that a warp's entries take one path
+                auto cls = [&](size_t q) {
+                    int c = ikind[q];
+                    for (int t = 0; t < 3; ++t) c = 3 * c + (iw[3 * q + t] < 1e-12 ? 0 : iw[3 * q + t] > 1.0 - 1e-12 ? 1 : 2);
+                    return c;
+                };
+                std::vector<std::vector<size_t>> bucket(4 * 27);
+                for (size_t q : ord) bucket[(size_t)cls(q)].push_back(q);
+                size_t n = 0;
+                for (const auto& bk : bucket) n = (size_t)(std::copy(bk.begin(), bk.end(), ord.begin() + (long)n) - ord.begin());
+            }
             std::vector<int32_t> d2(ord.size()), s2(ord.size());
             std::vector<double> w2(3 * ord.size()), r2(2 * ord.size());
             std::vector<uint8_t> k2(ord.size());

@@ -1109,33 +1109,280 @@ __device__ __forceinline__ void ghost_rotate(T (&val)[NV], T a, T c) {
     val[V_VT] = -(a * x2) - c * x3;
     val[V_VP] = -(a * x3) + c * x2;
 }
-// The values of one interpolated/rotated ghost entry (into val): the
-// reference's trilinear form and operand order.
-template <class T, bool CG = false>
-__device__ __forceinline__ void ghost_interp_vals(const double* u, const GhostInterpList& L, int ncell, int nip, int pl,
-                                                  int64_t e, double (&val)[NV]) {
-    const int kind = L.kind[e];
-    const size_t s = (size_t)L.src[e];
-    if (kind & 1) {
-        const double wi = L.w[3 * e], wj = L.w[3 * e + 1], wk = L.w[3 * e + 2];
-        const double ui = 1.0 - wi, uj = 1.0 - wj, uk = 1.0 - wk;
+// ---- FP64 ghost interpolation ------------------------------------------------
+// The reference's trilinear sum of a ghost entry: eight corners of three products
+// each, rounded operation by operation, 31 FP64 instructions a value at one warp
+// instruction in 16 cycles per SM. But nearly every entry lies on its source's grid
+// lines along two or three axes, up to the rounding of the coordinates: its weights
+// there are within some 1e-14 of 0 and 1 ("near" axes). Products with the small of
+// two such weights matter only to the last bits of the sum, and the exact bits of
+//   a (1 - D 2^-53)         a's significand less its D 2^-53, rounded, and
+//   S + t, |t| < 2^-35 |S|  S's significand plus t in units of its last place, rounded
+// follow from 32-bit integer and FP32 arithmetic, unless the exact result lies too
+// close to the middle between two numbers to tell, or near the end of a binade; then,
+// and for zeros, denormals and what is not finite, the value takes the reference's
+// form. 442k cells in 8^3 blocks, 604k entries a stage: 351 -> 121 us an exchange; what bounds it
+// now is half FP64 (entries near along one axis or none), half latency.
+constexpr unsigned kNearD = 1u << 13;   // a factor within kNearD 2^-53 of 1 is near
+
+// Weights of one entry. lo, hi: factors of the base and of the +1 corner along i, j, k.
+struct GhostWeights {
+    double lo[3], hi[3];
+    unsigned D[3];       // near axes: 1 - (the large factor), in units of 2^-53
+    unsigned near, up;   // bit a: axis a is near; its large factor is the +1 corner's
+};
+__device__ __forceinline__ GhostWeights ghost_weights(const double* w) {
+    GhostWeights g;
+    g.near = g.up = 0u;
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const double* f = u + s + (size_t)v * ncell;
-            val[v] = f[0] * ui * uj * uk + f[1] * wi * uj * uk + f[nip] * ui * wj * uk + f[pl] * ui * uj * wk +
-                     f[1 + nip] * wi * wj * uk + f[nip + pl] * ui * wj * wk + f[1 + pl] * wi * uj * wk +
-                     f[1 + nip + pl] * wi * wj * wk;
+    for (int a = 0; a < 3; ++a) {
+        g.hi[a] = w[a];
+        g.lo[a] = 1.0 - w[a];
+        const unsigned long long one = 0x3ff0000000000000ull;
+        const unsigned long long dl = one - (unsigned long long)__double_as_longlong(g.lo[a]);
+        const unsigned long long dh = one - (unsigned long long)__double_as_longlong(g.hi[a]);
+        g.D[a] = 0u;
+        if (dl <= kNearD) {
+            g.near |= 1u << a;
+            g.D[a] = (unsigned)dl;
+        } else if (dh <= kNearD) {
+            g.near |= 1u << a;
+            g.up |= 1u << a;
+            g.D[a] = (unsigned)dh;
         }
-    } else {
-        load_cell<CG>(u + s, ncell, val);
     }
-    if (kind & 2) ghost_rotate(val, L.rot[2 * e], L.rot[2 * e + 1]);
+    return g;
+}
+// the reference's form (f: the base corner; w: the weights)
+static __device__ __noinline__ double ghost_plain(const double* f, const double* w, int nip, int pl) {
+    const double wi = w[0], wj = w[1], wk = w[2], ui = 1.0 - wi, uj = 1.0 - wj, uk = 1.0 - wk;
+    return f[0] * ui * uj * uk + f[1] * wi * uj * uk + f[nip] * ui * wj * uk + f[pl] * ui * uj * wk +
+           f[1 + nip] * wi * wj * uk + f[nip + pl] * ui * wj * wk + f[1 + pl] * wi * uj * wk + f[1 + nip + pl] * wi * wj * wk;
+}
+// a's significand's leading 32 bits
+__device__ __forceinline__ unsigned top_bits(double a) {
+    return __funnelshift_l((unsigned)__double2loint(a), (unsigned)__double2hiint(a), 11) | 0x80000000u;
+}
+// round(M D 2^-53) for the significand M with leading bits Mt (M may have moved by
+// 2^16 since): the product of Mt and D has 32 fraction bits and is off by less than
+// D + 64 of their units; false if that leaves the rounding open
+__device__ __forceinline__ bool near_units(unsigned Mt, unsigned D, int& k) {
+    const unsigned long long x = (unsigned long long)Mt * D + 0x80000000ull;
+    k = (int)(x >> 32);
+    return (unsigned)x + (D + 64u) > 2u * (D + 64u);
+}
+// f W in units of the last place of a number with a's exponent and sign (W: times
+// 2^52), relative error 2^-22 beyond W's; 0 for an f beyond 2^-126 below it. d: f's exponent
+// less a's
+__device__ __forceinline__ float small_units(double f, float W, double a, int& d) {
+    const int hf = __double2hiint(f), ha = __double2hiint(a);
+    d = exp_field(f) - exp_field(a);
+    const unsigned m = __funnelshift_l((unsigned)__double2loint(f), (unsigned)hf, 3) & 0x7fffffu;
+    const unsigned bits = m | (unsigned)(d + 127) << 23 | ((unsigned)(hf ^ ha) & 0x80000000u);
+    return d < -126 ? 0.f : __fmul_rn(__int_as_float((int)bits), W);
+}
+// round(x) for an x off by less than 2^-21 m (m >= |x|); false if that leaves it open
+__device__ __forceinline__ bool round_units(float x, float m, int& k) {
+    const float r = __fadd_rn(x, 12582912.f);   // ulp 1: the integer in its low bits
+    k = __float_as_int(r) - 0x4B400000;
+    return __fmaf_rn(m, 4.7683716e-7f, fabsf(__fsub_rn(x, __fsub_rn(r, 12582912.f)))) < 0.499999f;
+}
+// exponents in the middle of the range: no underflow in the products, and what is
+// not finite lies more than 60 above
+__device__ __forceinline__ bool mid_range(double a) { return (unsigned)(exp_field(a) - 100) < 1800u; }
+
+// Entries near along all axes. Every rounding moves the large corner's significand by
+// a whole number of units that does not depend on the others, as long as the binade
+// does not end within 2^20 units: the three products with 1 - D 2^-53, the sum of the
+// terms before the large corner (the corners below it along its `up` axes), and each
+// term after it. Corners off along two or three axes add less than half a unit.
+struct NearEntry {
+    unsigned D[3], up;
+    int at, step[3];   // the large corner from the base, and from it to its neighbours
+    float W[3];        // weights of these, times 2^52
+};
+__device__ __forceinline__ NearEntry near_entry(const GhostWeights& g, int nip, int pl) {
+    NearEntry n;
+    n.up = g.up;
+    n.at = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int st = a == 0 ? 1 : a == 1 ? nip : pl;
+        const bool up = g.up >> a & 1u;
+        n.D[a] = g.D[a];
+        n.at += up ? st : 0;
+        n.step[a] = up ? -st : st;
+        n.W[a] = (float)(up ? g.lo[a] : g.hi[a]) * 4503599627370496.f;
+    }
+    return n;
+}
+__device__ __forceinline__ double ghost_near(const double* f, const double* w, const NearEntry& n, int nip, int pl) {
+    const double* fc = f + n.at;
+    const double a = fc[0];
+    double v[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) v[q] = fc[n.step[q]];
+    const int s01 = n.step[0] + n.step[1], s2 = n.step[2];
+    // the corners off along several axes: weights below 2^-75, so 2^20 |a| is small enough
+    const int hx = max(max(__double2hiint(fc[s01]) & 0x7ff00000, __double2hiint(fc[n.step[0] + s2]) & 0x7ff00000),
+                       max(__double2hiint(fc[n.step[1] + s2]) & 0x7ff00000, __double2hiint(fc[s01 + s2]) & 0x7ff00000));
+    const unsigned Mt = top_bits(a);
+    bool ok = mid_range(a) & (Mt - 0x80000001u < 0x7ffffffeu) & (hx - (__double2hiint(a) & 0x7ff00000) < (20 << 20));
+    int sum = 0, k;
+    float pre = 0.f, pre_m = 0.f, all_m = 0.f;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        ok &= near_units(Mt, n.D[q], k);
+        sum -= k;
+        int d;
+        const float y = small_units(v[q], n.W[q], a, d);
+        ok &= d < 60;
+        all_m += fabsf(y);
+        const bool before = n.up >> q & 1u;
+        pre += before ? y : 0.f;
+        pre_m += before ? fabsf(y) : 0.f;
+        ok &= round_units(before ? 0.f : y, fabsf(y), k);
+        sum += k;
+    }
+    ok &= round_units(pre, pre_m, k) & (all_m < 131072.f);
+    sum += k;
+    return ok ? __longlong_as_double(__double_as_longlong(a) + (long long)sum) : ghost_plain(f, w, nip, pl);
+}
+
+// Entries near along some axes. The main corners (all near factors large) are formed
+// in FP64 along the other axes; the rest are small terms, rounded one by one.
+__device__ __forceinline__ double move_units(double a, int k, bool& ok) {
+    const long long r = __double_as_longlong(a) + (long long)k;
+    ok &= (((int)(r >> 32) ^ __double2hiint(a)) >> 20 == 0) & (((unsigned long long)r << 12) != 0ull);   // inside the binade
+    return __longlong_as_double(r);
+}
+__device__ __forceinline__ constexpr int ghost_order(int p) { return 0x75634210 >> (4 * p) & 7; }   // the reference's order of summation
+struct MixedEntry {
+    GhostWeights g;
+    unsigned main;     // bit c: corner c (bit a of c: +1 along a) is a main corner
+    float W[8];        // the others: product of factors, times 2^52
+};
+__device__ __forceinline__ MixedEntry mixed_entry(const GhostWeights& g) {
+    MixedEntry n;
+    n.g = g;
+    n.main = 0xffu;
+    float lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const unsigned base = a == 0 ? 0x55u : a == 1 ? 0x33u : 0x0fu;   // corners with bit a clear
+        if (g.near >> a & 1u) n.main &= g.up >> a & 1u ? ~base : base;
+        lo[a] = (float)g.lo[a];
+        hi[a] = (float)g.hi[a];
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        n.W[c] = ((c & 1 ? hi[0] : lo[0]) * (c & 2 ? hi[1] : lo[1])) * (c & 4 ? hi[2] : lo[2]) * 4503599627370496.f;
+    return n;
+}
+__device__ __forceinline__ double ghost_mixed(const double* f, const double* w, const MixedEntry& n, int nip, int pl) {
+    double v[8], S = 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = f[(c & 1) + (c & 2 ? nip : 0) + (c & 4 ? pl : 0)];
+    bool ok = true;
+    auto main_term = [&](int c) {
+        double x = v[c];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (n.g.near >> a & 1u) {
+                int k;
+                ok &= near_units(top_bits(x), n.g.D[a], k) & mid_range(x);
+                x = move_units(x, -k, ok);
+            } else {
+                x = x * (c >> a & 1 ? n.g.hi[a] : n.g.lo[a]);
+            }
+        }
+        ok &= mid_range(x);
+        return x;
+    };
+    // the small terms before the first main corner are added to it when it is known
+    unsigned pending = 0u;
+    bool first = true;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        const int c = ghost_order(p);
+        int k, d;
+        if (n.main >> c & 1u) {
+            const double t = main_term(c);
+            if (first) {
+                S = t;
+                first = false;
+                if (pending) {
+                    float x = 0.f, m = 0.f;
+#pragma unroll
+                    for (int q = 0; q < p; ++q) {
+                        const int e = ghost_order(q);
+                        const float y = small_units(v[e], n.W[e], S, d);
+                        ok &= d < 60;
+                        x += y;
+                        m += fabsf(y);
+                    }
+                    ok &= round_units(x, 2.f * m, k);
+                    S = move_units(S, k, ok);
+                }
+            } else {
+                S = S + t;
+                ok &= mid_range(S);
+            }
+        } else if (first) {
+            pending = 1u;
+        } else {
+            const float y = small_units(v[c], n.W[c], S, d);
+            ok &= (d < 60) & round_units(y, 2.f * fabsf(y), k);   // (W: three rounded factors)
+            S = move_units(S, k, ok);
+        }
+    }
+    return ok ? S : ghost_plain(f, w, nip, pl);
+}
+
+// One interpolated/rotated ghost entry, put(variable, value) for each of the eight,
+// those that rotate together one after the other (a loop, not unrolled: the bodies
+// are long, and two at a time already miss the instruction cache).
+template <class F>
+__device__ __forceinline__ void ghost_interp_each(const double* u, const GhostInterpList& L, int ncell, int nip, int pl,
+                                                  int64_t e, F put) {
+    const int kind = L.kind[e];
+    const double *f = u + (size_t)L.src[e], *w = L.w + 3 * e;
+    const double ra = kind & 2 ? L.rot[2 * e] : 0.0, rc = kind & 2 ? L.rot[2 * e + 1] : 0.0;
+    auto each = [&](auto value) {
+        double a = 0.0;   // the first of a pair
+#pragma unroll 1
+        for (int q = 0; q < 8; ++q) {   // (rho1, vr), (vt, vp), (bt, bp), (br, s1)
+            const int v = 0x74653210 >> (4 * q) & 15;
+            double b = value(f + (size_t)v * ncell);
+            if ((kind & 2) && (q == 3 || q == 5)) {
+                const double x2 = a, x3 = b;
+                put(v - 1, -(ra * x2) - rc * x3);
+                b = -(ra * x3) + rc * x2;
+            }
+            if (!((kind & 2) && (q == 2 || q == 4))) put(v, b);
+            a = b;
+        }
+    };
+    if (!(kind & 1)) {
+        each([&](const double* x) { return x[0]; });
+        return;
+    }
+    const GhostWeights g = ghost_weights(w);
+    if (g.near == 7u) {
+        const NearEntry n = near_entry(g, nip, pl);
+        each([&](const double* x) { return ghost_near(x, w, n, nip, pl); });
+    } else if (g.near) {
+        const MixedEntry n = mixed_entry(g);
+        each([&](const double* x) { return ghost_mixed(x, w, n, nip, pl); });
+    } else {
+        each([&](const double* x) { return ghost_plain(x, w, nip, pl); });
+    }
 }
 // FP32 weights; the Yin-Yang seam is aligned in r (wi == 0 after snapping), so
 // most entries are bilinear in (j, k): four source cells. A cell is two 16-byte
 // reads, so an entry's gather touches 8 sectors where [var][cell] order touched 32
 // (21.2M cells, all entries of a stage: 114 -> 62 us).
-template <class T, bool CG = false>
+template <bool CG = false>
 __device__ __forceinline__ void ghost_interp_vals(const float* u, const GhostInterpList& L, int ncell, int nip, int pl,
                                                   int64_t e, float (&val)[NV]) {
     constexpr int CS = Layout<float>::cell;
@@ -1166,11 +1413,16 @@ __device__ __forceinline__ void ghost_interp_vals(const float* u, const GhostInt
     }
     if (kind & 2) ghost_rotate(val, L.rotf[2 * e], L.rotf[2 * e + 1]);
 }
-template <class T, bool CG = false>
-__device__ __forceinline__ void ghost_interp_one(T* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e) {
-    T val[NV];
-    ghost_interp_vals<T, CG>(u, L, ncell, nip, pl, e, val);
+template <bool CG = false>
+__device__ __forceinline__ void ghost_interp_one(float* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e) {
+    float val[NV];
+    ghost_interp_vals<CG>(u, L, ncell, nip, pl, e, val);
     store_cell(u + (size_t)L.dst[e], ncell, val);
+}
+template <bool CG = false>
+__device__ __forceinline__ void ghost_interp_one(double* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e) {
+    double* to = u + (size_t)L.dst[e];
+    ghost_interp_each(u, L, ncell, nip, pl, e, [&](int v, double x) { to[(size_t)v * ncell] = x; });
 }
 
 // ---- block sharding: the entries that cross ranks ---------------------------
@@ -1183,10 +1435,7 @@ template <class T>
 __global__ void __launch_bounds__(128) k_shard_pack(const T* u, GhostInterpList L, int ncell, int nip, int pl, T* pack) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= L.n) return;
-    T val[NV];
-    ghost_interp_vals<T>(u, L, ncell, nip, pl, e, val);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) pack[e * NV + v] = val[v];
+    ghost_interp_each(u, L, ncell, nip, pl, e, [&](int v, T x) { pack[e * NV + v] = x; });
 }
 template <class T>
 __global__ void __launch_bounds__(128) k_shard_unpack(T* u, const int32_t* dst, int64_t n, int ncell, const T* pack) {

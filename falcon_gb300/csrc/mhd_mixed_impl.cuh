@@ -1444,7 +1444,7 @@ k_step_persistent(StepBuffers sb, PushTable push, Geometry g, StepScalars* sc, G
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     auto exchange = [&](const GhostLists& G, float* u) {
         for (int64_t e = t0; e < G.ip.n; e += tstride)
-            ghost_interp_one<float, true>(u, G.ip, d.ncell, d.nip, d.nip * d.njp, e);
+            ghost_interp_one<true>(u, G.ip, d.ncell, d.nip, d.nip * d.njp, e);
         for (int64_t e = t0; e < G.ln.n; e += tstride) ghost_lin_one<float, true>(u, G.ln, d.ncell, e);
         for (int64_t e = t0; e < G.cp.n; e += tstride) ghost_copy_one<float, true>(u, G.cp, d.ncell, e);
     };
