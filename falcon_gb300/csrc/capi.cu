@@ -52,6 +52,7 @@ struct falcon_ctx {
     float *gi_f = nullptr, *gj_f = nullptr, *gs_f = nullptr;
     int32_t* flags = nullptr;
     StepScalars* sc = nullptr;
+    StepScalars* sc_host = nullptr;         // pinned copy of the scalars (read_scalars)
     GhostLists gl{};          // every ghost cell (the exchange after the diffusion pass)
     GhostLists gl_stage{};    // face ghosts not pushed by the stage kernel (exchanges after stages)
     GhostLists gl_final{};    // mixed: ghost entries the exchange ending a step fills (see setup_device)
@@ -407,19 +408,22 @@ int autotune(falcon_ctx* ctx) {
     return FALCON_OK;
 }
 
-int check_nan(falcon_ctx* ctx) {
-    int32_t flag = 0, stp = -1;
-    cudaError_t e = cudaMemcpy(&flag, &ctx->sc->nan_flag, sizeof(int32_t), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return ctx->cuda_fail(e, "nan flag");
-    cudaMemcpy(&stp, &ctx->sc->nan_step, sizeof(int32_t), cudaMemcpyDeviceToHost);
+// The step scalars into pinned memory, one copy behind the work queued so far (three
+// copies of single fields, two of them blocking, cost a small step 30 us)
+cudaError_t read_scalars(falcon_ctx* ctx) {
+    cudaError_t e = cudaMemcpyAsync(ctx->sc_host, ctx->sc, sizeof(StepScalars), cudaMemcpyDeviceToHost, ctx->st);
+    return e == cudaSuccess ? cudaStreamSynchronize(ctx->st) : e;
+}
+// the step flags of the scalars last read
+int step_flags(falcon_ctx* ctx) {
+    const int32_t flag = ctx->sc_host->nan_flag, stp = ctx->sc_host->nan_step;
     if (flag & 2) {
         // a step kernel's wait for a bulk copy ran out: its CTAs left cleanly,
         // the step's results are discarded (the state is undefined until the
         // next upload, synthetic initial condition or restart)
-        int32_t polls = 0;
-        cudaMemcpy(&polls, &ctx->sc->wait_polls, sizeof(int32_t), cudaMemcpyDeviceToHost);
         char buf[192];
-        snprintf(buf, sizeof buf, "a step kernel's bulk-copy wait ran out (poll limit %d); the state is undefined", polls);
+        snprintf(buf, sizeof buf, "a step kernel's bulk-copy wait ran out (poll limit %d); the state is undefined",
+                 ctx->sc_host->wait_polls);
         ctx->err = buf;
         return FALCON_ERR_TIMEOUT;
     }
@@ -430,6 +434,11 @@ int check_nan(falcon_ctx* ctx) {
         return FALCON_ERR_NAN_DETECTED;
     }
     return FALCON_OK;
+}
+
+int check_nan(falcon_ctx* ctx) {
+    cudaError_t e = read_scalars(ctx);
+    return e == cudaSuccess ? step_flags(ctx) : ctx->cuda_fail(e, "nan flag");
 }
 
 // global element offset of var 0 of padded cell (i,j,k) (Fortran indices) of block b
@@ -901,6 +910,7 @@ int setup_device(falcon_ctx* ctx) {
     s0.nan_step = -1;
     s0.wait_polls = kDefaultWaitPolls;
     CK(ctx->alloc(&ctx->sc, sizeof(StepScalars)), "alloc scalars");
+    CK(cudaMallocHost((void**)&ctx->sc_host, sizeof(StepScalars)), "alloc scalars");
     CK(cudaMemcpy(ctx->sc, &s0, sizeof s0, cudaMemcpyHostToDevice), "upload scalars");
     CK(cudaStreamSynchronize(ctx->st), "sync");
     ctx->on_device = true;
@@ -943,6 +953,7 @@ void falcon_destroy(falcon_ctx* ctx) {
         for (auto& r : ctx->pending) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
         for (auto e : ctx->pool) cudaEventDestroy(e);
         for (void* p : ctx->allocs) cudaFree(p);
+        if (ctx->sc_host) cudaFreeHost(ctx->sc_host);
         if (ctx->t0) cudaEventDestroy(ctx->t0);
         if (ctx->t1) cudaEventDestroy(ctx->t1);
         cudaStreamDestroy(ctx->st);
@@ -1359,10 +1370,10 @@ int falcon_step_rk4(falcon_ctx* ctx, double* dt_out) {
     rc = run(ctx, 1);
     if (rc) return rc;
     if (dt_out) {
-        CK(cudaMemcpyAsync(dt_out, &ctx->sc->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->st), "dt");
-        CK(cudaStreamSynchronize(ctx->st), "dt");
+        CK(read_scalars(ctx), "dt");
+        *dt_out = ctx->sc_host->dt;
         collect(ctx);
-        return check_nan(ctx);
+        return step_flags(ctx);
     }
     return FALCON_OK;
 }
