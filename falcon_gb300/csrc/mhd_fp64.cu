@@ -89,7 +89,10 @@ cudaError_t launch_shard_unpack_fp64(const StepDims& d, const int32_t* dst, int6
 
 // dt = min(1.e20, CFL*min(h/v_wave)) (3_6/ModTimeStep.f90:20-29); also the
 // per-stage FP32 factors of the mixed path and the reset of the accumulator.
-__global__ void k_finalize_dt(StepScalars* sc) { impl::finalize_dt_body(sc); }
+__global__ void k_finalize_dt(StepScalars* sc) {
+    impl::step_go();
+    impl::finalize_dt_body(sc);
+}
 cudaError_t launch_finalize_dt(StepScalars* sc, cudaStream_t st) {
     k_finalize_dt<<<1, 1, 0, st>>>(sc);
     return cudaGetLastError();

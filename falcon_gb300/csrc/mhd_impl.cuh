@@ -209,9 +209,13 @@ __device__ __forceinline__ void fence_proxy_async() {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
+// Programmatic dependent launch of the mixed step's kernels (launch_step): a kernel's
+// CTAs may start while the one before drains. What comes before step_wait reads only
+// what no kernel of a step writes (geometry, flags, lists, push table) and writes only
+// shared memory; after it, the work of every kernel before is complete and visible.
+// step_go lets the next kernel's CTAs take the slots that this one's leave.
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void step_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // 1-D bulk copy global -> shared, completion counted on `bar` (16-byte aligned, size % 16 == 0)
 // Hint: pull `bytes` (a multiple of 16, 16-byte aligned) of global memory into
 // L2 ahead of plain loads.
@@ -1080,24 +1084,29 @@ __global__ void __launch_bounds__(256) k_cfl(const T* u, Geometry g, StepScalars
 // (3_6/ModCommunication.f90:655-795). Exact copies first, then trilinear
 // entries (3_6/ModMath.f90:283-291) with the Yin-Yang vector rotation
 // (3_6/ModYinYang.f90:58-60).
-template <class T, bool CG = false>
+// WAIT: step_wait between the entry's own fields and the state.
+template <class T, bool CG = false, bool WAIT = false>
 __device__ __forceinline__ void ghost_copy_one(T* u, const GhostCopyList& L, int ncell, int64_t e) {
+    const size_t src = (size_t)L.src[e], dst = (size_t)L.dst[e];
+    if (WAIT) step_wait();
     T v[NV];
-    load_cell<CG>(u + (size_t)L.src[e], ncell, v);
-    store_cell(u + (size_t)L.dst[e], ncell, v);
+    load_cell<CG>(u + src, ncell, v);
+    store_cell(u + dst, ncell, v);
 }
 
 // one-dimensional linear interpolation (radial neighbours of different
 // spacing: the other two weights snapped to exactly 0), mixed path only
-template <class T, bool CG = false>
+template <class T, bool CG = false, bool WAIT = false>
 __device__ __forceinline__ void ghost_lin_one(T* u, const GhostLinList& L, int ncell, int64_t e) {
     const T w = (T)L.w[e], uw = T(1) - w;
+    const size_t src = (size_t)L.src[e], next = src + (size_t)L.stride[e], dst = (size_t)L.dst[e];
+    if (WAIT) step_wait();
     T v[NV], n[NV];
-    load_cell<CG>(u + (size_t)L.src[e], ncell, v);
-    load_cell<CG>(u + (size_t)L.src[e] + (size_t)L.stride[e], ncell, n);
+    load_cell<CG>(u + src, ncell, v);
+    load_cell<CG>(u + next, ncell, n);
 #pragma unroll
     for (int q = 0; q < NV; ++q) v[q] = blend(v[q], n[q], uw, w);
-    store_cell(u + (size_t)L.dst[e], ncell, v);
+    store_cell(u + dst, ncell, v);
 }
 
 template <class T>
@@ -1382,7 +1391,7 @@ __device__ __forceinline__ void ghost_interp_each(const double* u, const GhostIn
 // most entries are bilinear in (j, k): four source cells. A cell is two 16-byte
 // reads, so an entry's gather touches 8 sectors where [var][cell] order touched 32
 // (21.2M cells, all entries of a stage: 114 -> 62 us).
-template <bool CG = false>
+template <bool CG = false, bool WAIT = false>
 __device__ __forceinline__ void ghost_interp_vals(const float* u, const GhostInterpList& L, int ncell, int nip, int pl,
                                                   int64_t e, float (&val)[NV]) {
     constexpr int CS = Layout<float>::cell;
@@ -1390,7 +1399,8 @@ __device__ __forceinline__ void ghost_interp_vals(const float* u, const GhostInt
     const float* s = u + (size_t)L.src[e];
     auto at = [&](int off, float (&v)[NV]) { load_cell<CG>(s + (size_t)CS * off, ncell, v); };
     const float wi = L.wf[3 * e], wj = L.wf[3 * e + 1], wk = L.wf[3 * e + 2];
-    const float ui = 1.f - wi, uj = 1.f - wj, uk = 1.f - wk;
+    const float ui = 1.f - wi, uj = 1.f - wj, uk = 1.f - wk, ra = L.rotf[2 * e], rc = L.rotf[2 * e + 1];
+    if (WAIT) step_wait();
     if (!(kind & 1)) {
         at(0, val);
     } else if (wi == 0.f) {
@@ -1411,16 +1421,18 @@ __device__ __forceinline__ void ghost_interp_vals(const float* u, const GhostInt
                      f(1 + nip + pl) * wi * wj * wk;
         }
     }
-    if (kind & 2) ghost_rotate(val, L.rotf[2 * e], L.rotf[2 * e + 1]);
+    if (kind & 2) ghost_rotate(val, ra, rc);
 }
-template <bool CG = false>
+template <bool CG = false, bool WAIT = false>
 __device__ __forceinline__ void ghost_interp_one(float* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e) {
     float val[NV];
-    ghost_interp_vals<CG>(u, L, ncell, nip, pl, e, val);
-    store_cell(u + (size_t)L.dst[e], ncell, val);
+    const size_t dst = (size_t)L.dst[e];
+    ghost_interp_vals<CG, WAIT>(u, L, ncell, nip, pl, e, val);
+    store_cell(u + dst, ncell, val);
 }
-template <bool CG = false>
+template <bool CG = false, bool WAIT = false>
 __device__ __forceinline__ void ghost_interp_one(double* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e) {
+    if (WAIT) step_wait();
     double* to = u + (size_t)L.dst[e];
     ghost_interp_each(u, L, ncell, nip, pl, e, [&](int v, double x) { to[(size_t)v * ncell] = x; });
 }
@@ -1467,15 +1479,16 @@ __global__ void __launch_bounds__(128) k_ghost_interp(T* u, GhostInterpList L, i
 template <class T>
 __global__ void __launch_bounds__(128) k_ghost_all(T* u, GhostLists G, int ncell, int nip, int pl, int nb_ip, int nb_ln) {
     const int bx = blockIdx.x;
+    step_go();
     if (bx < nb_ip) {
         const int64_t e = (int64_t)bx * 128 + threadIdx.x;
-        if (e < G.ip.n) ghost_interp_one(u, G.ip, ncell, nip, pl, e);
+        if (e < G.ip.n) ghost_interp_one<false, true>(u, G.ip, ncell, nip, pl, e);
     } else if (bx < nb_ip + nb_ln) {
         const int64_t e = (int64_t)(bx - nb_ip) * 128 + threadIdx.x;
-        if (e < G.ln.n) ghost_lin_one(u, G.ln, ncell, e);
+        if (e < G.ln.n) ghost_lin_one<T, false, true>(u, G.ln, ncell, e);
     } else {
         const int64_t e = (int64_t)(bx - nb_ip - nb_ln) * 128 + threadIdx.x;
-        if (e < G.cp.n) ghost_copy_one(u, G.cp, ncell, e);
+        if (e < G.cp.n) ghost_copy_one<T, false, true>(u, G.cp, ncell, e);
     }
 }
 

@@ -30,8 +30,7 @@ cudaError_t stage_nd(const StepDims& d, const Geometry& g, const float* in, cons
         static const cudaError_t attr = allow_smem(kernel, smem);
         if (attr != cudaSuccess) return attr;
         const int split = in != out ? split_of(d, most) : 1;
-        kernel<<<d.nblocks * split, nt, smem, st>>>(in, un, out, lo, push, psi, g, sc, stage, bcw, split);
-        return cudaGetLastError();
+        return launch_step(d, kernel, d.nblocks * split, nt, smem, st, in, un, out, lo, push, psi, g, sc, stage, bcw, split);
     };
     if constexpr (KP == 0) return run(k_stage_march<N, N, N, DIVB>, SMarch<N, N, N>::smem, N * N, 8);
     else return run(k_stage_chunks<N, N, N, KP, DIVB>, QShape<N, N, N, KP>::smem, N * N * KP, N / KP);
@@ -57,8 +56,7 @@ cudaError_t diff_n(const StepDims& d, const Geometry& g, const float* u, float* 
     using S = DShape<N, N, N, KP>;
     static const cudaError_t attr = allow_smem(k_diffusion_quads<N, N, N, KP>, S::smem);
     if (attr != cudaSuccess) return attr;
-    k_diffusion_quads<N, N, N, KP><<<d.nblocks, S::NT, S::smem, st>>>(u, out, lo, push, g, sc, cfl_next);
-    return cudaGetLastError();
+    return launch_step(d, k_diffusion_quads<N, N, N, KP>, d.nblocks, S::NT, S::smem, st, u, out, lo, push, g, sc, cfl_next);
 }
 // 16^3 blocks: the k march
 cudaError_t diff_march16(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo,
@@ -67,8 +65,8 @@ cudaError_t diff_march16(const StepDims& d, const Geometry& g, const float* u, f
     static const cudaError_t attr = allow_smem(k_march_quads<16, 16, 16>, S::smem);
     if (attr != cudaSuccess) return attr;
     const int split = out != u ? split_of(d, 4) : 1;
-    k_march_quads<16, 16, 16><<<d.nblocks * split, S::NT, S::smem, st>>>(u, out, lo, push, g, sc, cfl_next, split);
-    return cudaGetLastError();
+    return launch_step(d, k_march_quads<16, 16, 16>, d.nblocks * split, S::NT, S::smem, st, u, out, lo, push, g, sc, cfl_next,
+                       split);
 }
 }  // namespace
 }  // namespace impl

@@ -528,13 +528,17 @@ __device__ __forceinline__ void stage_chunks(int b, int ch0, int ch1, const floa
     __shared__ PushBlock pb;
     load_push_block(push, b, &pb);
     const int tid = threadIdx.x, nch = ch1 - ch0;
-    if (tid == 0) {
+    const bool issuer = tid == S::NT - 32;   // requests the copies (the first warp loads the tables)
+    step_go();
+    if (issuer) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         fence_mbar_init();
+        step_wait();
         issue_quads<S>(blk_in, tile, ch0 * KPAR, ch0 * KPAR + KPAR + 4, 0, &bars[0]);
     }
     tab.load(g, b, NIP, S::NJP, S::NT);
+    step_wait();
     __syncthreads();   // barriers and tables are used by every thread below
 
     int i, j, kq;
@@ -580,7 +584,7 @@ __device__ __forceinline__ void stage_chunks(int b, int ch0, int ch1, const floa
             copy_wait_abort(sc, bars, n, n);
             return;
         }
-        if (tid == 0 && n + 1 < nch) issue_quads<S>(blk_in, tile, next, next + KPAR, 0, &bars[(n + 1) & 1]);
+        if (issuer && n + 1 < nch) issue_quads<S>(blk_in, tile, next, next + KPAR, 0, &bars[(n + 1) & 1]);
         const int kp = ch * KPAR + kq + 2;
         const size_t cell = (size_t)kp * PL + c0;
         int sl[5];
@@ -655,17 +659,21 @@ __device__ __forceinline__ void stage_march(int b, int ka, int kb, const float* 
     __shared__ PushBlock pb;
     load_push_block(push, b, &pb);
     const int tid = threadIdx.x, p0 = ka - 2, pe = kb + 2;   // planes [p0, pe) are read
-    int issued = p0;                                         // thread 0: planes [p0, issued) have been requested
+    const bool issuer = tid == S::NT - 32;                   // requests the copies (the first warp loads the tables)
+    int issued = p0;                                         // by the issuer: planes [p0, issued)
     auto issue = [&](int last) {
         for (; issued <= last && issued < pe; ++issued)
             issue_quads<S>(blk_in, tile, issued, issued + 1, p0, &bars[(issued - p0) % W]);
     };
-    if (tid == 0) {
+    step_go();
+    if (issuer) {
         for (int q = 0; q < W; ++q) mbar_init(&bars[q], 1);
         fence_mbar_init();
+        step_wait();
         issue(p0 + W - 1);
     }
     tab.load(g, b, NIP, S::NJP, S::NT);
+    step_wait();
     __syncthreads();   // barriers and tables are used by every thread below
     const int i = tid % NI, j = tid / NI, ii = i + 2, jj = j + 2, c0 = jj * NIP + ii;
     const float dtk = sc->dt_stage_f[stage - 1];
@@ -714,7 +722,7 @@ __device__ __forceinline__ void stage_march(int b, int ka, int kb, const float* 
     int s = 2;   // slot of plane kp
     for (int kp = ka; kp < kb; ++kp) {
         // everyone is through with the cells of plane kp - 1: plane kp - 3's slot is free
-        if (tid == 0 && !late) issue(kp + W - 3);
+        if (issuer && !late) issue(kp + W - 3);
         const int cell = kp * PL + c0;
         int2* ql = lo_b + (kp - 2) * S::PLI;
         const float4 ua = na, ub = nb;   // u^n (at stage 1 the input itself, in L2)
@@ -742,12 +750,12 @@ __device__ __forceinline__ void stage_march(int b, int ka, int kb, const float* 
             __syncthreads();
         }
     }
-    if (__syncthreads_or(late) && tid == 0) {
+    if (__syncthreads_or(late) && issuer) {
         atomicOr(&sc->nan_flag, 2);
         for (int p = issued - p0 < W ? p0 : issued - W; p < issued; ++p)   // the copies in flight
             mbar_wait(&bars[(p - p0) % W], (uint32_t)(((p - p0) / W) & 1), kWaitPolls);
     }
-    if (tid == 0)
+    if (issuer)
         for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
 }
 // split CTAs per block, each a run of planes
@@ -836,21 +844,24 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
     const bool copy_bc = out != u && (flb & 6);
     __shared__ PushBlock pb;
     load_push_block(push, b, &pb);
-    if (threadIdx.x == 0) {
+    const bool issuer = threadIdx.x == S::NT - 32;   // requests the copies
+    step_go();
+    if (issuer) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         fence_mbar_init();
+        step_wait();
+        issue_quads<S>(blk, tile, 0, KPAR + 4, 0, &bars[0]);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) issue_quads<S>(blk, tile, 0, KPAR + 4, 0, &bars[0]);
     // the int8 corrections of u^n are read with plain loads: warm L2 one chunk ahead
     auto prefetch_lo = [&](int kp_first) {
         if (ulo != nullptr && threadIdx.x == 0)
             prefetch_l2(ulo + ((size_t)b * S::NINT + (size_t)(kp_first - 2) * S::PLI) * NV, KPAR * S::PLI * NV);
     };
-    prefetch_lo(2);
     load_geometry<float, S>(g, b, gi, gj, gs, nullptr);
-    __syncthreads();   // the geometry tables are read by every thread below
+    step_wait();
+    prefetch_lo(2);
+    __syncthreads();   // barriers and tables are used by every thread below
     const int tid = threadIdx.x;
     const float* GCS = gi + GI_CS * NIP;
     const int kq = tid / (NI * NJ), i = tid % NI, j = tid / NI % NJ;
@@ -878,7 +889,7 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
             copy_wait_abort(sc, bars, ch - 1, ch);
             return;
         }
-        if (threadIdx.x == 0 && ch + 1 < nchunk) issue_quads<S>(blk, tile, hi, hi + KPAR, 0, &bars[(ch + 1) & 1]);
+        if (issuer && ch + 1 < nchunk) issue_quads<S>(blk, tile, hi, hi + KPAR, 0, &bars[(ch + 1) & 1]);
         if (ch + 1 < nchunk) prefetch_lo(k0 + KPAR + 1);
         const int kp0 = k0 + 1, kp = kp0 + kq;   // padded index of the chunk's first plane, this cell's plane
         // this thread's int8 corrections, loaded now so that their latency
@@ -1067,24 +1078,26 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
     const bool copy_bc = out != u && (flb & 6);
     __shared__ PushBlock pb;
     load_push_block(push, b, &pb);
-    if (tid == 0) {
-        for (int s = 0; s < W; ++s) mbar_init(&bars[s], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
+    const bool issuer = tid == S::NT - 32;   // requests the copies
     // planes are counted from pa, the first that [ka, kb) needs; pe: one past the last
     const int pa = ka - 2, pe = kb + 2;
-    int issued = pa;   // thread 0: planes [pa, issued) have been requested
+    int issued = pa;   // by the issuer: planes [pa, issued)
     auto issue = [&]() {
         issue_quads<S>(blk, tile, issued, issued + 1, pa, &bars[(issued - pa) % W]);
         ++issued;
     };
-    if (tid == 0)
-        while (issued < pa + W) issue();
     int8_t* blk_lo = ulo != nullptr ? ulo + (size_t)b * NV * S::NINT : nullptr;
-    if (blk_lo != nullptr && tid == 0) prefetch_l2(blk_lo + (size_t)(ka - 2) * S::PLI * NV, 2 * S::PLI * NV);
+    step_go();
+    if (issuer) {
+        for (int s = 0; s < W; ++s) mbar_init(&bars[s], 1);
+        fence_mbar_init();
+        step_wait();
+        while (issued < pa + W) issue();
+        if (blk_lo != nullptr) prefetch_l2(blk_lo + (size_t)(ka - 2) * S::PLI * NV, 2 * S::PLI * NV);
+    }
     load_geometry<float, S>(g, b, gi, gj, gs, nullptr);
-    __syncthreads();   // the geometry tables are read by every thread below
+    step_wait();
+    __syncthreads();   // barriers and tables are used by every thread below
     // this thread's column: warp w takes rows (w % 4) + 8 (w / 4) and that + 4
     const int wq = tid >> 5, i = tid & 15;
     const int j = (wq & 3) + 8 * (wq >> 2) + 4 * ((tid >> 4) & 1);
@@ -1098,7 +1111,7 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
     const int polls = sc->wait_polls;
     int late = 0;   // a wait of this thread for a plane ran out
     auto abort_cta = [&]() {   // after a uniform decision: flag, drain the copies in flight
-        if (tid != 0) return;
+        if (!issuer) return;
         atomicOr(&sc->nan_flag, 2);
         for (int p = issued - pa < W ? 0 : issued - pa - W; p < issued - pa; ++p)
             mbar_wait(&bars[p % W], (uint32_t)((p / W) & 1), kWaitPolls);
@@ -1141,7 +1154,7 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
     const float srho = __fsqrt_rn(gi[GI_RHO0 * NIP + ii]), srho_inv = __frcp_rn(srho);
     for (int kp = ka; kp < kb; ++kp) {
         const int p2 = kp + 2;
-        if (blk_lo != nullptr && tid == 0 && kp + 2 < kb)
+        if (blk_lo != nullptr && issuer && kp + 2 < kb)
             prefetch_l2(blk_lo + (size_t)kp * S::PLI * NV, S::PLI * NV);
         // this cell's int8 corrections, loaded before the wait
         int2 q8 = make_int2(0, 0);
@@ -1235,7 +1248,7 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
         __syncthreads();
         // planes below kp + 1 are done with: refill their slots, up to plane
         // kp + W (at kp = 2 that is planes 5, 6, 7; then one plane a step)
-        if (tid == 0)
+        if (issuer)
             while (issued < pe && issued <= kp + W) issue();
         // ---- phase C: sum the six faces in the reference's order, update
         const size_t cell = (size_t)kp * PL + c0;
@@ -1282,7 +1295,7 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
         abort_cta();
         return;
     }
-    if (tid == 0)   // every copy has been waited for
+    if (issuer)   // every copy has been waited for
         for (int q = 0; q < W; ++q) mbar_inval(&bars[q]);
     if (cfl_next) cfl_commit(cfl_column(wmax, rc, gj[GJ_SIN * S::NJP + jj], gs[GS_DXI], gs[GS_DXJ], gs[GS_DXK]), cnan, sc);
 }
