@@ -62,6 +62,33 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// eight channels of a voxel: BF16 in memory (16 bytes), FP32 in registers
+struct V8 { float v[8]; };
+__device__ __forceinline__ V8 load8(const __nv_bfloat16* p) {
+    const uint4 r = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+    V8 x;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        x.v[2 * q] = __uint_as_float(w[q] << 16);
+        x.v[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
+    }
+    return x;
+}
+__device__ __forceinline__ V8 load8(const float* p) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    return V8{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const V8& x) {
+    __nv_bfloat162 r[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        r[q].x = __float2bfloat16_rn(x.v[2 * q]);
+        r[q].y = __float2bfloat16_rn(x.v[2 * q + 1]);
+    }
+    *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(r);
+}
+
 // grid coordinates of voxel v (computed once per row, outside the tap loop)
 struct Vox { int64_t base; int d, h, w; bool ok; };   // base: first voxel of v's sample
 __device__ __forceinline__ Vox decompose(const Grid3& g, int64_t v, int64_t total) {
@@ -99,12 +126,15 @@ __device__ __forceinline__ int64_t neighbour(const Grid3& g, int64_t v, int dd, 
 // MODE 0: forward, out = bf16(relu?(acc + bias)), taps at +offset
 // MODE 1: forward of the last layer, out32[v] = acc(channel 0) + bias[0]
 // MODE 2: backward data, out32[v][c] = acc, taps at -offset
+// MODE 3: backward data into the next layer's masked gradient, out16 = bf16(acc) where
+//         y > 0, else 0 (y: that layer's output)
 // w: [27][NC][KC] BF16 (for MODE 2 the caller passes the transposed copy).
 // 4 warps, each 16 voxels x NC channels; a CTA covers 64 voxels.
 template <int KC, int NC, int MODE>
 __global__ void __launch_bounds__(128) k_conv(const __nv_bfloat16* __restrict__ x, Grid3 g,
                                               const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
-                                              int relu, __nv_bfloat16* __restrict__ out16, float* __restrict__ out32) {
+                                              int relu, __nv_bfloat16* __restrict__ out16, float* __restrict__ out32,
+                                              const __nv_bfloat16* __restrict__ y) {
     constexpr int NT = NC / 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gid = lane >> 2, tig = lane & 3;
@@ -116,7 +146,7 @@ __global__ void __launch_bounds__(128) k_conv(const __nv_bfloat16* __restrict__ 
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
     const Vox x0 = decompose(g, v0, total), x1 = decompose(g, v1, total);
     for (int tap = 0; tap < 27; ++tap) {
-        const int sgn = MODE == 2 ? -1 : 1;
+        const int sgn = MODE >= 2 ? -1 : 1;
         const int dd = sgn * (tap / 9 - 1), dh = sgn * ((tap / 3) % 3 - 1), dw = sgn * (tap % 3 - 1);
         const int64_t n0 = shifted(g, x0, dd, dh, dw);
         const int64_t n1 = shifted(g, x1, dd, dh, dw);
@@ -154,6 +184,12 @@ __global__ void __launch_bounds__(128) k_conv(const __nv_bfloat16* __restrict__ 
                 *reinterpret_cast<__nv_bfloat162*>(out16 + v * NC + co) = p;
             } else if (MODE == 1) {
                 if (co == 0) out32[v] = y0 + bias[0];
+            } else if (MODE == 3) {
+                const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(y + v * NC + co);
+                __nv_bfloat162 p;
+                p.x = __float2bfloat16_rn(__bfloat162float(m.x) > 0.f ? y0 : 0.f);
+                p.y = __float2bfloat16_rn(__bfloat162float(m.y) > 0.f ? y1 : 0.f);
+                *reinterpret_cast<__nv_bfloat162*>(out16 + v * NC + co) = p;
             } else {
                 out32[v * NC + co] = y0;
                 out32[v * NC + co + 1] = y1;
@@ -186,7 +222,6 @@ __global__ void __launch_bounds__(128) k_conv(const __nv_bfloat16* __restrict__ 
 // Every wait is bounded; one that runs out sets *err, the CTA waits (bounded)
 // for its copies in flight, frees its tensor memory and discards its tile.
 namespace tc {
-constexpr int kStages = 4;                          // ring depth of the weight-gradient tiles
 constexpr int kConvStages = 8;                      // ring depth of the convolutions' weight tiles
 constexpr int kBW = 8, kBH = 4, kBD = 4;            // voxel brick (w, h, d) of a weight-gradient tile
 constexpr int kRowW = 8, kRowH = 16;                // row block (w, h; one d) of a convolution tile
@@ -332,7 +367,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __nv_bfloat16* __restrict
                                                  const __grid_constant__ CUtensorMap wmap, Grid3 g,
                                                  const float* __restrict__ bias, int relu,
                                                  __nv_bfloat16* __restrict__ out16, float* __restrict__ out32,
-                                                 int32_t* err, int polls) {
+                                                 const __nv_bfloat16* __restrict__ y, int32_t* err, int polls) {
     using namespace tc;
     constexpr int ST = kConvStages;
     constexpr int HD = 3, HH = kRowH + 2, HW = kRowW + 2, HROWS = HD * HH * HW;
@@ -400,7 +435,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __nv_bfloat16* __restrict
             const int s = t % ST;
             if (!mbar_wait(&full[s], (uint32_t)((t / ST) & 1), polls)) { late = 1; break; }
             fence_after();
-            const int sgn = MODE == 2 ? -1 : 1;
+            const int sgn = MODE >= 2 ? -1 : 1;
             const int dd = sgn * (t / 9 - 1), dh = sgn * ((t / 3) % 3 - 1), dw = sgn * (t % 3 - 1);
             const uint32_t at = a0 + (uint32_t)((((dd + 1) * HH + dh + 1) * HW + dw + 1) * 16);
             const uint32_t b0 = smem_u32(bbase + s * B_STRIDE);
@@ -446,6 +481,15 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __nv_bfloat16* __restrict
             }
         } else if constexpr (MODE == 1) {
             out32[v] = acc[0] + bias[0];
+        } else if constexpr (MODE == 3) {
+#pragma unroll
+            for (int k = 0; k < 16; k += 8) {
+                const V8 m = load8(y + v * NC + c0 + k);
+                V8 r;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) r.v[q] = m.v[q] > 0.f ? acc[k + q] : 0.f;
+                store8(out16 + v * NC + c0 + k, r);
+            }
         } else {
 #pragma unroll
             for (int k = 0; k < 16; k += 4)
@@ -455,57 +499,64 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __nv_bfloat16* __restrict
     tile_release<NCOLS>(tmem);
 }
 
-// Weight gradient of one tap over a run of bricks: D[co][ci] (M = 128 rows,
-// co < CO real; N = CI) += sum over the bricks' voxels of gy[v][co] x[v +
-// off][ci]. Both tiles are [128 voxels][C] as copied, i.e. MN-major with the
-// voxels as K: 8 voxel rows form a swizzle atom (SBO = 8 rows), and the 16
-// voxels of one MMA are 16 rows further on. M = 128 covers CO with LBO = 0:
-// the rows past CO repeat the first ones and their accumulators are unused.
-// The sums of all bricks are added into dw[co][ci][tap] with FP32 atomics.
+// Weight gradient of T = 128 / CI taps over a run of bricks: D[tap, ci][co] (M = 128, N
+// = CO) += sum over the bricks' voxels of x[v + off(tap)][ci] gy[v][co]. The tiles are
+// [128 voxels][C] as copied, i.e. MN-major with the voxels as K: 8 voxel rows form a
+// swizzle atom (SBO = 8 rows), the 16 voxels of one MMA are 16 rows further on, and the
+// M index runs through the taps' tiles (LBO = a tile). An MMA reads its 128 rows of A
+// from shared memory whatever they hold, 4 KB at 128 bytes a cycle, which bounds it: with
+// gy as A, 16 of the 128 rows counted and a tap took as long as eight do here. Taps past
+// the 27th have no copy; their rows are not read. The sums of all bricks are added into
+// dw[co][ci][tap] with FP32 atomics. 393k voxels, 16 x 16 channels: 100 -> 60 us
+// (three taps to a gy tile with gy as A: 112).
+__host__ __device__ constexpr int kWgradStages(int co) { return co == 16 ? 3 : 2; }   // two CTAs per SM
 template <int CO, int CI>
 __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtensorMap gmap,
                                                   const __grid_constant__ CUtensorMap xmap, Grid3 g, int64_t nbricks,
                                                   int per_cta, int co_real, int ci_real, float* __restrict__ dw,
                                                   int32_t* err, int polls) {
     using namespace tc;
-    constexpr uint32_t SPAN_A = CO * 2, SPAN_B = CI * 2;
-    constexpr uint32_t A_BYTES = 128u * SPAN_A, B_BYTES = 128u * SPAN_B;
-    constexpr uint32_t A_STRIDE = up1024(A_BYTES), B_STRIDE = up1024(B_BYTES);
-    constexpr int NCOLS = CI < 32 ? 32 : CI;
-    constexpr uint32_t IDESC = idesc_bf16(128, CI, 1, 1);
+    constexpr int T = 128 / CI, ST = kWgradStages(CO);
+    constexpr uint32_t SPAN_X = CI * 2, SPAN_G = CO * 2;
+    constexpr uint32_t X_BYTES = 128u * SPAN_X, G_BYTES = 128u * SPAN_G;   // multiples of 1 KB
+    constexpr uint32_t STAGE = T * X_BYTES + G_BYTES;
+    constexpr int NCOLS = CO < 32 ? 32 : CO;
+    constexpr uint32_t IDESC = idesc_bf16(128, CO, 1, 1);
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint64_t bars[2 * kStages + 1];
+    __shared__ uint64_t bars[2 * ST + 1];
     __shared__ uint32_t tmem_slot;
-    unsigned char* abase = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);   // swizzle atoms: 1 KB aligned
-    unsigned char* bbase = abase + kStages * A_STRIDE;
+    unsigned char* base = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);   // swizzle atoms: 1 KB aligned
     const int tid = threadIdx.x, warp = tid >> 5;
-    uint64_t *full = bars, *empty = bars + kStages, *done = bars + 2 * kStages;
-    const int tap = blockIdx.y;
-    const int dd = tap / 9 - 1, dh = (tap / 3) % 3 - 1, dwo = tap % 3 - 1;
+    uint64_t *full = bars, *empty = bars + ST, *done = bars + 2 * ST;
+    const int tap0 = blockIdx.y * T, ntap = 27 - tap0 < T ? 27 - tap0 : T;
     const int64_t b0 = (int64_t)blockIdx.x * per_cta;
     const int nb = (int)((nbricks - b0) < per_cta ? (nbricks - b0) : per_cta);
-    const uint32_t tmem = tile_setup<NCOLS, kStages>(bars, &tmem_slot);
+    const uint32_t tmem = tile_setup<NCOLS, ST>(bars, &tmem_slot);
     int late = 0, issued = 0;
     if (tid == 0) {
         for (int t = 0; t < nb; ++t) {
-            const int s = t % kStages;
-            if (t >= kStages && !mbar_wait(&empty[s], (uint32_t)((t / kStages - 1) & 1), polls)) { late = 1; break; }
+            const int s = t % ST;
+            if (t >= ST && !mbar_wait(&empty[s], (uint32_t)((t / ST - 1) & 1), polls)) { late = 1; break; }
             const Brick bk = brick_of(g, b0 + t);
-            mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
-            tma_5d(abase + s * A_STRIDE, &gmap, &full[s], 0, bk.w0, bk.h0, bk.d0, bk.s);
-            tma_5d(bbase + s * B_STRIDE, &xmap, &full[s], 0, bk.w0 + dwo, bk.h0 + dh, bk.d0 + dd, bk.s);
+            mbar_expect_tx(&full[s], ntap * X_BYTES + G_BYTES);
+            tma_5d(base + s * STAGE + T * X_BYTES, &gmap, &full[s], 0, bk.w0, bk.h0, bk.d0, bk.s);
+            for (int u = 0; u < ntap; ++u) {
+                const int tap = tap0 + u;
+                tma_5d(base + s * STAGE + u * X_BYTES, &xmap, &full[s], 0, bk.w0 + tap % 3 - 1, bk.h0 + (tap / 3) % 3 - 1,
+                       bk.d0 + tap / 9 - 1, bk.s);
+            }
             issued = t + 1;
         }
     } else if (tid == 32) {
         for (int t = 0; t < nb; ++t) {
-            const int s = t % kStages;
-            if (!mbar_wait(&full[s], (uint32_t)((t / kStages) & 1), polls)) { late = 1; break; }
+            const int s = t % ST;
+            if (!mbar_wait(&full[s], (uint32_t)((t / ST) & 1), polls)) { late = 1; break; }
             fence_after();
-            const uint32_t a0 = smem_u32(abase + s * A_STRIDE), bb = smem_u32(bbase + s * B_STRIDE);
+            const uint32_t x0 = smem_u32(base + s * STAGE), g0 = x0 + T * X_BYTES;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-                mma(tmem, sdesc(a0 + kk * 16u * SPAN_A, 0u, 8 * SPAN_A, umma_layout(SPAN_A)),
-                    sdesc(bb + kk * 16u * SPAN_B, 0u, 8 * SPAN_B, umma_layout(SPAN_B)), IDESC,
+                mma(tmem, sdesc(x0 + kk * 16u * SPAN_X, X_BYTES, 8 * SPAN_X, umma_layout(SPAN_X)),
+                    sdesc(g0 + kk * 16u * SPAN_G, 0u, 8 * SPAN_G, umma_layout(SPAN_G)), IDESC,
                     (t > 0 || kk > 0) ? 1u : 0u);
             commit(&empty[s]);
         }
@@ -520,20 +571,20 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtens
     }
     late = __syncthreads_or(late);
     if (late && tid == 0) {
-        drain_copies<kStages>(full, issued);
+        drain_copies<ST>(full, issued);
         atomicOr(err, 1);
     }
     fence_after();
-    if (warp * 32 < CO && nb > 0) {                  // warp-uniform: TMEM lanes 32w.. hold co = 32w..
-        const int co = tid;
+    if (nb > 0) {                                    // TMEM lane tid: tap tap0 + tid / CI, input channel tid % CI
+        const int ci = tid % CI, tap = tap0 + tid / CI;
 #pragma unroll
-        for (int c0 = 0; c0 < CI; c0 += 16) {
+        for (int c0 = 0; c0 < CO; c0 += 16) {
             float acc[16];
             ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
-            if (late || co >= co_real) continue;
+            if (late || tap >= 27 || ci >= ci_real) continue;
 #pragma unroll
             for (int q = 0; q < 16; ++q)
-                if (c0 + q < ci_real) atomicAdd(&dw[((size_t)co * ci_real + c0 + q) * 27 + tap], acc[q]);
+                if (c0 + q < co_real) atomicAdd(&dw[((size_t)(c0 + q) * ci_real + ci) * 27 + tap], acc[q]);
         }
     }
     tile_release<NCOLS>(tmem);
@@ -617,124 +668,172 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(const __nv_bfloat16* __restr
 // ---- elementwise kernels -----------------------------------------------------
 #define GRID_STRIDE(i, n) for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
+// The elementwise kernels take eight channels of a voxel per thread (16-byte accesses;
+// C is a power of two times 8) and a row of a grid per CTA at a time, so that the
+// voxel's coordinates cost two divisions a row. 8 panels of 16 x 32 x 96: 383 -> 146 us
+// in a gradient's elementwise kernels.
+#define FOR_ROWS(r, rows) for (int64_t r = blockIdx.x; r < (rows); r += gridDim.x)
+#define FOR_ITEMS(i, n) for (int i = threadIdx.x; i < (n); i += blockDim.x)
+
 // fp32 [v][8] features -> bf16 [v][16] (channels 8..15 zero)
 __global__ void k_prep_input(const float* __restrict__ x, int64_t nv, __nv_bfloat16* __restrict__ out) {
-    GRID_STRIDE(i, nv * 16) {
-        const int64_t v = i >> 4;
-        const int c = (int)(i & 15);
-        out[i] = __float2bfloat16_rn(c < 8 ? x[v * 8 + c] : 0.f);
+    GRID_STRIDE(v, nv) {
+        store8(out + v * 16, load8(x + v * 8));
+        *reinterpret_cast<uint4*>(out + v * 16 + 8) = make_uint4(0u, 0u, 0u, 0u);
     }
+}
+
+// row (s, d, h) of grid g, and the first voxel of the fine (or coarse) row it touches
+struct Row { int64_t s; int d, h; };
+__device__ __forceinline__ Row row_of(int64_t r, int D, int H) {
+    const int64_t p = r / H, q = p / D;
+    return Row{q, (int)(p - q * D), (int)(r - p * H)};
+}
+// first voxel of the coarse row below a fine row of g
+__device__ __forceinline__ int64_t coarse_row(const Row& r, const Grid3& g) {
+    return ((r.s * (g.D / 2) + r.d / 2) * (g.H / 2) + r.h / 2) * (g.W / 2);
+}
+// sum of the eight fine children of a coarse cell, in the order d, h, w (row r of the
+// coarse grid, cell w), channels from `at` on; g is the fine grid
+template <class T>
+__device__ __forceinline__ V8 sum_children(const T* x, const Row& r, const Grid3& g, int w, int C, int at) {
+    V8 c[8], acc{};
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        c[q] = load8(x + (((r.s * g.D + 2 * r.d + (q >> 2)) * g.H + 2 * r.h + ((q >> 1) & 1)) * g.W + 2 * w + (q & 1)) * C + at);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc.v[k] += c[q].v[k];
+    return acc;
+}
+__device__ __forceinline__ void mask8(V8& x, const __nv_bfloat16* y) {
+    const V8 m = load8(y);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x.v[k] = m.v[k] > 0.f ? x.v[k] : 0.f;
 }
 
 // 2x2x2 average pool (grid g is the fine grid), C channels
 __global__ void k_pool(const __nv_bfloat16* __restrict__ x, Grid3 g, int C, __nv_bfloat16* __restrict__ out) {
-    const int D2 = g.D / 2, H2 = g.H / 2, W2 = g.W / 2;
-    const int64_t n = (int64_t)g.n * D2 * H2 * W2 * C;
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        int64_t v = i / C;
-        const int w = (int)(v % W2); v /= W2;
-        const int h = (int)(v % H2); v /= H2;
-        const int d = (int)(v % D2);
-        const int64_t s = v / D2;
-        float acc = 0.f;
-        for (int q = 0; q < 8; ++q) {
-            const int64_t f = ((s * g.D + 2 * d + (q >> 2)) * g.H + 2 * h + ((q >> 1) & 1)) * g.W + 2 * w + (q & 1);
-            acc += __bfloat162float(x[f * C + c]);
+    const int D2 = g.D / 2, H2 = g.H / 2, W2 = g.W / 2, G = C / 8;
+    FOR_ROWS(row, (int64_t)g.n * D2 * H2) {
+        const Row r = row_of(row, D2, H2);
+        FOR_ITEMS(i, W2 * G) {
+            const int w = i / G, at = i % G * 8;
+            V8 a = sum_children(x, r, g, w, C, at);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) a.v[k] *= 0.125f;
+            store8(out + (row * W2 + w) * C + at, a);
         }
-        out[i] = __float2bfloat16_rn(acc * 0.125f);
     }
 }
 
 // out = bf16(up2(a) + skip); g is the fine grid
 __global__ void k_up_add(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ skip, Grid3 g, int C,
                          __nv_bfloat16* __restrict__ out) {
-    const int64_t n = nvox(g) * C;
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        int64_t v = i / C;
-        const int w = (int)(v % g.W); v /= g.W;
-        const int h = (int)(v % g.H); v /= g.H;
-        const int d = (int)(v % g.D);
-        const int64_t s = v / g.D;
-        const int64_t cv = ((s * (g.D / 2) + d / 2) * (g.H / 2) + h / 2) * (g.W / 2) + w / 2;
-        out[i] = __float2bfloat16_rn(__bfloat162float(a[cv * C + c]) + __bfloat162float(skip[i]));
-    }
-}
-
-// G = bf16(dy * (y > 0)) for relu layers, bf16(dy) otherwise; channels C of
-// the padded layout (padded channels carry zeros)
-__global__ void k_relu_grad(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ y, int64_t n, int relu,
-                            __nv_bfloat16* __restrict__ g) {
-    GRID_STRIDE(i, n) {
-        float v = dy[i];
-        if (relu && !(__bfloat162float(y[i]) > 0.f)) v = 0.f;
-        g[i] = __float2bfloat16_rn(v);
-    }
-}
-
-// out[fine] = g[coarse] / 8 + skip[fine] (pool backward plus the skip gradient)
-__global__ void k_pool_back_add(const float* __restrict__ gc, const float* __restrict__ skip, Grid3 g, int C,
-                                float* __restrict__ out) {
-    const int64_t n = nvox(g) * C;
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        int64_t v = i / C;
-        const int w = (int)(v % g.W); v /= g.W;
-        const int h = (int)(v % g.H); v /= g.H;
-        const int d = (int)(v % g.D);
-        const int64_t s = v / g.D;
-        const int64_t cv = ((s * (g.D / 2) + d / 2) * (g.H / 2) + h / 2) * (g.W / 2) + w / 2;
-        out[i] = gc[cv * C + c] * 0.125f + (skip ? skip[i] : 0.f);
-    }
-}
-
-// out[coarse] = sum of the 8 fine children (up backward); g is the fine grid
-__global__ void k_up_back(const float* __restrict__ gf, Grid3 g, int C, float* __restrict__ out) {
-    const int D2 = g.D / 2, H2 = g.H / 2, W2 = g.W / 2;
-    const int64_t n = (int64_t)g.n * D2 * H2 * W2 * C;
-    GRID_STRIDE(i, n) {
-        const int c = (int)(i % C);
-        int64_t v = i / C;
-        const int w = (int)(v % W2); v /= W2;
-        const int h = (int)(v % H2); v /= H2;
-        const int d = (int)(v % D2);
-        const int64_t s = v / D2;
-        float acc = 0.f;
-        for (int q = 0; q < 8; ++q) {
-            const int64_t f = ((s * g.D + 2 * d + (q >> 2)) * g.H + 2 * h + ((q >> 1) & 1)) * g.W + 2 * w + (q & 1);
-            acc += gf[f * C + c];
+    const int G = C / 8;
+    FOR_ROWS(row, (int64_t)g.n * g.D * g.H) {
+        const int64_t cv = coarse_row(row_of(row, g.D, g.H), g);
+        FOR_ITEMS(i, g.W * G) {
+            const int w = i / G, at = i % G * 8;
+            const int64_t e = (row * g.W + w) * C + at;
+            const V8 u = load8(a + (cv + w / 2) * C + at);
+            V8 v = load8(skip + e);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v.v[k] = u.v[k] + v.v[k];
+            store8(out + e, v);
         }
-        out[i] = acc;
     }
 }
 
-// bias gradient: db[c] += sum_v g[v][c], c < creal
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ g, int64_t nv, int C, int creal, float* __restrict__ db) {
+// The gradient that reaches a relu layer's convolution is bf16(dy * (y > 0)), y the
+// layer's output; where dy has no other reader it is formed by the kernel that makes
+// dy (k_conv MODE 3, the two below, k_mse for the last layer, which has no relu).
+
+// dy[fine] = g[coarse] / 8 + skip[fine] (pool backward plus the skip gradient), masked
+__global__ void k_pool_back(const float* __restrict__ gc, const float* __restrict__ skip, const __nv_bfloat16* __restrict__ y,
+                            Grid3 g, int C, __nv_bfloat16* __restrict__ out) {
+    const int G = C / 8;
+    FOR_ROWS(row, (int64_t)g.n * g.D * g.H) {
+        const int64_t cv = coarse_row(row_of(row, g.D, g.H), g);
+        FOR_ITEMS(i, g.W * G) {
+            const int w = i / G, at = i % G * 8;
+            const int64_t e = (row * g.W + w) * C + at;
+            const V8 u = load8(gc + (cv + w / 2) * C + at);
+            V8 v = load8(skip + e);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v.v[k] = __fmaf_rn(u.v[k], 0.125f, v.v[k]);
+            mask8(v, y + e);
+            store8(out + e, v);
+        }
+    }
+}
+
+// dy[coarse] = sum of the 8 fine children (up backward), masked; g is the fine grid
+__global__ void k_up_back(const float* __restrict__ gf, const __nv_bfloat16* __restrict__ y, Grid3 g, int C,
+                          __nv_bfloat16* __restrict__ out) {
+    const int D2 = g.D / 2, H2 = g.H / 2, W2 = g.W / 2, G = C / 8;
+    FOR_ROWS(row, (int64_t)g.n * D2 * H2) {
+        const Row r = row_of(row, D2, H2);
+        FOR_ITEMS(i, W2 * G) {
+            const int w = i / G, at = i % G * 8;
+            const int64_t e = (row * W2 + w) * C + at;
+            V8 a = sum_children(gf, r, g, w, C, at);
+            mask8(a, y + e);
+            store8(out + e, a);
+        }
+    }
+}
+
+// bias gradient: db[c] += sum_v g[v][c], c < creal. A thread keeps its eight channels
+// (the stride is a multiple of C / 8), so that it adds in registers.
+__global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* __restrict__ g, int64_t nv, int C, int creal,
+                                                   float* __restrict__ db) {
     __shared__ float red[64];
-    for (int c = threadIdx.x; c < 64; c += blockDim.x) red[c] = 0.f;
+    if (threadIdx.x < 64) red[threadIdx.x] = 0.f;
     __syncthreads();
-    GRID_STRIDE(i, nv * C) {
-        const int c = (int)(i % C);
-        if (c < creal) atomicAdd(&red[c], __bfloat162float(g[i]));
+    const int G = C / 8, at = (int)(threadIdx.x % G) * 8;
+    float acc[8] = {};
+    constexpr int U = 4;   // loads in flight
+    const int64_t n = nv * G, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += U * step) {
+        V8 x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) x[u] = i + u * step < n ? load8(g + (i + u * step) * 8) : V8{};
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] += x[u].v[k];
     }
+    for (int o = 16; o >= G; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+    if ((threadIdx.x & 31) < G)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) atomicAdd(&red[at + k], acc[k]);
     __syncthreads();
-    for (int c = threadIdx.x; c < creal; c += blockDim.x) atomicAdd(&db[c], red[c]);
+    if (threadIdx.x < creal) atomicAdd(&db[threadIdx.x], red[threadIdx.x]);
 }
 
-// loss += sum (y - t)^2; dy = 2 (y - t) / count, written into the [v][16]
-// layout of the last layer (channel 0; the padded channels get 0)
+// loss += sum (y - t)^2; the last layer's gradient bf16(2 (y - t) / count) in its
+// [v][16] layout (channel 0; the padded channels get 0)
 __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ t, int64_t nv, float inv_count,
-                      float* __restrict__ dy16, double* __restrict__ loss) {
+                      __nv_bfloat16* __restrict__ g, double* __restrict__ loss) {
     double local = 0.0;
     GRID_STRIDE(v, nv) {
         const float d = y[v] - t[v];
         local += (double)d * d;
-        dy16[v * 16] = 2.f * d * inv_count;
-        for (int c = 1; c < 16; ++c) dy16[v * 16 + c] = 0.f;
+        store8(g + v * 16, V8{{2.f * d * inv_count}});
+        *reinterpret_cast<uint4*>(g + v * 16 + 8) = make_uint4(0u, 0u, 0u, 0u);
     }
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, local);
+    __shared__ double part[8];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {   // one atomic a CTA: all go to one address
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) local += part[w];
+        atomicAdd(loss, local);
+    }
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master parameters
@@ -769,6 +868,9 @@ __global__ void k_weights_bf16(const float* __restrict__ wm, int ci, int co, int
 #undef GRID_STRIDE
 
 // ---- launch helpers ----------------------------------------------------------
+inline unsigned row_grid(int64_t rows) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(rows, 152 * 32)); }
+// threads for the items of a row: whole warps, at most 256
+inline unsigned row_block(int64_t items) { return (unsigned)std::min<int64_t>(256, (items + 31) / 32 * 32); }
 inline unsigned ew_grid(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16)); }
 
 // cuTensorMapEncodeTiled, through the runtime's driver entry point
@@ -820,12 +922,10 @@ inline int64_t bricks(Grid3 g) {
     return (int64_t)g.n * ((g.D + tc::kBD - 1) / tc::kBD) * ((g.H + tc::kBH - 1) / tc::kBH) *
            ((g.W + tc::kBW - 1) / tc::kBW);
 }
-// dynamic shared memory of a ring with A and B tiles (plus 1 KB to align it)
-constexpr uint32_t ring_bytes(uint32_t a, uint32_t b) { return tc::kStages * (tc::up1024(a) + tc::up1024(b)) + 1024u; }
-
 template <int K, int N, int MODE>
 cudaError_t conv_tc_launch(const __nv_bfloat16* x, Grid3 g, const __nv_bfloat16* w, const float* bias, int relu,
-                           __nv_bfloat16* out16, float* out32, int32_t* err, int polls, cudaStream_t st) {
+                           __nv_bfloat16* out16, float* out32, const __nv_bfloat16* y, int32_t* err, int polls,
+                           cudaStream_t st) {
     // the weight ring, then the halo (3 x 18 x 10 voxels of K channels)
     constexpr uint32_t smem = tc::kConvStages * tc::up1024((uint32_t)N * K * 2) + 3u * (tc::kRowH + 2) * (tc::kRowW + 2) * K * 2 + 1024u;
     CUtensorMap wm;
@@ -834,14 +934,15 @@ cudaError_t conv_tc_launch(const __nv_bfloat16* x, Grid3 g, const __nv_bfloat16*
         e = cudaFuncSetAttribute(k_conv_tc<K, N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t blocks = (int64_t)g.n * g.D * ((g.H + tc::kRowH - 1) / tc::kRowH) * ((g.W + tc::kRowW - 1) / tc::kRowW);
-    k_conv_tc<K, N, MODE><<<(unsigned)blocks, 128, smem, st>>>(x, wm, g, bias, relu, out16, out32, err, polls);
+    k_conv_tc<K, N, MODE><<<(unsigned)blocks, 128, smem, st>>>(x, wm, g, bias, relu, out16, out32, y, err, polls);
     return cudaGetLastError();
 }
 
 template <int CO, int CI>
 cudaError_t wgrad_tc_launch(const __nv_bfloat16* gy, const __nv_bfloat16* x, Grid3 g, int co_real, int ci_real,
                             float* dw, int32_t* err, int polls, cudaStream_t st) {
-    constexpr uint32_t smem = ring_bytes(128u * CO * 2, 128u * CI * 2);
+    constexpr int T = 128 / CI;
+    constexpr uint32_t smem = kWgradStages(CO) * (T * 128u * CI * 2 + 128u * CO * 2) + 1024u;
     CUtensorMap gm, xm;
     cudaError_t e = act_map(&gm, gy, g, CO);
     if (e == cudaSuccess) e = act_map(&xm, x, g, CI);
@@ -850,7 +951,7 @@ cudaError_t wgrad_tc_launch(const __nv_bfloat16* gy, const __nv_bfloat16* x, Gri
     if (e != cudaSuccess) return e;
     const int64_t nb = bricks(g);
     const int per = (int)std::max<int64_t>(1, std::min<int64_t>(16, nb / 64));   // bricks (K = 128 each) per CTA
-    const dim3 grid((unsigned)((nb + per - 1) / per), 27);
+    const dim3 grid((unsigned)((nb + per - 1) / per), (27 + T - 1) / T);
     k_wgrad_tc<CO, CI><<<grid, 128, smem, st>>>(gm, xm, g, nb, per, co_real, ci_real, dw, err, polls);
     return cudaGetLastError();
 }
@@ -859,17 +960,20 @@ cudaError_t wgrad_tc_launch(const __nv_bfloat16* gy, const __nv_bfloat16* x, Gri
 template <int MODE>
 cudaError_t conv_launch(int kc, int nc, const __nv_bfloat16* x, Grid3 g, const __nv_bfloat16* w, const float* bias,
                         int relu, __nv_bfloat16* out16, float* out32, cudaStream_t st, bool tc = false,
-                        int32_t* err = nullptr, int polls = tc::kPolls) {
+                        int32_t* err = nullptr, int polls = tc::kPolls, const __nv_bfloat16* y = nullptr) {
     const int64_t nv = (int64_t)g.n * g.D * g.H * g.W;
     const unsigned blocks = (unsigned)((nv + 63) / 64);
 #define LCC_CONV(K, N)                                                                                   \
     if (kc == K && nc == N) {                                                                            \
-        if (tc) return conv_tc_launch<K, N, MODE>(x, g, w, bias, relu, out16, out32, err, polls, st);    \
-        k_conv<K, N, MODE><<<blocks, 128, 0, st>>>(x, g, w, bias, relu, out16, out32);                   \
+        if (tc) return conv_tc_launch<K, N, MODE>(x, g, w, bias, relu, out16, out32, y, err, polls, st); \
+        k_conv<K, N, MODE><<<blocks, 128, 0, st>>>(x, g, w, bias, relu, out16, out32, y);                \
         return cudaGetLastError();                                                                       \
     }
-    LCC_CONV(16, 16) LCC_CONV(16, 32) LCC_CONV(16, 64) LCC_CONV(32, 16) LCC_CONV(32, 32) LCC_CONV(32, 64)
-    LCC_CONV(64, 16) LCC_CONV(64, 32) LCC_CONV(64, 64)
+    LCC_CONV(16, 16) LCC_CONV(32, 32)
+    if constexpr (MODE != 3) {   // (mode 3: layers with as many channels in as out)
+        LCC_CONV(16, 32) LCC_CONV(16, 64) LCC_CONV(32, 16) LCC_CONV(32, 64) LCC_CONV(64, 16) LCC_CONV(64, 32)
+        LCC_CONV(64, 64)
+    }
 #undef LCC_CONV
     return cudaErrorInvalidValue;
 }
@@ -916,9 +1020,9 @@ struct falcon_lcc {
     int32_t* dflag = nullptr;         // device: a tcgen05 kernel's wait ran out
     int polls = tc::kPolls;           // the tcgen05 kernels' wait limit
     struct Acts {
-        bf16 *x0, *a1, *s0, *p0, *a2, *s1, *p1, *s2, *p2, *a5, *u2, *a6, *u1, *a7, *u0, *a8, *gb;
+        bf16 *x0, *a1, *s0, *p0, *a2, *s1, *p1, *s2, *p2, *a5, *u2, *a6, *u1, *a7, *u0, *a8, *gb, *gb2;
         float *y, *xin, *t;
-        float *dy9, *d_a8, *d_u0, *d_a7, *d_u1, *d_a6, *d_u2, *d_a5, *d_p2, *d_s2, *d_p1, *d_s1, *d_a2, *d_p0, *d_s0, *d_a1;
+        float *d_u0, *d_u1, *d_u2, *d_p2, *d_p1, *d_p0;
         double* loss;
     } A{};
     int fail(int c, const std::string& s) { err = s; return c; }
@@ -964,12 +1068,11 @@ cudaError_t ensure_shape(falcon_lcc* net, int n, int D, int H, int W) {
     b16(&A.a2, V1 * 32); b16(&A.s1, V1 * 32); b16(&A.p1, V2 * 32); b16(&A.s2, V2 * 64);
     b16(&A.p2, V3 * 64); b16(&A.a5, V3 * 64); b16(&A.u2, V2 * 64); b16(&A.a6, V2 * 32);
     b16(&A.u1, V1 * 32); b16(&A.a7, V1 * 16); b16(&A.u0, V0 * 16); b16(&A.a8, V0 * 16);
-    b16(&A.gb, V0 * 16);
+    // (the masked gradients: 16 channels of the finest grid hold every layer's)
+    b16(&A.gb, V0 * 16); b16(&A.gb2, V0 * 16);
     f32(&A.y, V0); f32(&A.xin, V0 * 8); f32(&A.t, V0);
-    f32(&A.dy9, V0 * 16); f32(&A.d_a8, V0 * 16); f32(&A.d_u0, V0 * 16); f32(&A.d_a7, V1 * 16);
-    f32(&A.d_u1, V1 * 32); f32(&A.d_a6, V2 * 32); f32(&A.d_u2, V2 * 64); f32(&A.d_a5, V3 * 64);
-    f32(&A.d_p2, V3 * 64); f32(&A.d_s2, V2 * 64); f32(&A.d_p1, V2 * 32); f32(&A.d_s1, V1 * 32);
-    f32(&A.d_a2, V1 * 32); f32(&A.d_p0, V1 * 16); f32(&A.d_s0, V0 * 16); f32(&A.d_a1, V0 * 16);
+    f32(&A.d_u0, V0 * 16); f32(&A.d_u1, V1 * 32); f32(&A.d_u2, V2 * 64);
+    f32(&A.d_p2, V3 * 64); f32(&A.d_p1, V2 * 32); f32(&A.d_p0, V1 * 16);
     if (e == cudaSuccess) e = net->alloc(&A.loss, 8, L);
     if (e == cudaSuccess) net->shape = s;
     return e;
@@ -981,17 +1084,17 @@ cudaError_t forward(falcon_lcc* net, cudaStream_t st) {
                 G3{G0.n, G0.D / 8, G0.H / 8, G0.W / 8};
     const int64_t V0 = (int64_t)G0.n * G0.D * G0.H * G0.W;
     cudaError_t e;
-    k_prep_input<<<ew_grid(V0 * 16), 256, 0, st>>>(A.xin, V0, A.x0);
+    k_prep_input<<<ew_grid(V0), 256, 0, st>>>(A.xin, V0, A.x0);
     auto conv = [&](int l, const bf16* x, Grid3 g, bf16* y) {
         return conv_launch<0>(pad16(kSpec[l].ci), pad16(kSpec[l].co), x, g, net->wf[l], net->p + net->boff[l],
                               kSpec[l].relu, y, nullptr, st, net->use_tc, net->dflag, net->polls);
     };
     auto pool = [&](const bf16* x, Grid3 g, int C, bf16* y) {
-        k_pool<<<ew_grid((int64_t)g.n * g.D * g.H * g.W * C / 8), 256, 0, st>>>(x, g, C, y);
+        k_pool<<<row_grid((int64_t)g.n * g.D / 2 * g.H / 2), row_block(g.W / 2 * C / 8), 0, st>>>(x, g, C, y);
         return cudaGetLastError();
     };
     auto upadd = [&](const bf16* a, const bf16* skip, Grid3 g, int C, bf16* y) {
-        k_up_add<<<ew_grid((int64_t)g.n * g.D * g.H * g.W * C), 256, 0, st>>>(a, skip, g, C, y);
+        k_up_add<<<row_grid((int64_t)g.n * g.D * g.H), row_block(g.W * C / 8), 0, st>>>(a, skip, g, C, y);
         return cudaGetLastError();
     };
     if ((e = conv(0, A.x0, G0, A.a1)) != cudaSuccess) return e;
@@ -1023,43 +1126,53 @@ cudaError_t backward(falcon_lcc* net, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(net->g, 0, (size_t)net->nparam * 4, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(A.loss, 0, 8, st);
     if (e != cudaSuccess) return e;
-    k_mse<<<ew_grid(V0), 256, 0, st>>>(A.y, A.t, V0, 1.f / (float)V0, A.dy9, A.loss);
-    // one layer: mask the upstream gradient, accumulate dW and db, propagate dX
-    auto back = [&](int l, const float* dy, const bf16* y, const bf16* x, Grid3 g, float* dx) -> cudaError_t {
+    k_mse<<<std::min(ew_grid(V0), 608u), 256, 0, st>>>(A.y, A.t, V0, 1.f / (float)V0, A.gb, A.loss);
+    // layer l, its masked gradient in A.gb: accumulate dW and db
+    auto weights = [&](int l, const bf16* x, Grid3 g) -> cudaError_t {
         const int ci = kSpec[l].ci, co = kSpec[l].co, cip = pad16(ci), cop = pad16(co);
-        const int64_t n = nv(g) * cop;
-        k_relu_grad<<<ew_grid(n), 256, 0, st>>>(dy, y, n, kSpec[l].relu ? 1 : 0, A.gb);
-        k_bias_grad<<<ew_grid(n), 256, 0, st>>>(A.gb, nv(g), cop, co, net->g + net->boff[l]);
-        cudaError_t e2 =
-            wgrad_launch(cop, cip, A.gb, x, g, co, ci, net->g + net->woff[l], st, net->use_tc, net->dflag, net->polls);
-        if (e2 != cudaSuccess || !dx) return e2;
-        return conv_launch<2>(cop, cip, A.gb, g, net->wb[l], nullptr, 0, nullptr, dx, st, net->use_tc, net->dflag,
-                              net->polls);
+        k_bias_grad<<<ew_grid(nv(g) * cop / 64), 256, 0, st>>>(A.gb, nv(g), cop, co, net->g + net->boff[l]);
+        return wgrad_launch(cop, cip, A.gb, x, g, co, ci, net->g + net->woff[l], st, net->use_tc, net->dflag, net->polls);
     };
-    auto upback = [&](const float* gf, Grid3 gfine, int C, float* out) {
-        k_up_back<<<ew_grid(nv(gfine) * C / 8), 256, 0, st>>>(gf, gfine, C, out);
+    // ... and propagate it: dX in FP32 ...
+    auto back = [&](int l, const bf16* x, Grid3 g, float* dx) -> cudaError_t {
+        cudaError_t e2 = weights(l, x, g);
+        if (e2 != cudaSuccess) return e2;
+        return conv_launch<2>(pad16(kSpec[l].co), pad16(kSpec[l].ci), A.gb, g, net->wb[l], nullptr, 0, nullptr, dx, st,
+                              net->use_tc, net->dflag, net->polls);
+    };
+    // ... or the masked gradient of the layer before, whose output is x (into A.gb)
+    auto back_masked = [&](int l, const bf16* x, Grid3 g) -> cudaError_t {
+        cudaError_t e2 = weights(l, x, g);
+        if (e2 != cudaSuccess) return e2;
+        e2 = conv_launch<3>(pad16(kSpec[l].co), pad16(kSpec[l].ci), A.gb, g, net->wb[l], nullptr, 0, A.gb2, nullptr, st,
+                            net->use_tc, net->dflag, net->polls, x);
+        std::swap(A.gb, A.gb2);
+        return e2;
+    };
+    auto upback = [&](const float* gf, const bf16* y, Grid3 g, int C) {
+        k_up_back<<<row_grid(nv(g) / g.W / 4), row_block(g.W / 2 * C / 8), 0, st>>>(gf, y, g, C, A.gb);
         return cudaGetLastError();
     };
-    auto poolback = [&](const float* gc, const float* skip, Grid3 gfine, int C, float* out) {
-        k_pool_back_add<<<ew_grid(nv(gfine) * C), 256, 0, st>>>(gc, skip, gfine, C, out);
+    auto poolback = [&](const float* gc, const float* skip, const bf16* y, Grid3 g, int C) {
+        k_pool_back<<<row_grid(nv(g) / g.W), row_block(g.W * C / 8), 0, st>>>(gc, skip, y, g, C, A.gb);
         return cudaGetLastError();
     };
-    if ((e = back(9, A.dy9, nullptr, A.a8, G0, A.d_a8)) != cudaSuccess) return e;
-    if ((e = back(8, A.d_a8, A.a8, A.u0, G0, A.d_u0)) != cudaSuccess) return e;
-    if ((e = upback(A.d_u0, G0, 16, A.d_a7)) != cudaSuccess) return e;
-    if ((e = back(7, A.d_a7, A.a7, A.u1, G1, A.d_u1)) != cudaSuccess) return e;
-    if ((e = upback(A.d_u1, G1, 32, A.d_a6)) != cudaSuccess) return e;
-    if ((e = back(6, A.d_a6, A.a6, A.u2, G2, A.d_u2)) != cudaSuccess) return e;
-    if ((e = upback(A.d_u2, G2, 64, A.d_a5)) != cudaSuccess) return e;
-    if ((e = back(5, A.d_a5, A.a5, A.p2, G3, A.d_p2)) != cudaSuccess) return e;
-    if ((e = poolback(A.d_p2, A.d_u2, G2, 64, A.d_s2)) != cudaSuccess) return e;
-    if ((e = back(4, A.d_s2, A.s2, A.p1, G2, A.d_p1)) != cudaSuccess) return e;
-    if ((e = poolback(A.d_p1, A.d_u1, G1, 32, A.d_s1)) != cudaSuccess) return e;
-    if ((e = back(3, A.d_s1, A.s1, A.a2, G1, A.d_a2)) != cudaSuccess) return e;
-    if ((e = back(2, A.d_a2, A.a2, A.p0, G1, A.d_p0)) != cudaSuccess) return e;
-    if ((e = poolback(A.d_p0, A.d_u0, G0, 16, A.d_s0)) != cudaSuccess) return e;
-    if ((e = back(1, A.d_s0, A.s0, A.a1, G0, A.d_a1)) != cudaSuccess) return e;
-    return back(0, A.d_a1, A.a1, A.x0, G0, nullptr);
+    if ((e = back_masked(9, A.a8, G0)) != cudaSuccess) return e;
+    if ((e = back(8, A.u0, G0, A.d_u0)) != cudaSuccess) return e;
+    if ((e = upback(A.d_u0, A.a7, G0, 16)) != cudaSuccess) return e;
+    if ((e = back(7, A.u1, G1, A.d_u1)) != cudaSuccess) return e;
+    if ((e = upback(A.d_u1, A.a6, G1, 32)) != cudaSuccess) return e;
+    if ((e = back(6, A.u2, G2, A.d_u2)) != cudaSuccess) return e;
+    if ((e = upback(A.d_u2, A.a5, G2, 64)) != cudaSuccess) return e;
+    if ((e = back(5, A.p2, G3, A.d_p2)) != cudaSuccess) return e;
+    if ((e = poolback(A.d_p2, A.d_u2, A.s2, G2, 64)) != cudaSuccess) return e;
+    if ((e = back(4, A.p1, G2, A.d_p1)) != cudaSuccess) return e;
+    if ((e = poolback(A.d_p1, A.d_u1, A.s1, G1, 32)) != cudaSuccess) return e;
+    if ((e = back_masked(3, A.a2, G1)) != cudaSuccess) return e;
+    if ((e = back(2, A.p0, G1, A.d_p0)) != cudaSuccess) return e;
+    if ((e = poolback(A.d_p0, A.d_u0, A.s0, G0, 16)) != cudaSuccess) return e;
+    if ((e = back_masked(1, A.a1, G0)) != cudaSuccess) return e;
+    return weights(0, A.x0, G0);
 }
 
 // a tcgen05 kernel's bounded wait that ran out (cleared when read)
