@@ -815,10 +815,13 @@ int setup_device(falcon_ctx* ctx) {
                     for (int t = 0; t < 3; ++t) c = 3 * c + (iw[3 * q + t] < 1e-12 ? 0 : iw[3 * q + t] > 1.0 - 1e-12 ? 1 : 2);
                     return c;
                 };
-                std::vector<std::vector<size_t>> bucket(4 * 27);
-                for (size_t q : ord) bucket[(size_t)cls(q)].push_back(q);
-                size_t n = 0;
-                for (const auto& bk : bucket) n = (size_t)(std::copy(bk.begin(), bk.end(), ord.begin() + (long)n) - ord.begin());
+                std::vector<uint8_t> c(ord.size());
+                std::array<size_t, 4 * 27 + 1> at{};
+                for (size_t q = 0; q < c.size(); ++q) ++at[(size_t)(c[q] = (uint8_t)cls(q)) + 1];
+                for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+                std::vector<size_t> by(ord.size());
+                for (size_t q : ord) by[at[c[q]]++] = q;
+                ord.swap(by);
             }
             std::vector<int32_t> d2(ord.size()), s2(ord.size());
             std::vector<double> w2(3 * ord.size()), r2(2 * ord.size());
