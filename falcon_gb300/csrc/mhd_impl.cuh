@@ -1054,6 +1054,16 @@ __device__ __forceinline__ void store_cell(float* p, size_t ncell, const float (
 // ---------------------------------------------------------------------------
 // Wave speed (3_6/ModWaveSpeed.f90:8-27), h/v_wave min-reduction
 // (3_6/ModTimeStep.f90:10-30) and the NaN scan of 3_6/ModCheck.f90:12-71.
+// |x| in FP32, truncated (0 below FP32's range, infinity above and for what is not finite)
+__device__ __forceinline__ float magnitude_f(double x) {
+    const int hi = __double2hiint(x) & 0x7fffffff, e = (hi >> 20) - 1023 + 127;
+    const unsigned m = __funnelshift_l((unsigned)__double2loint(x), (unsigned)hi, 3) & 0x7fffffu;
+    return e <= 0 ? 0.f : __int_as_float(e >= 255 ? 0x7f800000 : (int)(m | (unsigned)e << 23));
+}
+// FP64: the ratio takes about 100 FP64 instructions, and only the smallest counts. An
+// FP32 ratio, within 2e-6, first decides which cells can hold the minimum: those
+// within 1e-5 of the smallest of their CTA and of what other CTAs have committed so
+// far, and cells where FP32's range leaves it open. 442k cells: 67 -> 28 us.
 template <class T>
 __global__ void __launch_bounds__(256) k_cfl(const T* u, Geometry g, StepScalars* sc, StepDims d) {
     // R: the type the ratio and its block minimum are formed in (FP64 on the
@@ -1062,39 +1072,62 @@ __global__ void __launch_bounds__(256) k_cfl(const T* u, Geometry g, StepScalars
     const int nint = d.ni * d.nj * d.nk;
     const int b = blockIdx.y;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __shared__ R wmin[8];
+    __shared__ int wnan[8];
     R ratio = R(INFINITY);
     int nan = 0;
-    if (q < nint) {
-        const int i = q % d.ni + 2, j = (q / d.ni) % d.nj + 2, k = q / (d.ni * d.nj) + 2;
-        T x[NV];
-        load_cell<false>(u + Layout<T>::at(b, 0, ((size_t)k * d.njp + j) * d.nip + i, d.ncell), d.ncell, x);
+    const int i = q % d.ni + 2, j = (q / d.ni) % d.nj + 2, k = q / (d.ni * d.nj) + 2;
+    const T* Gi = gi_ptr<T>(g) + (size_t)b * GI_COUNT * d.nip + i;
+    const T* Gj = gj_ptr<T>(g) + (size_t)b * GJ_COUNT * d.njp + j;
+    const T* Gs = gs_ptr<T>(g) + (size_t)b * GS_COUNT;
+    T x[NV];
+    if (q < nint) load_cell<false>(u + Layout<T>::at(b, 0, ((size_t)k * d.njp + j) * d.nip + i, d.ncell), d.ncell, x);
+    if constexpr (Pol<T>::exact) {
+        float est = INFINITY;
+        bool open = false;
+        if (q < nint) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) nan |= abs_bits(x[v]) > 0x7ff0000000000000ull;
+            const float vr = magnitude_f(x[V_VR]), vt = magnitude_f(x[V_VT]), vp = magnitude_f(x[V_VP]);
+            const float br = magnitude_f(x[V_BR]), bt = magnitude_f(x[V_BT]), bp = magnitude_f(x[V_BP]);
+            const float r = magnitude_f(Gi[GI_R * d.nip]);
+            const float w = magnitude_f(Gi[GI_CS * d.nip]) + sqrtf(vr * vr + vt * vt + vp * vp) +
+                            sqrtf(br * br + bt * bt + bp * bp) / sqrtf(magnitude_f(Gi[GI_RHO0 * d.nip]));
+            const float h = fminf(fminf(magnitude_f(Gs[GS_DXI]), r * magnitude_f(Gs[GS_DXJ])),
+                                  r * magnitude_f(Gj[GJ_SIN * d.njp]) * magnitude_f(Gs[GS_DXK]));
+            // (squares that vanished or overflowed in FP32 are too small to count or out of this range)
+            open = !(w > 1e-10f && w < 1e15f && h > 1e-15f && h < 1e15f && magnitude_f(Gi[GI_RHO0 * d.nip]) > 1e-20f);
+            if (!open) est = h / w;
+        }
+        float m = est;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        __shared__ float west[8];
+        if (lane == 0) west[wid] = m;
+        __syncthreads();
+        m = (float)__longlong_as_double((long long)*(volatile unsigned long long*)&sc->min_ratio_bits);
+        for (int w2 = 0; w2 < (int)(blockDim.x >> 5); ++w2) m = fminf(m, west[w2]);
+        if (q < nint && (open || est <= m * 1.00001f)) {
+            // h_LLL = min(dxi, r*dxj, r*sin(theta)*dxk) (3_6/ModBlock.f90:416-425)
+            const T r = Gi[GI_R * d.nip];
+            const T h = fmin(fmin(Gs[GS_DXI], r * Gs[GS_DXJ]), r * Gj[GJ_SIN * d.njp] * Gs[GS_DXK]);
+            T w = Gi[GI_CS * d.nip] + sqrt(x[V_VR] * x[V_VR] + x[V_VT] * x[V_VT] + x[V_VP] * x[V_VP]);
+            w = w + sqrt(x[V_BR] * x[V_BR] + x[V_BT] * x[V_BT] + x[V_BP] * x[V_BP]) / sqrt(Gi[GI_RHO0 * d.nip]);
+            ratio = h / w;                 // the reference's h_LLL/v_wave
+        }
+    } else if (q < nint) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) nan |= (x[v] != x[v]);
-        const T* Gi = gi_ptr<T>(g) + (size_t)b * GI_COUNT * d.nip;
-        const T* Gj = gj_ptr<T>(g) + (size_t)b * GJ_COUNT * d.njp;
-        const T* Gs = gs_ptr<T>(g) + (size_t)b * GS_COUNT;
-        // h_LLL = min(dxi, r*dxj, r*sin(theta)*dxk) (3_6/ModBlock.f90:416-425)
-        const T r = Gi[GI_R * d.nip + i];
-        if constexpr (Pol<T>::exact) {
-            const T h = fmin(fmin(Gs[GS_DXI], r * Gs[GS_DXJ]), r * Gj[GJ_SIN * d.njp + j] * Gs[GS_DXK]);
-            T w = Gi[GI_CS * d.nip + i] + sqrt(x[V_VR] * x[V_VR] + x[V_VT] * x[V_VT] + x[V_VP] * x[V_VP]);
-            w = w + sqrt(x[V_BR] * x[V_BR] + x[V_BT] * x[V_BT] + x[V_BP] * x[V_BP]) / sqrt(Gi[GI_RHO0 * d.nip + i]);
-            ratio = h / w;                 // the reference's h_LLL/v_wave
-        } else {
-            ratio = cfl_ratio_f(cfl_sq3(x[V_VR], x[V_VT], x[V_VP]), cfl_sq3(x[V_BR], x[V_BT], x[V_BP]),
-                                Gi[GI_CS * d.nip + i], Gi[GI_RHO0 * d.nip + i], r, Gj[GJ_SIN * d.njp + j],
-                                Gs[GS_DXI], Gs[GS_DXJ], Gs[GS_DXK]);
-        }
-        if (ratio != ratio) { nan = 1; ratio = R(INFINITY); }
+        ratio = cfl_ratio_f(cfl_sq3(x[V_VR], x[V_VT], x[V_VP]), cfl_sq3(x[V_BR], x[V_BT], x[V_BP]), Gi[GI_CS * d.nip],
+                            Gi[GI_RHO0 * d.nip], Gi[GI_R * d.nip], Gj[GJ_SIN * d.njp], Gs[GS_DXI], Gs[GS_DXJ], Gs[GS_DXK]);
     }
+    if (ratio != ratio) { nan = 1; ratio = R(INFINITY); }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         ratio = fmin(ratio, __shfl_xor_sync(0xffffffffu, ratio, o));
         nan |= __shfl_xor_sync(0xffffffffu, nan, o);
     }
-    __shared__ R wmin[8];
-    __shared__ int wnan[8];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) { wmin[wid] = ratio; wnan[wid] = nan; }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1102,7 +1135,7 @@ __global__ void __launch_bounds__(256) k_cfl(const T* u, Geometry g, StepScalars
         int n = wnan[0];
         for (int w2 = 1; w2 < (int)(blockDim.x >> 5); ++w2) { m = fmin(m, wmin[w2]); n |= wnan[w2]; }
         // positive doubles order like their bit patterns
-        atomicMin(&sc->min_ratio_bits, (unsigned long long)__double_as_longlong((double)m));
+        if (m < R(INFINITY)) atomicMin(&sc->min_ratio_bits, (unsigned long long)__double_as_longlong((double)m));
         if (n) atomicOr(&sc->nan_flag, 1);
     }
 }
