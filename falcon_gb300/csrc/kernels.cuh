@@ -222,7 +222,7 @@ cudaError_t launch_psi_diffusion_mixed(const StepDims& d, const Geometry& g, con
 cudaError_t launch_psi_ghost_mixed(const StepDims& d, const GhostLists& gl, float* psi, cudaStream_t st);
 // diffusion of u into out: in place (out == u, push.tgt == nullptr) or out of
 // place with the regular faces pushed into out and the radial boundary ghost
-// columns copied (see k_diffusion)
+// columns copied (see k_march_quads)
 // One whole mixed step of 16^3 blocks as one persistent cooperative launch
 // (after the CFL minimum of u^n is formed): dt, four stages with their face
 // exchanges, diffusion into R2, the final exchange. bar: 8 device words

@@ -1556,7 +1556,7 @@ __global__ void __launch_bounds__(128) k_ghost_all(T* u, GhostLists G, int ncell
 // ---------------------------------------------------------------------------
 // GLM psi: artificial diffusion (3_6/ModDiffusion.f90:9-150 applies to every
 // variable, psi included) into psi_out = psi + dt/2 R_psi, the same formulas
-// as k_diffusion with psi read from global memory; wave speeds from u.
+// as the diffusion of u, with psi read from global memory; wave speeds from u.
 template <class T>
 __global__ void __launch_bounds__(256) k_psi_diffusion(const T* u, const T* psi, T* psi_out, Geometry g,
                                                        StepScalars* sc, StepDims d) {
