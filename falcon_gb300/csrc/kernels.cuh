@@ -163,6 +163,7 @@ struct PushTable {
 
 struct StepDims {
     int nblocks, ni, nj, nk, nip, njp, nkp, ncell;
+    int overlap;   // launch the mixed step's kernels with programmatic dependencies (launch_step)
 };
 
 // The u^n correction of the mixed path is stored for interior cells only,
