@@ -332,8 +332,10 @@ __global__ void k_ghost_ff(GhostFF H, const float* z, const float* scale, const 
 // beta A' p, so that beta, alpha and the update follow from one pass over the operator
 // and no halo of p is kept.
 template <int M>   // m, or 0
-__global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, const float* z, const float* scale, const float2* G,
-                                                   const float2* p, const float2* r, const float2* Ap, float2* w, Dots D) {
+__global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, const float* __restrict__ z, const float* scale,
+                                                   const float2* __restrict__ G, const float2* __restrict__ p,
+                                                   const float2* __restrict__ r, const float2* __restrict__ Ap,
+                                                   float2* __restrict__ w, Dots D) {
     const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d), pb = D.bprob[b];
     if (!D.active[pb]) return;
     const int m = M > 0 ? M : d.m0, mm = m * m;
@@ -341,6 +343,10 @@ __global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, const fl
     const float* zb = z + (size_t)b * d.nint;
     const float2* Gb = G + (size_t)b * 6 * mm;
     FFSum zw, za, pw, zr;
+    const float2 *__restrict__ Aii = A.Aii, *__restrict__ Ai = A.Ai, *__restrict__ Aj = A.Aj, *__restrict__ Ak = A.Ak;
+    // two cells at a time (the pointers' promise lets their loads overlap): a 6.3M-cell
+    // iteration 0.885 -> 0.845 ms; four at a time 0.870
+#pragma unroll 2
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
         const int i = c % m, row = c / m, j = row % m, k = row / m;
         const size_t fi = ((size_t)b * mm + row) * (m + 1) + i;
@@ -349,13 +355,13 @@ __global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, const fl
         auto inside = [&](int y) { return make_float2(zb[y] * s, 0.f); };
         const float2 zc = inside(c);
         FFSum y;
-        y.add(A.Aii[q], zc);
-        y.add(A.Ai[fi], i > 0 ? inside(c - 1) : Gb[row]);
-        y.add(A.Ai[fi + 1], i < m - 1 ? inside(c + 1) : Gb[mm + row]);
-        y.add(A.Aj[fj], j > 0 ? inside(c - m) : Gb[2 * mm + k * m + i]);
-        y.add(A.Aj[fj + m], j < m - 1 ? inside(c + m) : Gb[3 * mm + k * m + i]);
-        y.add(A.Ak[fk], k > 0 ? inside(c - mm) : Gb[4 * mm + j * m + i]);
-        y.add(A.Ak[fk + mm], k < m - 1 ? inside(c + mm) : Gb[5 * mm + j * m + i]);
+        y.add(Aii[q], zc);
+        y.add(Ai[fi], i > 0 ? inside(c - 1) : Gb[row]);
+        y.add(Ai[fi + 1], i < m - 1 ? inside(c + 1) : Gb[mm + row]);
+        y.add(Aj[fj], j > 0 ? inside(c - m) : Gb[2 * mm + k * m + i]);
+        y.add(Aj[fj + m], j < m - 1 ? inside(c + m) : Gb[3 * mm + k * m + i]);
+        y.add(Ak[fk], k > 0 ? inside(c - mm) : Gb[4 * mm + j * m + i]);
+        y.add(Ak[fk + mm], k < m - 1 ? inside(c + mm) : Gb[5 * mm + j * m + i]);
         const float2 wv = y.value();
         w[q] = wv;
         zw.add(zc, wv);
