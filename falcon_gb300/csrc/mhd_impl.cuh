@@ -14,14 +14,12 @@ namespace impl {
 template <class T> struct Pol;
 template <> struct Pol<double> {
     static constexpr bool exact = true;
-    __device__ static __forceinline__ double dv(double a, double b, double binv) { return a / b; }
     __device__ static __forceinline__ double mmthr() { return (double)1.e-30f; }
     __device__ static __forceinline__ double mmscale() { return 1.e10; }
     __device__ static __forceinline__ double ratio(double a, double b) { return a / b; }
 };
 template <> struct Pol<float> {
     static constexpr bool exact = false;
-    __device__ static __forceinline__ float dv(float a, float, float binv) { return a * binv; }
     __device__ static __forceinline__ float mmthr() { return 1.e-30f; }
     __device__ static __forceinline__ float mmscale() { return 1.e10f; }
     // limiter ratio: an approximate quotient is enough (0/0 still gives NaN -> phi = 0)
@@ -319,7 +317,6 @@ struct Shape {
     static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * NIP * sizeof(T);
     static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * NJP * sizeof(T);
     static constexpr size_t smem_stage = off_gs + GS_COUNT * sizeof(T);
-    static constexpr size_t smem_diff = smem_stage;
     // FP32 stage: as many CTAs per SM as the shared memory holds (228 KB per
     // SM, 1 KB reserved per CTA), so the register allocation must fit them
     // too (at least 32 registers a thread). FP64 keeps the compiler's choice.
@@ -352,17 +349,7 @@ __device__ __forceinline__ void load_geometry(const Geometry& g, int b, T* gi, T
         const double* Gd = g.gi + (size_t)b * GI_COUNT * S::NIP;
         for (int x = threadIdx.x; x < 2 * S::NIP; x += S::NT) {
             const double a = Gd[(x < S::NIP ? GI_A1 * S::NIP : GI_A2 * S::NIP - S::NIP) + x];
-            if constexpr (Pol<T>::exact) {
-                a12[x] = a;
-            } else {
-                // FP32 pairs (hi, lo) with hi + lo = a to about 2^-48:
-                // [a1 hi | a1 lo | a2 hi | a2 lo], NIP floats each
-                float* f = reinterpret_cast<float*>(a12);
-                const int c = x % S::NIP, which = x / S::NIP;
-                const float hi = (float)a;
-                f[(2 * which) * S::NIP + c] = hi;
-                f[(2 * which + 1) * S::NIP + c] = (float)(a - (double)hi);
-            }
+            a12[x] = a;
         }
     }
 }
