@@ -52,11 +52,6 @@ __device__ __forceinline__ float2 half_slope2(float2 ul, float2 u, float2 ur) {
 // saturates to [0, 1] without clipping phi from above; one saturating FMA forms it,
 // 0/0 as 0. The quotient is num times the approximate reciprocal of den, which flushes
 // a denormal den: there the saturated phi keeps the flux as small as num.
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float eighth_phi(float r) { return __saturatef(__fmaf_rn(r, 0.25f, -0.125f)); }
 __device__ __forceinline__ float face_flux(float fl, float fr, float hL, float hR, float cc) {
     const float num = __fsub_rn(__fsub_rn(__fsub_rn(fr, hR), fl), hL);

@@ -1,0 +1,30 @@
+"""The FP64 kernels' short forms (falcon_gb300/csrc/exact64.cuh) compiled for the CPU:
+each gives the bits of the reference's expression."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def _compile(tmp, *flags):
+    exe = str(tmp / "exact64_host")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", *flags, os.path.join(HERE, "exact64_host.cpp"), "-o", exe],
+                   check=True)
+    return exe
+
+
+def _run(*cmd):
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.fixture(scope="module")
+def exe(tmp_path_factory):
+    return _compile(tmp_path_factory.mktemp("exact64"))
+
+
+@pytest.mark.parametrize("form", ["slopes", "fluxes", "quotients", "limiters", "ghosts"])
+def test_short_form_is_the_expression(exe, form):
+    _run(exe, form, "2000000", "7")
