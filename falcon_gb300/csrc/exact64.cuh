@@ -227,7 +227,9 @@ __device__ __forceinline__ bool mid_range(double a) { return (unsigned)(exp_fiel
 // a whole number of units that does not depend on the others, as long as the binade
 // does not end within 2^20 units: the three products with 1 - D 2^-53, the sum of the
 // terms before the large corner (the corners below it along its `up` axes), and each
-// term after it. Corners off along two or three axes add less than half a unit.
+// term after it. Corners off along two or three axes are left out: added after the
+// large corner they move nothing, being less than half a unit; before it (`up` set
+// along j or k) they are part of the sum that is rounded, and count as its error.
 struct NearEntry {
     unsigned D[3], up;
     int at, step[3];   // the large corner from the base, and from it to its neighbours
@@ -255,13 +257,16 @@ __device__ __forceinline__ double ghost_near(const double* f, const double* w, c
 #pragma unroll
     for (int q = 0; q < 3; ++q) v[q] = fc[n.step[q]];
     const int s01 = n.step[0] + n.step[1], s2 = n.step[2];
-    // the corners off along several axes: weights below 2^-75, so 2^20 |a| is small enough
+    // the corners off along several axes: weights up to kNearD^2 2^-106 = 2^-80. With
+    // exponents up to `rise` above a's their sum is below 2^(rise - 25) units of a's last place
     const int hx = max(max(__double2hiint(fc[s01]) & 0x7ff00000, __double2hiint(fc[n.step[0] + s2]) & 0x7ff00000),
                        max(__double2hiint(fc[n.step[1] + s2]) & 0x7ff00000, __double2hiint(fc[s01 + s2]) & 0x7ff00000));
     const unsigned Mt = top_bits(a);
-    bool ok = mid_range(a) & (Mt - 0x80000001u < 0x7ffffffeu) & (hx - (__double2hiint(a) & 0x7ff00000) < (20 << 20));
+    const int rise = (hx - (__double2hiint(a) & 0x7ff00000)) >> 20;
+    bool ok = mid_range(a) & (Mt - 0x80000001u < 0x7ffffffeu) & (rise < 20);
     int sum = 0, k;
-    float pre = 0.f, pre_m = 0.f, all_m = 0.f;
+    // (pre_m counts 2^-21 of itself as error)
+    float pre = 0.f, pre_m = n.up > 1u ? __int_as_float((127 - 4 + max(rise, -100)) << 23) : 0.f, all_m = 0.f;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         ok &= near_units(Mt, n.D[q], k);

@@ -130,6 +130,25 @@ static void ghosts() {
           : rng() % 64 ? sym() : bits<double>((uint64_t)rng());
     ghost(v, w);
 }
+// all three axes near, with factors over the whole accepted range, and corners far
+// above the large one: those off along several axes reach its rounding
+static void far_ghosts() {
+    double v[8], w[3];
+    const int large = (int)(rng() % 8);
+    for (int a = 0; a < 3; ++a) {
+        const double e = (double)(1 + rng() % kNearD) * 0x1p-53;
+        w[a] = large >> a & 1 ? 1.0 - e : e;
+    }
+    for (int c = 0; c < 8; ++c) v[c] = c == large ? 1.0 + unit() : wide(-3, 21);
+    ghost(v, w);
+}
+// a sum within 2^-9 of a unit of the middle between two numbers
+static void far_ghost_case() {
+    const double w[3] = {0x1.ffffffffff82p-1, 0x1.fffffffffff1p-1, 0.0};
+    const double v[8] = {-0x1.ffffffffffffcp+30, -0x1.aaaa34ep+6,      0x1.0000000000002p+5,  -0x1.4688ff63e2b77p+11,
+                         0x1.0000000000002p+21,  -0x1.e5396d33293fep+26, 0x1.ffffffffffffdp+20, -0x1.cc5025p+34};
+    ghost(v, w);
+}
 
 int main(int argc, char** argv) {
     const char* form = argc > 1 ? argv[1] : "";
@@ -141,6 +160,8 @@ int main(int argc, char** argv) {
         else if (!std::strcmp(form, "quotients")) quotients();
         else if (!std::strcmp(form, "limiters")) limiters();
         else if (!std::strcmp(form, "ghosts")) ghosts();
+        else if (!std::strcmp(form, "far_ghosts")) far_ghosts();
+        else if (!std::strcmp(form, "far_ghost_case")) far_ghost_case();
         else return 2;
     }
     std::printf("%s: %ld of %ld differ\n", form, bad, n);

@@ -28,3 +28,10 @@ def exe(tmp_path_factory):
 @pytest.mark.parametrize("form", ["slopes", "fluxes", "quotients", "limiters", "ghosts"])
 def test_short_form_is_the_expression(exe, form):
     _run(exe, form, "2000000", "7")
+
+
+@pytest.mark.parametrize("form,count", [("far_ghost_case", 1), ("far_ghosts", 5000000)])
+def test_ghost_with_large_corners_off_along_several_axes(exe, form, count):
+    """Corners off along several axes weigh up to 2^-80, and those that the reference adds
+    before the large corner take part in its rounding."""
+    _run(exe, form, str(count), "11")
