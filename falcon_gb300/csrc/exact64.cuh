@@ -98,14 +98,16 @@ __device__ __forceinline__ double quarter_phi(unsigned long long an, unsigned lo
     long long R = (long long)(((an ^ ad) >> 52 & 1ull) ? A : A << 1) - (long long)B;   // N; exponents equal or one apart
     // 2^k / B for the digits: y = 2^52 / B from its leading 24 bits
     const float y = rcp_approx(__int_as_float(0x3f800000 | (int)((B >> 29) & 0x7fffffull)));
-    auto digit = [&](int bits) {   // round(R 2^bits / B), off by at most 1; R becomes the remainder
+    // round(R 2^bits / B), off by at most 1; R becomes the remainder (both products leave 64
+    // bits, their difference does not: modulo 2^64)
+    auto digit = [&](int bits) {
         const float t = __fmul_rn(__fmul_rn((float)(int)(R >> 22), y), __int_as_float((127 + bits - 30) << 23));
         const int k = __float_as_int(__fadd_rn(t, 12582912.f)) - 0x4B400000;
-        R = (R << bits) - (long long)k * (long long)B;
+        R = (long long)(((unsigned long long)R << bits) - (unsigned long long)(long long)k * B);
         return (long long)k;
     };
-    long long K = digit(18) << 34;
-    K += digit(17) << 17;
+    long long K = digit(18) * (1ll << 34);
+    K += digit(17) * (1ll << 17);
     K += digit(17);
     K += (2 * R > (long long)B) - (2 * R < -(long long)B);
     // K as a double: 2^52 + K less 2^52; K = 0 and K = 2^52 keep the form's values
@@ -216,7 +218,7 @@ __device__ __forceinline__ float small_units(double f, float W, double a, int& d
 // round(x) for an x off by less than 2^-21 m (m >= |x|); false if that leaves it open
 __device__ __forceinline__ bool round_units(float x, float m, int& k) {
     const float r = __fadd_rn(x, 12582912.f);   // ulp 1: the integer in its low bits
-    k = __float_as_int(r) - 0x4B400000;
+    k = (int)((unsigned)__float_as_int(r) - 0x4B400000u);
     return __fmaf_rn(m, 4.7683716e-7f, fabsf(__fsub_rn(x, __fsub_rn(r, 12582912.f)))) < 0.499999f;
 }
 // exponents in the middle of the range: no underflow in the products, and what is
@@ -264,13 +266,14 @@ __device__ __forceinline__ double ghost_near(const double* f, const double* w, c
     const unsigned Mt = top_bits(a);
     const int rise = (hx - (__double2hiint(a) & 0x7ff00000)) >> 20;
     bool ok = mid_range(a) & (Mt - 0x80000001u < 0x7ffffffeu) & (rise < 20);
-    int sum = 0, k;
+    unsigned sum = 0u;   // (modulo 2^32: a term out of range fails a test below)
+    int k;
     // (pre_m counts 2^-21 of itself as error)
-    float pre = 0.f, pre_m = n.up > 1u ? __int_as_float((127 - 4 + max(rise, -100)) << 23) : 0.f, all_m = 0.f;
+    float pre = 0.f, pre_m = n.up > 1u ? __int_as_float((127 - 4 + min(max(rise, -100), 20)) << 23) : 0.f, all_m = 0.f;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         ok &= near_units(Mt, n.D[q], k);
-        sum -= k;
+        sum -= (unsigned)k;
         int d;
         const float y = small_units(v[q], n.W[q], a, d);
         ok &= d < 60;
@@ -279,17 +282,17 @@ __device__ __forceinline__ double ghost_near(const double* f, const double* w, c
         pre += before ? y : 0.f;
         pre_m += before ? fabsf(y) : 0.f;
         ok &= round_units(before ? 0.f : y, fabsf(y), k);
-        sum += k;
+        sum += (unsigned)k;
     }
     ok &= round_units(pre, pre_m, k) & (all_m < 131072.f);
-    sum += k;
-    return ok ? __longlong_as_double(__double_as_longlong(a) + (long long)sum) : ghost_plain(f, w, nip, pl);
+    sum += (unsigned)k;
+    return ok ? __longlong_as_double(__double_as_longlong(a) + (long long)(int)sum) : ghost_plain(f, w, nip, pl);
 }
 
 // Entries near along some axes. The main corners (all near factors large) are formed
 // in FP64 along the other axes; the rest are small terms, rounded one by one.
 __device__ __forceinline__ double move_units(double a, int k, bool& ok) {
-    const long long r = __double_as_longlong(a) + (long long)k;
+    const long long r = (long long)((unsigned long long)__double_as_longlong(a) + (unsigned long long)(long long)k);
     ok &= (((int)(r >> 32) ^ __double2hiint(a)) >> 20 == 0) & (((unsigned long long)r << 12) != 0ull);   // inside the binade
     return __longlong_as_double(r);
 }

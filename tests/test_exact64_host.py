@@ -35,3 +35,10 @@ def test_ghost_with_large_corners_off_along_several_axes(exe, form, count):
     """Corners off along several axes weigh up to 2^-80, and those that the reference adds
     before the large corner take part in its rounding."""
     _run(exe, form, str(count), "11")
+
+
+@pytest.mark.parametrize("form", ["slopes", "fluxes", "quotients", "limiters", "ghosts"])
+def test_short_forms_have_no_undefined_arithmetic(tmp_path, form):
+    """Signed overflow and shifts of negative values end the program."""
+    exe = _compile(tmp_path, "-fsanitize=undefined", "-fsanitize-undefined-trap-on-error")
+    _run(exe, form, "200000", "3")
