@@ -75,7 +75,7 @@ EXPORTS = (
     "falcon_set_background", "falcon_solver_set_operator", "falcon_solver_set_magnetogram",
     "falcon_solver_magnetogram", "falcon_solver_set_guess", "falcon_solver_block_ranges",
     "falcon_solver_block_flags", "falcon_solver_magnetogram_sources", "falcon_solver_vcycle_op",
-    "falcon_solver_tuning", "falcon_solver_set_tile", "falcon_shard_ranges", "falcon_shard_plan",
+    "falcon_solver_tuning", "falcon_solver_set_tile", "falcon_solver_coarse_form", "falcon_shard_ranges", "falcon_shard_plan",
     "falcon_set_shard", "falcon_shard_counts", "falcon_shard_pack", "falcon_shard_unpack",
     "falcon_shard_min_ratio", "falcon_shard_set_min_ratio", "falcon_lcc_set_tensor_path", "falcon_set_tuning",
     "falcon_set_step_mode", "falcon_lcc_set_wait_limit",

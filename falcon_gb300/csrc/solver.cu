@@ -895,6 +895,14 @@ cudaError_t coarse_sweeps(falcon_solver* sv, int sweeps, float* zout) {
                                          sv->coarse_slots},
                               (const float*)L.r, zout);
 }
+// A kernel's opt-ins hold for every solver of the process, whichever set them last: all
+// set the same, the most shared memory that a plan may ask for.
+constexpr size_t kCoarseSmemMax = 232448;
+cudaError_t allow_coarse(CoarseKernel kern, int cluster) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmemMax);
+    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
 // Whether the coarsest level's sweeps run as one launch, and with how many CTAs
 // per problem: the smallest cluster that holds the largest problem at two
 // cells per thread and colour, one cell where that fits too. Batches whose
@@ -924,8 +932,7 @@ int plan_coarse(falcon_solver* sv, const std::vector<int32_t>& ghost, const std:
             cudaLaunchAttribute at[1];
             coarse_config(sv, &cfg, at);
             cfg.dynamicSmemBytes = coarse_smem(r, 4 * kCoarseThreads);
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
-            if (e == cudaSuccess && c > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            cudaError_t e = allow_coarse(kern, c);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
             if (e != cudaSuccess || n < 1) {
                 cudaGetLastError();
@@ -1025,10 +1032,9 @@ int plan_coarse(falcon_solver* sv, const std::vector<int32_t>& ghost, const std:
     sv->coarse_r = R;
     sv->coarse_slots = slots;
     const CoarseKernel kern = coarse_kernel(m, R, cl > 1);
-    cudaError_t e = coarse_smem(R, slots) > 232448 || 2 * R * kCoarseThreads + 1 + slots > 65536 ? cudaErrorInvalidValue
-                                                   : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                                          (int)coarse_smem(R, slots));
-    if (e == cudaSuccess && cl > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaError_t e = coarse_smem(R, slots) > kCoarseSmemMax || 2 * R * kCoarseThreads + 1 + slots > 65536
+                        ? cudaErrorInvalidValue
+                        : allow_coarse(kern, cl);
     int n = 1;
     if (e == cudaSuccess && cl > 1) {
         cudaLaunchConfig_t cfg;
@@ -1861,6 +1867,14 @@ int falcon_solver_tuning(const falcon_solver* sv, int32_t* tile, double* ms_per_
     tile[1] = sv->tile_tpb;
     tile[2] = sv->tuned ? 1 : 0;
     if (ms_per_iteration) *ms_per_iteration = sv->tuned_ms;
+    return FALCON_OK;
+}
+
+int falcon_solver_coarse_form(const falcon_solver* sv, int32_t* form) {
+    if (!sv || !form) return FALCON_ERR_INVALID_ARG;
+    form[0] = sv->coarse_cluster;
+    form[1] = sv->coarse_cluster ? sv->coarse_r : 0;
+    form[2] = sv->coarse_cluster ? sv->coarse_slots : 0;
     return FALCON_OK;
 }
 

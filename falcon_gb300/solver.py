@@ -43,7 +43,8 @@ _SYMS = ("falcon_solver_create", "falcon_solver_last_error", "falcon_solver_info
          "falcon_solver_set_smoothing", "falcon_solver_problem_residuals", "falcon_solver_set_operator",
          "falcon_solver_set_magnetogram", "falcon_solver_magnetogram", "falcon_solver_set_guess",
          "falcon_solver_block_ranges", "falcon_solver_block_flags", "falcon_solver_magnetogram_sources",
-         "falcon_solver_vcycle_op", "falcon_solver_tuning", "falcon_solver_set_tile")
+         "falcon_solver_vcycle_op", "falcon_solver_tuning", "falcon_solver_set_tile",
+         "falcon_solver_coarse_form")
 
 
 def _ptr(a):
@@ -218,6 +219,12 @@ class Solver:
 
     def set_tile(self, cells_per_cta, threads_per_cta):
         self._ck(self.L.falcon_solver_set_tile(self.h, C.c_int32(cells_per_cta), C.c_int32(threads_per_cta)))
+
+    def coarse_form(self):
+        """How the coarsest level's sweeps run (see falcon_solver_coarse_form)."""
+        t = (C.c_int32 * 3)()
+        self._ck(self.L.falcon_solver_coarse_form(self.h, t))
+        return {"ctas": t[0], "cells": t[1], "slots": t[2]}
 
     def block_ranges(self):
         out = np.zeros((self.nblocks, 3, 2))

@@ -510,6 +510,11 @@ int  falcon_solver_magnetogram(const falcon_solver* sv, double* br);
  * falcon_solver_set_tile fixes the shape instead (no autotuning). */
 int  falcon_solver_tuning(const falcon_solver* sv, int32_t* tile, double* ms_per_iteration);
 int  falcon_solver_set_tile(falcon_solver* sv, int32_t cells_per_cta, int32_t threads_per_cta);
+/* How the coarsest level's sweeps run when a V-cycle makes more than two of them
+ * there: form[0] CTAs per problem of the one launch that makes them all (0: a
+ * launch per half sweep), form[1] cells of each colour per thread, form[2] ghosts
+ * that a CTA gathers per half sweep, at most */
+int  falcon_solver_coarse_form(const falcon_solver* sv, int32_t* form);
 /* Verification: one kernel of the V-cycle on host arrays at `level`, eagerly
  * and synchronously (as falcon_step_phase is for the step). Arrays are FP32,
  * interior cells [block][k][j][i] of their level.
