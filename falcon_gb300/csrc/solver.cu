@@ -277,12 +277,24 @@ struct FFSum {
     __device__ __forceinline__ float2 value() const { return ff_quick(s, e); }
 };
 
-// Ghosts of z (FP32, scaled by the problem's sA) at the finest level as FF
-// values, one slot per ghost in the layout of VLevel::ghost. A copied cell's map
-// weights are 0 or 1 up to eps (about 1e-14, see kSnapFF): the ghost is z0 + sum of eps_d
-// (z_d - z0) over the three directions, z_d one cell on (eps > 0) or back (eps
-// < 0); second-order terms are below 2^-64. Other ghosts sum eight cells with
-// FF weights.
+// The search's z: the preconditioner's FP32 output scaled by the problem's sA, or
+// without a preconditioner the residual itself, all of its bits.
+struct Z32 {
+    const float *__restrict__ z, *__restrict__ scale;
+    __device__ __forceinline__ float of_problem(int pb) const { return scale[pb]; }
+    __device__ __forceinline__ float2 operator()(size_t q, float s) const { return make_float2(z[q] * s, 0.f); }
+};
+struct ZFF {
+    const float2* r;
+    __device__ __forceinline__ float of_problem(int) const { return 1.f; }
+    __device__ __forceinline__ float2 operator()(size_t q, float) const { return r[q]; }
+};
+
+// Ghosts of z at the finest level as FF values, one slot per ghost in the layout of
+// VLevel::ghost. A copied cell's map weights are 0 or 1 up to eps (about 1e-14, see
+// kSnapFF): the ghost is z0 + sum of eps_d (z_d - z0) over the three directions, z_d
+// one cell on (eps > 0) or back (eps < 0); second-order terms are below 2^-64. Other
+// ghosts sum eight cells with FF weights.
 struct GhostFF {
     const int32_t* ghost;   // [slot] >= 0 source cell, -1 none, <= -2 entry -(v + 2)
     const float* eps;       // [slot][3]
@@ -292,55 +304,56 @@ struct GhostFF {
     int m;
     int64_t n;              // slots
 };
-__global__ void k_ghost_ff(GhostFF H, const float* z, const float* scale, const int32_t* bprob, float2* G) {
+template <class Z>
+__global__ void k_ghost_ff(GhostFF H, Z z, const int32_t* bprob, float2* G) {
     const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= H.n) return;
     const int d = H.ghost[x];
     if (d == -1) return;   // stays 0
     const int m = H.m, mm = m * m;
-    const float s = scale ? scale[bprob[x / (6 * mm)]] : 1.f;
+    const float s = z.of_problem(bprob[x / (6 * mm)]);
     if (d >= 0) {
-        const float z0 = z[d] * s;
+        const float2 z0 = z((size_t)d, s);
         float lo = 0.f;
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const float ep = H.eps[3 * x + q];
             const int st = q == 0 ? 1 : q == 1 ? m : mm;
-            if (ep != 0.f) lo = fmaf(fabsf(ep), z[ep > 0.f ? d + st : d - st] * s - z0, lo);
+            if (ep != 0.f) lo = fmaf(fabsf(ep), z((size_t)(ep > 0.f ? d + st : d - st), s).x - z0.x, lo);
         }
-        G[x] = ff_two_sum(z0, lo);
+        const float2 t = ff_two_sum(z0.x, lo);
+        G[x] = ff_quick(t.x, t.y + z0.y);
         return;
     }
     const int e = -(d + 2), cd = H.code[e];
     const int a = (cd & 1) ? 1 : 0, b = (cd & 2) ? m : 0, c = (cd & 4) ? mm : 0;
     const int off[8] = {0, a, b, c, a + b, b + c, a + c, a + b + c};
-    const float* f = z + H.src[e];
+    const size_t f = (size_t)H.src[e];
     const float4* w = reinterpret_cast<const float4*>(H.w8 + 8 * (size_t)e);
     FFSum y;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
         const float4 w2 = w[t];
-        y.add(make_float2(w2.x, w2.y), make_float2(f[off[2 * t]] * s, 0.f));
-        y.add(make_float2(w2.z, w2.w), make_float2(f[off[2 * t + 1]] * s, 0.f));
+        y.add(make_float2(w2.x, w2.y), z(f + off[2 * t], s));
+        y.add(make_float2(w2.z, w2.w), z(f + off[2 * t + 1], s));
     }
     G[x] = y.value();
 }
 
 // w = A' z, the reference's operand order, with the four products that the
-// step needs: z.w, z.Ap, p.w, z.r. z is the preconditioner's FP32 output (or
-// the residual's FP32 part): the direction is p' = z + beta p and A' p' = w +
+// step needs: z.w, z.Ap, p.w, z.r. The direction is p' = z + beta p and A' p' = w +
 // beta A' p, so that beta, alpha and the update follow from one pass over the operator
 // and no halo of p is kept.
-template <int M>   // m, or 0
-__global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, const float* __restrict__ z, const float* scale,
-                                                   const float2* __restrict__ G, const float2* __restrict__ p,
+template <int M, class Z>   // M: m, or 0
+__global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, Z z, const float2* __restrict__ G,
+                                                   const float2* __restrict__ p,
                                                    const float2* __restrict__ r, const float2* __restrict__ Ap,
                                                    float2* __restrict__ w, Dots D) {
     const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d), pb = D.bprob[b];
     if (!D.active[pb]) return;
     const int m = M > 0 ? M : d.m0, mm = m * m;
-    const float s = scale ? scale[pb] : 1.f;
-    const float* zb = z + (size_t)b * d.nint;
+    const float s = z.of_problem(pb);
+    const size_t zb = (size_t)b * d.nint;
     const float2* Gb = G + (size_t)b * 6 * mm;
     FFSum zw, za, pw, zr;
     const float2 *__restrict__ Aii = A.Aii, *__restrict__ Ai = A.Ai, *__restrict__ Aj = A.Aj, *__restrict__ Ak = A.Ak;
@@ -352,7 +365,7 @@ __global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, const fl
         const size_t fi = ((size_t)b * mm + row) * (m + 1) + i;
         const size_t fj = ((size_t)b * m * (m + 1) + (size_t)k * (m + 1) + j) * m + i;
         const size_t fk = ((size_t)b * (m + 1) * m + row) * m + i, q = (size_t)b * d.nint + c;
-        auto inside = [&](int y) { return make_float2(zb[y] * s, 0.f); };
+        auto inside = [&](int y) { return z(zb + y, s); };
         const float2 zc = inside(c);
         FFSum y;
         y.add(Aii[q], zc);
@@ -388,7 +401,8 @@ __device__ __forceinline__ StepFF step_ff(const Dots& D, int pb, int restart) {
 
 // p = z + beta p; Ap = w + beta Ap; x += alpha p; r -= alpha Ap; rr += r.r; rf =
 // hi(r), the V-cycle's input
-__global__ void __launch_bounds__(512) k_step_ff(LevelDims d, const float* z, const float* scale, const float2* w, float2* x,
+template <class Z>
+__global__ void __launch_bounds__(512) k_step_ff(LevelDims d, Z z, const float2* w, float2* x,
                                                  float2* p, float2* r, float2* Ap, float* rf, Dots D, int restart) {
     const int b = cell_block(d), c0 = cell_first(d), c1 = cell_end(d), pb = D.bprob[b];
     if (!D.active[pb]) return;
@@ -400,11 +414,11 @@ __global__ void __launch_bounds__(512) k_step_ff(LevelDims d, const float* z, co
     }
     __syncthreads();
     const float2 al = ab[0], be = ab[1], nal = ff_neg(al);
-    const float s = scale ? scale[pb] : 1.f;
+    const float s = z.of_problem(pb);
     FFSum rr;
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
         const size_t q = (size_t)b * d.nint + c;
-        const float2 pv = ff_add(make_float2(z[q] * s, 0.f), ff_mul(be, p[q]));
+        const float2 pv = ff_add(z(q, s), ff_mul(be, p[q]));   // (z may be r: read before it changes)
         const float2 av = ff_add(w[q], ff_mul(be, Ap[q]));
         const float2 rv = ff_add(r[q], ff_mul(nal, av));
         p[q] = pv;
@@ -1614,8 +1628,7 @@ bool all_finite(const double* v, size_t n) {
 }
 
 // ---- the inner solve: one FCG iteration, as a graph or eagerly ----------------
-// One iteration unit on the stream: z = M r (the residual's FP32 part without
-// a preconditioner), its ghosts, w = A z with the products that give beta
+// One iteration unit on the stream: z = M r (r without a preconditioner), its ghosts, w = A z with the products that give beta
 // (`first`: 0, a restart) and alpha, the update of p, A p, x and r with r.r, and
 // the device-side check (k_inner_check), which sets the WHILE condition when
 // `set_cond`. Inactive problems take no step. (Forming p first, with its own
@@ -1632,15 +1645,16 @@ cudaError_t enqueue_iteration(falcon_solver* sv, int pc, bool first, cudaGraphCo
         sv->use_net = false;
         if (e != cudaSuccess) return e;
     }
-    const bool none = pc == FALCON_PRECOND_NONE;
-    const float* z = none ? sv->lv[0].r : sv->lv[0].z;
-    const float* scale = none ? nullptr : sv->dsA;   // the V-cycle inverts the unscaled FP32 operator
-    k_ghost_ff<<<(unsigned)((sv->gff.n + 255) / 256), 256, 0, sv->st>>>(sv->gff, z, scale, sv->bprob, sv->ghosts2);
-    const auto spmv = d.m0 == 8 ? k_spmv_z_ff<8> : d.m0 == 16 ? k_spmv_z_ff<16> : k_spmv_z_ff<0>;
-    spmv<<<g, std::min(tpb(d), 512u), 0, sv->st>>>(sv->lv[0].ops2(), d, z, scale, sv->ghosts2, sv->p2, sv->r2, sv->Ap2,
-                                                   sv->w2, sv->D());
-    k_step_ff<<<g, std::min(tpb(d), 512u), 0, sv->st>>>(d, z, scale, sv->w2, sv->x2, sv->p2, sv->r2, sv->Ap2, sv->lv[0].r,
-                                                        sv->D(), first ? 1 : 0);
+    auto step = [&](auto z) {
+        using Z = decltype(z);
+        const unsigned t = std::min(tpb(d), 512u);
+        k_ghost_ff<Z><<<(unsigned)((sv->gff.n + 255) / 256), 256, 0, sv->st>>>(sv->gff, z, sv->bprob, sv->ghosts2);
+        const auto spmv = d.m0 == 8 ? k_spmv_z_ff<8, Z> : d.m0 == 16 ? k_spmv_z_ff<16, Z> : k_spmv_z_ff<0, Z>;
+        spmv<<<g, t, 0, sv->st>>>(sv->lv[0].ops2(), d, z, sv->ghosts2, sv->p2, sv->r2, sv->Ap2, sv->w2, sv->D());
+        k_step_ff<Z><<<g, t, 0, sv->st>>>(d, z, sv->w2, sv->x2, sv->p2, sv->r2, sv->Ap2, sv->lv[0].r, sv->D(), first ? 1 : 0);
+    };
+    if (pc == FALCON_PRECOND_NONE) step(ZFF{sv->r2});
+    else step(Z32{sv->lv[0].z, sv->dsA});   // the V-cycle inverts the unscaled FP32 operator
     k_inner_check<<<1, 256, 0, sv->st>>>(np, sv->D(), first ? 1 : 0, sv->rr0, sv->eta, sv->active, sv->ictl, h, set_cond);
     return cudaGetLastError();
 }
