@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "../../include/falcon_gb300.h"
+#include "ff.cuh"
 #include "lcc.h"
 #include "solver.h"
 #include "vcycle.cuh"
@@ -195,51 +196,19 @@ __global__ void k_residual64(Ops64 A, LevelDims d, const double* x, const double
 // with sA, sr powers of two (exact): every vector and dot product is O(1).
 struct Ops2 { const float2 *Aii, *Ai, *Aj, *Ak; };
 
-__device__ __forceinline__ float2 ff_quick(float s, float e) {
-    const float h = s + e;
-    return make_float2(h, e - (h - s));
-}
-__device__ __forceinline__ float2 ff_two_sum(float a, float b) {
-    const float s = a + b;
-    const float bb = s - a;
-    return make_float2(s, (a - (s - bb)) + (b - bb));
-}
-__device__ __forceinline__ float2 ff_add(float2 a, float2 b) {
-    float2 s = ff_two_sum(a.x, b.x);
-    const float2 t = ff_two_sum(a.y, b.y);
-    s.y += t.x;
-    s = ff_quick(s.x, s.y);
-    s.y += t.y;
-    return ff_quick(s.x, s.y);
-}
-__device__ __forceinline__ float2 ff_mul(float2 a, float2 b) {
-    const float p = a.x * b.x;
-    float e = fmaf(a.x, b.x, -p);
-    e = fmaf(a.x, b.y, e);
-    e = fmaf(a.y, b.x, e);
-    return ff_quick(p, e);
-}
-__device__ __forceinline__ float2 ff_neg(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 ff_from(double v) {   // a few FP64 operations: per thread, not per cell
-    const float h = (float)v;
-    return make_float2(h, (float)(v - (double)h));
-}
-__device__ __forceinline__ double ff_to(float2 a) { return (double)a.x + (double)a.y; }
-
 __device__ __forceinline__ float2 ff_shfl_xor(float2 v, int o) {
     return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
 }
-// per-problem FF sums -> one FP64 atomic per CTA and sum. FP64 instructions are
-// the scarce ones (16 cycles each per SM), so the sums stay FF across the warps and only the
-// CTA's totals are converted, one lane each.
+// per-problem FF sums -> one FP64 atomic per CTA and sum (FP64 work once per warp)
 __device__ __forceinline__ void block_sum_atomic_ff(float2 v, double* slot) {
     for (int o = 16; o > 0; o >>= 1) v = ff_add(v, ff_shfl_xor(v, o));
-    __shared__ float2 ws[32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __shared__ double ws[32];
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = ff_to(v);
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = ff_add(v, ws[w]);
-        atomicAdd(slot, ff_to(v));
+        double t = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
+        atomicAdd(slot, t);
     }
 }
 // four sums at once: each exchange of the first two folds two sums into one
@@ -251,41 +220,28 @@ __device__ __forceinline__ void block_sum4_atomic_ff(const float2 (&v)[4], doubl
     const float2 b = ff_add(hi ? v[3] : v[2], ff_shfl_xor(hi ? v[2] : v[3], 16));
     float2 s = ff_add(top ? b : a, ff_shfl_xor(top ? a : b, 8));
     for (int o = 4; o > 0; o >>= 1) s = ff_add(s, ff_shfl_xor(s, o));
-    __shared__ float2 ws[32][4];
-    if ((lane & 7) == 0) ws[threadIdx.x >> 5][(hi ? 1 : 0) + (top ? 2 : 0)] = s;
+    __shared__ double ws[32][4];
+    if ((lane & 7) == 0) ws[threadIdx.x >> 5][(hi ? 1 : 0) + (top ? 2 : 0)] = ff_to(s);
     __syncthreads();
     if (threadIdx.x < 4) {
-        s = ws[0][threadIdx.x];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) s = ff_add(s, ws[w][threadIdx.x]);
+        double t = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w][threadIdx.x];
         double* p = threadIdx.x == 0 ? slot[0] : threadIdx.x == 1 ? slot[1] : threadIdx.x == 2 ? slot[2] : slot[3];
-        atomicAdd(p, ff_to(s));
+        atomicAdd(p, t);
     }
 }
-
-// Sums of products of FF numbers in compensated form (Ogita, Rump and Oishi's
-// Dot2 with the low parts added to the error): s the running sum, e the rounding
-// errors of the sums and products, about 2^-46 of the summed magnitudes in a
-// third of the instructions of an FF addition per term.
-struct FFSum {
-    float s = 0.f, e = 0.f;
-    __device__ __forceinline__ void add(float2 a, float2 b) {
-        const float p = a.x * b.x;
-        const float t = s + p, bb = t - s;
-        e += ((s - (t - bb)) + (p - bb)) + fmaf(a.y, b.x, fmaf(a.x, b.y, fmaf(a.x, b.x, -p)));
-        s = t;
-    }
-    __device__ __forceinline__ float2 value() const { return ff_quick(s, e); }
-};
 
 // The search's z: the preconditioner's FP32 output scaled by the problem's sA, or
 // without a preconditioner the residual itself, all of its bits.
 struct Z32 {
     const float *__restrict__ z, *__restrict__ scale;
+    static constexpr int kUnroll = 2;
     __device__ __forceinline__ float of_problem(int pb) const { return scale[pb]; }
     __device__ __forceinline__ float2 operator()(size_t q, float s) const { return make_float2(z[q] * s, 0.f); }
 };
 struct ZFF {
     const float2* r;
+    static constexpr int kUnroll = 1;
     __device__ __forceinline__ float of_problem(int) const { return 1.f; }
     __device__ __forceinline__ float2 operator()(size_t q, float) const { return r[q]; }
 };
@@ -357,9 +313,8 @@ __global__ void __launch_bounds__(512) k_spmv_z_ff(Ops2 A, LevelDims d, Z z, con
     const float2* Gb = G + (size_t)b * 6 * mm;
     FFSum zw, za, pw, zr;
     const float2 *__restrict__ Aii = A.Aii, *__restrict__ Ai = A.Ai, *__restrict__ Aj = A.Aj, *__restrict__ Ak = A.Ak;
-    // two cells at a time (the pointers' promise lets their loads overlap): a 6.3M-cell
-    // iteration 0.885 -> 0.845 ms; four at a time 0.870
-#pragma unroll 2
+    // two cells at a time with an FP32 z (the pointers' promise lets their loads overlap)
+#pragma unroll Z::kUnroll
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
         const int i = c % m, row = c / m, j = row % m, k = row / m;
         const size_t fi = ((size_t)b * mm + row) * (m + 1) + i;
