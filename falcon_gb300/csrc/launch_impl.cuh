@@ -2,13 +2,17 @@
 // mhd_mixed.cu): CFL, ghost fill, psi.
 #pragma once
 #include "mhd_impl.cuh"
+#include "once_per_device.h"
 
 namespace falcon {
 namespace impl {
 
-// Dynamic shared memory above 48 KB for a kernel, set once per process and kernel.
-template <class K> cudaError_t allow_smem(K kernel, size_t bytes) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+// Dynamic shared memory above 48 KB for a kernel, set once per device (`once`: the kernel's own).
+template <class K> cudaError_t allow_smem(OncePerDevice& once, K kernel, size_t bytes) {
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return once(device, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 // Launch of a kernel that calls step_wait: with d.overlap (grids of up to 2^20 cells

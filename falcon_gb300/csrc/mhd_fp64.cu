@@ -15,7 +15,8 @@ template <int N, int KP, int DIVB>
 cudaError_t stage_nd(const StepDims& d, const Geometry& g, const double* in, const double* un, double* out,
                      const DivBArgs& psi, int stage, int bcw, StepScalars* sc, cudaStream_t st) {
     using S = Shape<double, N, N, N, KP>;
-    static const cudaError_t attr = allow_smem(k_stage<N, N, N, KP, DIVB>, S::smem_stage);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, k_stage<N, N, N, KP, DIVB>, S::smem_stage);
     if (attr != cudaSuccess) return attr;
     k_stage<N, N, N, KP, DIVB><<<d.nblocks, S::NT, S::smem_stage, st>>>(in, un, out, psi, g, sc, stage, bcw);
     return cudaGetLastError();
@@ -38,7 +39,8 @@ cudaError_t stage_n(const StepDims& d, const Geometry& g, const double* in, cons
 template <int N, int VPT>
 cudaError_t diff_march64(const StepDims& d, const Geometry& g, double* u, StepScalars* sc, cudaStream_t st) {
     using S = M64Shape<N, N, N, VPT>;
-    static const cudaError_t attr = allow_smem(k_diffusion_march64<N, N, N, VPT>, S::smem);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, k_diffusion_march64<N, N, N, VPT>, S::smem);
     if (attr != cudaSuccess) return attr;
     k_diffusion_march64<N, N, N, VPT><<<d.nblocks, S::NT, S::smem, st>>>(u, g, sc);
     return cudaGetLastError();

@@ -27,7 +27,8 @@ template <int N, int KP, int DIVB>
 cudaError_t stage_nd(const StepDims& d, const Geometry& g, const float* in, const float* un, float* out, int8_t* lo,
                      const PushTable& push, const DivBArgs& psi, int stage, int bcw, StepScalars* sc, cudaStream_t st) {
     auto run = [&](auto kernel, size_t smem, int nt, int most) {
-        static const cudaError_t attr = allow_smem(kernel, smem);
+        static OncePerDevice once;
+        const cudaError_t attr = allow_smem(once, kernel, smem);
         if (attr != cudaSuccess) return attr;
         const int split = in != out ? split_of(d, most) : 1;
         return launch_step(d, kernel, d.nblocks * split, nt, smem, st, in, un, out, lo, push, psi, g, sc, stage, bcw, split);
@@ -54,7 +55,8 @@ template <int N, int KP>
 cudaError_t diff_n(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo, const PushTable& push,
                    StepScalars* sc, int cfl_next, cudaStream_t st) {
     using S = DShape<N, N, N, KP>;
-    static const cudaError_t attr = allow_smem(k_diffusion_quads<N, N, N, KP>, S::smem);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, k_diffusion_quads<N, N, N, KP>, S::smem);
     if (attr != cudaSuccess) return attr;
     return launch_step(d, k_diffusion_quads<N, N, N, KP>, d.nblocks, S::NT, S::smem, st, u, out, lo, push, g, sc, cfl_next);
 }
@@ -62,7 +64,8 @@ cudaError_t diff_n(const StepDims& d, const Geometry& g, const float* u, float* 
 cudaError_t diff_march16(const StepDims& d, const Geometry& g, const float* u, float* out, int8_t* lo,
                          const PushTable& push, StepScalars* sc, int cfl_next, cudaStream_t st) {
     using S = MShape<16, 16, 16>;
-    static const cudaError_t attr = allow_smem(k_march_quads<16, 16, 16>, S::smem);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, k_march_quads<16, 16, 16>, S::smem);
     if (attr != cudaSuccess) return attr;
     const int split = out != u ? split_of(d, 4) : 1;
     return launch_step(d, k_march_quads<16, 16, 16>, d.nblocks * split, S::NT, S::smem, st, u, out, lo, push, g, sc, cfl_next,
