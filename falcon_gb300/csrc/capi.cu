@@ -16,6 +16,7 @@
 #include "../../include/falcon_gb300.h"
 #include "host_setup.h"
 #include "kernels.cuh"
+#include "restart_order.h"
 #include "synth.cuh"
 
 namespace falcon {
@@ -1579,41 +1580,31 @@ RestartHeader restart_header(const falcon_ctx* ctx) {
     h.bytes_psi = ctx->P ? cells * ctx->elem : 0;
     return h;
 }
-constexpr size_t kIoChunk = 64u << 20;
+// Piece of a restart file moved at a time: small enough to stay in the host's caches from
+// the copy to the write, and for its first pages to cost little (64 MB: 2.7 ms for a 6 MB
+// file, 0.6 for the pieces)
+constexpr size_t kIoChunk = 8u << 20;
 
-// Restart files hold the state as [block][var][cell] and the correction as
-// [block][var][interior cell]; the mixed device arrays hold a cell's variables
-// side by side (Layout). Whole blocks of either, in host memory, from one
-// order to the other: n values of `item` bytes per variable and block, `group`
-// variables side by side on the device.
-void reorder_blocks(const unsigned char* src, unsigned char* dst, size_t nblocks, size_t n, int item, int group, bool to_file) {
-    const size_t block = n * NV * (size_t)item;
-#pragma omp parallel for schedule(static)
-    for (long b = 0; b < (long)nblocks; ++b)
-        for (int v = 0; v < NV; ++v)
-            for (size_t c = 0; c < n; ++c) {
-                const size_t file = (size_t)b * block + ((size_t)v * n + c) * item;
-                const size_t dev = (size_t)b * block + (((size_t)(v / group) * n + c) * group + v % group) * item;
-                std::memcpy(dst + (to_file ? file : dev), src + (to_file ? dev : file), (size_t)item);
-            }
-}
 // The restart file's arrays: device pointer, bytes, and for the mixed state and
-// correction the values per variable and block (0: stored as on the device)
+// correction the values per variable and block (0: stored as on the device) of `item` bytes
 struct RestartPart {
     void* dev;
     uint64_t bytes;
     size_t n;
-    int item, group;
-    size_t chunk() const {   // whole blocks, about kIoChunk
-        const size_t block = n * NV * (size_t)item;
-        return n ? std::max<size_t>(1, kIoChunk / block) * block : kIoChunk;
+    int item;
+    size_t block() const { return n * NV * (size_t)item; }
+    size_t chunk() const { return n ? std::max<size_t>(1, kIoChunk / block()) * block() : kIoChunk; }   // whole blocks
+    void to_file(const std::vector<unsigned char>& from, std::vector<unsigned char>& to) const {
+        const size_t nb = from.size() / block();
+        if (item == 4) blocks_to_file<float, 4>(from.data(), to.data(), nb, n);
+        else blocks_to_file<int8_t, NV>(from.data(), to.data(), nb, n);
     }
 };
 std::array<RestartPart, 3> restart_parts(falcon_ctx* ctx, const RestartHeader& h) {
     const bool m = ctx->mixed();
     const size_t nint = (size_t)ctx->dims.ni * ctx->dims.nj * ctx->dims.nk;
-    return {RestartPart{ctx->U, h.bytes_state, m ? (size_t)ctx->dims.ncell : 0, 4, 4},
-            RestartPart{ctx->Ulo, h.bytes_lo, nint, 1, NV}, RestartPart{ctx->P, h.bytes_psi, 0, 0, 0}};
+    return {RestartPart{ctx->U, h.bytes_state, m ? (size_t)ctx->dims.ncell : 0, 4},
+            RestartPart{ctx->Ulo, h.bytes_lo, nint, 1}, RestartPart{ctx->P, h.bytes_psi, 0, 0}};
 }
 }  // namespace
 
@@ -1729,7 +1720,7 @@ int falcon_save_restart(falcon_ctx* ctx, const char* path) {
             ok = e == cudaSuccess;
             if (ok && p.n) {
                 file.resize(n);
-                reorder_blocks(buf.data(), file.data(), n / (p.n * NV * (size_t)p.item), p.n, p.item, p.group, true);
+                p.to_file(buf, file);
             }
             ok = ok && std::fwrite(p.n ? file.data() : buf.data(), 1, n, f) == n;
         }
@@ -1771,7 +1762,7 @@ int falcon_load_restart(falcon_ctx* ctx, const char* path) {
         return ctx->fail(FALCON_ERR_INVALID_ARG, std::string("restart ") + path + ": " + why);
     }
     CK(cudaStreamSynchronize(ctx->st), "restart");
-    std::vector<unsigned char> buf, file;
+    std::vector<unsigned char> buf;
     cudaError_t e = cudaSuccess;
     bool ok = true;
     for (const RestartPart& p : restart_parts(ctx, h))
@@ -1779,17 +1770,13 @@ int falcon_load_restart(falcon_ctx* ctx, const char* path) {
             const size_t n = (size_t)std::min<uint64_t>(p.chunk(), p.bytes - off);
             buf.resize(n);
             ok = std::fread(buf.data(), 1, n, f) == n;
-            if (ok && p.n) {
-                file.swap(buf);
-                buf.resize(n);
-                reorder_blocks(file.data(), buf.data(), n / (p.n * NV * (size_t)p.item), p.n, p.item, p.group, false);
-            }
             if (ok) e = cudaMemcpy((unsigned char*)p.dev + off, buf.data(), n, cudaMemcpyHostToDevice);
             ok = ok && e == cudaSuccess;
         }
     std::fclose(f);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "restart");
     if (!ok) return ctx->fail(FALCON_ERR_INVALID_ARG, std::string("restart ") + path + ": short read");
+    if (ctx->mixed()) CK(launch_state_from_file((float*)ctx->U, ctx->Ulo, ctx->dims, ctx->st), "restart");
     // the stage arrays start equal to the state, as after falcon_upload_state
     CK(mirror_state(ctx, true), "restart");
     ctx->stale_edges = false;

@@ -233,6 +233,8 @@ cudaError_t launch_psi_ghost_mixed(const StepDims& d, const GhostLists& gl, floa
 cudaError_t launch_clear_outside_core_mixed(const StepDims& d, float* u, int nvar, cudaStream_t st);
 // the regular faces of a mixed state pushed and its CFL minimum formed, as the
 // diffusion pass closing a step leaves them (after a core upload)
+// in place: the order of restart files ([block][var][cell], lo: interior cells) to the device's (Layout)
+cudaError_t launch_state_from_file(float* U, int8_t* lo, const StepDims& d, cudaStream_t st);
 cudaError_t launch_push_state_mixed(const StepDims& d, const Geometry& g, float* u, const PushTable& push,
                                     StepScalars* sc, cudaStream_t st);
 cudaError_t launch_step_persistent_mixed(const StepDims& d, const Geometry& g, float* U, float* RK, float* R2,

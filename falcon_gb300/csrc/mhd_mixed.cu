@@ -130,6 +130,23 @@ cudaError_t launch_clear_outside_core_mixed(const StepDims& d, float* u, int nva
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
+namespace impl {
+namespace {
+template <class T, int G> cudaError_t interleave(T* a, int64_t arrays, int n, cudaStream_t st) {
+    const size_t smem = (size_t)G * n * sizeof(T);
+    static OncePerDevice once;
+    const cudaError_t e = allow_smem(once, k_interleave<T, G>, 232448);
+    if (e != cudaSuccess) return e;
+    if (smem > 232448 || smem % 16 != 0 || arrays > INT32_MAX) return cudaErrorInvalidValue;
+    k_interleave<T, G><<<(unsigned)arrays, 512, smem, st>>>(a, n);
+    return cudaGetLastError();
+}
+}  // namespace
+}  // namespace impl
+cudaError_t launch_state_from_file(float* U, int8_t* lo, const StepDims& d, cudaStream_t st) {
+    const cudaError_t e = impl::interleave<float, 4>(U, (int64_t)d.nblocks * 2, d.ncell, st);
+    return e == cudaSuccess && lo ? impl::interleave<int8_t, NV>(lo, d.nblocks, d.ni * d.nj * d.nk, st) : e;
+}
 cudaError_t launch_push_state_mixed(const StepDims& d, const Geometry& g, float* u, const PushTable& push,
                                     StepScalars* sc, cudaStream_t st) {
     if (d.ni == 16 && d.nj == 16 && d.nk == 16) impl::k_push_state<16, 16, 16><<<d.nblocks, 256, 0, st>>>(u, push, g, sc);

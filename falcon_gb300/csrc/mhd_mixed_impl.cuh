@@ -1304,6 +1304,32 @@ k_march_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geometry 
 }
 
 // ---------------------------------------------------------------------------
+// [G][n] to [n][G] in place, an array per CTA through shared memory (a half of a 16^3
+// block: 125 KB).
+template <class T, int G>
+__global__ void __launch_bounds__(512) k_interleave(T* a, int n) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    int4* s = reinterpret_cast<int4*>(smem);
+    int4* g = reinterpret_cast<int4*>(a + (size_t)blockIdx.x * G * n);
+    const int vecs = (int)((size_t)G * n * sizeof(T) / 16);
+    for (int x = threadIdx.x; x < vecs; x += blockDim.x) s[x] = g[x];
+    __syncthreads();
+    constexpr int V = 16 / sizeof(T);
+    const T* t = reinterpret_cast<const T*>(smem);
+    for (int x = threadIdx.x; x < vecs; x += blockDim.x) {
+        T o[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            const int y = x * V + q;
+            o[q] = t[y % G * n + y / G];
+        }
+        int4 r;
+        memcpy(&r, o, 16);
+        g[x] = r;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Every cell outside the core of each block and variable set to 0 (the k ghost
 // planes and, in the interior planes, the j ghost rows: per block and
 // variable, (NJP-4)*NIP-wide gaps between the core runs). A core upload clears
