@@ -249,17 +249,19 @@ bool wide_ok(const void* p, int64_t ncell) { return ((uintptr_t)p % 16) == 0 && 
 // psi last), the interior planes and within them the interior rows, each
 // row whole (its radial ghost columns, which hold the radial boundary
 // condition, included). The interior rows of one plane are one contiguous
-// run of (NJP-4)*NIP host elements. A warp takes the runs of one plane of one
-// group of a block's variables at a time -- four that the mixed state holds side
-// by side (FP64: one), or psi -- so no element pays a 64-bit division and the
-// mixed state's side is whole 16-byte cells; each lane's 16-byte host accesses of
-// a pass (two cells of every variable, kPass passes) are issued before any is
-// used. Offsets are even and NIP is even, so a pair (ip, ip+1) is either two
-// radial ghost columns or two interior cells.
-template <class T> struct CoreRun {
+// run of (NJP-4)*NIP host elements. A warp takes pieces of the runs of one plane of one
+// group of a block's variables -- four that the mixed state holds side by side (FP64:
+// one), or psi -- so no element pays a 64-bit division (a piece does) and the mixed
+// state's side is whole 16-byte cells; a lane's 16-byte host accesses of a piece (two
+// cells of every variable, PASS passes) are issued before any is used. Offsets are
+// even and NIP is even, so a pair (ip, ip+1) is either two radial ghost columns or
+// two interior cells.
+template <class T, int PASS> struct CoreRun {
     static constexpr int G = sizeof(T) == 4 ? 4 : 1;    // variables of a group
     static constexpr int NG = NV / G + 1;               // groups, psi last
-    static constexpr int kPass = sizeof(T) == 4 ? 2 : 5;
+    static constexpr int kPass = PASS;
+    __host__ __device__ static int length(const StepDims& dm) { return (dm.njp - 4) * dm.nip; }
+    __host__ __device__ static int pieces(const StepDims& dm) { return (length(dm) + 64 * kPass - 1) / (64 * kPass); }
     int64_t b, cell0;   // block, padded cell of the run's first element
     int g;
     int kp;
@@ -287,116 +289,123 @@ template <class T> struct CoreRun {
 };
 // host core -> device: state cells narrowed (FP32 with its correction) or
 // copied (FP64); psi converted into P, or, without P, tested for 0 (flag)
-template <class T>
+template <class T, int PASS>
 __global__ void k_core_up(const double* s, T* U, int8_t* lo, T* P, int32_t* flag, int64_t nruns, StepDims dm) {
-    using R = CoreRun<T>;
-    const int lane2 = 2 * (threadIdx.x & 31), len = (dm.njp - 4) * dm.nip;
+    using R = CoreRun<T, PASS>;
+    const int lane2 = 2 * (threadIdx.x & 31), len = R::length(dm), pieces = R::pieces(dm);
     int any = 0;
-    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nruns;
-         r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nruns * pieces;
+         w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        const int64_t r = w / pieces;
         const R c(r, dm);
         const int nv = c.vars();
-        for (int o0 = 0; o0 < len; o0 += 64 * R::kPass) {
-            double2 v[R::kPass][R::G];
+        const int o0 = (int)(w - r * pieces) * 64 * R::kPass;
+        double2 v[R::kPass][R::G];
 #pragma unroll
-            for (int q = 0; q < R::kPass; ++q)
+        for (int q = 0; q < R::kPass; ++q)
 #pragma unroll
-                for (int g = 0; g < R::G; ++g)
-                    if (o0 + 64 * q + lane2 < len && g < nv)
-                        v[q][g] = *reinterpret_cast<const double2*>(s + c.host(g, o0 + 64 * q + lane2, dm));
+            for (int g = 0; g < R::G; ++g)
+                if (o0 + 64 * q + lane2 < len && g < nv)
+                    v[q][g] = *reinterpret_cast<const double2*>(s + c.host(g, o0 + 64 * q + lane2, dm));
 #pragma unroll
-            for (int q = 0; q < R::kPass; ++q) {
-                const int o = o0 + 64 * q + lane2;
-                if (o >= len) continue;
-                const int64_t pc = c.b * dm.ncell + c.cell0 + o;   // the cells in a [b][cell] array
-                if (c.psi()) {
-                    if (!P) {
-                        any |= (v[q][0].x != 0.0) | (v[q][0].y != 0.0);
-                    } else if constexpr (sizeof(T) == 4) {
-                        *reinterpret_cast<float2*>(P + pc) = make_float2((float)v[q][0].x, (float)v[q][0].y);
-                    } else {
-                        *reinterpret_cast<double2*>(P + pc) = v[q][0];
-                    }
-                    continue;
-                }
-                if constexpr (sizeof(T) == 4) {
-                    float4* out = reinterpret_cast<float4*>(U) + (c.b * 2 + c.g) * dm.ncell + c.cell0 + o;
-                    const float4 a = make_float4((float)v[q][0].x, (float)v[q][1].x, (float)v[q][2].x, (float)v[q][3].x);
-                    const float4 e = make_float4((float)v[q][0].y, (float)v[q][1].y, (float)v[q][2].y, (float)v[q][3].y);
-                    out[0] = a;
-                    out[1] = e;
-                    if (lo && c.interior(o, dm)) {
-                        int8_t* l = lo + c.lo(o, dm);
-                        *reinterpret_cast<char4*>(l) =
-                            make_char4(lo_encode64(a.x, v[q][0].x - (double)a.x), lo_encode64(a.y, v[q][1].x - (double)a.y),
-                                       lo_encode64(a.z, v[q][2].x - (double)a.z), lo_encode64(a.w, v[q][3].x - (double)a.w));
-                        *reinterpret_cast<char4*>(l + NV) =
-                            make_char4(lo_encode64(e.x, v[q][0].y - (double)e.x), lo_encode64(e.y, v[q][1].y - (double)e.y),
-                                       lo_encode64(e.z, v[q][2].y - (double)e.z), lo_encode64(e.w, v[q][3].y - (double)e.w));
-                    }
+        for (int q = 0; q < R::kPass; ++q) {
+            const int o = o0 + 64 * q + lane2;
+            if (o >= len) continue;
+            const int64_t pc = c.b * dm.ncell + c.cell0 + o;   // the cells in a [b][cell] array
+            if (c.psi()) {
+                if (!P) {
+                    any |= (v[q][0].x != 0.0) | (v[q][0].y != 0.0);
+                } else if constexpr (sizeof(T) == 4) {
+                    *reinterpret_cast<float2*>(P + pc) = make_float2((float)v[q][0].x, (float)v[q][0].y);
                 } else {
-                    *reinterpret_cast<double2*>(U + Layout<T>::at((size_t)c.b, c.g, (size_t)(c.cell0 + o), (size_t)dm.ncell)) = v[q][0];
+                    *reinterpret_cast<double2*>(P + pc) = v[q][0];
                 }
+                continue;
+            }
+            if constexpr (sizeof(T) == 4) {
+                float4* out = reinterpret_cast<float4*>(U) + (c.b * 2 + c.g) * dm.ncell + c.cell0 + o;
+                const float4 a = make_float4((float)v[q][0].x, (float)v[q][1].x, (float)v[q][2].x, (float)v[q][3].x);
+                const float4 e = make_float4((float)v[q][0].y, (float)v[q][1].y, (float)v[q][2].y, (float)v[q][3].y);
+                out[0] = a;
+                out[1] = e;
+                if (lo && c.interior(o, dm)) {
+                    int8_t* l = lo + c.lo(o, dm);
+                    *reinterpret_cast<char4*>(l) =
+                        make_char4(lo_encode64(a.x, v[q][0].x - (double)a.x), lo_encode64(a.y, v[q][1].x - (double)a.y),
+                                   lo_encode64(a.z, v[q][2].x - (double)a.z), lo_encode64(a.w, v[q][3].x - (double)a.w));
+                    *reinterpret_cast<char4*>(l + NV) =
+                        make_char4(lo_encode64(e.x, v[q][0].y - (double)e.x), lo_encode64(e.y, v[q][1].y - (double)e.y),
+                                   lo_encode64(e.z, v[q][2].y - (double)e.z), lo_encode64(e.w, v[q][3].y - (double)e.w));
+                }
+            } else {
+                *reinterpret_cast<double2*>(U + Layout<T>::at((size_t)c.b, c.g, (size_t)(c.cell0 + o), (size_t)dm.ncell)) = v[q][0];
             }
         }
     }
     if (flag && __any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) *flag = 1;
 }
 // device -> host core (psi 0 without P)
-template <class T>
+template <class T, int PASS>
 __global__ void k_core_down(const T* U, const int8_t* lo, const T* P, double* out, int64_t nruns, StepDims dm) {
-    using R = CoreRun<T>;
-    const int lane2 = 2 * (threadIdx.x & 31), len = (dm.njp - 4) * dm.nip;
-    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nruns;
-         r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    using R = CoreRun<T, PASS>;
+    const int lane2 = 2 * (threadIdx.x & 31), len = R::length(dm), pieces = R::pieces(dm);
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nruns * pieces;
+         w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        const int64_t r = w / pieces;
         const R c(r, dm);
         const int nv = c.vars();
-        for (int o0 = 0; o0 < len; o0 += 64 * R::kPass) {
-            double2 v[R::kPass][R::G];
+        const int o0 = (int)(w - r * pieces) * 64 * R::kPass;
+        double2 v[R::kPass][R::G];
 #pragma unroll
-            for (int q = 0; q < R::kPass; ++q) {
-                const int o = o0 + 64 * q + lane2;
-                if (o >= len) continue;
-                const int64_t pc = c.b * dm.ncell + c.cell0 + o;
-                if (c.psi()) {
-                    v[q][0] = make_double2(0.0, 0.0);
-                    if (P) v[q][0] = make_double2((double)P[pc], (double)P[pc + 1]);
-                    continue;
-                }
-                if constexpr (sizeof(T) == 4) {
-                    const float4* in = reinterpret_cast<const float4*>(U) + (c.b * 2 + c.g) * dm.ncell + c.cell0 + o;
-                    const float4 a = in[0], e = in[1];
-                    const float h0[4] = {a.x, a.y, a.z, a.w}, h1[4] = {e.x, e.y, e.z, e.w};
-                    char4 l0 = make_char4(0, 0, 0, 0), l1 = l0;
-                    const bool add = lo && c.interior(o, dm);
-                    if (add) {
-                        const int8_t* l = lo + c.lo(o, dm);
-                        l0 = *reinterpret_cast<const char4*>(l);
-                        l1 = *reinterpret_cast<const char4*>(l + NV);
-                    }
-                    const int8_t q0[4] = {l0.x, l0.y, l0.z, l0.w}, q1[4] = {l1.x, l1.y, l1.z, l1.w};
-#pragma unroll
-                    for (int g = 0; g < R::G; ++g) {
-                        v[q][g] = make_double2((double)h0[g], (double)h1[g]);
-                        if (add) {
-                            v[q][g].x += (double)q0[g] * (double)lo_unit(h0[g]);
-                            v[q][g].y += (double)q1[g] * (double)lo_unit(h1[g]);
-                        }
-                    }
-                } else {
-                    v[q][0] = *reinterpret_cast<const double2*>(U + Layout<T>::at((size_t)c.b, c.g, (size_t)(c.cell0 + o), (size_t)dm.ncell));
-                }
+        for (int q = 0; q < R::kPass; ++q) {
+            const int o = o0 + 64 * q + lane2;
+            if (o >= len) continue;
+            const int64_t pc = c.b * dm.ncell + c.cell0 + o;
+            if (c.psi()) {
+                v[q][0] = make_double2(0.0, 0.0);
+                if (P) v[q][0] = make_double2((double)P[pc], (double)P[pc + 1]);
+                continue;
             }
+            if constexpr (sizeof(T) == 4) {
+                const float4* in = reinterpret_cast<const float4*>(U) + (c.b * 2 + c.g) * dm.ncell + c.cell0 + o;
+                const float4 a = in[0], e = in[1];
+                const float h0[4] = {a.x, a.y, a.z, a.w}, h1[4] = {e.x, e.y, e.z, e.w};
+                char4 l0 = make_char4(0, 0, 0, 0), l1 = l0;
+                const bool add = lo && c.interior(o, dm);
+                if (add) {
+                    const int8_t* l = lo + c.lo(o, dm);
+                    l0 = *reinterpret_cast<const char4*>(l);
+                    l1 = *reinterpret_cast<const char4*>(l + NV);
+                }
+                const int8_t q0[4] = {l0.x, l0.y, l0.z, l0.w}, q1[4] = {l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+                for (int g = 0; g < R::G; ++g) {
+                    v[q][g] = make_double2((double)h0[g], (double)h1[g]);
+                    if (add) {
+                        v[q][g].x += (double)q0[g] * (double)lo_unit(h0[g]);
+                        v[q][g].y += (double)q1[g] * (double)lo_unit(h1[g]);
+                    }
+                }
+            } else {
+                v[q][0] = *reinterpret_cast<const double2*>(U + Layout<T>::at((size_t)c.b, c.g, (size_t)(c.cell0 + o), (size_t)dm.ncell));
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < R::G; ++g)
 #pragma unroll
             for (int q = 0; q < R::kPass; ++q)
-#pragma unroll
-                for (int g = 0; g < R::G; ++g)
-                    if (o0 + 64 * q + lane2 < len && g < nv)
-                        *reinterpret_cast<double2*>(out + c.host(g, o0 + 64 * q + lane2, dm)) = v[q][g];
-        }
+                if (o0 + 64 * q + lane2 < len && g < nv)
+                    *reinterpret_cast<double2*>(out + c.host(g, o0 + 64 * q + lane2, dm)) = v[q][g];
     }
 }
-template <class T> int64_t core_runs(const StepDims& dm) { return (int64_t)dm.nblocks * CoreRun<T>::NG * (dm.nkp - 4); }
+template <class T> int64_t core_runs(const StepDims& dm) { return (int64_t)dm.nblocks * CoreRun<T, 1>::NG * (dm.nkp - 4); }
+constexpr unsigned kCoreGrid = 1216, kCoreThreads = 256;
+// Mixed: pieces of two passes while they outnumber the grid's warps, else of one. 12
+// blocks of 8^3 to the host 21 / 18 us, 192 blocks 71 / 69; 5,184 blocks of 16^3 from the
+// host 10.42 / 10.74 ms. (A whole run per warp: 12 blocks of 16^3 39 us, in pieces 36.)
+bool core_short_pieces(const StepDims& dm) {
+    return core_runs<float>(dm) * CoreRun<float, 2>::pieces(dm) < (int64_t)kCoreGrid * kCoreThreads / 32;
+}
 bool core_ok(const void* host, const StepDims& dm) {
     return ((uintptr_t)host % 16) == 0 && dm.ncell % 2 == 0 && dm.nip % 2 == 0;
 }
@@ -445,15 +454,25 @@ cudaError_t launch_core_up(const double* host, void* U, int8_t* lo, void* P, int
         cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int32_t), st);
         if (e != cudaSuccess) return e;
     }
-    if (fp32) k_core_up<float><<<1216, 256, 0, st>>>(host, (float*)U, lo, (float*)P, flag, core_runs<float>(dm), dm);
-    else k_core_up<double><<<1216, 256, 0, st>>>(host, (double*)U, nullptr, (double*)P, flag, core_runs<double>(dm), dm);
+    if (fp32) {
+        const auto kern = core_short_pieces(dm) ? k_core_up<float, 1> : k_core_up<float, 2>;
+        kern<<<kCoreGrid, kCoreThreads, 0, st>>>(host, (float*)U, lo, (float*)P, flag, core_runs<float>(dm), dm);
+    } else {
+        k_core_up<double, 5><<<kCoreGrid, kCoreThreads, 0, st>>>(host, (double*)U, nullptr, (double*)P, flag,
+                                            core_runs<double>(dm), dm);
+    }
     return cudaGetLastError();
 }
 cudaError_t launch_core_down(const void* U, const int8_t* lo, const void* P, bool fp32, double* host, const StepDims& dm,
                              cudaStream_t st) {
     if (!core_ok(host, dm)) return cudaErrorInvalidValue;
-    if (fp32) k_core_down<float><<<1216, 256, 0, st>>>((const float*)U, lo, (const float*)P, host, core_runs<float>(dm), dm);
-    else k_core_down<double><<<1216, 256, 0, st>>>((const double*)U, nullptr, (const double*)P, host, core_runs<double>(dm), dm);
+    if (fp32) {
+        const auto kern = core_short_pieces(dm) ? k_core_down<float, 1> : k_core_down<float, 2>;
+        kern<<<kCoreGrid, kCoreThreads, 0, st>>>((const float*)U, lo, (const float*)P, host, core_runs<float>(dm), dm);
+    } else {
+        k_core_down<double, 5><<<kCoreGrid, kCoreThreads, 0, st>>>((const double*)U, nullptr, (const double*)P, host,
+                                            core_runs<double>(dm), dm);
+    }
     return cudaGetLastError();
 }
 
