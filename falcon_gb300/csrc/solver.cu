@@ -1029,6 +1029,25 @@ int plan_coarse(falcon_solver* sv, const std::vector<int32_t>& ghost, const std:
     return FALCON_OK;
 }
 
+// Whether `sweeps` red-black sweeps of level l from z = 0 are one launch: on a small
+// coarsest level, where several launches are saved
+bool sweeps_in_one_launch(const falcon_solver* sv, int l, int sweeps) {
+    const int nl = (int)sv->lv.size();
+    return l == nl - 1 && nl > 1 && sv->coarse_cluster > 0 && sweeps > 2;
+}
+// `sweeps` (at least one) red-black sweeps of level l on its r from z = 0. z: the first
+// launch's output, next(): the output of each launch after it
+template <class F> cudaError_t smooth_from_zero(falcon_solver* sv, int l, int sweeps, float* z, F next) {
+    if (sweeps_in_one_launch(sv, l, sweeps)) return coarse_sweeps(sv, sweeps, z);
+    cudaError_t e = vsweep<V_FIRST>(sv, l, nullptr, nullptr, z, 1);
+    for (int s = 2; s < 2 * sweeps && e == cudaSuccess; ++s) {
+        float* out = next();
+        e = vsweep<V_PLAIN>(sv, l, z, nullptr, out, s & 1);
+        z = out;
+    }
+    return e;
+}
+
 // z_0 = M r_0: one V-cycle on the FP32 residual stored in lv[0].r, into lv[0].z
 cudaError_t vcycle_body(falcon_solver* sv) {
     const int nl = (int)sv->lv.size(), nb = sv->S.nblocks;
@@ -1047,8 +1066,7 @@ cudaError_t vcycle_body(falcon_solver* sv) {
         SvLevel& L = sv->lv[l];
         const bool coarsest = l == nl - 1 && nl > 1, net = coarsest && sv->use_net;
         const int sweeps = net ? sv->net_sweeps : l == nl - 1 ? sv->nu_coarse : sv->nu_pre;
-        // the whole smoothing of a small coarsest level in one launch where several launches are saved
-        const bool one = coarsest && !net && sv->coarse_cluster > 0 && sweeps > 2;
+        const bool one = !net && sweeps_in_one_launch(sv, l, sweeps);
         left[l] = (net ? 1 + 2 * sweeps : one || sweeps == 0 ? 1 : 2 * sweeps - 1) +
                   (l < nl - 1 ? std::max(1, 2 * sv->nu_post) : 0);
         if (coarsest && sv->rec && sv->rec_n < sv->rec_max)
@@ -1072,11 +1090,8 @@ cudaError_t vcycle_body(falcon_solver* sv) {
             for (int s = 0; s < 2 * sweeps; ++s) plain(l, s & 1);
         } else if (sweeps == 0) {
             e = cudaMemsetAsync(zc[l], 0, (size_t)nb * L.d.nint * 4, sv->st);
-        } else if (one) {
-            e = coarse_sweeps(sv, sweeps, zc[l]);
         } else {
-            e = vsweep<V_FIRST>(sv, l, nullptr, nullptr, zc[l], 1);
-            for (int s = 2; s < 2 * sweeps; ++s) plain(l, s & 1);
+            e = smooth_from_zero(sv, l, sweeps, zc[l], [&] { return zc[l] = next(l); });
         }
         if (l + 1 < nl && e == cudaSuccess) e = vresid_restrict(sv, l, zc[l], sv->lv[l + 1].r);
     }
@@ -1799,9 +1814,12 @@ int falcon_solver_vcycle_op(falcon_solver* sv, int32_t op, int32_t level, const 
     if (!sv || !in0 || !out) return FALCON_ERR_INVALID_ARG;
     if (!sv->st) return sv->fail(FALCON_ERR_NO_DEVICE, "solver created without a device");
     const int nl = sv->S.nlevels, nb = sv->S.nblocks;
-    const bool needs_coarse = op == FALCON_VCYCLE_RESTRICT || op == FALCON_VCYCLE_PROLONG_ADD;
-    if (op < FALCON_VCYCLE_RESTRICT || op > FALCON_VCYCLE_RESIDUAL || level < 0 || level >= nl ||
-        (needs_coarse && level + 1 >= nl) || (op != FALCON_VCYCLE_RESTRICT && !in1))
+    const bool needs_coarse = op == FALCON_VCYCLE_RESTRICT || op == FALCON_VCYCLE_PROLONG_ADD ||
+                              op == FALCON_VCYCLE_RESIDUAL_RESTRICT || op == FALCON_VCYCLE_PROLONG_SWEEP;
+    const bool only_in0 = op == FALCON_VCYCLE_RESTRICT || op == FALCON_VCYCLE_FIRST_SWEEP || op == FALCON_VCYCLE_COARSE_SWEEPS;
+    if (op < FALCON_VCYCLE_RESTRICT || op > FALCON_VCYCLE_COARSE_SWEEPS || level < 0 || level >= nl ||
+        (needs_coarse && level + 1 >= nl) || (!only_in0 && !in1) ||
+        (op == FALCON_VCYCLE_COARSE_SWEEPS && (level == 0 || level != nl - 1 || sv->nu_coarse < 1)))
         return sv->fail(FALCON_ERR_INVALID_ARG, "falcon_solver_vcycle_op: bad operation, level or input");
     cudaSetDevice(sv->device);
     SvLevel& L = sv->lv[level];
@@ -1819,6 +1837,27 @@ int falcon_solver_vcycle_op(falcon_solver* sv, int32_t op, int32_t level, const 
         SCK(cudaMemcpyAsync(L.z, in1, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
         SCK(vsweep<V_PROLONG>(sv, level, L.z, Cl.z, L.zb, -1), "vcycle op");
         SCK(cudaMemcpyAsync(out, L.zb, nf, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
+    } else if (op == FALCON_VCYCLE_RESIDUAL_RESTRICT) {
+        SvLevel& Cl = sv->lv[level + 1];
+        SCK(cudaMemcpyAsync(L.r, in0, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(cudaMemcpyAsync(L.z, in1, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(vresid_restrict(sv, level, L.z, Cl.r), "vcycle op");
+        SCK(cudaMemcpyAsync(out, Cl.r, (size_t)nb * Cl.d.nint * 4, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
+    } else if (op == FALCON_VCYCLE_PROLONG_SWEEP) {
+        SvLevel& Cl = sv->lv[level + 1];
+        SCK(cudaMemcpyAsync(Cl.z, in0, (size_t)nb * Cl.d.nint * 4, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(cudaMemcpyAsync(L.r, in1, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(cudaMemcpyAsync(L.z, in1 + nf / 4, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        SCK(vsweep<V_PROLONG>(sv, level, L.z, Cl.z, L.zb, 1), "vcycle op");
+        SCK(cudaMemcpyAsync(out, L.zb, nf, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
+    } else if (op == FALCON_VCYCLE_FIRST_SWEEP || op == FALCON_VCYCLE_COARSE_SWEEPS) {
+        SCK(cudaMemcpyAsync(L.r, in0, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
+        float* z = L.z;
+        SCK(smooth_from_zero(sv, level, op == FALCON_VCYCLE_FIRST_SWEEP ? 1 : sv->nu_coarse, L.z, [&] {
+                z = z == L.z ? L.zb : L.z;
+                return z;
+            }), "vcycle op");
+        SCK(cudaMemcpyAsync(out, z, nf, cudaMemcpyDeviceToHost, sv->st), "vcycle op");
     } else {   // one red-black half sweep of a colour from z = in1, or the residual r - A z
         SCK(cudaMemcpyAsync(L.r, in0, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");
         SCK(cudaMemcpyAsync(L.z, in1, nf, cudaMemcpyHostToDevice, sv->st), "vcycle op");

@@ -19,6 +19,7 @@ PRECOND_NONE = 0
 PRECOND_MG = 1
 PRECOND_MG_LCC = 2
 VCYCLE_RESTRICT, VCYCLE_PROLONG_ADD, VCYCLE_SMOOTH_RED, VCYCLE_SMOOTH_BLACK, VCYCLE_RESIDUAL = range(5)
+VCYCLE_RESIDUAL_RESTRICT, VCYCLE_FIRST_SWEEP, VCYCLE_PROLONG_SWEEP, VCYCLE_COARSE_SWEEPS = range(5, 9)
 
 
 class SolverSpec(C.Structure):
@@ -204,7 +205,8 @@ class Solver:
         shp = lambda l: (self.nblocks,) + self.level_shape(l)[::-1]
         a = np.ascontiguousarray(in0, dtype=np.float32)
         b = None if in1 is None else np.ascontiguousarray(in1, dtype=np.float32)
-        out = np.zeros(shp(level + 1) if op == VCYCLE_RESTRICT else shp(level), dtype=np.float32)
+        to_coarse = op in (VCYCLE_RESTRICT, VCYCLE_RESIDUAL_RESTRICT)
+        out = np.zeros(shp(level + 1) if to_coarse else shp(level), dtype=np.float32)
         self._ck(self.L.falcon_solver_vcycle_op(self.h, C.c_int32(op), C.c_int32(level), _ptr(a),
                                                 None if b is None else _ptr(b), _ptr(out)))
         return out

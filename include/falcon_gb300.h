@@ -530,12 +530,24 @@ int  falcon_solver_coarse_form(const falcon_solver* sv, int32_t* form);
  *               i+j+k even / odd) with the halo filled from z first; each
  *               updated cell takes the Jacobi formula of
  *               ModMultigrid_Jacobi_Mz_r (3_5/ModMultigrid.f90:316-324)
- *   RESIDUAL:   in0 = r, in1 = z -> out = r - A z (halo filled from z) */
+ *   RESIDUAL:   in0 = r, in1 = z -> out = r - A z (halo filled from z)
+ * and the forms that a V-cycle makes of them:
+ *   RESIDUAL_RESTRICT: in0 = r, in1 = z -> out = the residual, restricted (level+1)
+ *   FIRST_SWEEP: in0 = r -> out = z after a red and a black half sweep from z = 0
+ *   PROLONG_SWEEP: in0 = coarse correction (level+1), in1 = r and behind it z ->
+ *               out = z + injection of in0, after a black half sweep
+ *   COARSE_SWEEPS: the coarsest of several levels, in0 = r -> out = z after the
+ *               coarsest level's red-black sweeps (falcon_solver_set_smoothing)
+ *               from z = 0; falcon_solver_coarse_form tells how they run */
 #define FALCON_VCYCLE_RESTRICT     0
 #define FALCON_VCYCLE_PROLONG_ADD  1
 #define FALCON_VCYCLE_SMOOTH_RED   2
 #define FALCON_VCYCLE_SMOOTH_BLACK 3
 #define FALCON_VCYCLE_RESIDUAL     4
+#define FALCON_VCYCLE_RESIDUAL_RESTRICT 5
+#define FALCON_VCYCLE_FIRST_SWEEP       6
+#define FALCON_VCYCLE_PROLONG_SWEEP     7
+#define FALCON_VCYCLE_COARSE_SWEEPS     8
 int  falcon_solver_vcycle_op(falcon_solver* sv, int32_t op, int32_t level, const float* in0, const float* in1,
                              float* out);
 /* level-0 block geometry, for a driver that evaluates its own fields on the
