@@ -21,7 +21,9 @@ __device__ __forceinline__ float rcp_approx(float x) {   // infinity of what FP3
 // sign and exponent changes of doubles run on the integer pipes instead (a
 // positive double orders as its bit pattern), and a division by a value that
 // many cells share goes through its reciprocal. Every function below gives the
-// bits of the expression that it stands for.
+// bits of the expression that it stands for; face_flux_h does so for speeds within
+// 2^-590 .. 2^440, between which the halvings that it moves are exact (a face's
+// speed is at least two sound speeds).
 __device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
     return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
@@ -61,7 +63,7 @@ __device__ __forceinline__ double div_by(double a, const Divisor& d) {
     return q;
 }
 
-// Half the minmod slope of a cell (minmod() below times 0.5) from its
+// Half the minmod slope of a cell (minmod() times 0.5) from its
 // differences dl = u - ul, dr = ur - u and da = ur - ul. With a = da/2, b =
 // 2 dr, c = 2 dl the selector max(0,ab) max(0,bc) 1e10 >= 1e-30 needs equal
 // signs and |a| |b|^2 |c| >= 1e-40: the exponents' sum E puts that product in

@@ -3,7 +3,7 @@
 // Instantiated twice:
 //   mhd_fp64.cu  (T = double, compiled with -fmad=false): every operation in the
 //                reference's order, bit-comparable with the CPU oracle;
-//   mhd_mixed.cu (T = float): FP32 state and stencil RHS, p1 assembled in FP64.
+//   mhd_mixed.cu (T = float): FP32 state and stencil RHS, p1 in float-float.
 //
 // Data layout in HBM (one state buffer), cells kp, jp, ip with ip fastest, padded
 // extents nip = ni + 4 etc.:

@@ -18,7 +18,7 @@ template <class K> cudaError_t allow_smem(OncePerDevice& once, K kernel, size_t 
 // Launch of a kernel that calls step_wait: with d.overlap (grids of up to 2^20 cells
 // without psi, whose kernels run on a branch of their own) it may start while the
 // kernel before it in the stream drains (and, if that calls step_go, as soon as all
-// its CTAs run). Step without / with: 8^3 blocks, 111k cells 71 / 69 us, 442k 178
+// its CTAs run). Step without / with: 8^3 blocks, 111k cells 61 / 54 us, 442k 178
 // / 174; 16^3, 442k 158 / 153, 885k 290 / 287. Larger grids lose by it, their slots
 // taken by waiting CTAs while many remain to run: 16^3, 5.3M cells 1,150 / 1,167, 21M
 // 3,982 / 4,074; 8^3, 2.7M 740 / 806.

@@ -192,13 +192,6 @@ struct Shape {
     static constexpr size_t off_gj = off_gi + (size_t)GI_COUNT * NIP * sizeof(T);
     static constexpr size_t off_gs = off_gj + (size_t)GJ_COUNT * NJP * sizeof(T);
     static constexpr size_t smem_stage = off_gs + GS_COUNT * sizeof(T);
-    // FP32 stage: as many CTAs per SM as the shared memory holds (228 KB per
-    // SM, 1 KB reserved per CTA), so the register allocation must fit them
-    // too (at least 32 registers a thread). FP64 keeps the compiler's choice.
-    static constexpr int by_smem = (int)(233472 / (smem_stage + 1024));
-    static constexpr int reg_cap = 2048 / NT;
-    static constexpr int min_blocks =
-        sizeof(T) != 4 || by_smem < 2 ? 1 : (by_smem < reg_cap ? by_smem : (reg_cap < 1 ? 1 : reg_cap));
 };
 
 // Thread 0: bulk-copy planes kp in [lo,hi) of all variables of the block into
@@ -311,30 +304,18 @@ __device__ __forceinline__ void load_push_block(const PushTable& P, int b, PushB
     }
 }
 
-// Cell (i, j, kq) of a thread in a k-chunk. With 16-wide rows and an even
-// chunk depth a warp takes one row of two adjacent planes (lanes 0-15 plane
-// kq, 16-31 plane kq+1): a plane is 400 floats, 16 banks apart, so every
-// shared-memory access of the stencil is free of bank conflicts (two rows of
-// one plane, 20 floats apart, share 4 banks). Otherwise rows of one plane.
-// i stays the fastest index within 16 or 8 lanes either way.
-template <int NI, int NJ, int KPAR>
+// Cell (i, j, kq) of a thread in a k-chunk: rows of one plane, then the next plane.
+template <int NI, int NJ>
 __device__ __forceinline__ void cell_of_thread(int tid, int& i, int& j, int& kq) {
-    if constexpr (NI == 16 && KPAR % 2 == 0) {
-        i = tid % NI;
-        const int pair = (tid / NI) % 2;
-        j = (tid / (2 * NI)) % NJ;
-        kq = 2 * (tid / (2 * NI * NJ)) + pair;
-    } else {
-        i = tid % NI;
-        j = (tid / NI) % NJ;
-        kq = tid / (NI * NJ);
-    }
+    i = tid % NI;
+    j = (tid / NI) % NJ;
+    kq = tid / (NI * NJ);
 }
 
 // ---------------------------------------------------------------------------
 // One RK stage of one block: boundary -> RHS (3_6/ModEquation.f90:24-162) ->
 // u_out = u^n + dt*R/(5-s) (3_6/ModAdvance.f90:87-93).
-// FP64 (the mixed stage: stage_quads).
+// FP64 (the mixed stage: stage_march, stage_chunks).
 template <int NI, int NJ, int NK, int KPAR, int DIVB>
 __global__ void __launch_bounds__(NI* NJ* KPAR)
 k_stage(const double* in, const double* un, double* out, DivBArgs psi, Geometry g, StepScalars* sc, int stage,
@@ -388,7 +369,7 @@ k_stage(const double* in, const double* un, double* out, DivBArgs psi, Geometry 
 
     const int tid = threadIdx.x;
     int i, j, kq;
-    cell_of_thread<NI, NJ, KPAR>(tid, i, j, kq);
+    cell_of_thread<NI, NJ>(tid, i, j, kq);
     const int ii = i + 2, jj = j + 2;
     const T c1 = gs[GS_C1], c2 = gs[GS_C2], c3 = gs[GS_C3];
     const T* GR = gi + GI_R * NIP;
@@ -400,8 +381,8 @@ k_stage(const double* in, const double* un, double* out, DivBArgs psi, Geometry 
     const T rho0c = GRHO0[ii];
     const T gor0 = gi[GI_GOR0 * NIP + ii], heat = gi[GI_HEAT * NIP + ii], xi2inv = gi[GI_XI2INV * NIP + ii];
     const double dt = sc->dt;
-    // (dt R) / (5 - stage): for 4, 2, 1 (stages 1, 3, 4) the division is exact
-    // and goes into dt, the same bits; stage 2 divides by 3
+    // (dt R) / (5 - stage): for 4, 2, 1 (stages 1, 3, 4) the division is exact and goes
+    // into dt, the same bits while dt R / 4 is a normal number; stage 2 divides by 3
     const Divisor three{3.0, 1.0 / 3.0, 1000u};
     const double dts = stage == 2 ? dt : dt / (double)(5.0f - (float)stage);
     auto advance = [&](double R) {   // (dt R) / (5 - stage)
@@ -664,8 +645,8 @@ k_stage(const double* in, const double* un, double* out, DivBArgs psi, Geometry 
 // plus one integer selector, 17 in the formula), a face's difference is the
 // slopes' own, its speed sum is formed once for all variables, only faces near
 // an extremum divide (face_flux_h) and the sums divide by reciprocals (div_by).
-// 442,368 cells, CUDA events: 8^3 blocks 1678 -> 768 us (251 -> 105 FP64
-// instructions per cell and variable), 16^3 blocks 2385 (chunked kernel) -> 971 us.
+// 442,368 cells, CUDA events: 8^3 blocks 1678 -> 587 us, 16^3 blocks 2385 (chunked
+// kernel) -> 731 us (768 and 971 before the limiter's quotient was formed by digits).
 template <int NI, int NJ, int NK, int VPT>
 struct M64Shape {
     static constexpr int NG = 2, NIP = NI + 4, NJP = NJ + 4, NKP = NK + 4;

@@ -538,7 +538,7 @@ __device__ __forceinline__ void stage_chunks(int b, int ch0, int ch1, const floa
     __syncthreads();   // barriers and tables are used by every thread below
 
     int i, j, kq;
-    cell_of_thread<NI, NJ, KPAR>(tid, i, j, kq);
+    cell_of_thread<NI, NJ>(tid, i, j, kq);
     const int ii = i + 2, jj = j + 2, c0 = jj * NIP + ii;
     const float dtk = sc->dt_stage_f[stage - 1];
     const int polls = sc->wait_polls;
@@ -1031,7 +1031,6 @@ struct MShape {
     static constexpr int W = 5;                          // plane ring slots
     static constexpr int PLI = NI * NJ, NINT = PLI * NK;
     static constexpr int NP = NV / 2;                    // variable pairs
-    static constexpr uint32_t PLB = PL * 4u;
     static constexpr int P = 20;                         // row pitch (pairs) of the slope and face arrays
     // per pair (float2): SI[NJ][P] slopes along i of cells i = -1..NI at i + 1;
     // SJ[NJ + 2][P] slopes along j of rows j = -1..NJ at row j + 1;
@@ -1216,7 +1215,7 @@ __device__ __forceinline__ void march_quads(int b, int ka, int kb, const float* 
             pairs(s0, c0 - NIP, d);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-                                const float2* si = SI + q * S::NSI + j * P + i;
+                const float2* si = SI + q * S::NSI + j * P + i;
                 const float2* sj = SJ + q * S::NSJ + j * P + i;
                 fi0[q] = face_flux2(l[q], u0[q], si[0], si[1], cci);
                 fj0[q] = face_flux2(d[q], u0[q], sj[0], sj[P], ccj);

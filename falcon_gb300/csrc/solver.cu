@@ -17,9 +17,9 @@
 //     Galerkin coarse operators;
 //   - every problem of a batch is advanced by the same launches: kernels index
 //     block -> problem, scalars are per problem, converged problems freeze.
-// Kernels are launched with one CTA per block (grid.x = block) looping over the
-// block's cells, so a CTA never mixes problems and its reductions go to one
-// per-problem slot with one atomic.
+// The cell kernels' CTAs take chunks of one block's cells, so a CTA never mixes problems
+// and its reductions go to one per-problem slot with one atomic; the V-cycle's threads
+// take pairs of cells of a row (vcycle.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -860,8 +860,7 @@ cudaError_t coarse_sweeps(falcon_solver* sv, int sweeps, float* zout) {
     coarse_config(sv, &cfg, at);
     const SvLevel& L = sv->lv.back();
     return cudaLaunchKernelEx(&cfg, coarse_kernel(L.d.m0, sv->coarse_r, sv->coarse_cluster > 1), L.view(sv->S.nblocks),
-                              CoarseArgs{sv->first, sv->cghost, sv->ceat, sv->cew, sv->clist, sweeps, sv->coarse_cluster,
-                                         sv->coarse_slots},
+                              CoarseArgs{sv->first, sv->cghost, sv->ceat, sv->cew, sv->clist, sweeps, sv->coarse_cluster},
                               (const float*)L.r, zout);
 }
 // A kernel's opt-ins hold for every solver of the process, whichever set them last: all
@@ -872,11 +871,13 @@ cudaError_t allow_coarse(CoarseKernel kern, int cluster) {
     if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
-// Whether the coarsest level's sweeps run as one launch, and with how many CTAs
-// per problem: the smallest cluster that holds the largest problem at two
-// cells per thread and colour, one cell where that fits too. Batches whose
-// clusters would take more than three waves of SMs keep a launch per half
-// sweep, which advances all problems at once. Builds the neighbour words.
+// Whether the coarsest level's sweeps run as one launch, and with how many CTAs per
+// problem: the cluster with the shortest estimated half sweep -- 0.35 us of barriers in a
+// single CTA, 1 in a cluster, and 0.25 per cell of a thread and colour -- times the waves
+// that the batch's clusters take. Above 4 us (four waves of clusters, say) a launch per
+// half sweep, which advances all problems at once, is the faster form. The constants follow
+// the measured sums: 64 half sweeps of a 24 x 45 problem 48 us in one CTA with two cells,
+// of eight problems in clusters of eight with four cells 315 us. Builds the neighbour words.
 int plan_coarse(falcon_solver* sv, const std::vector<int32_t>& ghost, const std::vector<int32_t>& isrc,
                 const std::vector<uint8_t>& icode, const std::vector<float>& iw) {
     const SolverProblemSet& S = sv->S;
@@ -1714,13 +1715,13 @@ cudaError_t run_inner(falcon_solver* sv, int pc, int max_it, InnerCtl* ctl) {
     }
 }
 
-// The solver's autotuner: times one eager FCG iteration (V-cycle with the
-// solver's smoothing, the float-float kernels, halo fills) for each candidate
-// tile -- cells per CTA in {512, 1024, 2048, 4096} (a multiple of the row
-// length, so the red-black sweep's colour-only form applies) x threads per
-// CTA in {128, 256, 512} -- on this solver's own grid, and keeps the fastest.
-// Runs once, at the first solve, on scratch vectors that the solve
-// initialises afterwards.
+// The solver's autotuner: times two eager FCG iterations for each candidate tile of the
+// cell kernels -- cells per CTA in {512, 1024, 2048, 4096}, whole rows, x threads per
+// CTA in {128, 256, 512} -- on this solver's own grid, and keeps the fastest. What
+// differs between candidates is the operator and the update; the V-cycle, which does
+// not use the tile, brings the vectors through the caches between them as in a solve.
+// Runs once, at the first solve, on scratch vectors that the solve initialises
+// afterwards.
 int autotune_tile(falcon_solver* sv) {
     if (sv->tuned) return FALCON_OK;
     const int np = sv->S.nproblems;

@@ -346,7 +346,6 @@ struct CoarseArgs {
     const int4* list;
     int sweeps;                // red-black sweeps
     int cluster;               // CTAs per problem
-    int slots;                 // most entries of one colour in a CTA
 };
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
