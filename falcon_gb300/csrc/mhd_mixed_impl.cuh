@@ -47,25 +47,28 @@ __device__ __forceinline__ float2 half_slope2(float2 ul, float2 u, float2 ur) {
 
 // The limited flux through a face (3_6/ModDiffusion.f90:40-60) from its two cells'
 // values and half slopes: -(phi/2 num) speed/2 with phi = max(0, 1 + 2 (num/den - 1)),
-// den = fr - fl, num the jump left between the reconstructions; cc = -speed/4, speed
+// den = fr - fl, num the jump left between the reconstructions; cc = -2 speed, speed
 // the sum of the cells' |v_dir| + c_s. Slopes have den's sign or are 0, so num/den is at
-// most 1 and phi lies in [0, 1]; one saturating FMA forms it, 0/0 as 0. The quotient is
-// num times the approximate reciprocal of den, infinite for a denormal den, which makes
-// phi 1: right, since the slopes' selector has den's square and is 0 there unless the
-// cells' other differences exceed 5e17.
-__device__ __forceinline__ float limiter_phi(float r) { return __saturatef(__fmaf_rn(r, 2.f, -1.f)); }
+// most 1, and the quotient, num times the approximate reciprocal of den, at most 1 + 2^-22:
+// phi/8 saturates to [0, 1] without rounding it again from above; one saturating FMA
+// forms it, 0/0 as 0. The reciprocal flushes a denormal den, whose quotient is infinite:
+// the bound above makes phi 1 there, the value for slopes of 0, which the selector gives
+// (it has den's square) unless the cells' other differences exceed 5e17.
+__device__ __forceinline__ float eighth_phi(float r) {
+    return fminf(__saturatef(__fmaf_rn(r, 0.25f, -0.125f)), 0.125f * (1.f + 1.f / (1 << 21)));
+}
 __device__ __forceinline__ float face_flux(float fl, float fr, float hL, float hR, float cc) {
     const float num = __fsub_rn(__fsub_rn(__fsub_rn(fr, hR), fl), hL);
-    return __fmul_rn(__fmul_rn(limiter_phi(__fmul_rn(num, rcp_approx(__fsub_rn(fr, fl)))), num), cc);
+    return __fmul_rn(__fmul_rn(eighth_phi(__fmul_rn(num, rcp_approx(__fsub_rn(fr, fl)))), num), cc);
 }
 __device__ __forceinline__ float2 face_flux2(float2 fl, float2 fr, float2 hL, float2 hR, float2 cc) {
     const float2 num = sub2(sub2(sub2(fr, hR), fl), hL), den = sub2(fr, fl);
     const float2 r = __fmul2_rn(num, f2(rcp_approx(den.x), rcp_approx(den.y)));
-    return __fmul2_rn(__fmul2_rn(f2(limiter_phi(r.x), limiter_phi(r.y)), num), cc);
+    return __fmul2_rn(__fmul2_rn(f2(eighth_phi(r.x), eighth_phi(r.y)), num), cc);
 }
 // cc of a face: uL, uR the velocity across it, csL, csR the sound speeds of its cells
 __device__ __forceinline__ float face_speed(float uL, float csL, float uR, float csR) {
-    return -0.25f * ((fabsf(uR) + csR) + (fabsf(uL) + csL));
+    return -2.f * ((fabsf(uR) + csR) + (fabsf(uL) + csL));
 }
 
 // (hi + q*unit(hi)) + d for four values, rounded to the nearest (hi', q') pairs: two
