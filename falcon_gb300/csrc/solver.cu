@@ -872,12 +872,13 @@ cudaError_t allow_coarse(CoarseKernel kern, int cluster) {
     return e;
 }
 // Whether the coarsest level's sweeps run as one launch, and with how many CTAs per
-// problem: the cluster with the shortest estimated half sweep -- 0.35 us of barriers in a
-// single CTA, 1 in a cluster, and 0.25 per cell of a thread and colour -- times the waves
-// that the batch's clusters take. Above 4 us (four waves of clusters, say) a launch per
-// half sweep, which advances all problems at once, is the faster form. The constants follow
-// the measured sums: 64 half sweeps of a 24 x 45 problem 48 us in one CTA with two cells,
-// of eight problems in clusters of eight with four cells 315 us. Builds the neighbour words.
+// problem: the cluster with the shortest estimated half sweep -- barriers (a cluster's
+// take about three times a CTA's) plus a share per cell of a thread and colour -- times
+// the waves that the batch's clusters take, as far as the estimate stays below 4. A launch
+// per half sweep advances all problems at once and is as fast from there on. us per
+// iteration with 32 sweeps, one launch / launches: 24 x 45 127 / 416, 64 x 180 (16 CTAs of
+// four cells) 780 / 916, 16 x 24 x 45 262 / 603, batch of 8 1,012 / 1,180; above the
+// limit 16 problems 2,494 / 2,475, 32 problems 4,724 / 4,424. Builds the neighbour words.
 int plan_coarse(falcon_solver* sv, const std::vector<int32_t>& ghost, const std::vector<int32_t>& isrc,
                 const std::vector<uint8_t>& icode, const std::vector<float>& iw) {
     const SolverProblemSet& S = sv->S;
