@@ -845,36 +845,46 @@ int setup_device(falcon_ctx* ctx) {
         {   // interpolated entries in target order: a warp's eight stores per
             // entry then write neighbouring ghost cells (its gathers still read
             // neighbouring source rows; measured faster than source order)
-            std::vector<size_t> ord(idst.size());
-            for (size_t q = 0; q < ord.size(); ++q) ord[q] = q;
-            std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return idst[a] < idst[b]; });
-            if (!snap) {
-                // FP64: entries of one kind together (which axes are near, to which
-                // side: ghost_weights), so that a warp's entries take one path
-                auto cls = [&](size_t q) {
+            // A block's entries are sorted on their own: target offsets ascend with the block.
+            const size_t n = idst.size();
+            std::vector<size_t> ord(n);
+            // FP64: entries of one class together (which axes are near, to which side:
+            // ghost_weights), so that a warp's entries take one path; in target order within
+            constexpr size_t kClasses = 4 * 27;
+            std::vector<uint8_t> cls(snap ? 0 : n);
+            std::vector<std::array<size_t, kClasses>> place(snap ? 0 : nb);   // of a block's next entry, by class
+#pragma omp parallel for schedule(dynamic, 16)
+            for (int b = 0; b < nb; ++b) {
+                for (size_t q = oi[b]; q < oi[b + 1]; ++q) ord[q] = q;
+                std::sort(ord.begin() + (long)oi[b], ord.begin() + (long)oi[b + 1], [&](size_t x, size_t y) { return idst[x] < idst[y]; });
+                if (snap) continue;
+                place[b].fill(0);
+                for (size_t q = oi[b]; q < oi[b + 1]; ++q) {
                     int c = ikind[q];
                     for (int t = 0; t < 3; ++t) c = 3 * c + (iw[3 * q + t] < 1e-12 ? 0 : iw[3 * q + t] > 1.0 - 1e-12 ? 1 : 2);
-                    return c;
-                };
-                std::vector<uint8_t> c(ord.size());
-                std::array<size_t, 4 * 27 + 1> at{};
-                for (size_t q = 0; q < c.size(); ++q) ++at[(size_t)(c[q] = (uint8_t)cls(q)) + 1];
-                for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
-                std::vector<size_t> by(ord.size());
-                for (size_t q : ord) by[at[c[q]]++] = q;
-                ord.swap(by);
+                    ++place[b][cls[q] = (uint8_t)c];
+                }
             }
-            std::vector<int32_t> d2(ord.size()), s2(ord.size());
-            std::vector<double> w2(3 * ord.size()), r2(2 * ord.size());
-            std::vector<uint8_t> k2(ord.size());
-            for (size_t q = 0; q < ord.size(); ++q) {
-                const size_t o = ord[q];
-                d2[q] = idst[o];
-                s2[q] = isrc[o];
-                for (int t = 0; t < 3; ++t) w2[3 * q + t] = iw[3 * o + t];
-                for (int t = 0; t < 2; ++t) r2[2 * q + t] = irot[2 * o + t];
-                k2[q] = ikind[o];
-            }
+            if (!snap)
+                for (size_t k = 0, at = 0; k < kClasses; ++k)
+                    for (int b = 0; b < nb; ++b) {
+                        const size_t m = place[b][k];
+                        place[b][k] = at;
+                        at += m;
+                    }
+            std::vector<int32_t> d2(n), s2(n);
+            std::vector<double> w2(3 * n), r2(2 * n);
+            std::vector<uint8_t> k2(n);
+#pragma omp parallel for schedule(dynamic, 16)
+            for (int b = 0; b < nb; ++b)
+                for (size_t x = oi[b]; x < oi[b + 1]; ++x) {
+                    const size_t o = ord[x], q = snap ? x : place[b][cls[o]]++;
+                    d2[q] = idst[o];
+                    s2[q] = isrc[o];
+                    for (int t = 0; t < 3; ++t) w2[3 * q + t] = iw[3 * o + t];
+                    for (int t = 0; t < 2; ++t) r2[2 * q + t] = irot[2 * o + t];
+                    k2[q] = ikind[o];
+                }
             idst.swap(d2);
             isrc.swap(s2);
             iw.swap(w2);
