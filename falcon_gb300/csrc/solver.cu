@@ -647,7 +647,9 @@ struct SvLevel {
     Ops2 ops2() const { return Ops2{Aii2, Ai2, Aj2, Ak2}; }
     Ops64 ops64() const { return Ops64{Aii, Ai, Aj, Ak}; }
     VLevel view(int nb) const {
-        return VLevel{d.m0, d.nint, nb, fAii, fAi, fAj, fAk, ghost, isrc, icode, iw, nbr};
+        const uint32_t h = (uint32_t)d.m0 / 2, mh = h * d.m0;
+        auto inverse = [](uint32_t x) { return x > 1 ? (uint32_t)((1ull << 32) / x + 1) : 0u; };
+        return VLevel{d.m0, d.nint, nb, inverse(h), inverse(mh), fAii, fAi, fAj, fAk, ghost, isrc, icode, iw, nbr};
     }
 };
 
@@ -787,6 +789,17 @@ void vsweep_pairs(falcon_solver* sv, int l, const float* zin, const float* zc, f
     const VLevel V = L.view(sv->S.nblocks);
     k_vsweep<M, MODE><<<vgrid((int64_t)V.nb * V.nint / 2), kVThreads, 0, sv->st>>>(V, L.r, zin, zc, zout, colour);
 }
+// of the kernels for any m (Cell)
+struct AnyGrid {
+    unsigned threads, ctas;
+    explicit AnyGrid(const VLevel& V)
+        : threads((unsigned)std::min(kVThreads, (V.nint + 31) / 32 * 32)), ctas((unsigned)V.nb * ((V.nint + threads - 1) / threads)) {}
+};
+// m not a power of two: pairs of cells above 1e5 cells of an even m, else a thread per
+// cell with all its ghosts' loads at once. us per iteration by pairs / by cells: levels of
+// 83k cells 137 / 109, of 166k 149 / 179, of 384k 126 / 160, of 2.2M 423 / 774
+bool even_pairs(const VLevel& V) { return V.m % 2 == 0 && (int64_t)V.nb * V.nint > 100000; }
+unsigned even_grid(const VLevel& V) { return (unsigned)V.nb * (((unsigned)V.nint / 2 + kVThreads - 1) / kVThreads); }
 template <int MODE>
 cudaError_t vsweep(falcon_solver* sv, int l, const float* zin, const float* zc, float* zout, int colour) {
     const SvLevel& L = sv->lv[l];
@@ -798,8 +811,18 @@ cudaError_t vsweep(falcon_solver* sv, int l, const float* zin, const float* zc, 
     case 32: vsweep_pairs<32, MODE>(sv, l, zin, zc, zout, colour); break;
     default: {
         const VLevel V = L.view(sv->S.nblocks);
-        k_vsweep_any<MODE><<<vgrid((int64_t)V.nb * V.nint), kVThreads, 0, sv->st>>>(V, L.r, zin, zc, zout,
-                                                                                                  colour);
+        const AnyGrid g(V);
+        if constexpr (MODE == V_FIRST) {   // the red half sweep into the level's other buffer
+            float* red = zout == L.z ? L.zb : L.z;
+            k_vfirst_any<<<g.ctas, g.threads, 0, sv->st>>>(V, L.r, red);
+            zin = red;
+        } else if constexpr (MODE == V_PROLONG) {   // in place where a sweep follows
+            float* sum = colour < 0 ? zout : zin == L.z ? L.z : L.zb;
+            k_vprolong_any<<<g.ctas, g.threads, 0, sv->st>>>(V, zin, zc, sum);
+            if (colour < 0) break;
+        }
+        if (even_pairs(V)) k_vsweep_even<<<even_grid(V), kVThreads, 0, sv->st>>>(V, L.r, zin, zout, colour);
+        else k_vsweep_any<<<g.ctas, g.threads, 0, sv->st>>>(V, L.r, zin, zout, colour);
     }
     }
     return cudaGetLastError();
@@ -807,7 +830,9 @@ cudaError_t vsweep(falcon_solver* sv, int l, const float* zin, const float* zc, 
 cudaError_t vresid(falcon_solver* sv, int l, const float* z, float* res) {
     const SvLevel& L = sv->lv[l];
     const VLevel V = L.view(sv->S.nblocks);
-    k_vresid<<<vgrid((int64_t)V.nb * V.nint), kVThreads, 0, sv->st>>>(V, L.r, z, res);
+    const AnyGrid g(V);
+    if (even_pairs(V)) k_vresid_even<<<even_grid(V), kVThreads, 0, sv->st>>>(V, L.r, z, res);
+    else k_vresid<<<g.ctas, g.threads, 0, sv->st>>>(V, L.r, z, res);
     return cudaGetLastError();
 }
 // rc = R (r - A z)

@@ -29,6 +29,7 @@ __device__ __forceinline__ float gs_value(float r, float off, float aii) { retur
 
 struct VLevel {
     int m, nint, nb;           // cells per block edge and block, blocks
+    uint32_t inv_h, inv_mh;    // 2^32 / (m / 2) and 2^32 / (m^2 / 2), rounded up (EvenPair)
     const float *Aii, *Ai, *Aj, *Ak;
     const int32_t* ghost;      // [nb][6 m^2]: faces i-, i+ [k][j], j-, j+ [k][i], k-, k+ [j][i];
                                // >= 0 source cell, -1 none (0), <= -2 interpolation entry -(v + 2)
@@ -148,29 +149,96 @@ struct Coef7 {
     }
 };
 
-// One half sweep of `colour` (0 red: i + j + k even counted from 1; -1: none)
-// out of place; with V_FIRST the whole first red-black sweep (colour = 1).
-// m not a power of two: a thread per cell.
-template <int MODE>
-__global__ void k_vsweep_any(const __grid_constant__ VLevel V, const float* __restrict__ r, const float* __restrict__ zin,
-                             const float* __restrict__ zc, float* __restrict__ zout, int colour) {
-    const int m = V.m, q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= V.nb * V.nint) return;
-    const Start<0, MODE> f{r, V.Aii, zin, zc, m};
-    const int i = q % m, row = q / m, j = row % m, k = (row / m) % m, b = row / (m * m);
-    float v = f(q);
-    if (((i + j + k + 1) & 1) == colour) {
-        const Faces F(V, b);
-        const Coef7 A(V, m, b, i, j, k, q);
-        float off = A.c[0] * neighbour<0>(V, F, b, i, j, k, q, f);
-        off = fmaf(A.c[1], neighbour<1>(V, F, b, i, j, k, q, f), off);
-        off = fmaf(A.c[2], neighbour<2>(V, F, b, i, j, k, q, f), off);
-        off = fmaf(A.c[3], neighbour<3>(V, F, b, i, j, k, q, f), off);
-        off = fmaf(A.c[4], neighbour<4>(V, F, b, i, j, k, q, f), off);
-        off = fmaf(A.c[5], neighbour<5>(V, F, b, i, j, k, q, f), off);
-        v = gs_value(r[q], off, A.c[6]);
+// Cells of the kernels for any m: a thread per cell, CTAs within one block. Lanes without
+// a cell (on = false) take part in the warp's votes.
+struct Cell {
+    int b, i, j, k, q;
+    bool on;
+    __device__ __forceinline__ Cell(const VLevel& V) {
+        const int m = V.m, n = (V.nint + blockDim.x - 1) / blockDim.x;
+        b = blockIdx.x / n;
+        const int c = (blockIdx.x - b * n) * blockDim.x + threadIdx.x, row = c / m;
+        on = c < V.nint;
+        i = c - row * m;
+        j = row % m;
+        k = row / m;
+        q = b * V.nint + c;
     }
-    zout[q] = v;
+};
+// The six neighbours' values of a cell (0 for lanes that want none). What bounds these
+// kernels is latency: a ghost is its descriptor, an entry's fields and its corners, one
+// after the other, so each of the three is loaded for all faces at once.
+__device__ __forceinline__ void six_neighbours(const VLevel& V, const Cell& C, bool want, const float* __restrict__ z, float (&n)[6]) {
+    const int m = V.m, mm = m * m;
+    int src[6];
+    bool entry = false;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+        const int on = f < 2 ? C.i : f < 4 ? C.j : C.k, st = f < 2 ? 1 : f < 4 ? m : mm;
+        const int t = f < 2 ? C.k * m + C.j : f < 4 ? C.k * m + C.i : C.j * m + C.i;
+        src[f] = C.q + ((f & 1) ? st : -st);
+        if (!((f & 1) ? on < m - 1 : on > 0)) src[f] = want ? V.ghost[((size_t)C.b * 6 + f) * mm + t] : -1;
+        entry |= want && src[f] <= -2;
+    }
+#pragma unroll
+    for (int f = 0; f < 6; ++f) n[f] = want && src[f] >= 0 ? z[src[f]] : 0.f;
+    if (!__any_sync(0xffffffffu, entry)) return;
+    int s[6], cd[6];
+    float w[6][3];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+        const bool is = want && src[f] <= -2;
+        const int e = is ? -(src[f] + 2) : 0;
+        s[f] = is ? V.isrc[e] : 0;
+        cd[f] = is ? V.icode[e] : -1;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) w[f][d] = is ? V.iw[3 * e + d] : 0.f;
+    }
+    float c[6][8];   // corner t: bit d of t one cell on along d; those of weight 0 are not read
+#pragma unroll
+    for (int f = 0; f < 6; ++f)
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+            c[f][t] = cd[f] >= 0 && (t & ~cd[f]) == 0 ? z[s[f] + (t & 1) + (t & 2 ? m : 0) + (t & 4 ? mm : 0)] : 0.f;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+        if (cd[f] < 0) continue;
+        const float wi = w[f][0], wj = w[f][1], wk = w[f][2], ui = 1.f - wi, uj = 1.f - wj, uk = 1.f - wk;
+        n[f] = c[f][0] * ui * uj * uk + c[f][1] * wi * uj * uk + c[f][2] * ui * wj * uk + c[f][4] * ui * uj * wk +
+               c[f][3] * wi * wj * uk + c[f][6] * ui * wj * wk + c[f][5] * wi * uj * wk + c[f][7] * wi * wj * wk;
+    }
+}
+
+// For m not a power of two: z = r / Aii on red cells, 0 on black ones (the red half sweep
+// from 0); z plus the coarse correction of the cell's parent; one half sweep of `colour`
+// (0 red: i + j + k even counted from 1) out of place.
+__global__ void k_vfirst_any(const __grid_constant__ VLevel V, const float* __restrict__ r, float* __restrict__ z) {
+    const Cell C(V);
+    if (C.on) z[C.q] = ((C.i + C.j + C.k + 1) & 1) == 0 ? gs_value(r[C.q], 0.f, V.Aii[C.q]) : 0.f;
+}
+__global__ void k_vprolong_any(const __grid_constant__ VLevel V, const float* zin, const float* __restrict__ zc, float* zout) {
+    const Cell C(V);
+    const int h = V.m >> 1;
+    if (C.on) zout[C.q] = zin[C.q] + zc[((C.b * h + (C.k >> 1)) * h + (C.j >> 1)) * h + (C.i >> 1)];
+}
+__global__ void k_vsweep_any(const __grid_constant__ VLevel V, const float* __restrict__ r, const float* __restrict__ zin,
+                             float* __restrict__ zout, int colour) {
+    const Cell C(V);
+    const bool upd = C.on && ((C.i + C.j + C.k + 1) & 1) == colour;
+    float v = C.on && !upd ? zin[C.q] : 0.f, rq = 0.f, n[6];
+    float a[7] = {};
+    if (upd) {
+        const Coef7 A(V, V.m, C.b, C.i, C.j, C.k, C.q);
+#pragma unroll
+        for (int f = 0; f < 7; ++f) a[f] = A.c[f];
+        rq = r[C.q];
+    }
+    six_neighbours(V, C, upd, zin, n);
+    float off = a[0] * n[0];
+#pragma unroll
+    for (int f = 1; f < 6; ++f) off = fmaf(a[f], n[f], off);
+    if (upd) v = gs_value(rq, off, a[6]);
+    if (C.on) zout[C.q] = v;
 }
 
 constexpr int kVThreads = 128;   // of a V-cycle kernel's CTA
@@ -200,16 +268,33 @@ struct Pair {
     }
 };
 
+// ... and of any even m: CTAs within one block, divisions by multiplication (exact here:
+// the dividends stay below 2^32 / m^2).
+struct EvenPair {
+    int b, k, j, i0, q0;
+    bool on;
+    __device__ __forceinline__ EvenPair(const VLevel& V) {
+        const int m = V.m, h = m >> 1, per = m * m * h, n = (per + kVThreads - 1) / kVThreads;
+        b = blockIdx.x / n;
+        const unsigned y = (blockIdx.x - b * n) * kVThreads + threadIdx.x;
+        on = y < (unsigned)per;
+        k = __umulhi(y, V.inv_mh);
+        const unsigned x = y - k * (m * h);
+        j = __umulhi(x, V.inv_h);
+        i0 = 2 * (x - j * h);
+        q0 = ((b * m + k) * m + j) * m + i0;
+    }
+};
+
+// One half sweep of `colour` (-1: none) on the pair at q0, out of place; with V_FIRST the
+// whole first red-black sweep (colour = 1).
 template <int M, int MODE>
-__global__ void __launch_bounds__(kVThreads)
-k_vsweep(const __grid_constant__ VLevel V, const float* __restrict__ r, const float* __restrict__ zin,
-         const float* __restrict__ zc, float* __restrict__ zout, int colour) {
-    const Pair<M> C;
-    const int b = C.b, j = C.j, k = C.k, q0 = C.q0;
-    if (b >= V.nb) return;
-    const Start<M, MODE> f{r, V.Aii, zin, zc, M};
-    const int odd = (colour + j + k + 1) & 1;   // which of the two cells has the colour
-    const int i = C.i0 + odd, q = q0 + odd;
+__device__ __forceinline__ void vsweep_pair(const VLevel& V, const float* __restrict__ r, const float* __restrict__ zin,
+                                            const float* __restrict__ zc, float* __restrict__ zout, int colour, int b, int i0,
+                                            int j, int k, int q0) {
+    const Start<M, MODE> f{r, V.Aii, zin, zc, V.m};
+    const int m = f.m(), odd = (colour + j + k + 1) & 1;   // which of the two cells has the colour
+    const int i = i0 + odd, q = q0 + odd;
     const Faces F(V, b);
     float2 z;
     if constexpr (MODE == V_FIRST) {
@@ -219,14 +304,14 @@ k_vsweep(const __grid_constant__ VLevel V, const float* __restrict__ r, const fl
     } else {
         z = *reinterpret_cast<const float2*>(zin + q0);
         if constexpr (MODE == V_PROLONG) {
-            constexpr int h = M / 2;
-            const float c = zc[((b * h + (k >> 1)) * h + (j >> 1)) * h + (C.i0 >> 1)];
+            const int h = m >> 1;
+            const float c = zc[((b * h + (k >> 1)) * h + (j >> 1)) * h + (i0 >> 1)];
             z.x += c;
             z.y += c;
         }
     }
     if (colour >= 0) {
-        const Coef7 A(V, M, b, i, j, k, q);
+        const Coef7 A(V, m, b, i, j, k, q);
         const float rq = r[q];
         const float o = odd ? neighbour<1>(V, F, b, i, j, k, q, f) : neighbour<0>(V, F, b, i, j, k, q, f);
         const float n2 = neighbour<2>(V, F, b, i, j, k, q, f), n3 = neighbour<3>(V, F, b, i, j, k, q, f);
@@ -242,6 +327,19 @@ k_vsweep(const __grid_constant__ VLevel V, const float* __restrict__ r, const fl
         else z.x = v;
     }
     *reinterpret_cast<float2*>(zout + q0) = z;
+}
+template <int M, int MODE>
+__global__ void __launch_bounds__(kVThreads)
+k_vsweep(const __grid_constant__ VLevel V, const float* __restrict__ r, const float* __restrict__ zin,
+         const float* __restrict__ zc, float* __restrict__ zout, int colour) {
+    const Pair<M> C;
+    if (C.b < V.nb) vsweep_pair<M, MODE>(V, r, zin, zc, zout, colour, C.b, C.i0, C.j, C.k, C.q0);
+}
+__global__ void __launch_bounds__(kVThreads)
+k_vsweep_even(const __grid_constant__ VLevel V, const float* __restrict__ r, const float* __restrict__ zin,
+              float* __restrict__ zout, int colour) {
+    const EvenPair C(V);
+    if (C.on) vsweep_pair<0, V_PLAIN>(V, r, zin, nullptr, zout, colour, C.b, C.i0, C.j, C.k, C.q0);
 }
 
 // r - A z at a cell with value z, the reference's operand order
@@ -262,13 +360,31 @@ __device__ __forceinline__ float resid_cell(const VLevel& V, const Faces& F, int
 // res = r - A z
 __global__ void k_vresid(const __grid_constant__ VLevel V, const float* __restrict__ r, const float* __restrict__ z,
                          float* __restrict__ res) {
-    const int m = V.m, q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= V.nb * V.nint) return;
-    const int i = q % m, row = q / m, j = row % m, k = (row / m) % m, b = row / (m * m);
-    const Start<0, V_PLAIN> f{r, V.Aii, z, nullptr, m};
+    const Cell C(V);
+    float n[6];
+    six_neighbours(V, C, C.on, z, n);
+    if (!C.on) return;
+    const Coef7 A(V, V.m, C.b, C.i, C.j, C.k, C.q);
+    float y = A.c[6] * z[C.q];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) y = y + A.c[f] * n[f];
+    res[C.q] = r[C.q] - y;
+}
+// ... on pairs of cells (m even)
+template <int M>
+__device__ __forceinline__ float2 resid_pair(const VLevel& V, const float* __restrict__ r, const float* __restrict__ z, int b, int i,
+                                             int j, int k, int q) {
+    const Start<M, V_PLAIN> f{r, V.Aii, z, nullptr, V.m};
     const Faces F(V, b);
-    res[q] = resid_cell(V, F, b, i, j, k, q, r[q], z[q], neighbour<0>(V, F, b, i, j, k, q, f),
-                        neighbour<1>(V, F, b, i, j, k, q, f), f);
+    const float2 r2 = *reinterpret_cast<const float2*>(r + q), z2 = *reinterpret_cast<const float2*>(z + q);
+    const float v0 = resid_cell(V, F, b, i, j, k, q, r2.x, z2.x, neighbour<0>(V, F, b, i, j, k, q, f), z2.y, f);
+    const float v1 = resid_cell(V, F, b, i + 1, j, k, q + 1, r2.y, z2.y, z2.x, neighbour<1>(V, F, b, i + 1, j, k, q + 1, f), f);
+    return make_float2(v0, v1);
+}
+__global__ void __launch_bounds__(kVThreads)
+k_vresid_even(const __grid_constant__ VLevel V, const float* __restrict__ r, const float* __restrict__ z, float* __restrict__ res) {
+    const EvenPair C(V);
+    if (C.on) *reinterpret_cast<float2*>(res + C.q0) = resid_pair<0>(V, r, z, C.b, C.i0, C.j, C.k, C.q0);
 }
 // rc = the sum of the eight children of res (R = P^T), in the reference's order
 __global__ void k_vrestrict(int m, int ncoarse, const float* __restrict__ res, float* __restrict__ rc) {
@@ -301,12 +417,8 @@ k_vresid_restrict(const __grid_constant__ VLevel V, const float* __restrict__ r,
     b = min(b, V.nb - 1);   // every lane takes part in the shuffles
     const int ih = y % h, sub = (y / h) & 3, brick = y / (4 * h), J = brick % h, K = brick / h;
     const int j = 2 * J + (sub & 1), k = 2 * K + (sub >> 1), q = ((b * M + k) * M + j) * M + 2 * ih;
-    const Start<M, V_PLAIN> f{r, V.Aii, z, nullptr, M};
-    const Faces F(V, b);
-    const float2 r2 = *reinterpret_cast<const float2*>(r + q), z2 = *reinterpret_cast<const float2*>(z + q);
-    const float v0 = resid_cell(V, F, b, 2 * ih, j, k, q, r2.x, z2.x, neighbour<0>(V, F, b, 2 * ih, j, k, q, f), z2.y, f);
-    const float v1 = resid_cell(V, F, b, 2 * ih + 1, j, k, q + 1, r2.y, z2.y, z2.x,
-                                neighbour<1>(V, F, b, 2 * ih + 1, j, k, q + 1, f), f);
+    const float2 v = resid_pair<M>(V, r, z, b, 2 * ih, j, k, q);
+    const float v0 = v.x, v1 = v.y;
     float s = 0.f;
     s += v0;
     s += v1;

@@ -18,7 +18,9 @@ SPECS = {
     "m8": dict(sizes=[(24, 45), (16, 30)]),                    # 8, 4, 2 cells
     "m16": dict(sizes=[(32, 60)], block=16, nlevels=4),        # 16, 8, 4, 2
     "m32": dict(sizes=[(32, 64)], block=32, nlevels=5),
-    "m12": dict(sizes=[(24, 48)], block=12, nlevels=3),        # 12, 6, 3
+    "m12": dict(sizes=[(24, 48)], block=12, nlevels=3),        # 12, 6, 3: a thread per cell
+    "m10": dict(sizes=[(40, 80)], block=10, nlevels=2),        # 10 by pairs, 5
+    "m24": dict(sizes=[(48, 96)], block=24, nlevels=4),        # 24 by pairs, 12, 6, 3
 }
 
 
