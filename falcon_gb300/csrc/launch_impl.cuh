@@ -62,13 +62,20 @@ cudaError_t cfl_any(const StepDims& d, const Geometry& g, const T* u, StepScalar
     return cudaGetLastError();
 }
 
+// Threads per interpolated FP64 entry, each a share of its variables: an entry's eight
+// values one after the other are a long chain, which few entries do not hide. us per
+// exchange with 1 / 2 / 4 threads: 7.5k entries 31.5 / 20.2 / 12.7, 30k 33 / 24.2 / 22.4,
+// 69k 34.8 / 28.4 / 26.0, 152k 53.8 / 47.4 / 47.6, 276k 77.0 / 73.7 / 78.0, 303k 77.8 /
+// 75.0 / 83.2, 604k 121.6 / 129.2 / 150.8.
+inline int ghost_parts(int64_t n) { return n <= 100000 ? 4 : n <= 320000 ? 2 : 1; }
 template <class T>
 cudaError_t ghost_any(const StepDims& d, const GhostLists& gl, T* u, cudaStream_t st) {
-    const int64_t nb_ip = (gl.ip.n + 127) / 128, nb_ln = (gl.ln.n + 127) / 128, nb_cp = (gl.cp.n + 127) / 128;
+    const int parts = sizeof(T) == 8 ? ghost_parts(gl.ip.n) : 1;
+    const int64_t nb_ip = (gl.ip.n * parts + 127) / 128, nb_ln = (gl.ln.n + 127) / 128, nb_cp = (gl.cp.n + 127) / 128;
     if (nb_ip + nb_ln + nb_cp == 0) return cudaSuccess;
     if (nb_ip + nb_ln + nb_cp < (int64_t)INT32_MAX) {
         return launch_step(d, k_ghost_all<T>, (unsigned)(nb_ip + nb_ln + nb_cp), 128, 0, st, u, gl, d.ncell, d.nip,
-                           d.nip * d.njp, (int)nb_ip, (int)nb_ln);
+                           d.nip * d.njp, (int)nb_ip, (int)nb_ln, parts);
     }
     if (gl.cp.n > 0) {
         k_ghost_copy<T><<<(unsigned)((gl.cp.n + 255) / 256), 256, 0, st>>>(u, gl.cp, d.ncell);

@@ -208,6 +208,7 @@ __device__ __forceinline__ double gather_one(const T* U, const int8_t* lo, const
                                              const StepDims& dm) {
     const int64_t b = h / ((NV + 1) * ncell), r = h - b * (NV + 1) * ncell;
     if (r < NV * ncell) {
+        if constexpr (sizeof(T) == 8) return U[b * NV * ncell + r];   // the host's order
         const int v = (int)(r / ncell), c = (int)(r - v * ncell);
         const T hi = U[Layout<T>::at((size_t)b, v, (size_t)c, (size_t)ncell)];
         double x = (double)hi;

@@ -1022,19 +1022,20 @@ __device__ __forceinline__ void ghost_rotate(T (&val)[NV], T a, T c) {
     val[V_VT] = -(a * x2) - c * x3;
     val[V_VP] = -(a * x3) + c * x2;
 }
-// One interpolated/rotated ghost entry, put(variable, value) for each of the eight,
-// those that rotate together one after the other (a loop, not unrolled: the bodies
-// are long, and two at a time already miss the instruction cache).
+// One interpolated/rotated ghost entry, put(variable, value) for the variables of its
+// pairs part, part + parts, .. of four, those that rotate together one after the other
+// (a loop, not unrolled: the bodies are long, and two at a time already miss the
+// instruction cache).
 template <class F>
 __device__ __forceinline__ void ghost_interp_each(const double* u, const GhostInterpList& L, int ncell, int nip, int pl,
-                                                  int64_t e, F put) {
+                                                  int64_t e, F put, int part = 0, int parts = 1) {
     const int kind = L.kind[e];
     const double *f = u + (size_t)L.src[e], *w = L.w + 3 * e;
     const double ra = kind & 2 ? L.rot[2 * e] : 0.0, rc = kind & 2 ? L.rot[2 * e + 1] : 0.0;
     auto each = [&](auto value) {
         double a = 0.0;   // the first of a pair
 #pragma unroll 1
-        for (int q = 0; q < 8; ++q) {   // (rho1, vr), (vt, vp), (bt, bp), (br, s1)
+        for (int q = 2 * part; q < 8; q += (q & 1) ? 2 * parts - 1 : 1) {   // (rho1, vr), (vt, vp), (bt, bp), (br, s1)
             const int v = 0x74653210 >> (4 * q) & 15;
             double b = value(f + (size_t)v * ncell);
             if ((kind & 2) && (q == 3 || q == 5)) {
@@ -1105,10 +1106,11 @@ __device__ __forceinline__ void ghost_interp_one(float* u, const GhostInterpList
     store_cell(u + dst, ncell, val);
 }
 template <bool CG = false, bool WAIT = false>
-__device__ __forceinline__ void ghost_interp_one(double* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e) {
+__device__ __forceinline__ void ghost_interp_one(double* u, const GhostInterpList& L, int ncell, int nip, int pl, int64_t e,
+                                                 int part = 0, int parts = 1) {
     if (WAIT) step_wait();
     double* to = u + (size_t)L.dst[e];
-    ghost_interp_each(u, L, ncell, nip, pl, e, [&](int v, double x) { to[(size_t)v * ncell] = x; });
+    ghost_interp_each(u, L, ncell, nip, pl, e, [&](int v, double x) { to[(size_t)v * ncell] = x; }, part, parts);
 }
 
 // ---- block sharding: the entries that cross ranks ---------------------------
@@ -1149,14 +1151,20 @@ __global__ void __launch_bounds__(128) k_ghost_interp(T* u, GhostInterpList L, i
 }
 // The three lists of one exchange in one launch: every entry reads interior
 // cells and writes a ghost cell that no other entry writes, so the lists are
-// independent. The interpolated entries (the longest) take the first CTAs.
+// independent. The interpolated entries (the longest) take the first CTAs, FP64 ones
+// `parts` threads each (1, 2 or 4: ghost_parts).
 template <class T>
-__global__ void __launch_bounds__(128) k_ghost_all(T* u, GhostLists G, int ncell, int nip, int pl, int nb_ip, int nb_ln) {
+__global__ void __launch_bounds__(128) k_ghost_all(T* u, GhostLists G, int ncell, int nip, int pl, int nb_ip, int nb_ln, int parts) {
     const int bx = blockIdx.x;
     step_go();
     if (bx < nb_ip) {
-        const int64_t e = (int64_t)bx * 128 + threadIdx.x;
-        if (e < G.ip.n) ghost_interp_one<false, true>(u, G.ip, ncell, nip, pl, e);
+        const int64_t x = (int64_t)bx * 128 + threadIdx.x;
+        if constexpr (sizeof(T) == 8) {
+            const int64_t e = x >> (parts >> 1);   // parts 1, 2, 4: shifts 0, 1, 2
+            if (e < G.ip.n) ghost_interp_one<false, true>(u, G.ip, ncell, nip, pl, e, (int)(x & (parts - 1)), parts);
+        } else {
+            if (x < G.ip.n) ghost_interp_one<false, true>(u, G.ip, ncell, nip, pl, x);
+        }
     } else if (bx < nb_ip + nb_ln) {
         const int64_t e = (int64_t)(bx - nb_ip) * 128 + threadIdx.x;
         if (e < G.ln.n) ghost_lin_one<T, false, true>(u, G.ln, ncell, e);
