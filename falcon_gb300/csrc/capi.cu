@@ -511,24 +511,46 @@ std::vector<int64_t> shard_entries(const Grid& g, const std::vector<int>& first,
     return out;
 }
 
+// Class of an FP64 entry: which axes are near, to which side (ghost_weights). A warp's
+// entries of one class take one path.
+constexpr size_t kInterpClasses = 4 * 27;
+int interp_class(int kind, const double* w) {
+    for (int t = 0; t < 3; ++t) kind = 3 * kind + (w[t] < 1e-12 ? 0 : w[t] > 1.0 - 1e-12 ? 1 : 2);
+    return kind;
+}
+
 // FP64 device lists of the given map entries: the trilinear/rotated form of
-// the exchange for every entry (a copy is an entry of kind 0), target offsets
-// and source base offsets into the state.
-cudaError_t upload_interp_list(falcon_ctx* ctx, const std::vector<int64_t>& ks, GhostInterpList& out, int32_t** dst_out) {
+// the exchange for every entry (a copy is an entry of kind 0), source base offsets
+// into the state and, by what the list is for, target offsets into it (a rank's own
+// entries, those it receives) or places in the pack buffer (those it sends). The lists
+// that interpolate are in the order of their classes, received ones in the map's.
+enum class ListFor { kOwn, kSend, kReceive };
+cudaError_t upload_interp_list(falcon_ctx* ctx, const std::vector<int64_t>& ks, ListFor what, GhostInterpList& out, int32_t** dst_out) {
     const Grid& g = ctx->grid;
     const size_t n = ks.size();
     std::vector<int32_t> dst(n), src(n);
     std::vector<double> w(3 * n), rot(2 * n);
     std::vector<uint8_t> kind(n);
-    for (size_t q = 0; q < n; ++q) {
-        const GhostMapEntry& e = g.ghosts[ks[q]];
-        dst[q] = (int32_t)cell_off(g, e.e.tblock, e.e.ti, e.e.tj, e.e.tk, Layout<double>::cell);
+    auto kind_of = [&](size_t m) {
+        const GhostMapEntry& e = g.ghosts[ks[m]];
+        return (e.w[0] != 0.0 || e.w[1] != 0.0 || e.w[2] != 0.0 ? 1 : 0) | (e.rotate ? 2 : 0);
+    };
+    std::array<size_t, kInterpClasses + 1> at{};
+    if (what != ListFor::kReceive) {
+        for (size_t m = 0; m < n; ++m) ++at[(size_t)interp_class(kind_of(m), g.ghosts[ks[m]].w) + 1];
+        for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+    }
+    for (size_t m = 0; m < n; ++m) {
+        const GhostMapEntry& e = g.ghosts[ks[m]];
+        const int kd = kind_of(m);
+        const size_t q = what == ListFor::kReceive ? m : at[(size_t)interp_class(kd, e.w)]++;
+        dst[q] = what == ListFor::kSend ? (int32_t)m
+                                        : (int32_t)cell_off(g, e.e.tblock, e.e.ti, e.e.tj, e.e.tk, Layout<double>::cell);
         src[q] = (int32_t)cell_off(g, e.e.sblock, e.i0, e.j0, e.k0, Layout<double>::cell);
-        const int nz = (e.w[0] != 0.0) + (e.w[1] != 0.0) + (e.w[2] != 0.0);
         for (int t = 0; t < 3; ++t) w[3 * q + t] = e.w[t];
         rot[2 * q] = e.rotate ? e.rot[0] : 0.0;
         rot[2 * q + 1] = e.rotate ? e.rot[1] : 0.0;
-        kind[q] = (uint8_t)((nz ? 1 : 0) | (e.rotate ? 2 : 0));
+        kind[q] = (uint8_t)kd;
     }
     auto up = [&](auto** dptr, const auto& vec) -> cudaError_t {
         using E = typename std::decay_t<decltype(vec)>::value_type;
@@ -848,11 +870,9 @@ int setup_device(falcon_ctx* ctx) {
             // A block's entries are sorted on their own: target offsets ascend with the block.
             const size_t n = idst.size();
             std::vector<size_t> ord(n);
-            // FP64: entries of one class together (which axes are near, to which side:
-            // ghost_weights), so that a warp's entries take one path; in target order within
-            constexpr size_t kClasses = 4 * 27;
+            // FP64: entries of one class together, in target order within
             std::vector<uint8_t> cls(snap ? 0 : n);
-            std::vector<std::array<size_t, kClasses>> place(snap ? 0 : nb);   // of a block's next entry, by class
+            std::vector<std::array<size_t, kInterpClasses>> place(snap ? 0 : nb);   // of a block's next entry, by class
 #pragma omp parallel for schedule(dynamic, 16)
             for (int b = 0; b < nb; ++b) {
                 for (size_t q = oi[b]; q < oi[b + 1]; ++q) ord[q] = q;
@@ -860,13 +880,12 @@ int setup_device(falcon_ctx* ctx) {
                 if (snap) continue;
                 place[b].fill(0);
                 for (size_t q = oi[b]; q < oi[b + 1]; ++q) {
-                    int c = ikind[q];
-                    for (int t = 0; t < 3; ++t) c = 3 * c + (iw[3 * q + t] < 1e-12 ? 0 : iw[3 * q + t] > 1.0 - 1e-12 ? 1 : 2);
-                    ++place[b][cls[q] = (uint8_t)c];
+                    cls[q] = (uint8_t)interp_class(ikind[q], &iw[3 * q]);
+                    ++place[b][cls[q]];
                 }
             }
             if (!snap)
-                for (size_t k = 0, at = 0; k < kClasses; ++k)
+                for (size_t k = 0, at = 0; k < kInterpClasses; ++k)
                     for (int b = 0; b < nb; ++b) {
                         const size_t m = place[b][k];
                         place[b][k] = at;
@@ -1840,7 +1859,7 @@ int falcon_set_shard(falcon_ctx* ctx, int32_t nranks, int32_t rank) {
     S.last = f[rank + 1];
     // entries within the rank: copies and interpolated/rotated entries as one list
     GhostInterpList loc{};
-    CK(upload_interp_list(ctx, shard_entries(ctx->grid, f, rank, rank), loc, nullptr), "shard lists");
+    CK(upload_interp_list(ctx, shard_entries(ctx->grid, f, rank, rank), ListFor::kOwn, loc, nullptr), "shard lists");
     S.local = GhostLists{GhostCopyList{0, nullptr, nullptr}, GhostLinList{0, nullptr, nullptr, nullptr, nullptr}, loc};
     S.send.assign(nranks, GhostInterpList{});
     S.recv_dst.assign(nranks, nullptr);
@@ -1848,9 +1867,9 @@ int falcon_set_shard(falcon_ctx* ctx, int32_t nranks, int32_t rank) {
     size_t most = 0;
     for (int p = 0; p < nranks; ++p) {
         if (p == rank) continue;
-        CK(upload_interp_list(ctx, shard_entries(ctx->grid, f, rank, p), S.send[p], nullptr), "shard lists");
+        CK(upload_interp_list(ctx, shard_entries(ctx->grid, f, rank, p), ListFor::kSend, S.send[p], nullptr), "shard lists");
         GhostInterpList in{};
-        CK(upload_interp_list(ctx, shard_entries(ctx->grid, f, p, rank), in, &S.recv_dst[p]), "shard lists");
+        CK(upload_interp_list(ctx, shard_entries(ctx->grid, f, p, rank), ListFor::kReceive, in, &S.recv_dst[p]), "shard lists");
         S.nrecv[p] = in.n;
         most = std::max(most, (size_t)std::max(S.send[p].n, in.n));
     }

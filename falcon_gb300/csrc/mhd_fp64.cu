@@ -79,7 +79,8 @@ cudaError_t launch_ghost_fp64(const StepDims& d, const GhostLists& gl, double* u
 cudaError_t launch_shard_pack_fp64(const StepDims& d, const GhostInterpList& L, const double* u, double* pack,
                                    cudaStream_t st) {
     if (L.n == 0) return cudaSuccess;
-    impl::k_shard_pack<double><<<(unsigned)((L.n + 127) / 128), 128, 0, st>>>(u, L, d.ncell, d.nip, d.nip * d.njp, pack);
+    const int parts = impl::ghost_parts(L.n);
+    impl::k_shard_pack<double><<<(unsigned)((L.n * parts + 127) / 128), 128, 0, st>>>(u, L, d.ncell, d.nip, d.nip * d.njp, pack, parts);
     return cudaGetLastError();
 }
 cudaError_t launch_shard_unpack_fp64(const StepDims& d, const int32_t* dst, int64_t n, const double* pack, double* u,

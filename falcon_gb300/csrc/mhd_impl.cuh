@@ -1115,15 +1115,16 @@ __device__ __forceinline__ void ghost_interp_one(double* u, const GhostInterpLis
 
 // ---- block sharding: the entries that cross ranks ---------------------------
 // The sender evaluates each outgoing ghost entry from its own blocks (the
-// same values as the single-GPU ghost fill) into a pack buffer pack[e][NV];
-// the receiver writes pack[e] into its ghost cells (dst[e], the entries in
-// the same order), as the reference's per-peer send/receive buffers
+// same values as the single-GPU ghost fill) into a pack buffer, entry e at
+// pack[dst[e]][NV]; the receiver writes pack[e] into its ghost cells (its dst[e], in
+// the map's order), as the reference's per-peer send/receive buffers
 // (3_6/ModCommunication.f90:725-765).
 template <class T>
-__global__ void __launch_bounds__(128) k_shard_pack(const T* u, GhostInterpList L, int ncell, int nip, int pl, T* pack) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) k_shard_pack(const T* u, GhostInterpList L, int ncell, int nip, int pl, T* pack, int parts) {
+    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, e = x >> (parts >> 1);   // parts 1, 2, 4
     if (e >= L.n) return;
-    ghost_interp_each(u, L, ncell, nip, pl, e, [&](int v, T x) { pack[e * NV + v] = x; });
+    T* to = pack + (size_t)L.dst[e] * NV;
+    ghost_interp_each(u, L, ncell, nip, pl, e, [&](int v, T y) { to[v] = y; }, (int)(x & (parts - 1)), parts);
 }
 template <class T>
 __global__ void __launch_bounds__(128) k_shard_unpack(T* u, const int32_t* dst, int64_t n, int ncell, const T* pack) {
