@@ -1022,9 +1022,9 @@ k_diffusion_quads(const float* u, float* out, int8_t* ulo, PushTable push, Geome
 // (half-warps of 16 cells), so a half-warp holds one row, as the pushed
 // radial faces need.
 //
-// What bounds it is the issue (16 warps per SM, 128 registers a thread): 1,124 warp
+// What bounds it is the issue (16 warps per SM, 128 registers a thread): 1,139 warp
 // instructions per 32 cells, issued in 58% of the cycles. 21.2M cells: 1,229 ->
-// 1,022 us; 442k cells with split blocks: 60 -> 34 us. Two threads per column with
+// 1,019 us; 442k cells with split blocks: 60 -> 34 us. Two threads per column with
 // 64 registers each: 1,367 us (of 1,135 then).
 template <int NI, int NJ, int NK>
 struct MShape {
