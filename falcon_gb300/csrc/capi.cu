@@ -18,6 +18,7 @@
 #include "kernels.cuh"
 #include "restart_order.h"
 #include "synth.cuh"
+#include "uploads.h"
 
 namespace falcon {
 // state_range.cu: range download through the library's static device array
@@ -647,7 +648,7 @@ int upload_tables(falcon_ctx* ctx, bool first) {
     CK(cudaMemcpy(ctx->gi_f, gif.data(), gif.size() * 4, cudaMemcpyHostToDevice), "upload gi_f");
     CK(cudaMemcpy(ctx->gj_f, gjf.data(), gjf.size() * 4, cudaMemcpyHostToDevice), "upload gj_f");
     CK(cudaMemcpy(ctx->gs_f, gsf.data(), gsf.size() * 4, cudaMemcpyHostToDevice), "upload gs_f");
-
+    CK(uploads_arrived(), "upload tables");
     return FALCON_OK;
 }
 
@@ -985,6 +986,7 @@ int setup_device(falcon_ctx* ctx) {
     CK(ctx->alloc(&ctx->sc, sizeof(StepScalars)), "alloc scalars");
     CK(cudaMallocHost((void**)&ctx->sc_host, sizeof(StepScalars)), "alloc scalars");
     CK(cudaMemcpy(ctx->sc, &s0, sizeof s0, cudaMemcpyHostToDevice), "upload scalars");
+    CK(uploads_arrived(), "upload");
     CK(cudaStreamSynchronize(ctx->st), "sync");
     ctx->on_device = true;
     return FALCON_OK;
@@ -1805,6 +1807,7 @@ int falcon_load_restart(falcon_ctx* ctx, const char* path) {
     std::fclose(f);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "restart");
     if (!ok) return ctx->fail(FALCON_ERR_INVALID_ARG, std::string("restart ") + path + ": short read");
+    CK(uploads_arrived(), "restart");
     if (ctx->mixed()) CK(launch_state_from_file((float*)ctx->U, ctx->Ulo, ctx->dims, ctx->st), "restart");
     // the stage arrays start equal to the state, as after falcon_upload_state
     CK(mirror_state(ctx, true), "restart");
@@ -1877,6 +1880,7 @@ int falcon_set_shard(falcon_ctx* ctx, int32_t nranks, int32_t rank) {
     CK(ctx->alloc(&S.pack, std::max<size_t>(S.pack_elems, 1) * sizeof(double)), "shard pack");
     S.last_out = ctx->U;
     S.on = true;
+    CK(uploads_arrived(), "shard lists");
     CK(cudaStreamSynchronize(ctx->st), "shard");
     return FALCON_OK;
 }

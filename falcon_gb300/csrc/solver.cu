@@ -35,6 +35,7 @@
 #include "ff.cuh"
 #include "lcc.h"
 #include "solver.h"
+#include "uploads.h"
 #include "vcycle.cuh"
 
 namespace falcon {
@@ -1436,6 +1437,7 @@ int setup(falcon_solver* sv) {
     SCK(sv->alloc(&sv->first, (size_t)(S.nproblems + 1) * 4), "scalars");
     SCK(cudaMemcpy(sv->first, S.problem_first_block.data(), (size_t)(S.nproblems + 1) * 4, cudaMemcpyHostToDevice), "scalars");
     apply_tile(sv, sv->tile_chunk, sv->tile_tpb);
+    SCK(uploads_arrived(), "setup");
     SCK(cudaStreamSynchronize(sv->st), "setup");
     return FALCON_OK;
 }
@@ -1524,6 +1526,7 @@ int ensure_coarse_map(falcon_solver* sv) {
     }
     SCK(sv->alloc(&sv->gmap, gm.size() * 4), "coarse map");
     SCK(cudaMemcpy(sv->gmap, gm.data(), gm.size() * 4, cudaMemcpyHostToDevice), "coarse map");
+    SCK(uploads_arrived(), "coarse map");
     SCK(sv->alloc(&sv->feat, (size_t)2 * D * H * W * 8 * 4), "coarse features");
     SCK(sv->alloc(&sv->yout, (size_t)2 * D * H * W * 4), "coarse features");
     SCK(sv->alloc(&sv->csum, 8), "coarse features");
@@ -1609,6 +1612,7 @@ int reupload_operators(falcon_solver* sv) {
     }
     std::vector<float> fa(sv->sA.begin(), sv->sA.end());
     SCK(cudaMemcpy(sv->dsA, fa.data(), fa.size() * 4, cudaMemcpyHostToDevice), "operator");
+    SCK(uploads_arrived(), "operator");
     if (sv->cmap_ok) {
         SvLevel& Lc = sv->lv[S.nlevels - 1];
         k_lcc_static<<<grid_cells(Lc.d, nb), tpb(Lc.d), 0, sv->st>>>(Lc.ops64(), Lc.d, sv->gmap, sv->feat);
@@ -1826,6 +1830,7 @@ int falcon_solver_set_magnetogram(falcon_solver* sv, const double* br) {
     cudaSetDevice(sv->device);
     SCK(cudaStreamSynchronize(sv->st), "rhs");
     SCK(cudaMemcpy(sv->bvec, S.b.data(), S.b.size() * 8, cudaMemcpyHostToDevice), "rhs");
+    SCK(uploads_arrived(), "rhs");
     return FALCON_OK;
 }
 
@@ -2354,6 +2359,7 @@ int falcon_solver_set_rhs(falcon_solver* sv, const double* b) {
         cudaSetDevice(sv->device);
         SCK(cudaStreamSynchronize(sv->st), "rhs");
         SCK(cudaMemcpy(sv->bvec, b, sv->S.b.size() * 8, cudaMemcpyHostToDevice), "rhs");
+        SCK(uploads_arrived(), "rhs");
     }
     return FALCON_OK;
 }

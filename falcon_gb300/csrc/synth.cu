@@ -13,6 +13,7 @@
 // them to it), converted to the block's frame, then scaled to rms Mach `mach`
 // against the local c_s(r).
 #include "synth.cuh"
+#include "uploads.h"
 
 #include <cmath>
 #include <random>
@@ -181,6 +182,7 @@ std::string synth_initial_state(const Grid& g, const Geometry& geo, void* U, boo
     if (e == cudaSuccess) e = cudaMemcpy(dxj, g.xj.data(), g.xj.size() * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(dxk, g.xk.data(), g.xk.size() * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(dmodes, modes.data(), sizeof(Mode) * NMODE, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = uploads_arrived();
     if (e != cudaSuccess) { cleanup(); return std::string("synth setup: ") + cudaGetErrorString(e); }
     if (mixed) k_synth<float><<<grid, 256, 0, st>>>((float*)U, dxj, dxk, geo, d, sp, dmodes, dsum);
     else k_synth<double><<<grid, 256, 0, st>>>((double*)U, dxj, dxk, geo, d, sp, dmodes, dsum);
